@@ -1,0 +1,348 @@
+// In-shared-memory building blocks of the panel kernels (panel.cuh, trsm.cuh): the
+// factor of a diagonal block, the triangular solve of rows below it, and the updates
+// between them, all in 16-column sub-panels.
+//
+// What bounds them is latency: a pivot must be known before the next column starts, so
+// the code is written around that chain, and everything that is not on it is done by
+// other warps at the same time.
+//   * factor16 (one warp): lane i holds row i of the sub-panel, 16 columns in registers.
+//     Per pivot the chain is one warp shuffle (the pivot), the reciprocal square root,
+//     one multiplication and one fused multiply-add: the next pivot d' = a' - |l|^2 needs
+//     only values of its own lane.  The column itself goes through shared memory to the
+//     other lanes in the shadow of the next pivot's square root.  The loop is rolled:
+//     every step shifts the register columns down by one (x[q] := x[q+1] - l v[q]), so
+//     one body of about 60 instructions serves all 16 steps and is fetched once.  (The
+//     kernels run once per block column from a cold instruction cache, where unrolled
+//     code costs more than the FMAs it saves.)
+//   * solve16 (one thread per row): the same shifted loop, right-looking.
+//   * tile_update (one warp): C(32 x 16) -= P Q^H over 16 columns; FP64 on DMMA.
+// A column of L is kept twice: in place, and "shifted" in Lsh[j][q] = L(j+1+q, j), zero
+// past the block, so that the loops read it with aligned 16-byte loads.
+#pragma once
+#include <stdint.h>
+#include <type_traits>
+#include "scalar.cuh"
+
+namespace cuchol {
+
+// Asynchronous global -> shared copy of one element (cp.async: no register
+// staging, every copy of a loop is in flight at once); valid = false writes zeros.
+template <typename T>
+__device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool valid) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  const int n = valid ? (int)sizeof(T) : 0;
+  if constexpr (sizeof(T) == 16) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(sizeof(T)), "r"(n)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
+constexpr int kSub = 16;             // sub-panel columns
+constexpr int kSubRows = 32;         // rows factor16 covers: the 16 x 16 block and 16 rows below
+
+// Shared leading dimensions are = 4 (mod 16): a DMMA fragment load (8 rows x 4 k) then
+// touches 16 distinct 8-byte banks per half warp.
+constexpr int kLdPad = 4;
+
+// 1 / sqrt(d) for the pivot chain.  FP64: the hardware estimate y (relative error below
+// 2^-20) refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, to second order
+// (the dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations after the
+// estimate.  Outside a safe exponent range (where d y^2 could leave it) rsqrt().
+__device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrtf(d); }
+__device__ __forceinline__ double pivot_rsqrt(double d) {
+  if (d >= 0x1p-900 && d <= 0x1p900) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+  }
+  return rsqrt(d);
+}
+
+// 16 elements at a 16-byte aligned shared address.
+template <typename T>
+__device__ __forceinline__ void load_row16(const T* p, T (&v)[kSub]) {
+  constexpr int per = 16 / sizeof(T);
+  const int4* q = reinterpret_cast<const int4*>(p);
+#pragma unroll
+  for (int u = 0; u < kSub / per; ++u) {
+    const int4 w = q[u];
+    memcpy(&v[u * per], &w, 16);
+  }
+}
+
+__device__ __forceinline__ void fms(float& acc, float a, float b) { acc = fmaf(-a, b, acc); }
+__device__ __forceinline__ void fms(double& acc, double a, double b) { acc = fma(-a, b, acc); }
+__device__ __forceinline__ void fms(cuFloatComplex& acc, cuFloatComplex a, cuFloatComplex b) {
+  acc.x = fmaf(-a.x, b.x, acc.x); acc.x = fmaf(a.y, b.y, acc.x);
+  acc.y = fmaf(-a.x, b.y, acc.y); acc.y = fmaf(-a.y, b.x, acc.y);
+}
+__device__ __forceinline__ void fms(cuDoubleComplex& acc, cuDoubleComplex a, cuDoubleComplex b) {
+  acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(a.y, b.y, acc.x);
+  acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(-a.y, b.x, acc.y);
+}
+__device__ __forceinline__ float minus_abs2(float a, float l) { return fmaf(-l, l, a); }
+__device__ __forceinline__ double minus_abs2(double a, double l) { return fma(-l, l, a); }
+__device__ __forceinline__ float minus_abs2(cuFloatComplex a, cuFloatComplex l) { return fmaf(-l.y, l.y, fmaf(-l.x, l.x, a.x)); }
+__device__ __forceinline__ double minus_abs2(cuDoubleComplex a, cuDoubleComplex l) { return fma(-l.y, l.y, fma(-l.x, l.x, a.x)); }
+
+// One warp.  S: the sub-panel's top-left element (column-major, ld), rows 0 .. 31 of it,
+// of which those below nrows exist; factors the 16 columns in place, writes Lsh and the
+// reciprocal pivots rd[0..15].  Returns the first failing column (pivot <= 0 or NaN) or
+// -1, the same in every lane; the columns before it are then done.
+template <typename T>
+__device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Lsh, RealOf<T>* rd) {
+  using R = RealOf<T>;
+  const int i = threadIdx.x & 31;
+  const bool mine = i < nrows;
+  T x[kSub];
+#pragma unroll
+  for (int q = 0; q < kSub; ++q) x[q] = mine ? S[q * ld + i] : zero<T>();
+  R dn = re(x[0]);
+#pragma unroll 1
+  for (int j = 0; j < kSub; ++j) {
+    const R d = __shfl_sync(0xffffffffu, dn, j);
+    if (!(d > R(0))) return j;
+    const R r = pivot_rsqrt(d);
+    const T l = (i == j) ? from_real<T>(d * r) : scale(x[0], r);
+    dn = minus_abs2(x[1], l);                  // the next pivot, on lane j + 1
+    if (mine && i >= j) S[j * ld + i] = l;
+    if (i < kSub) Lsh[j * kSub + ((i - j - 1) & (kSub - 1))] = (i > j) ? l : zero<T>();
+    if (i == 0) rd[j] = r;
+    __syncwarp();
+    T v[kSub];
+    load_row16(Lsh + j * kSub, v);
+#pragma unroll
+    for (int q = 0; q < kSub - 1; ++q) {
+      T t = x[q + 1];
+      fms(t, l, cj(v[q]));
+      x[q] = t;
+    }
+  }
+  return -1;
+}
+
+// One thread: the row x of 16 columns (elements ld apart from S) solved against the
+// factored block: x := x L^-H, the first ncols columns of it.  Unrolled: 120 FMAs whose
+// chain is one multiplication and one FMA per column; the same loop rolled like
+// factor16's would issue twice as many.
+template <typename T>
+__device__ __forceinline__ void solve16(T* S, int ld, const T* __restrict__ Lsh, const RealOf<T>* __restrict__ rd,
+                                        int ncols = kSub) {
+  T x[kSub];
+#pragma unroll
+  for (int q = 0; q < kSub; ++q) x[q] = S[q * ld];
+#pragma unroll
+  for (int j = 0; j < kSub; ++j) {
+    if (j >= ncols) break;
+    T v[kSub];
+    load_row16(Lsh + j * kSub, v);             // only v[0 .. 14 - j] is used
+    x[j] = scale(x[j], rd[j]);
+#pragma unroll
+    for (int q = j + 1; q < kSub; ++q) fms(x[q], x[j], cj(v[q - j - 1]));
+  }
+  // stored at the end: a store between them would hold back the loads of Lsh
+#pragma unroll
+  for (int q = 0; q < kSub; ++q) S[q * ld] = x[q];
+}
+
+__device__ __forceinline__ void dmma16n8k4(double (&d)[4], double a0, double a1, double b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a0), "d"(a1), "d"(b));
+}
+
+// One warp: C(r, c) -= sum_{k < 16} P(r, k) conj(Q(c, k)), r < 32, c < 16, all
+// column-major in shared memory.  Rows of C and P at or past nr (a multiple of 16) are
+// neither read nor written.
+// The tile is 32 x 16 because eight warps then cover 128 x 32 or 64 x 64 with every
+// lane holding 4 x 4 outputs.  FP64 runs on DMMA: the same flop rate as DFMA, but 6
+// shared loads per 4 k instead of 32.
+template <typename T>
+__device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, const T* Q, int ldq, int nr) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (std::is_same<T, double>::value) {
+    const int g = lane >> 2, t = lane & 3;
+    const bool hi = nr > 16;
+    double acc[2][2][4];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[a][b][e] = 0.0;
+#pragma unroll
+    for (int k4 = 0; k4 < kSub; k4 += 4) {
+      const double* p = P + (k4 + t) * ldp + g;
+      const double* q = Q + (k4 + t) * ldq + g;
+      const double b0 = q[0], b1 = q[8];
+      const double a0 = p[0], a1 = p[8];
+      dmma16n8k4(acc[0][0], a0, a1, b0);
+      dmma16n8k4(acc[0][1], a0, a1, b1);
+      if (hi) {
+        const double a2 = p[16], a3 = p[24];
+        dmma16n8k4(acc[1][0], a2, a3, b0);
+        dmma16n8k4(acc[1][1], a2, a3, b1);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      if (a == 1 && !hi) break;
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) C[(8 * b + 2 * t + (e & 1)) * ldc + 16 * a + g + 8 * (e >> 1)] -= acc[a][b][e];
+    }
+  } else {
+    // lane: rows lr + 8u, columns lc + 4v
+    const int lr = lane & 7, lc = lane >> 3;
+    const int nu = nr > 16 ? 4 : 2;
+    T acc[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = zero<T>();
+    if (nu == 4) {
+#pragma unroll 8
+      for (int k = 0; k < kSub; ++k) {
+        T a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = P[k * ldp + lr + 8 * u];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) b[v] = cj(Q[k * ldq + lc + 4 * v]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) fms(acc[u][v], a[u], b[v]);
+      }
+    } else {
+#pragma unroll 8
+      for (int k = 0; k < kSub; ++k) {
+        T a[2], b[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) a[u] = P[k * ldp + lr + 8 * u];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) b[v] = cj(Q[k * ldq + lc + 4 * v]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) fms(acc[u][v], a[u], b[v]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u < nu) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          T* c = C + (lc + 4 * v) * ldc + lr + 8 * u;
+          *c = add(*c, acc[u][v]);
+        }
+      }
+  }
+}
+
+// All NT threads: C(r, c) -= sum_{k < 16} P(r, k) conj(Q(c, k)), r < R (32 or 64; rows
+// at or past nr, a multiple of 16, are left alone), c < 16: the step between two
+// sub-panels that is on the critical path.  FP64: one 16 x 8 DMMA tile per warp and pass
+// (two independent chains of two DMMAs); otherwise a warp takes two columns and a lane
+// one row.
+template <typename T, int R, int NT>
+__device__ __forceinline__ void strip_update(T* C, int ldc, const T* P, int ldp, const T* Q, int ldq, int nr) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr (std::is_same<T, double>::value) {
+    const int g = lane >> 2, t = lane & 3;
+    for (int w = warp; w < (R / 16) * 2; w += NT / 32) {
+      const int r0 = 16 * (w >> 1), n0 = 8 * (w & 1);
+      if (r0 >= nr) continue;
+      double acc[2][4] = {};
+#pragma unroll
+      for (int k4 = 0; k4 < kSub; k4 += 4) {
+        const double* p = P + (k4 + t) * ldp + r0 + g;
+        dmma16n8k4(acc[(k4 >> 2) & 1], p[0], p[8], Q[(k4 + t) * ldq + n0 + g]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) C[(n0 + 2 * t + (e & 1)) * ldc + r0 + g + 8 * (e >> 1)] -= acc[0][e] + acc[1][e];
+    }
+  } else {
+    for (int w = warp; w < (R / 32) * 8; w += NT / 32) {
+      const int r = 32 * (w >> 3) + lane, c = 2 * (w & 7);
+      if (r >= nr) continue;
+      T a0 = C[c * ldc + r], a1 = C[(c + 1) * ldc + r];
+#pragma unroll
+      for (int k = 0; k < kSub; ++k) {
+        const T p = P[k * ldp + r];
+        fms(a0, p, cj(Q[k * ldq + c]));
+        fms(a1, p, cj(Q[k * ldq + c + 1]));
+      }
+      C[c * ldc + r] = a0;
+      C[(c + 1) * ldc + r] = a1;
+    }
+  }
+}
+
+// Shared memory of the factor of one block of order up to NB.
+template <typename T, int NB>
+struct FactorSmem {
+  static constexpr int LD = NB + kLdPad;
+  static constexpr size_t S = sizeof(T) * NB * LD;
+  static constexpr size_t LSH = sizeof(T) * kSub * kSub;
+  static constexpr size_t RD = sizeof(RealOf<T>) * NB;
+  static constexpr size_t bytes = S + LSH + RD;
+};
+
+// Cholesky factor of the block in S (order n16, a multiple of 16 up to NB; lower part),
+// by the whole CTA of NT threads, NT / 32 >= 2 warps.  rd[c] = 1 / L(c, c).  done(c0)
+// is called by the threads of warps 1 .. (t - 32 counts them) as soon as the columns
+// c0 .. c0 + 15 are final, and by all warps for the last ones, with (thread, threads).
+// s_fail (shared, -1 at entry) becomes the first failing column.  Starts and ends with a
+// barrier.
+//
+// Per sub-panel: warp 0 factors the diagonal 16 x 16 (and 16 rows below); one thread per
+// remaining row solves; the 32 x 16 elements warp 0 needs next are updated by all
+// threads; then warp 0 goes on while the other warps update the rest of the block.
+template <typename T, int NB, int NT, typename Done>
+__device__ __forceinline__ void factor_block(T* S, T* Lsh, RealOf<T>* rd, int n16, int* s_fail, Done done) {
+  constexpr int LD = FactorSmem<T, NB>::LD;
+  const int t = threadIdx.x, warp = t >> 5;
+  __syncthreads();
+  for (int c0 = 0; c0 < n16; c0 += kSub) {
+    const int c1 = c0 + kSub;
+    if (warp == 0) {
+      const int f = factor16<T>(S + c0 * LD + c0, LD, n16 - c0, Lsh, rd + c0);
+      if (t == 0 && f >= 0) *s_fail = c0 + f;
+    } else if (c0 > 0) {
+      // the rest of the update by the previous sub-panel: 32 x 16 tiles of the columns
+      // from c0 on, from the diagonal down (the 32 rows warp 0 works on are done already)
+      const int cp = c0 - kSub;
+      int w = warp - 1;
+      for (int cb = c0; cb < n16; cb += kSub)
+        for (int rb = (cb == c0) ? c0 + kSubRows : cb; rb < n16; rb += 32) {
+          if (w == 0)
+            tile_update<T>(S + cb * LD + rb, LD, S + cp * LD + rb, LD, S + cp * LD + cb, LD, n16 - rb);
+          w = (w == 0) ? NT / 32 - 2 : w - 1;
+        }
+      done(cp, t - 32, NT - 32);
+    }
+    __syncthreads();
+    const int fail = *s_fail;
+    const int ncols = fail < 0 ? kSub : fail - c0;
+    for (int r = c0 + kSubRows + t; r < n16; r += NT) solve16<T>(S + c0 * LD + r, LD, Lsh, rd + c0, ncols);
+    __syncthreads();
+    if (fail >= 0 || c1 >= n16) {
+      done(c0, t, NT);
+      break;
+    }
+    // the 32 x 16 elements the next factor16 works on
+    strip_update<T, kSubRows, NT>(S + c1 * LD + c1, LD, S + c0 * LD + c1, LD, S + c0 * LD + c1, LD, n16 - c1);
+    __syncthreads();
+  }
+  __syncthreads();
+}
+
+}  // namespace cuchol

@@ -457,6 +457,42 @@ CUresult set_smem(const void* fn, size_t bytes) {
   return CUDA_SUCCESS;
 }
 
+// ---- diagonal block and panel solve ------------------------------------------------
+constexpr int kDiagThreads2 = 256;
+
+// Factor of the jb x jb diagonal block at A (logical lower view), queued on s; T: the
+// computing type, TA: the storage type.
+template <typename T, typename TA, int NB>
+CUresult diag_factor(CULAPACKhandle h, TA* A, long long rs, long long cs, int jb, long long info_base,
+                     double* logdet, cudaStream_t s) {
+  constexpr int smem = (int)FactorSmem<T, NB>::bytes;
+  auto* kernel = diag_factor_kernel<T, TA, NB, kDiagThreads2>;
+  CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
+  kernel<<<1, kDiagThreads2, smem, s>>>(A, rs, cs, jb, info_base, h->d_words, logdet);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
+// Panel solve of the m rows at B below the factored block L (trsm.cuh), queued on s.
+template <typename T, typename O2, int MODE, int NB>
+CUresult panel_solve(CULAPACKhandle h, T* B, int m, int jb, const T* L, long long rs, long long cs, O2* out2,
+                     long long o_rs, long long o_cs, O2* out3, cudaStream_t s) {
+  constexpr int R = 32, smem = (int)SolveSmem<T, NB, R>::bytes;
+  auto* kernel = trsm_rows_kernel<T, O2, MODE, NB, R>;
+  static bool attr = false;
+  if (!attr) {
+    CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
+    // several CTAs per SM: ask for the whole unified L1/shared carve-out
+    CUCHOL_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    attr = true;
+  }
+  kernel<<<(m + R - 1) / R, 256, smem, s>>>(B, rs, cs, m, jb, L, rs, cs, out2, o_rs, o_cs, h->d_words, out3);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
 // ---- FP32 updates on the TF32 tensor cores, split in three (tc.cuh, SPLIT3) -------
 // C -= Q(r) Q(c)^T on the logical lower trapezoid m x ncols whose corner is the
 // diagonal element (r0, r0) of A (column-major, lda), with Q = qhi + qlo k-major (row
@@ -537,8 +573,6 @@ CUresult tc3_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
 // P (ping-pong pair) holds rows from the first sub-panel's diagonal block down:
 // P(r, c) = L(j + nb + r, j + c).  Failure: the diagonal kernel sets the device
 // info word, and every later kernel exits at entry when it is set.
-constexpr int kDiagThreads2 = 256;
-
 // `on_final`, when given, is called once per diagonal block c .. c + jb - 1 in
 // order, as soon as the queued work that finishes that block column of the factor
 // (logical rows c .. n-1) has been issued, with the stream that work is on: a
@@ -555,7 +589,6 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   constexpr int nb = Tune<T>::nb;
   // outer block: sub diagonal blocks, from the handle's override or the tuning table
   const int NB = (h->potrf_sub > 0 ? h->potrf_sub : tuned_potrf_sub(type_char<T>(), n)) * nb;
-  using Smem = DiagSmem<T, nb>;
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel, su = h->s_update;
@@ -574,12 +607,6 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   T* qbuf[4] = {static_cast<T*>(h->ws), static_cast<T*>(h->ws) + (size_t)n * ldq,
                 static_cast<T*>(h->ws) + 2 * (size_t)n * ldq, static_cast<T*>(h->ws) + 3 * (size_t)n * ldq};
 
-  CUCHOL_CHECK_CU(set_smem<T>((const void*)diag_factor_kernel<T, nb, kDiagThreads2>, Smem::bytes));
-  // the panel solve is a row-parallel triangular solve (no inverse of the diagonal
-  // block) that writes the solved rows into A and into P
-  CUCHOL_CHECK_CU(set_smem<T>((const void*)trsm_rows_kernel<T, T, T, T, OUT_CONVERT>, trsm_rows_smem<T>()));
-  if constexpr (std::is_same<T, float>::value)
-    CUCHOL_CHECK_CU(set_smem<T>((const void*)trsm_rows_kernel<T, T, T, T, OUT_SPLIT>, trsm_rows_smem<T>()));
   CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
   CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
   // the update stream starts after the panel stream's initialisation
@@ -618,10 +645,7 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;                 // rows below this diagonal block
-      diag_factor_kernel<T, nb, kDiagThreads2><<<1, kDiagThreads2, Smem::bytes, sp>>>(
-          at(c, c), rs, cs, jb, nullptr, nb, c, d_info, h->d_logdet);
-      ++h->launches;
-      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, h->d_logdet, sp)));
       if (mr == 0) {
         if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
         break;
@@ -633,18 +657,14 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
       if constexpr (std::is_same<T, float>::value) {
         if (tc3) {
           const long long qo = (long long)s0 * ldq + s0;
-          trsm_rows_kernel<T, T, T, T, OUT_SPLIT><<<(mr + 63) / 64, 256, trsm_rows_smem<T>(), sp>>>(
-              at(c + jb, c), rs, cs, mr, jb, at(c, c), rs, cs, Qh + qo, ldq, 1, d_info, Ql + qo);
+          CUCHOL_CHECK_CU((panel_solve<T, T, OUT_SPLIT, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Qh + qo, ldq, 1,
+                                                            Ql + qo, sp)));
           split = true;
         }
       }
-      if (!split) {
-        T* Ps = P + s0 + (long long)s0 * ldp;
-        trsm_rows_kernel<T, T, T, T, OUT_CONVERT><<<(mr + 63) / 64, 256, trsm_rows_smem<T>(), sp>>>(
-            at(c + jb, c), rs, cs, mr, jb, at(c, c), rs, cs, Ps, 1, ldp, d_info, nullptr);
-      }
-      ++h->launches;
-      CUCHOL_CHECK(cudaGetLastError());
+      if (!split)
+        CUCHOL_CHECK_CU((panel_solve<T, T, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs,
+                                                         P + s0 + (long long)s0 * ldp, 1, ldp, nullptr, sp)));
       CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
       if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
       if (s0 + nb < jB) {

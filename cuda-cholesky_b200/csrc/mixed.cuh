@@ -11,7 +11,7 @@
 //      the operand unit roundoff) and grows 8x after a breakdown.
 //   2. Right-looking blocked Cholesky of W with the two-stream schedule of ?potrf
 //      (outer blocks of 512 columns = four 128-column sub-panels, lookahead 1):
-//        - diagonal blocks in FP64 (the ?potrf diagonal kernel on an FP64 copy),
+//        - diagonal blocks in FP64 (the ?potrf diagonal kernel, FP32 in and out),
 //        - panel solve P = W21 inv(L11)^T in FP32 (SIMT engine) into a k-major
 //          buffer, then copied into W and rounded to the operand type Q (BF16 or
 //          TF32),
@@ -81,22 +81,6 @@ __global__ void build_kernel(const double* __restrict__ a, long long rs, long lo
       W[i + (long long)j * ldw] = w;
     }
   }
-}
-
-// FP32 diagonal block of W -> FP64 copy D (ld SB); column j = blockIdx.x.
-__global__ void diag_in_kernel(const float* __restrict__ W, long long ldw, int jb, double* __restrict__ D,
-                               const int* __restrict__ stop) {
-  if (cta_aborted(stop)) return;
-  const int j = blockIdx.x, i = threadIdx.x;
-  if (i < jb && i >= j) D[i + j * SB] = (double)W[i + (long long)j * ldw];
-}
-
-// Factored FP64 block -> W (FP32).
-__global__ void diag_out_kernel(const double* __restrict__ D, int jb, float* __restrict__ W, long long ldw,
-                                const int* __restrict__ stop) {
-  if (cta_aborted(stop)) return;
-  const int j = blockIdx.x, i = threadIdx.x;
-  if (i < jb && i >= j) W[i + (long long)j * ldw] = (float)D[i + j * SB];
 }
 
 // ---- triangular solves ------------------------------------------------------------
@@ -1130,25 +1114,14 @@ CUresult tc_update(CULAPACKhandle h, const Op* q, long long ldq, int q_rows, int
 // store of the plan, ld NBT) at its place in its NBT-wide block.
 template <typename Op>
 CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* info) {
-  using Smem = DiagSmem<double, SB>;
   cudaStream_t sp = h->s_panel, su = h->s_update;
   int* d_info = h->d_words;
   const long long ldq = OB;
   const size_t rows = round_up((size_t)n, 128) + 128;
-  const size_t small = round_up(sizeof(double) * SB * SB, 256);
   const size_t qbytes = round_up(sizeof(Op) * rows * ldq, 256);
-  CUCHOL_CHECK_CU(ensure_workspace(h, small + 2 * qbytes));
+  CUCHOL_CHECK_CU(ensure_workspace(h, 2 * qbytes));
   char* ws = static_cast<char*>(h->ws);
-  double* D = reinterpret_cast<double*>(ws);
-  Op* Q[2] = {reinterpret_cast<Op*>(ws + small), reinterpret_cast<Op*>(ws + small + qbytes)};
-  static bool attr = false;
-  if (!attr) {
-    CUCHOL_CHECK(cudaFuncSetAttribute(trsm_rows_kernel<float, float, double, Op, OUT_ROUND>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_rows_smem<float>()));
-    attr = true;
-  }
-
-  CUCHOL_CHECK_CU(set_smem<double>((const void*)diag_factor_kernel<double, SB, kDiagThreads2>, Smem::bytes));
+  Op* Q[2] = {reinterpret_cast<Op*>(ws), reinterpret_cast<Op*>(ws + qbytes)};
   CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
   CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
   CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
@@ -1163,19 +1136,12 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
     const int q_rows = n - j - SB;   // P / Q row r = global row j + SB + r
     for (int s0 = 0; s0 < jB; s0 += SB) {
       const int c = j + s0, jb = std::min(SB, j + jB - c), mr = n - c - jb;
-      diag_in_kernel<<<jb, SB, 0, sp>>>(at(c, c), ldw, jb, D, d_info);
-      diag_factor_kernel<double, SB, kDiagThreads2><<<1, kDiagThreads2, Smem::bytes, sp>>>(
-          D, 1, SB, jb, nullptr, SB, c, d_info, h->d_logdet);
-      diag_out_kernel<<<jb, SB, 0, sp>>>(D, jb, at(c, c), ldw, d_info);
-      h->launches += 3;
-      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK_CU((diag_factor<double, float, SB>(h, at(c, c), 1, ldw, jb, c, h->d_logdet, sp)));
       if (mr == 0) break;
       // panel rows c + jb .. n-1 solved in place; they are Q rows s0 .., columns s0 ..
       Op* Qs = Qj + (long long)s0 * ldq + s0;
-      trsm_rows_kernel<float, float, double, Op, OUT_ROUND><<<(mr + 63) / 64, kThreads, trsm_rows_smem<float>(), sp>>>(
-          at(c + jb, c), 1, ldw, mr, jb, D, 1, SB, Qs, ldq, 1, d_info, nullptr);
-      ++h->launches;
-      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK_CU((panel_solve<float, Op, OUT_ROUND, SB>(h, at(c + jb, c), mr, jb, at(c, c), 1, ldw, Qs, ldq, 1,
+                                                             nullptr, sp)));
       if (s0 + SB < jB)   // the outer block's remaining columns by this sub-panel
         CUCHOL_CHECK_CU(tc_update<Op>(h, Qs, ldq, q_rows - s0, jb, 0, 0, at(c + jb, c + jb), ldw, mr,
                                       jB - s0 - SB, sp, d_info));

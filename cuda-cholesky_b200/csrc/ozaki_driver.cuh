@@ -55,7 +55,6 @@ CUresult ozaki_update(CULAPACKhandle h, const int8_t* sl, int R, int S, long lon
 CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long long lda, int S, long* info) {
   constexpr int nb = 128;
   const int NB = (h->potrf_sub > 0 ? h->potrf_sub : tuned_sub(TUNE_OZAKI, 'D', n)) * nb;
-  using Smem = DiagSmem<double, nb>;
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel, su = h->s_update;
@@ -71,9 +70,6 @@ CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long lo
   int* ebuf[2] = {reinterpret_cast<int*>(ws + pbytes + 2 * sbytes),
                   reinterpret_cast<int*>(ws + pbytes + 2 * sbytes + ebytes)};
 
-  CUCHOL_CHECK_CU(set_smem<double>((const void*)diag_factor_kernel<double, nb, kDiagThreads2>, Smem::bytes));
-  CUCHOL_CHECK_CU(set_smem<double>((const void*)trsm_rows_kernel<double, double, double, double, OUT_CONVERT>,
-                                   trsm_rows_smem<double>()));
   CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
   CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
   CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
@@ -87,16 +83,11 @@ CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long lo
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;
-      diag_factor_kernel<double, nb, kDiagThreads2><<<1, kDiagThreads2, Smem::bytes, sp>>>(
-          at(c, c), rs, cs, jb, nullptr, nb, c, d_info, h->d_logdet);
-      ++h->launches;
-      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK_CU((diag_factor<double, double, nb>(h, at(c, c), rs, cs, jb, c, h->d_logdet, sp)));
       if (mr == 0) break;
       double* Ps = P + s0 + (long long)s0 * ldp;   // P(r, .) = rows from j + nb
-      trsm_rows_kernel<double, double, double, double, OUT_CONVERT><<<(mr + 63) / 64, 256, trsm_rows_smem<double>(), sp>>>(
-          at(c + jb, c), rs, cs, mr, jb, at(c, c), rs, cs, Ps, 1, ldp, d_info, nullptr);
-      ++h->launches;
-      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK_CU((panel_solve<double, double, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Ps, 1, ldp,
+                                                                    nullptr, sp)));
       if (s0 + nb < jB) {   // the outer block's remaining sub-panel columns by this one (DMMA)
         GemmProblem<double> u = problem<double>();
         u.a = Ps; u.a_rs = 1; u.a_ks = ldp;

@@ -23,26 +23,10 @@
 // reference copied it to the host for a CPU dpotrf every step
 // (lapack/dpotrf.c:263-276).
 #pragma once
+#include "block.cuh"
 #include "scalar.cuh"
 
 namespace cuchol {
-
-// Asynchronous global -> shared copy of one element (cp.async: no register
-// staging, every copy of a loop is in flight at once); valid = false writes zeros.
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  const int n = valid ? (int)sizeof(T) : 0;
-  if constexpr (sizeof(T) == 16) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-  } else {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(sizeof(T)), "r"(n)
-                 : "memory");
-  }
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
 
 template <typename T>
 __device__ __forceinline__ T shfl(T v, int src) {
@@ -390,14 +374,86 @@ __device__ __forceinline__ void diag_factor_block(T* __restrict__ A, long long r
   }
 }
 
-// In-place inverse of the diagonal blocks [b*nb, b*nb + jb) of a triangular matrix
-// (blockIdx.x = b), nb <= NB.  Only the lower triangle of each block is read or
-// written; unit: the diagonal is taken as 1 and left untouched.
-template <typename T, int NB, int NT>
+// Lower part of the logical block A(r, c) (strides rs, cs) -> S (column-major, ld LD),
+// order jb padded to n16 with the identity.
+template <typename T, typename TA, int LD, int NT>
+__device__ __forceinline__ void load_lower(T* S, const TA* __restrict__ A, long long rs, long long cs, int jb, int n16) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto put = [&](int r, int c) {
+    const bool v = r < jb && c < jb;
+    if constexpr (std::is_same<T, TA>::value) {
+      if (v || r != c) cp_async_elem<T>(&S[c * LD + r], v ? A + r * rs + c * cs : A, v);
+      else S[c * LD + r] = from_real<T>(RealOf<T>(1));
+    } else {
+      S[c * LD + r] = v ? (T)A[r * rs + c * cs] : T(r == c ? 1 : 0);
+    }
+  };
+  if (rs == 1) {               // rows contiguous: a warp per column
+    for (int c = warp; c < n16; c += NT / 32)
+      for (int r = (c & ~31) + lane; r < n16; r += 32)
+        if (r >= c) put(r, c);
+  } else {                     // columns contiguous: 4 rows x 8 columns per warp and step
+    const int dr = lane >> 3, dc = lane & 7;
+    for (int r0 = 4 * warp; r0 < n16; r0 += 4 * (NT / 32))
+      for (int c0 = 0; c0 <= r0 + 3; c0 += 8)
+        if (r0 + dr >= c0 + dc) put(r0 + dr, c0 + dc);
+  }
+}
+
+// Cholesky factor of one jb x jb diagonal block, jb <= NB, in place (block.cuh); T:
+// computing type, TA: storage type.  On failure at local column k: *d_info = info_base
+// + k + 1 (if still 0), and the columns before k are written back.
+//
+// Bound by the chain of pivots.  One 128-column block, launch included, B200: FP64 73 ->
+// MEASURE us, FP32 52 -> , complex 75 -> , 64-column complex double 52 -> .
+template <typename T, typename TA, int NB, int NT>
 __global__ void __launch_bounds__(NT)
-diag_factor_kernel(T* __restrict__ A, long long rs, long long cs, int jb, T* __restrict__ W, int ldw,
-                   long long info_base, int* __restrict__ d_info, double* __restrict__ logdet) {
-  diag_factor_block<T, NB, NT>(A, rs, cs, jb, W, ldw, info_base, d_info, logdet);
+diag_factor_kernel(TA* __restrict__ A, long long rs, long long cs, int jb, long long info_base,
+                   int* __restrict__ d_info, double* __restrict__ logdet) {
+  using F = FactorSmem<T, NB>;
+  constexpr int LD = F::LD;
+  if (cta_aborted(d_info)) return;   // an earlier block already failed
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* S = reinterpret_cast<T*>(smem_raw);
+  T* Lsh = reinterpret_cast<T*>(smem_raw + F::S);
+  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem_raw + F::S + F::LSH);
+  __shared__ int s_fail;
+  __shared__ double s_log[NT / 32];
+  const int tid = threadIdx.x, n16 = (jb + kSub - 1) & ~(kSub - 1);
+  load_lower<T, TA, LD, NT>(S, A, rs, cs, jb, n16);
+  if (tid == 0) s_fail = -1;
+  cp_async_wait_all();
+  factor_block<T, NB, NT>(S, Lsh, rd, n16, &s_fail, [&](int c0, int t, int nt) {
+    // columns c0 .. c0 + 15 of the factor back to A
+    const int rows = jb - c0;
+    if (rs == 1) {
+      for (int e = t >> 5; e < 4 * kSub; e += nt >> 5) {       // a warp per column and quarter
+        const int c = c0 + (e & (kSub - 1));
+        const int r = c0 + 32 * (e / kSub) + (t & 31);
+        if (c < jb && r < jb && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
+      }
+    } else {
+      for (int e = t; e < rows * kSub; e += nt) {
+        const int c = c0 + (e & (kSub - 1)), r = c0 + e / kSub;
+        if (c < jb && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
+      }
+    }
+  });
+  if (s_fail >= 0) {
+    if (tid == 0) atomicCAS(d_info, 0, (int)(info_base + s_fail + 1));
+    return;
+  }
+  if (logdet != nullptr) {
+    // 2 sum log L(j,j), one column per thread, reduced in a fixed order (deterministic)
+    double s = (tid < jb) ? log((double)re(S[tid * LD + tid])) : 0.0;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((tid & 31) == 0) s_log[tid >> 5] = s;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < (NB + 31) / 32; ++w) s += s_log[w];
+      *logdet += 2.0 * s;
+    }
+  }
 }
 
 // One diagonal block of one matrix of a batch (batched factor: one CTA per task).
@@ -423,6 +479,9 @@ template <typename T, int NB, int NT>
 __device__ __forceinline__ void diag_invert_block(T* __restrict__ B, long long rs, long long cs, int jb,
                                                   int unit);
 
+// In-place inverse of the diagonal blocks [b*nb, b*nb + jb) of a triangular matrix
+// (blockIdx.x = b), nb <= NB.  Only the lower triangle of each block is read or
+// written; unit: the diagonal is taken as 1 and left untouched.
 template <typename T, int NB, int NT>
 __global__ void __launch_bounds__(NT)
 diag_invert_kernel(T* __restrict__ A, long long rs, long long cs, int n, int nb, int unit) {

@@ -1,10 +1,11 @@
 // Row-parallel panel solve of the blocked Cholesky factorisations (?potrf and the
 // mixed-precision factor): the rows below a factored diagonal block are
-// independent right-hand sides of L x = b, so one CTA solves 64 of them with the
+// independent right-hand sides of L x = b, so one CTA solves 32 or 64 of them with the
 // block in shared memory, with no inverse of the block and no extra pass.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "block.cuh"
 #include "scalar.cuh"
 
 namespace cuchol {
@@ -20,119 +21,177 @@ template <typename Op> __device__ __forceinline__ Op to_op(float x);
 template <> __device__ __forceinline__ __nv_bfloat16 to_op<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 template <> __device__ __forceinline__ float to_op<float>(float x) { return round_tf32(x); }
 
-// Conversions between the element types the panel solve reads and writes (the
-// complex types are only ever converted to themselves).
-template <typename D, typename S> __device__ __forceinline__ D cvt(S x) {
-  if constexpr (Traits<D>::complex) return x;
-  else return (D)x;
-}
-// acc -= a * b
-__device__ __forceinline__ void msub(float& acc, float a, float b) { acc = fmaf(-a, b, acc); }
-__device__ __forceinline__ void msub(double& acc, double a, double b) { acc = fma(-a, b, acc); }
-__device__ __forceinline__ void msub(cuFloatComplex& acc, cuFloatComplex a, cuFloatComplex b) {
-  acc.x = fmaf(-a.x, b.x, acc.x); acc.x = fmaf(a.y, b.y, acc.x);
-  acc.y = fmaf(-a.x, b.y, acc.y); acc.y = fmaf(-a.y, b.x, acc.y);
-}
-__device__ __forceinline__ void msub(cuDoubleComplex& acc, cuDoubleComplex a, cuDoubleComplex b) {
-  acc.x = fma(-a.x, b.x, acc.x); acc.x = fma(a.y, b.y, acc.x);
-  acc.y = fma(-a.x, b.y, acc.y); acc.y = fma(-a.y, b.x, acc.y);
-}
-
 // How the panel solve writes its second copy of X (out2, and out3 for the split).
 enum : int {
-  OUT_CONVERT = 0,   // out2 = X converted to O2
+  OUT_COPY = 0,      // out2 = X
   OUT_ROUND = 1,     // out2 = X rounded to the tensor-core operand type O2 (BF16 or TF32)
   OUT_SPLIT = 2,     // out2 = hi = tf32(X), out3 = lo = tf32(X - hi): X = hi + lo to 2^-22
+                     // (complex: the two-row form of tcgemm.cuh)
+};
+
+// Shared memory of the panel solve of R rows: the row tile Xs (column-major), the parts
+// of L below its 16 x 16 diagonal blocks (one column-major strip per sub-panel, from the
+// row below the block), the shifted diagonal blocks and the reciprocal pivots.
+template <typename T, int NB, int R>
+struct SolveSmem {
+  static constexpr bool dmma = std::is_same<T, double>::value;
+  static constexpr int NP = NB / kSub;
+  static constexpr int LDX = R + (dmma ? kLdPad : 1);
+  static constexpr size_t X = (sizeof(T) * NB * LDX + 15) / 16 * 16;
+  // strip p: rows 16(p+1) .. NB-1, ld = NB - 16(p+1) + kLdPad, 16 columns
+  __host__ __device__ static constexpr int strip_ld(int p) { return NB - kSub * (p + 1) + kLdPad; }
+  __host__ __device__ static constexpr int strip_off(int p) {
+    return kSub * (p * (NB - kSub + kLdPad) - kSub * (p * (p - 1) / 2));
+  }
+  static constexpr size_t L = sizeof(T) * strip_off(NP - 1);
+  static constexpr size_t LSH = sizeof(T) * NP * kSub * kSub;
+  static constexpr size_t RD = sizeof(RealOf<T>) * NB;
+  static constexpr size_t bytes = X + L + LSH + RD;
 };
 
 // Panel solve X = B L^-H in place (L^-T for real types), row-parallel: B (m x jb,
-// jb <= 128, logical view B(i, j) = B[i*brs + j*bcs]) is overwritten by X, and X
+// jb <= NB, logical view B(i, j) = B[i*brs + j*bcs]) is overwritten by X, and X
 // also goes to out2 (out2[i*o_rs + j*o_cs]) and, for OUT_SPLIT, out3 (same strides),
-// as MODE says.  L: the factored jb x jb
-// diagonal block (view strides lrs, lcs).  Each row x of X solves x L^H = b:
-//   x_k = (b_k - sum_{j<k} x_j conj(L(k, j))) / L(k, k),
-// so the block is staged as conj(L).  CTA: 64 rows; thread (r, cg) holds columns
-// [32cg, 32cg + 32) of row r in registers.  Column block b is solved by the threads
-// with cg == b (forward substitution, right-looking inside the block), published
-// through shared memory, and subtracted by the threads with cg > b.  Computes in T.
-// Complex double rows need up to 255 registers: one CTA per SM for that type.
-template <typename T, typename TB, typename TL, typename O2, int MODE>
-__global__ void __launch_bounds__(256, sizeof(T) == 16 ? 1 : 2)
-    trsm_rows_kernel(TB* __restrict__ B, long long brs, long long bcs, int m, int jb, const TL* __restrict__ L,
-                     long long lrs, long long lcs, O2* __restrict__ out2, long long o_rs, long long o_cs,
+// as MODE says.  L: the factored jb x jb diagonal block (view strides lrs, lcs; real
+// diagonal).  One CTA of 8 warps solves R rows with the tile and the block in shared
+// memory, in 16-column sub-panels: one thread per row substitutes through the 16
+// columns; all warps update the next sub-panel; then the next substitution runs while
+// the other warps update the columns further right (block.cuh).  Computes in T.
+//
+// Bound by latency on its critical path (8 sub-panels of about 1000 cycles) and, with
+// many rows, by the FP64 rate.
+template <typename T, typename O2, int MODE, int NB, int R>
+__global__ void __launch_bounds__(256)
+    trsm_rows_kernel(T* __restrict__ B, long long brs, long long bcs, int m, int jb, const T* __restrict__ L, long long lrs,
+                     long long lcs, O2* __restrict__ out2, long long o_rs, long long o_cs,
                      const int* __restrict__ stop, O2* __restrict__ out3) {
+  using SM = SolveSmem<T, NB, R>;
+  constexpr int NT = 256, LDX = SM::LDX, SW = R / 32;   // SW warps substitute
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Ls = reinterpret_cast<T*>(smem_raw);   // [128][33]: conj L(32b + j, 32b + k)
-  T* Xs = Ls + 128 * 33;                    // [64][33]: solved block
-  T* rd = Xs + 64 * 33;                     // [32]: 1 / L(32b + j, 32b + j)
+  T* Xs = reinterpret_cast<T*>(smem_raw);                       // Xs[col * LDX + row]
+  T* Ls = reinterpret_cast<T*>(smem_raw + SM::X);
+  T* Lsh = reinterpret_cast<T*>(smem_raw + SM::X + SM::L);
+  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem_raw + SM::X + SM::L + SM::LSH);
   if (cta_aborted(stop)) return;
-  const int t = threadIdx.x, r = t & 63, cg = t >> 6;
-  const int row = blockIdx.x * 64 + r;
-  T x[32];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int n16 = (jb + kSub - 1) & ~(kSub - 1);
+  const long long row0 = (long long)blockIdx.x * R;
+  const int rows = min((long long)R, m - row0);
+
+  // Everything comes in with cp.async, a warp walking its columns (or rows) with one
+  // pointer: no index divisions, and no load waits for another.
+  if (brs == 1) {                                // row tile: a warp per column
+    for (int c = warp; c < n16; c += NT / 32) {
+      const T* src = B + row0 + (long long)c * bcs;
 #pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const int col = cg * 32 + k;
-    x[k] = (row < m && col < jb) ? cvt<T>(B[(long long)row * brs + (long long)col * bcs]) : zero<T>();
-  }
-  const int nblk = (jb + 31) / 32;
-  for (int b = 0; b < nblk; ++b) {
-    const int rows = 128 - 32 * b;   // rows of L from 32b down (zero past jb)
-    __syncthreads();
-    for (int e = t; e < rows * 32; e += 256) {
-      const int j = e >> 5, kk = e & 31;
-      const int gi = 32 * b + j, gk = 32 * b + kk;
-      Ls[j * 33 + kk] =
-          (gi < jb && gk < jb && gi >= gk) ? cj(cvt<T>(L[(long long)gi * lrs + (long long)gk * lcs])) : zero<T>();
-    }
-    __syncthreads();
-    if (t < 32) rd[t] = (32 * b + t < jb) ? recip(Ls[t * 33 + t]) : zero<T>();
-    __syncthreads();
-    if (cg == b) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        x[j] = mul(x[j], rd[j]);
-#pragma unroll
-        for (int kk = j + 1; kk < 32; ++kk) msub(x[kk], Ls[kk * 33 + j], x[j]);
+      for (int r = lane; r < R; r += 32) {
+        const bool v = r < rows && c < jb;
+        cp_async_elem<T>(&Xs[c * LDX + r], v ? src + r : B, v);
       }
-#pragma unroll
-      for (int kk = 0; kk < 32; ++kk) Xs[r * 33 + kk] = x[kk];
     }
-    __syncthreads();
-    if (cg > b) {
-      const T* Lb = Ls + (cg - b) * 32 * 33;
-#pragma unroll 4
-      for (int kk = 0; kk < 32; ++kk) {
-        const T xk = Xs[r * 33 + kk];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) msub(x[j], Lb[j * 33 + kk], xk);
+  } else {                                       // 4 rows x 8 columns per warp and step
+    const int dr = lane >> 3, dc = lane & 7;
+    for (int r = 4 * warp + dr; r < R; r += 4 * (NT / 32)) {
+      const T* src = B + (row0 + r) * brs;
+      for (int c = dc; c < n16; c += 8) {
+        const bool v = r < rows && c < jb;
+        cp_async_elem<T>(&Xs[c * LDX + r], v ? src + (long long)c * bcs : B, v);
       }
     }
   }
-  // the solved 64-row tile, staged in shared memory (the L / X buffers are idle now),
-  // goes to each output in the order that is contiguous in that output
+  // the diagonal 16 x 16 blocks, shifted: global column j, row j + 1 + q
+  for (int e = t; e < n16 * kSub; e += NT) {
+    const int j = e / kSub, q = e & (kSub - 1), i = j + 1 + q;
+    const bool v = q < kSub - 1 - (j & (kSub - 1)) && i < jb;
+    cp_async_elem<T>(&Lsh[e], v ? L + (long long)i * lrs + (long long)j * lcs : L, v);
+  }
+  // the strips of L below them
+  if (lrs == 1) {
+    for (int j = warp; j < n16 - kSub; j += NT / 32) {
+      const int r0 = (j & ~(kSub - 1)) + kSub, p = j / kSub;
+      T* S = Ls + SM::strip_off(p) + (j & (kSub - 1)) * SM::strip_ld(p) - r0;
+      const T* src = L + (long long)j * lcs;
+      for (int r = r0 + lane; r < n16; r += 32) {
+        const bool v = r < jb;
+        cp_async_elem<T>(&S[r], v ? src + r : L, v);
+      }
+    }
+  } else {
+    const int dr = lane >> 3, dc = lane & 7;
+    for (int r = kSub + 4 * warp + dr; r < n16; r += 4 * (NT / 32)) {
+      const T* src = L + (long long)r * lrs;
+      const int ce = r & ~(kSub - 1);
+      for (int j = dc; j < ce; j += 8) {
+        const int p = j / kSub;
+        const bool v = r < jb;
+        cp_async_elem<T>(&Ls[SM::strip_off(p) + (j & (kSub - 1)) * SM::strip_ld(p) + r - kSub * (p + 1)],
+                         v ? src + (long long)j * lcs : L, v);
+      }
+    }
+  }
+  if (t < n16) rd[t] = (t < jb) ? RealOf<T>(1) / re(L[(long long)t * (lrs + lcs)]) : RealOf<T>(0);
+  cp_async_wait_all();
   __syncthreads();
-  T* Xt = reinterpret_cast<T*>(smem_raw);   // [64][129]: Xt[r * 129 + col]
-#pragma unroll
-  for (int k = 0; k < 32; ++k) Xt[r * 129 + cg * 32 + k] = x[k];
-  __syncthreads();
-  const int rows = min(64, m - (int)blockIdx.x * 64);
-  const long long row0 = (long long)blockIdx.x * 64;
+
+  for (int c0 = 0; c0 < n16; c0 += kSub) {
+    const int p = c0 / kSub, c1 = c0 + kSub;
+    if (warp < SW) {
+      solve16<T>(Xs + c0 * LDX + t, LDX, Lsh + p * kSub * kSub, rd + c0);
+    } else if (p > 0) {
+      // columns past this sub-panel, by the previous one
+      int w = warp - SW;
+      for (int cb = c1; cb < n16; cb += kSub)
+        for (int rb = 0; rb < R; rb += 32) {
+          if (w == 0)
+            tile_update<T>(Xs + cb * LDX + rb, LDX, Xs + (c0 - kSub) * LDX + rb, LDX,
+                           Ls + SM::strip_off(p - 1) + (cb - c0), SM::strip_ld(p - 1), 32);
+          w = (w == 0) ? NT / 32 - SW - 1 : w - 1;
+        }
+    }
+    __syncthreads();
+    if (c1 >= n16) break;
+    strip_update<T, R, NT>(Xs + c1 * LDX, LDX, Xs + c0 * LDX, LDX, Ls + SM::strip_off(p), SM::strip_ld(p), R);
+    __syncthreads();
+  }
+
+  // the solved tile to each output in the order that is contiguous in that output
   auto put = [&](auto* out, long long rs_, long long cs_, auto conv) {
-    if (rs_ == 1) {        // rows contiguous: consecutive threads take consecutive rows
-      for (int e = t; e < 64 * jb; e += 256) {
-        const int rr = e & 63, c = e >> 6;
-        if (rr < rows) out[(row0 + rr) * rs_ + (long long)c * cs_] = conv(Xt[rr * 129 + c]);
+    if (rs_ == 1) {
+      for (int c = warp; c < jb; c += NT / 32) {
+        auto* dst = out + row0 + (long long)c * cs_;
+#pragma unroll
+        for (int r = lane; r < R; r += 32)
+          if (r < rows) dst[r] = conv(Xs[c * LDX + r]);
       }
-    } else {               // columns contiguous (or neither): consecutive threads take consecutive columns
-      for (int e = t; e < rows * jb; e += 256) {
-        const int rr = e / jb, c = e - rr * jb;
-        out[(row0 + rr) * rs_ + (long long)c * cs_] = conv(Xt[rr * 129 + c]);
+    } else if (SM::dmma) {
+      const int dr = lane >> 3, dc = lane & 7;
+      for (int r = 4 * warp + dr; r < rows; r += 4 * (NT / 32)) {
+        auto* dst = out + (row0 + r) * rs_;
+        for (int c = dc; c < jb; c += 8) dst[(long long)c * cs_] = conv(Xs[c * LDX + r]);
+      }
+    } else {
+      for (int r = warp; r < rows; r += NT / 32) {
+        auto* dst = out + (row0 + r) * rs_;
+        for (int c = lane; c < jb; c += 32) dst[(long long)c * cs_] = conv(Xs[c * LDX + r]);
       }
     }
   };
-  put(B, brs, bcs, [](T v) { return cvt<TB>(v); });
+  put(B, brs, bcs, [](T v) { return v; });
   if constexpr (MODE == OUT_ROUND) {
     put(out2, o_rs, o_cs, [](T v) { return to_op<O2>((float)v); });
+  } else if constexpr (MODE == OUT_SPLIT && Traits<T>::complex) {
+    // two rows of the split per row: (re, im) and (-im, re); o_rs floats per row of the split
+    for (int r = warp; r < rows; r += NT / 32)
+    for (int c = lane; c < jb; c += 32) {
+      const T v = Xs[c * LDX + r];
+      const float re = (float)v.x, im = (float)v.y, rh = round_tf32(re), ih = round_tf32(im);
+      const float rl = round_tf32(re - rh), il = round_tf32(im - ih);
+      const long long o = 2 * (row0 + r) * o_rs + 2 * c;
+      *reinterpret_cast<float2*>(out2 + o) = make_float2(rh, ih);
+      *reinterpret_cast<float2*>(out2 + o + o_rs) = make_float2(-ih, rh);
+      *reinterpret_cast<float2*>(out3 + o) = make_float2(rl, il);
+      *reinterpret_cast<float2*>(out3 + o + o_rs) = make_float2(-il, rl);
+    }
   } else if constexpr (MODE == OUT_SPLIT) {
     put(out2, o_rs, o_cs, [](T v) { return round_tf32((float)v); });
     put(out3, o_rs, o_cs, [](T v) {
@@ -140,15 +199,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 16 ? 1 : 2)
       return round_tf32((float)v - hi);
     });
   } else {
-    put(out2, o_rs, o_cs, [](T v) { return cvt<O2>(v); });
+    put(out2, o_rs, o_cs, [](T v) { return v; });
   }
-}
-
-// Shared memory of trsm_rows_kernel: the diagonal block rows, the published solved
-// block and the reciprocal pivots, and later the 64 x 128 output tile (padded).
-template <typename T>
-constexpr size_t trsm_rows_smem() {
-  return sizeof(T) * ((128 * 33 + 64 * 33 + 32) > 64 * 129 ? (128 * 33 + 64 * 33 + 32) : 64 * 129);
 }
 
 }  // namespace cuchol
