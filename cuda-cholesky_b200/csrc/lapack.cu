@@ -22,6 +22,7 @@
 #include "panel.cuh"
 #include "tc.cuh"
 #include "trsm.cuh"
+#include "tcgemm.cuh"
 #include "tuning.cuh"
 
 using namespace cuchol;
@@ -556,6 +557,108 @@ CUresult tc3_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
   return CUDA_SUCCESS;
 }
 
+// ---- FP32 products, real and complex, on the TF32 tensor cores (tcgemm.cuh) ---------
+template <typename T> constexpr bool is_fp32() { return std::is_same<T, float>::value || std::is_same<T, cuFloatComplex>::value; }
+template <typename T> constexpr int real_per() { return Traits<T>::complex ? 2 : 1; }
+
+// A pack (k-major, `rows` rows of pitch ld floats) as a TMA map of 128-row x 32-k tiles;
+// step 2 takes every other row (the A form of a complex B pack).
+bool make_pack_map(CUtensorMap* map, const float* base, long long rows, long long ld, int step) {
+  EncodeTiledFn fn = encode_tiled();
+  if (fn == nullptr) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)((rows + step - 1) / step)};
+  const cuuint64_t str[1] = {(cuuint64_t)ld * step * sizeof(float)};
+  const cuuint32_t box[2] = {(cuuint32_t)tcg::BK, (cuuint32_t)tcg::BM}, es[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, str, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+struct PackRef { const float *hi, *lo; long long rows, ld; int step; };
+
+CUresult tcg_launch(CULAPACKhandle h, const PackRef& A, const PackRef& B, tcg::Params p, cudaStream_t s,
+                    const int* stop) {
+  CUtensorMap ah, al, bh, bl;
+  if (!make_pack_map(&ah, A.hi, A.rows, A.ld, A.step) || !make_pack_map(&al, A.lo, A.rows, A.ld, A.step) ||
+      !make_pack_map(&bh, B.hi, B.rows, B.ld, B.step) || !make_pack_map(&bl, B.lo, B.rows, B.ld, B.step))
+    return CUDA_ERROR_INVALID_VALUE;
+  p.tiles_m = (p.m + tcg::BM - 1) / tcg::BM;
+  p.tiles_n = (p.n + tcg::BN - 1) / tcg::BN;
+  p.vec = (p.cs == p.cx) && aligned16(p.c) && (p.rs % 4) == 0 && (p.c_node % 4) == 0;
+  p.err = h->d_words + 3;
+  static bool attr = false;
+  if (!attr) {
+    CUCHOL_CHECK(cudaFuncSetAttribute(tcg::gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcg::SMEM_BYTES));
+    attr = true;
+  }
+  tcg::gemm_kernel<<<p.nodes * p.tiles_m * p.tiles_n, tcg::THREADS, tcg::SMEM_BYTES, s>>>(ah, al, bh, bl, p, stop);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
+CUresult pack_launch(CULAPACKhandle h, const tcg::Packs& ps, cudaStream_t s) {
+  int gx = 0, gy = 0, gz = 0;
+  for (int i = 0; i < ps.count; ++i) {
+    const tcg::Pack& p = ps.p[i];
+    gx = std::max(gx, (std::max(p.kk, p.kk_last) + 31) / 32);
+    gy = std::max(gy, (std::max(p.rows, p.rows_last) + 31) / 32);
+    gz = std::max(gz, p.nodes);
+  }
+  tcg::pack_kernel<<<dim3(gx, gy, gz * ps.count), 256, 0, s>>>(ps);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
+// C -= Q(r) Q(c)^H on the logical lower trapezoid m x ncols of A (corner at r0 on the
+// diagonal) from the split panel of the panel solve (pack rows from qrow, columns koff ..
+// koff + k): any alignment and both storages.
+template <typename T>
+CUresult tcg_update(CULAPACKhandle h, const float* qhi, const float* qlo, long long ldq, int q_rows, int qrow, int koff,
+                    int k, T* corner, long long rs, long long cs, int m, int ncols, cudaStream_t s, const int* stop) {
+  constexpr int cx = real_per<T>();
+  if (m <= 0 || ncols <= 0 || k <= 0) return CUDA_SUCCESS;
+  tcg::Params p{};
+  p.nodes = 1;
+  p.m = p.m_last = m;
+  p.n = ncols * cx;
+  p.k = p.k_last = k * cx;
+  p.kmode = tcg::K_FULL;
+  p.cx = cx;
+  p.a_row0 = qrow;
+  p.b_row0 = qrow * cx;
+  p.k0 = koff * cx;
+  p.c = reinterpret_cast<float*>(corner);
+  p.rs = rs * cx;
+  p.cs = cs * cx;
+  p.beta = 1;
+  p.neg = 1;
+  p.lower_only = 1;
+  p.real_diag = 1;
+  return tcg_launch(h, PackRef{qhi, qlo, (long long)q_rows * cx, ldq, cx}, PackRef{qhi, qlo, (long long)q_rows * cx, ldq, 1},
+                    p, s, stop);
+}
+
+// Grows the workspace like ensure_workspace, but an allocation that fails is not an
+// error: false, and the caller takes a path that needs less.
+constexpr size_t kTcgWorkspace = size_t(8) << 30;
+bool try_workspace(CULAPACKhandle h, size_t bytes) {
+  if (bytes <= h->ws_bytes) return true;
+  if (bytes > kTcgWorkspace || cudaStreamSynchronize(h->s_panel) != cudaSuccess ||
+      cudaStreamSynchronize(h->s_update) != cudaSuccess)
+    return false;
+  void* p = nullptr;
+  if (dev_malloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaFree(h->ws);
+  h->ws = p;
+  h->ws_bytes = bytes;
+  return true;
+}
+
 // ---- ?POTRF ---------------------------------------------------------------------
 // Right-looking blocked Cholesky, outer blocks of NB = sub*nb columns (each factored
 // as sub nb-wide sub-panels; sub from the tuning table, 2 to 8 by n for FP64),
@@ -595,17 +698,23 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   int* d_info = h->d_words;
 
   const long long ldp = (long long)round_up((size_t)n, 2);
-  // FP32 with an aligned A: the updates run on the TF32 tensor cores as split
+  // FP32 (real and complex): the updates run on the TF32 tensor cores as split
   // products, from hi / lo copies of the solved panel in k-major buffers Q (row
-  // r = P row r, pitch ldq), ping-pong like P; P itself is then not needed
-  bool tc3 = false;
-  if constexpr (std::is_same<T, float>::value) tc3 = !h->force_simt && tc3_usable(A, lda) && n > 128;
-  const long long ldq = (long long)round_up((size_t)NB, 32);
-  const size_t ws = tc3 ? sizeof(T) * 4 * (size_t)n * ldq : sizeof(T) * (2 * (size_t)ldp * NB);
+  // r = P row r, pitch ldq; complex: two rows, 2r = (re, im) and 2r + 1 = (-im, re)),
+  // ping-pong like P; P itself is then not needed.  An aligned real A takes the kernel
+  // that adds into C with TMA, the others the one that reads and writes C itself.  n % 4:
+  // TMA clips its last row piece to 16 bytes, not to elements, and would add to the
+  // padding rows below an order that is not a multiple of four.
+  constexpr int cx = real_per<T>();
+  const bool tc3 = is_fp32<T>() && !h->force_simt && n > 128;
+  const bool tc3_tma = tc3 && n % 4 == 0 && tc3_usable(reinterpret_cast<const float*>(A), lda);
+  const long long ldq = (long long)round_up((size_t)NB, 32) * cx;
+  const size_t qsize = (size_t)n * cx * ldq;   // floats of one buffer
+  const size_t ws = tc3 ? sizeof(float) * 4 * qsize : sizeof(T) * (2 * (size_t)ldp * NB);
   CUCHOL_CHECK_CU(ensure_workspace(h, ws));
   T* pbuf[2] = {static_cast<T*>(h->ws), static_cast<T*>(h->ws) + (size_t)ldp * NB};
-  T* qbuf[4] = {static_cast<T*>(h->ws), static_cast<T*>(h->ws) + (size_t)n * ldq,
-                static_cast<T*>(h->ws) + 2 * (size_t)n * ldq, static_cast<T*>(h->ws) + 3 * (size_t)n * ldq};
+  float* qbuf[4];
+  for (int i = 0; i < 4; ++i) qbuf[i] = static_cast<float*>(h->ws) + i * qsize;
 
   CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
   CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
@@ -617,11 +726,14 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   const T minus_one = from_real<T>(RealOf<T>(-1)), one = from_real<T>(RealOf<T>(1));
   // C -= Phat Phat^H on the lower trapezoid m x ncols of A with its corner on the
   // diagonal at r0; operand rows from P row prow (both sides), k columns [koff, koff + k)
-  auto update = [&](const T* P, const T* Qh, const T* Ql, int r0, int m, int ncols, int prow, int koff, int k,
+  auto update = [&](const T* P, const float* Qh, const float* Ql, int r0, int m, int ncols, int prow, int koff, int k,
                     cudaStream_t s) -> CUresult {
     if constexpr (std::is_same<T, float>::value) {
-      if (tc3)
+      if (tc3_tma)
         return tc3_update(h, Qh, Ql, ldq, n, prow, koff, k, A, lda, upper, r0, m, ncols, s, d_info);
+    }
+    if constexpr (is_fp32<T>()) {
+      if (tc3) return tcg_update<T>(h, Qh, Ql, ldq, n, prow, koff, k, at(r0, r0), rs, cs, m, ncols, s, d_info);
     }
     const T* pa = P + prow + (long long)koff * ldp;
     GemmProblem<T> u = problem<T>();
@@ -640,8 +752,8 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     const int m = n - j - jB;                    // rows below the outer block
     const int mc = ncols - j - jB;               // columns right of it (in the panel)
     T* P = pbuf[step & 1];
-    T* Qh = qbuf[2 * (step & 1)];
-    T* Ql = qbuf[2 * (step & 1) + 1];
+    float* Qh = qbuf[2 * (step & 1)];
+    float* Ql = qbuf[2 * (step & 1) + 1];
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;                 // rows below this diagonal block
@@ -653,18 +765,16 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
       // panel solve into P: rows c + jb .. n-1 are P rows s0 .. (P starts at j + nb)
       // row-parallel triangular solve: A21 := A21 L11^-H in place, and into P (or its
       // hi / lo split into Q)
-      bool split = false;
-      if constexpr (std::is_same<T, float>::value) {
-        if (tc3) {
-          const long long qo = (long long)s0 * ldq + s0;
-          CUCHOL_CHECK_CU((panel_solve<T, T, OUT_SPLIT, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Qh + qo, ldq, 1,
-                                                            Ql + qo, sp)));
-          split = true;
+      if (tc3) {
+        if constexpr (is_fp32<T>()) {
+          const long long qo = (long long)s0 * cx * ldq + s0 * cx;
+          CUCHOL_CHECK_CU((panel_solve<T, float, OUT_SPLIT, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Qh + qo, ldq,
+                                                                1, Ql + qo, sp)));
         }
-      }
-      if (!split)
+      } else {
         CUCHOL_CHECK_CU((panel_solve<T, T, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs,
-                                                         P + s0 + (long long)s0 * ldp, 1, ldp, nullptr, sp)));
+                                                            P + s0 + (long long)s0 * ldp, 1, ldp, nullptr, sp)));
+      }
       CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
       if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
       if (s0 + nb < jB) {
@@ -720,6 +830,100 @@ int build_tree(int o, int s, int nb, std::vector<Node>& out) {
   return hgt;
 }
 
+// FP32 orders from which ?trtri and ?lauum run on the TF32 tensor cores.
+constexpr int kTcgMinOrder = 256;
+
+// Whether the split products are safe for the triangle of A: every entry finite and at
+// most 2^62, every diagonal entry (unless unit) at least 2^-62, so that no hi part
+// rounds to infinity, no product of two entries overflows, and what underflow drops
+// from a lo part (below 2^-126) is below 2^-60 of the larger entries.  Others take the
+// SIMT engine.  Synchronises.
+template <typename T>
+CUresult tcg_in_range(CULAPACKhandle h, const T* A, long long rs, long long cs, int n, bool unit, bool* ok) {
+  int* bad = h->d_words + 6;
+  cudaStream_t s = h->s_panel;
+  CUCHOL_CHECK(cudaMemsetAsync(bad, 0, sizeof(int), s));
+  const dim3 grid((n + 63) / 64, (n + 63) / 64);
+  tcg::range_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const float*>(A), rs * real_per<T>(), cs * real_per<T>(), n,
+                                         real_per<T>(), unit ? 1 : 0, bad);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words + 6, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CUCHOL_CHECK(cudaStreamSynchronize(s));
+  *ok = h->h_words[6] == 0;
+  return CUDA_SUCCESS;
+}
+
+// The levels of ?trtri above the inverted 128-wide diagonal blocks, bottom-up, for FP32:
+// level s joins pairs of inverted blocks of order s.  Per level one launch packs, for
+// all pairs, inv(T22), T21 and inv(T11); one forms X = inv(T22) T21 straight into pack
+// form; one writes T21 := -X inv(T11).  *done = false when the workspace is refused.
+template <typename T>
+CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs, long long cs, bool* done) {
+  constexpr int cx = real_per<T>(), nb = Tune<T>::nb;
+  static_assert(nb == tcg::BM, "levels are multiples of the tile");
+  auto pairs = [&](int s) { return (n - s + 2 * s - 1) / (2 * s); };
+  // buffers of a level, in floats (hi and lo alike): inv(T22) and X (pairs*s rows), T21^T
+  // and inv(T11)^T (cx rows per row), all of pitch s*cx
+  size_t need = 0;
+  for (int s = nb; s < n; s *= 2) need = std::max(need, (size_t)pairs(s) * s * s * cx * (2 + 2 * cx) * 2);
+  *done = need == 0 || try_workspace(h, sizeof(float) * need);
+  if (!*done) return CUDA_SUCCESS;
+  cudaStream_t sp = h->s_panel;
+  float* a = reinterpret_cast<float*>(A);
+  for (int s = nb; s < n; s *= 2) {
+    const int np = pairs(s), s2_last = std::min(s, n - 2 * s * (np - 1) - s);
+    const long long ld = (long long)s * cx;
+    const size_t rows = (size_t)np * s, one = rows * ld;
+    float* w = static_cast<float*>(h->ws);
+    float *ia = w, *x = w + 2 * one, *b1 = w + 4 * one, *b2 = b1 + 2 * one * cx;   // each: hi, then lo
+    auto at = [&](long long i, long long j) { return a + (i * rs + j * cs) * cx; };
+    tcg::Packs ps{};
+    ps.count = 3;
+    for (int i = 0; i < 3; ++i) {
+      tcg::Pack& p = ps.p[i];
+      p.cx = cx;
+      p.nodes = np;
+      p.node_rows = s;
+      p.src_node = 2LL * s * (rs + cs) * cx;
+      p.ld = ld;
+      p.rows = p.rows_last = p.kk = p.kk_last = s;
+    }
+    tcg::Pack& p0 = ps.p[0];                    // A(i, k) = inv(T22)(i, k)
+    p0.src = at(s, s); p0.rs = rs * cx; p0.cs = cs * cx; p0.tri = TRI_LOWER; p0.unit = unit;
+    p0.rows_last = p0.kk_last = s2_last;
+    p0.hi = ia; p0.lo = ia + one;
+    tcg::Pack& p1 = ps.p[1];                    // B(j, k) = T21(k, j)
+    p1.src = at(s, 0); p1.rs = cs * cx; p1.cs = rs * cx; p1.two = cx == 2;
+    p1.kk_last = s2_last;
+    p1.hi = b1; p1.lo = b1 + one * cx;
+    tcg::Pack& p2 = ps.p[2];                    // B(j, k) = inv(T11)(k, j)
+    p2.src = at(0, 0); p2.rs = cs * cx; p2.cs = rs * cx; p2.two = cx == 2; p2.tri = TRI_UPPER; p2.unit = unit;
+    p2.hi = b2; p2.lo = b2 + one * cx;
+    CUCHOL_CHECK_CU(pack_launch(h, ps, sp));
+    tcg::Params g{};
+    g.nodes = np;
+    g.m = s; g.m_last = s2_last; g.n = s * cx;
+    g.cx = cx;
+    g.a_node = s; g.b_node = s * cx;
+    g.kmode = tcg::K_A_LOWER;
+    g.k = s * cx; g.k_last = s2_last * cx;
+    g.xhi = x; g.xlo = x + one; g.xld = ld;
+    const PackRef rb1{b1, b1 + one * cx, (long long)rows * cx, ld, 1}, rb2{b2, b2 + one * cx, (long long)rows * cx, ld, 1};
+    CUCHOL_CHECK_CU(tcg_launch(h, PackRef{ia, ia + one, (long long)rows, ld, 1}, rb1, g, sp, nullptr));
+    g.xhi = g.xlo = nullptr;
+    g.kmode = tcg::K_B_UPPER;
+    g.k_last = g.k;
+    g.c = at(s, 0);
+    g.rs = rs * cx; g.cs = cs * cx; g.c_node = p0.src_node;
+    g.neg = 1;
+    CUCHOL_CHECK_CU(tcg_launch(h, PackRef{x, x + one, (long long)rows, ld, 1}, rb2, g, sp, nullptr));
+  }
+  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
+  CUCHOL_CHECK(cudaStreamSynchronize(sp));
+  return check_engine(h);
+}
+
 template <typename T>
 CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long long lda, long* info) {
   const int nb = Tune<T>::nb;
@@ -727,6 +931,10 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel;
   *info = 0;
+  bool tensor = false;
+  if constexpr (is_fp32<T>()) {
+    if (!h->force_simt && n >= kTcgMinOrder) CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, unit, &tensor));
+  }
   if (!unit) {
     int init[3] = {0, 0, INT_MAX};
     CUCHOL_CHECK(cudaMemcpyAsync(h->d_words, init, sizeof(init), cudaMemcpyHostToDevice, sp));
@@ -747,6 +955,11 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
 
+  if constexpr (is_fp32<T>()) {
+    bool done = false;
+    if (tensor) CUCHOL_CHECK_CU(trtri_levels_tcg<T>(h, unit, n, A, rs, cs, &done));
+    if (done) return CUDA_SUCCESS;
+  }
   std::vector<Node> nodes;
   const int height = build_tree(0, n, nb, nodes);
   // workspace: X blocks of all nodes of one height side by side
@@ -813,6 +1026,41 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel;
+  if constexpr (is_fp32<T>()) {
+    // one pack of the whole triangle, from which the product is written straight over A
+    constexpr int cx = real_per<T>();
+    const long long ld = (long long)round_up((size_t)n, 32) * cx;
+    const size_t one = (size_t)n * cx * ld;
+    bool tensor = false;
+    if (!h->force_simt && n >= kTcgMinOrder && h->lauum_cols == 0)
+      CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, false, &tensor));
+    if (tensor && try_workspace(h, sizeof(float) * 2 * one)) {
+      float* w = static_cast<float*>(h->ws);
+      tcg::Packs ps{};
+      ps.count = 1;
+      tcg::Pack& p = ps.p[0];                   // B(j, k) = L(k, j); A(i, k) = conj(L(k, i)) is its even rows
+      p.src = reinterpret_cast<const float*>(A);
+      p.rs = cs * cx; p.cs = rs * cx;
+      p.nodes = 1; p.node_rows = p.rows = p.rows_last = p.kk = p.kk_last = n;
+      p.tri = TRI_UPPER; p.cx = cx; p.two = cx == 2;
+      p.hi = w; p.lo = w + one; p.ld = ld;
+      CUCHOL_CHECK_CU(pack_launch(h, ps, sp));
+      tcg::Params g{};
+      g.nodes = 1;
+      g.m = g.m_last = n; g.n = n * cx;
+      g.k = g.k_last = n * cx;
+      g.kmode = tcg::K_LAUUM;
+      g.cx = cx;
+      g.c = reinterpret_cast<float*>(A);
+      g.rs = rs * cx; g.cs = cs * cx;
+      g.lower_only = 1; g.real_diag = 1;
+      CUCHOL_CHECK_CU(tcg_launch(h, PackRef{w, w + one, (long long)n * cx, ld, cx}, PackRef{w, w + one, (long long)n * cx, ld, 1},
+                                 g, sp, nullptr));
+      CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
+      CUCHOL_CHECK(cudaStreamSynchronize(sp));
+      return check_engine(h);
+    }
+  }
   const int w = lauum_width<T>(h, n);
   const long long ldw = (long long)round_up((size_t)n, 2);
   CUCHOL_CHECK_CU(ensure_workspace(h, sizeof(T) * (size_t)ldw * w));
