@@ -42,6 +42,32 @@ __global__ void copy_view_kernel(const T* __restrict__ src, long long s_rs, long
   }
 }
 
+// dst(i, j) = sum over the slabs q that reach row i ((q + 1) slab > i) of
+// W[q * stride + i + j * ldw], in order, for i >= j (the k slabs of ?lauum).  32 x 32
+// tiles; through shared memory when the destination's rows are not contiguous.
+template <typename T>
+__global__ void sum_slabs_kernel(const T* __restrict__ W, long long ldw, long long stride, int slabs, int slab,
+                                 T* __restrict__ dst, long long rs, long long cs, int n) {
+  __shared__ T tile[32][33];
+  const int bi = blockIdx.x * 32, bj = blockIdx.y * 32;
+  if (bj > bi + 31) return;
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  for (int q = ty; q < 32; q += 8) {
+    const int i = bi + tx, j = bj + q;
+    if (i >= n || j > i) continue;
+    T v = zero<T>();
+    for (int s = i / slab; s < slabs; ++s) v = add(v, W[s * stride + i + j * ldw]);
+    if (rs == 1) dst[i + j * cs] = v;
+    else tile[q][tx] = v;
+  }
+  if (rs == 1) return;
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int i = bi + q, j = bj + tx;
+    if (i < n && j <= i) dst[i * rs + j * cs] = tile[tx][q];
+  }
+}
+
 // log det from a strided diagonal: 2 * sum log(Re x[i*incx]) in double, one pass.
 // Partial sums go to part[blockIdx.x]; the last CTA to finish (retirement counter,
 // as in the reference's lapack/dlogdet.cu:35,93-117) adds them in index order, so

@@ -48,7 +48,7 @@ template <int MB>
 struct Shape {
   static constexpr int BM = 32 * MB;
   static constexpr int STAGES = 4;
-  static constexpr int MIN_CTAS = MB == 4 ? 2 : 3;  // CTAs per SM the registers allow
+  static constexpr int MIN_CTAS = MB == 4 ? 2 : MB == 2 ? 3 : 4;  // CTAs per SM the registers allow
   static constexpr int A_STAGE = BM * BK * 8;       // 16 KB (MB = 4) or 8 KB
   static constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;   // + 1 KB alignment slack
@@ -57,6 +57,19 @@ constexpr unsigned kSpinLimit = 1u << 26;          // bounded mbarrier waits: at
 constexpr unsigned long long kWaitNs = 1000000000ull;   // and at most one second
 
 enum : int { LAYOUT_R = 0, LAYOUT_K = 1 };
+
+// Several problems of one shape in one launch of a TRI kernel (count >= 1; count = 1
+// and the rest zero: one problem).  Node q reads operand rows and k shifted by (row, k)
+// + q * (node_row, node_k) in the tensor maps and writes at c + q * c_node; the last
+// node has m_last rows and k_last k.  slab > 0: the nodes are instead the k ranges
+// [q slab, (q + 1) slab) of one problem (slab a multiple of 128), whose partial products
+// go to c + q * c_node; tiles without any k in a slab are not written.
+struct Nodes {
+  int count, m_last, k_last, slab;
+  int a_row, a_k, b_row, b_k;
+  int a_node_row, a_node_k, b_node_row, b_node_k;
+  long long c_node;
+};
 
 struct Params {
   double* c; long long c_rs, c_cs;
@@ -71,6 +84,7 @@ struct Params {
                          // the k loop, so its latency hides under the TMA fill)
   int neg;               // alpha = -1 (with preload): B fragments are negated
   int* err;              // set when a bounded wait gave up
+  Nodes nd;              // TRI kernels only
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -150,21 +164,33 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   // This CTA's tiles: blockIdx.x, blockIdx.x + gridDim.x, ...  The host picks the
   // grid so that a CTA handles several tiles: the TMA ring keeps streaming across
   // tile boundaries, while CTAs still retire often enough for other streams' kernels.
-  const int ntiles = P.tiles_m * P.tiles_n;
+  const int per = P.tiles_m * P.tiles_n;
+  const int ntiles = TRI ? per * P.nd.count : per;
   // rows i0, columns j0 and k range [kbase, kbase + KT*BK) of a tile (triangular
   // views limit it); false for a tile wholly above the diagonal of a lower-only output
-  auto tile_range = [&](int tile, int& i0, int& j0, int& kbase, int& KT) -> bool {
+  auto tile_range = [&](int tile, int& node, int& i0, int& j0, int& kbase, int& KT) -> bool {
+    node = TRI ? tile / per : 0;
+    if (TRI) tile -= node * per;
     i0 = (tile / P.tiles_n) * BM;
     j0 = (tile % P.tiles_n) * BN;
     if (P.lower_only && j0 > i0 + BM - 1) return false;
     int kb = 0, ke = P.k;
+    if (TRI) {
+      if (P.nd.slab > 0) {
+        kb = node * P.nd.slab;
+        ke = min(ke, kb + P.nd.slab);
+      } else if (node == P.nd.count - 1 && P.nd.count > 1) {
+        ke = P.nd.k_last;
+        if (i0 >= P.nd.m_last) return false;
+      }
+    }
     if (P.tri_a == TRI_LOWER) ke = min(ke, i0 + BM);
     if (P.tri_a == TRI_UPPER) kb = max(kb, i0);
     if (P.tri_b == TRI_LOWER) ke = min(ke, j0 + BN);
     if (P.tri_b == TRI_UPPER) kb = max(kb, j0);
     kbase = (kb / BK) * BK;
     KT = (ke > kbase) ? (ke - kbase + BK - 1) / BK : 0;
-    return true;
+    return !(TRI && P.nd.slab > 0 && KT == 0);
   };
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -185,20 +211,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   __syncthreads();
   // Thread 0 fills the ring in the order the tiles consume it: item q (the q-th
   // k block of this CTA, over all its tiles) goes to stage q % STAGES.
-  int p_tile = (int)blockIdx.x - (int)gridDim.x, p_kt = 0, p_KT = 0, p_i0 = 0, p_j0 = 0, p_kbase = 0;
+  int p_tile = (int)blockIdx.x - (int)gridDim.x, p_kt = 0, p_KT = 0, p_i0 = 0, p_j0 = 0, p_kbase = 0, p_node = 0;
   long long issued = 0, consumed = 0;
   auto produce = [&]() -> bool {   // issue the next item; false when none is left
     while (p_kt >= p_KT) {
       p_tile += gridDim.x;
       if (p_tile >= ntiles) return false;
       p_kt = 0;
-      if (!tile_range(p_tile, p_i0, p_j0, p_kbase, p_KT)) p_KT = 0;
+      if (!tile_range(p_tile, p_node, p_i0, p_j0, p_kbase, p_KT)) p_KT = 0;
     }
     const int s = (int)(issued % STAGES);
     unsigned char* st = smem + s * STAGE_BYTES;
     mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-    load_operand<LA, BM>(&mapA, &full_bar[s], st, p_i0, p_kbase + p_kt * BK);
-    load_operand<LB, BN>(&mapB, &full_bar[s], st + A_STAGE, p_j0, p_kbase + p_kt * BK);
+    int ar = p_i0, ak = p_kbase + p_kt * BK, br = p_j0, bk = ak;
+    if (TRI && P.nd.slab == 0) {
+      ar += P.nd.a_row + p_node * P.nd.a_node_row;
+      ak += P.nd.a_k + p_node * P.nd.a_node_k;
+      br += P.nd.b_row + p_node * P.nd.b_node_row;
+      bk += P.nd.b_k + p_node * P.nd.b_node_k;
+    }
+    load_operand<LA, BM>(&mapA, &full_bar[s], st, ar, ak);
+    load_operand<LB, BN>(&mapB, &full_bar[s], st + A_STAGE, br, bk);
     ++p_kt;
     ++issued;
     return true;
@@ -228,11 +261,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   const int arow1 = (LA == LAYOUT_R) ? 2 * g + 1 : fg + 8;
   bool ok = true;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-  int i0, j0, kbase, KT;
-  if (!tile_range(tile, i0, j0, kbase, KT)) continue;
+  int node, i0, j0, kbase, KT;
+  if (!tile_range(tile, node, i0, j0, kbase, KT)) continue;
+  const int pm = (TRI && P.nd.count > 1 && P.nd.slab == 0 && node == P.nd.count - 1) ? P.nd.m_last : P.m;
+  const long long cshift = TRI ? node * P.nd.c_node : 0;
   double acc[MB][4][4];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < MB; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -245,7 +280,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
     if constexpr (LB == LAYOUT_R) return (nb8 >> 1) * 16 + 4 * t + 2 * e1 + (nb8 & 1);
     else return nb8 * 8 + t + 4 * e1;
   };
-  const bool full_tile = (i0 + BM <= P.m) && (j0 + BN <= P.n) && (!P.lower_only || j0 + BN - 1 <= i0);
+  const bool full_tile = (i0 + BM <= pm) && (j0 + BN <= P.n) && (!P.lower_only || j0 + BN - 1 <= i0);
   const bool vec_rows = (LA == LAYOUT_R) && full_tile && P.vec_ok && P.c_rs == 1;
   const bool vec_cols = !vec_rows && (LB == LAYOUT_R) && full_tile && P.vec_ok && P.c_cs == 1;
   if (P.preload && P.cin != nullptr) {
@@ -283,7 +318,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
           for (int e = 0; e < 4; ++e) {
             const int row = wrow + mb * 16 + (e < 2 ? arow0 : arow1);
             const int col = wcol + colof(nb8, e & 1);
-            if (row < P.m && col < P.n && (!P.lower_only || row >= col))
+            if (row < pm && col < P.n && (!P.lower_only || row >= col))
               acc[mb][nb8][e] = P.beta * P.cin[row * P.cin_rs + (long long)col * P.cin_cs];
           }
     }
@@ -465,7 +500,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
 #pragma unroll
         for (int e1 = 0; e1 < 2; ++e1) {
           const int row = wrow + mb * 16 + arow0, col = wcol + colof(nb8, e1);
-          double2* ptr = reinterpret_cast<double2*>(P.c + row + (long long)col * P.c_cs);
+          double2* ptr = reinterpret_cast<double2*>(P.c + cshift + row + (long long)col * P.c_cs);
           double2 v = make_double2(alpha * acc[mb][nb8][e1], alpha * acc[mb][nb8][2 + e1]);
           if (has_cin) {
             const double2 o = *ptr;
@@ -484,7 +519,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
         for (int p = 0; p < 2; ++p) {
           const int row = wrow + mb * 16 + (e < 2 ? arow0 : arow1);
           const int col = wcol + colof(2 * p, e & 1);
-          double2* ptr = reinterpret_cast<double2*>(P.c + (long long)row * P.c_rs + col);
+          double2* ptr = reinterpret_cast<double2*>(P.c + cshift + (long long)row * P.c_rs + col);
           double2 v = make_double2(alpha * acc[mb][2 * p][e], alpha * acc[mb][2 * p + 1][e]);
           if (has_cin) {
             const double2 o = *ptr;
@@ -502,10 +537,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
         for (int e = 0; e < 4; ++e) {
           const int row = wrow + mb * 16 + (e < 2 ? arow0 : arow1);
           const int col = wcol + colof(nb8, e & 1);
-          if (row < P.m && col < P.n && (!P.lower_only || row >= col)) {
+          if (row < pm && col < P.n && (!P.lower_only || row >= col)) {
             double v = alpha * acc[mb][nb8][e];
             if (has_cin) v = fma(P.beta, P.cin[row * P.cin_rs + (long long)col * P.cin_cs], v);
-            P.c[row * P.c_rs + (long long)col * P.c_cs] = v;
+            P.c[cshift + row * P.c_rs + (long long)col * P.c_cs] = v;
           }
         }
   }

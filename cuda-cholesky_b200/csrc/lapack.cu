@@ -216,16 +216,37 @@ CUresult launch_dmma_layouts(CULAPACKhandle h, int la, int lb, const CUtensorMap
   return launch_dmma<1, 1, TRI, MB>(h, ma, mb, q, tiles, s, abort);
 }
 
+// What a launch over several problems adds to a GemmProblem (which then describes one
+// of them, its views starting at the first element of the matrices that the tensor maps
+// cover: a_rows x a_ks and b_rows x b_ks).
+struct NodeLaunch {
+  dmma::Nodes nd;
+  long long a_rows, a_ks, b_rows, b_ks;
+};
+
+// Tiles of height bm (width 64) of a launch.
+template <typename T>
+inline long long count_tiles(const GemmProblem<T>& p, const NodeLaunch* nl, int bm) {
+  const long long tm = (p.m + bm - 1) / bm, tn = (p.n + 63) / 64;
+  return (nl != nullptr ? nl->nd.count : 1) * (p.lower_only ? tm * tn - std::min(tm * bm / 64, tn) * tn / 2 : tm * tn);
+}
+
 // Warp tile height of the FP64 engine for a problem (m16 blocks per warp): 64 x 64
 // tiles, three CTAs per SM, for the updates of the factorizations (k up to about a
 // thousand: more resident warps and finer waves measured faster), 128 x 64 tiles,
-// two per SM, for long products (fewer operand bytes per flop).
-inline int dmma_mb(const GemmProblem<double>& p) { return p.k >= 2048 ? 4 : 2; }
+// two per SM, for long products that fill the SMs several times (fewer operand bytes
+// per flop), and 32 x 64 tiles for launches that would leave SMs without one: an SM
+// runs a lone tile at its full FP64 rate, so the launch takes as long as one tile.
+inline int dmma_mb(const GemmProblem<double>& p, const NodeLaunch* nl, int sms) {
+  if (p.k >= 2048 && count_tiles(p, nl, 128) >= 8LL * sms) return 4;
+  return count_tiles(p, nl, 64) <= sms ? 1 : 2;
+}
 
 // Runs the problem on the FP64 tensor-core engine if its views fit the engine
 // (each view row- or k-contiguous, 16-byte aligned, even leading dimension);
 // returns false (nothing launched) otherwise.
-bool try_dmma(CULAPACKhandle h, const GemmProblem<double>& p, cudaStream_t s, const int* abort, CUresult* rc) {
+bool try_dmma(CULAPACKhandle h, const GemmProblem<double>& p, cudaStream_t s, const int* abort, CUresult* rc,
+              const NodeLaunch* nl = nullptr) {
   const int la = (p.a_rs == 1) ? dmma::LAYOUT_R : (p.a_ks == 1 ? dmma::LAYOUT_K : -1);
   const int lb = (p.b_rs == 1) ? dmma::LAYOUT_R : (p.b_ks == 1 ? dmma::LAYOUT_K : -1);
   if (la < 0 || lb < 0 || p.k <= 0) return false;
@@ -233,10 +254,14 @@ bool try_dmma(CULAPACKhandle h, const GemmProblem<double>& p, cudaStream_t s, co
   const long long ldb = (lb == dmma::LAYOUT_R) ? p.b_ks : p.b_rs;
   if ((lda & 1) || (ldb & 1) || !aligned16(p.a) || !aligned16(p.b)) return false;
   CUtensorMap ma, mb;
-  const int mbk = dmma_mb(p), bm = 32 * mbk;
-  if (!make_map(&ma, p.a, la, p.m, p.k, lda, bm) || !make_map(&mb, p.b, lb, p.n, p.k, ldb, dmma::BN))
+  const int mbk = dmma_mb(p, nl, h->num_sms), bm = 32 * mbk;
+  if (!make_map(&ma, p.a, la, nl ? nl->a_rows : p.m, nl ? nl->a_ks : p.k, lda, bm) ||
+      !make_map(&mb, p.b, lb, nl ? nl->b_rows : p.n, nl ? nl->b_ks : p.k, ldb, dmma::BN))
     return false;
   dmma::Params q;
+  q.nd = dmma::Nodes{};
+  q.nd.count = 1;
+  if (nl != nullptr) q.nd = nl->nd;
   q.c = p.c; q.c_rs = p.c_rs; q.c_cs = p.c_cs;
   q.cin = p.cin; q.cin_rs = p.cin_rs; q.cin_cs = p.cin_cs;
   q.m = p.m; q.n = p.n; q.k = p.k;
@@ -252,11 +277,13 @@ bool try_dmma(CULAPACKhandle h, const GemmProblem<double>& p, cudaStream_t s, co
   q.neg = q.preload && p.alpha == -1.0;
   q.err = h->d_words + 3;
   q.tiles_m = (p.m + bm - 1) / bm;
-  const int all_tiles = q.tiles_m * q.tiles_n;
   // one tile per CTA: several tiles per CTA measured slower (tails, uneven skipping)
-  const int tiles = all_tiles;
+  const int tiles = q.tiles_m * q.tiles_n * q.nd.count;
   const bool tri = p.tri_a || p.tri_b || p.unit_a || p.unit_b;
-  if (mbk == 2)
+  if (mbk == 1)
+    *rc = tri ? launch_dmma_layouts<true, 1>(h, la, lb, ma, mb, q, tiles, s, abort)
+              : launch_dmma_layouts<false, 1>(h, la, lb, ma, mb, q, tiles, s, abort);
+  else if (mbk == 2)
     *rc = tri ? launch_dmma_layouts<true, 2>(h, la, lb, ma, mb, q, tiles, s, abort)
               : launch_dmma_layouts<false, 2>(h, la, lb, ma, mb, q, tiles, s, abort);
   else
@@ -317,15 +344,18 @@ CUresult launch_zmma_layouts(CULAPACKhandle h, int la, int lb, const CUtensorMap
 // Warp tile height of the complex engine for a problem (m16 blocks per warp): 32 x 64
 // tiles, three CTAs per SM, for k < 1024 (the updates of zpotrf up to n = 16384: their
 // CTAs retire twice as often, so the panel chain finds SMs sooner; zpotrf n = 8192
-// 38.2 -> 36.9 ms, n = 4096 9.7 -> 8.7 ms), 64 x 64 otherwise.
+// 38.2 -> 36.9 ms, n = 4096 9.7 -> 8.7 ms) and for launches that do not fill the SMs
+// several times, 64 x 64 otherwise.
 constexpr int kZmmaShortK = 1024;
-inline int zmma_mb(const GemmProblem<cuDoubleComplex>& p) { return p.k < kZmmaShortK ? 1 : 2; }
+inline int zmma_mb(const GemmProblem<cuDoubleComplex>& p, const NodeLaunch* nl, int sms) {
+  return p.k < kZmmaShortK || count_tiles(p, nl, 64) < 8LL * sms ? 1 : 2;
+}
 
 // Runs a complex double problem on the FP64 tensor-core engine when both operand
 // views are row- or k-contiguous and 16-byte aligned; false (nothing launched)
 // otherwise.
 bool try_zmma(CULAPACKhandle h, const GemmProblem<cuDoubleComplex>& p, cudaStream_t s, const int* abort,
-              CUresult* rc) {
+              CUresult* rc, const NodeLaunch* nl = nullptr) {
   const int la = (p.a_rs == 1) ? dmma::LAYOUT_R : (p.a_ks == 1 ? dmma::LAYOUT_K : -1);
   const int lb = (p.b_rs == 1) ? dmma::LAYOUT_R : (p.b_ks == 1 ? dmma::LAYOUT_K : -1);
   if (la < 0 || lb < 0 || p.k <= 0) return false;
@@ -333,10 +363,14 @@ bool try_zmma(CULAPACKhandle h, const GemmProblem<cuDoubleComplex>& p, cudaStrea
   const long long ldb = (lb == dmma::LAYOUT_R) ? p.b_ks : p.b_rs;
   if (!aligned16(p.a) || !aligned16(p.b)) return false;
   CUtensorMap ma, mb;
-  const int mbk = zmma_mb(p), bm = 32 * mbk;
-  if (!make_zmap(&ma, p.a, la, p.m, p.k, lda, bm) || !make_zmap(&mb, p.b, lb, p.n, p.k, ldb, zmma::BN))
+  const int mbk = zmma_mb(p, nl, h->num_sms), bm = 32 * mbk;
+  if (!make_zmap(&ma, p.a, la, nl ? nl->a_rows : p.m, nl ? nl->a_ks : p.k, lda, bm) ||
+      !make_zmap(&mb, p.b, lb, nl ? nl->b_rows : p.n, nl ? nl->b_ks : p.k, ldb, zmma::BN))
     return false;
   zmma::Params q;
+  q.nd = dmma::Nodes{};
+  q.nd.count = 1;
+  if (nl != nullptr) q.nd = nl->nd;
   q.c = p.c; q.c_rs = p.c_rs; q.c_cs = p.c_cs;
   q.cin = p.cin; q.cin_rs = p.cin_rs; q.cin_cs = p.cin_cs;
   q.m = p.m; q.n = p.n; q.k = p.k;
@@ -351,7 +385,7 @@ bool try_zmma(CULAPACKhandle h, const GemmProblem<cuDoubleComplex>& p, cudaStrea
               (p.cin == nullptr || (p.cin_rs == p.c_rs && p.cin_cs == p.c_cs) || p.cin != p.c);
   q.neg = q.preload && p.alpha.x == -1.0;
   q.err = h->d_words + 3;
-  const int tiles = q.tiles_m * q.tiles_n;
+  const int tiles = q.tiles_m * q.tiles_n * q.nd.count;
   const bool tri = p.tri_a || p.tri_b || p.unit_a || p.unit_b;
   if (mbk == 1)
     *rc = tri ? launch_zmma_layouts<true, 1>(h, la, lb, ma, mb, q, tiles, s, abort)
@@ -924,6 +958,67 @@ CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs
   return check_engine(h);
 }
 
+template <typename T> constexpr bool is_fp64() { return std::is_same<T, double>::value || std::is_same<T, cuDoubleComplex>::value; }
+
+// Whether the FP64 tensor-core engines read views of A directly (16-byte aligned, real:
+// even leading dimension).
+template <typename T>
+bool fp64_aligned(const T* A, long long lda) {
+  return aligned16(A) && (sizeof(T) == 16 || !(lda & 1));
+}
+
+template <typename T>
+CUresult gemm_nodes(CULAPACKhandle h, const GemmProblem<T>& p, const NodeLaunch& nl, cudaStream_t s) {
+  CUresult rc = CUDA_ERROR_NOT_SUPPORTED;
+  bool ran = false;
+  if constexpr (std::is_same<T, double>::value) ran = try_dmma(h, p, s, nullptr, &rc, &nl);
+  if constexpr (std::is_same<T, cuDoubleComplex>::value) ran = try_zmma(h, p, s, nullptr, &rc, &nl);
+  return ran ? rc : CUDA_ERROR_NOT_SUPPORTED;
+}
+
+// The levels of ?trtri above the inverted nb-wide diagonal blocks, bottom-up, FP64: level
+// s joins all pairs of inverted blocks of order s in two launches, X = inv(T22) T21 into
+// workspace (the X of pair q are rows q s .. of it) and T21 := -X inv(T11).  One launch
+// per pair and product, as the recursive splits took for up to eight pairs, ran small
+// levels one after the other on a nearly idle GPU: n = 2048 30 launches, 970 us.
+template <typename T>
+CUresult trtri_levels_fp64(CULAPACKhandle h, bool unit, int n, T* A, long long lda, bool upper, T* X, cudaStream_t sp) {
+  constexpr int nb = Tune<T>::nb;
+  const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
+  for (int s = nb; s < n; s *= 2) {
+    const int np = (n - s + 2 * s - 1) / (2 * s), s2 = std::min(s, n - 2 * s * (np - 1) - s);
+    const int m = np > 1 ? s : s2;
+    const long long ldx = (long long)np * s;
+    NodeLaunch nl{};
+    nl.nd.count = np;
+    nl.nd.m_last = s2;
+    GemmProblem<T> a = problem<T>();            // X = inv(T22) T21
+    a.a = A; a.a_rs = rs; a.a_ks = cs; a.tri_a = TRI_LOWER; a.unit_a = unit;
+    a.b = A; a.b_rs = cs; a.b_ks = rs;          // B(j, k) = T21(k, j)
+    a.c = X; a.c_rs = 1; a.c_cs = ldx;
+    a.m = m; a.n = s; a.k = m;
+    nl.a_rows = nl.a_ks = nl.b_rows = nl.b_ks = n;
+    nl.nd.k_last = s2;
+    nl.nd.a_row = nl.nd.a_k = nl.nd.b_k = s;
+    nl.nd.a_node_row = nl.nd.a_node_k = nl.nd.b_node_row = nl.nd.b_node_k = 2 * s;
+    nl.nd.c_node = s;
+    CUCHOL_CHECK_CU(gemm_nodes<T>(h, a, nl, sp));
+    GemmProblem<T> b = problem<T>();            // T21 = -X inv(T11)
+    b.a = X; b.a_rs = 1; b.a_ks = ldx;
+    b.b = A; b.b_rs = cs; b.b_ks = rs; b.tri_b = TRI_UPPER; b.unit_b = unit;   // B(j, k) = inv(T11)(k, j)
+    b.c = A + s * rs; b.c_rs = rs; b.c_cs = cs;
+    b.alpha = from_real<T>(RealOf<T>(-1));
+    b.m = m; b.n = s; b.k = s;
+    nl.a_rows = ldx; nl.a_ks = s;
+    nl.nd.k_last = s;
+    nl.nd.a_row = nl.nd.a_k = nl.nd.b_k = 0;
+    nl.nd.a_node_row = s; nl.nd.a_node_k = 0;
+    nl.nd.c_node = 2LL * s * (rs + cs);
+    CUCHOL_CHECK_CU(gemm_nodes<T>(h, b, nl, sp));
+  }
+  return CUDA_SUCCESS;
+}
+
 template <typename T>
 CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long long lda, long* info) {
   const int nb = Tune<T>::nb;
@@ -955,6 +1050,27 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
 
+  if constexpr (is_fp64<T>()) {
+    if (!h->force_simt && n > nb) {
+      // X of the largest level, and an aligned copy of the triangle when A itself is not
+      size_t x = 0;
+      for (int s = nb; s < n; s *= 2) x = std::max(x, (size_t)((n - s + 2 * s - 1) / (2 * s)) * s * s);
+      const bool direct = fp64_aligned(A, lda);
+      const long long ldc = (long long)round_up((size_t)n, 2);
+      const size_t need = sizeof(T) * (x + (direct ? 0 : (size_t)ldc * n));
+      if (try_workspace(h, need)) {
+        T* X = static_cast<T*>(h->ws);
+        T* W = direct ? A : X + x;
+        if (!direct) CUCHOL_CHECK_CU(copy_view<T>(h, A, rs, cs, W, upper ? ldc : 1, upper ? 1 : ldc, n, n, true, sp, nullptr));
+        CUCHOL_CHECK_CU(trtri_levels_fp64<T>(h, unit, n, W, direct ? lda : ldc, upper, X, sp));
+        if (!direct)
+          CUCHOL_CHECK_CU(copy_view<T>(h, W, upper ? ldc : 1, upper ? 1 : ldc, A, rs, cs, n, n, true, sp, nullptr));
+        CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
+        CUCHOL_CHECK(cudaStreamSynchronize(sp));
+        return check_engine(h);
+      }
+    }
+  }
   if constexpr (is_fp32<T>()) {
     bool done = false;
     if (tensor) CUCHOL_CHECK_CU(trtri_levels_tcg<T>(h, unit, n, A, rs, cs, &done));
@@ -1063,6 +1179,43 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
   }
   const int w = lauum_width<T>(h, n);
   const long long ldw = (long long)round_up((size_t)n, 2);
+  if constexpr (is_fp64<T>()) {
+    // Orders whose product fits the workspace: the k range in slabs, one node of one
+    // launch each, summed in order on the way back into A.  The tiles' k ranges run from
+    // n down to one tile, and without slabs the launch takes as long as an SM's share
+    // of the longest ones (n = 2048: 285 us for 82 us of FP64 work).
+    const long long tiles = (long long)((n + 63) / 64) * ((n + 63) / 64 + 1) / 2;
+    const int want = (int)std::min<long long>((24LL * h->num_sms + tiles - 1) / tiles, std::max(1, n / 512));
+    const int slab = (int)round_up((size_t)(n + want - 1) / want, 128), slabs = (n + slab - 1) / slab;
+    const bool direct = fp64_aligned(A, lda);
+    const size_t need = sizeof(T) * (size_t)ldw * n * (slabs + (direct ? 0 : 1));
+    if (!h->force_simt && h->lauum_cols == 0 && (slabs > 1 || !direct) && need <= kLauumWorkspace && try_workspace(h, need)) {
+      T* W = static_cast<T*>(h->ws);
+      T* S = W + (size_t)ldw * n * slabs;
+      if (!direct) CUCHOL_CHECK_CU(copy_view<T>(h, A, rs, cs, S, upper ? ldw : 1, upper ? 1 : ldw, n, n, true, sp, nullptr));
+      GemmProblem<T> p = problem<T>();
+      p.a = p.b = direct ? A : S;
+      p.a_rs = p.b_rs = direct ? cs : (upper ? 1 : ldw);
+      p.a_ks = p.b_ks = direct ? rs : (upper ? ldw : 1);
+      p.conj_a = 1; p.tri_a = p.tri_b = TRI_UPPER;
+      p.c = W; p.c_rs = 1; p.c_cs = ldw;
+      p.m = p.n = p.k = n;
+      p.lower_only = 1; p.real_diag = 1;
+      NodeLaunch nl{};
+      nl.nd.count = slabs;
+      nl.nd.slab = slab;
+      nl.nd.c_node = (long long)ldw * n;
+      nl.a_rows = nl.a_ks = nl.b_rows = nl.b_ks = n;
+      CUCHOL_CHECK_CU(gemm_nodes<T>(h, p, nl, sp));
+      const int nt = (n + 31) / 32;
+      sum_slabs_kernel<T><<<dim3(nt, nt), 256, 0, sp>>>(W, ldw, nl.nd.c_node, slabs, slab, A, rs, cs, n);
+      ++h->launches;
+      CUCHOL_CHECK(cudaGetLastError());
+      CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
+      CUCHOL_CHECK(cudaStreamSynchronize(sp));
+      return check_engine(h);
+    }
+  }
   CUCHOL_CHECK_CU(ensure_workspace(h, sizeof(T) * (size_t)ldw * w));
   T* W = static_cast<T*>(h->ws);
   for (int j0 = 0; j0 < n; j0 += w) {

@@ -70,6 +70,7 @@ struct Params {
   int preload;      // alpha = +-1: accumulators start at beta * Cin
   int neg;          // alpha = -1 (with preload): the B fragments are negated
   int* err;         // set when a bounded wait gave up
+  dmma::Nodes nd;   // TRI kernels only
 };
 
 // x with its sign bit XORed by `m` (0 or 0x80000000), on the integer pipe
@@ -119,19 +120,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   constexpr int BM = Shape<MB>::BM, STAGES = Shape<MB>::STAGES;
   constexpr int A_STAGE = Shape<MB>::A_STAGE, STAGE_BYTES = Shape<MB>::STAGE_BYTES;
   if (cta_aborted(abort_flag)) return;
-  const int ntiles = P.tiles_m * P.tiles_n;
-  auto tile_range = [&](int tile, int& i0, int& j0, int& kbase, int& KT) -> bool {
+  const int per = P.tiles_m * P.tiles_n;
+  const int ntiles = TRI ? per * P.nd.count : per;
+  auto tile_range = [&](int tile, int& node, int& i0, int& j0, int& kbase, int& KT) -> bool {
+    node = TRI ? tile / per : 0;
+    if (TRI) tile -= node * per;
     i0 = (tile / P.tiles_n) * BM;
     j0 = (tile % P.tiles_n) * BN;
     if (P.lower_only && j0 > i0 + BM - 1) return false;
     int kb = 0, ke = P.k;
+    if (TRI) {
+      if (P.nd.slab > 0) {
+        kb = node * P.nd.slab;
+        ke = min(ke, kb + P.nd.slab);
+      } else if (node == P.nd.count - 1 && P.nd.count > 1) {
+        ke = P.nd.k_last;
+        if (i0 >= P.nd.m_last) return false;
+      }
+    }
     if (P.tri_a == TRI_LOWER) ke = min(ke, i0 + BM);
     if (P.tri_a == TRI_UPPER) kb = max(kb, i0);
     if (P.tri_b == TRI_LOWER) ke = min(ke, j0 + BN);
     if (P.tri_b == TRI_UPPER) kb = max(kb, j0);
     kbase = (kb / BK) * BK;
     KT = (ke > kbase) ? (ke - kbase + BK - 1) / BK : 0;
-    return true;
+    return !(TRI && P.nd.slab > 0 && KT == 0);
   };
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -151,20 +164,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   }
   __syncthreads();
   // thread 0 fills the ring in consumption order: item q -> stage q % STAGES
-  int p_tile = (int)blockIdx.x - (int)gridDim.x, p_kt = 0, p_KT = 0, p_i0 = 0, p_j0 = 0, p_kbase = 0;
+  int p_tile = (int)blockIdx.x - (int)gridDim.x, p_kt = 0, p_KT = 0, p_i0 = 0, p_j0 = 0, p_kbase = 0, p_node = 0;
   long long issued = 0, consumed = 0;
   auto produce = [&]() -> bool {
     while (p_kt >= p_KT) {
       p_tile += gridDim.x;
       if (p_tile >= ntiles) return false;
       p_kt = 0;
-      if (!tile_range(p_tile, p_i0, p_j0, p_kbase, p_KT)) p_KT = 0;
+      if (!tile_range(p_tile, p_node, p_i0, p_j0, p_kbase, p_KT)) p_KT = 0;
     }
     const int s = (int)(issued % STAGES);
     unsigned char* st = smem + s * STAGE_BYTES;
     dmma::mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-    load_operand<LA, BM>(&mapA, &full_bar[s], st, p_i0, p_kbase + p_kt * BK);
-    load_operand<LB, BN>(&mapB, &full_bar[s], st + A_STAGE, p_j0, p_kbase + p_kt * BK);
+    int ar = p_i0, ak = p_kbase + p_kt * BK, br = p_j0, bk = ak;
+    if (TRI && P.nd.slab == 0) {
+      ar += P.nd.a_row + p_node * P.nd.a_node_row;
+      ak += P.nd.a_k + p_node * P.nd.a_node_k;
+      br += P.nd.b_row + p_node * P.nd.b_node_row;
+      bk += P.nd.b_k + p_node * P.nd.b_node_k;
+    }
+    load_operand<LA, BM>(&mapA, &full_bar[s], st, ar, ak);
+    load_operand<LB, BN>(&mapB, &full_bar[s], st + A_STAGE, br, bk);
     ++p_kt;
     ++issued;
     return true;
@@ -193,8 +213,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
   const uint32_t m_bi = ((P.conj_b != 0) != (P.neg != 0)) ? SIGN : 0u;
   bool ok = true;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    int i0, j0, kbase, KT;
-    if (!tile_range(tile, i0, j0, kbase, KT)) continue;
+    int node, i0, j0, kbase, KT;
+    if (!tile_range(tile, node, i0, j0, kbase, KT)) continue;
+  const int pm = (TRI && P.nd.count > 1 && P.nd.slab == 0 && node == P.nd.count - 1) ? P.nd.m_last : P.m;
+  const long long cshift = TRI ? node * P.nd.c_node : 0;
     // acc[mb][nb8][e]: Re (accr) and Im (acci) of row wrow + mb*16 + g (+8 for e >= 2),
     // column wcol + nb8*8 + 2t + (e & 1)
     double accr[MB][4][4], acci[MB][4][4];
@@ -214,7 +236,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
           for (int e = 0; e < 4; ++e) {
             const int row = wrow + mb * 16 + g + (e >> 1) * 8;
             const int col = wcol + nb8 * 8 + 2 * t + (e & 1);
-            if (row < P.m && col < P.n && (!P.lower_only || row >= col)) {
+            if (row < pm && col < P.n && (!P.lower_only || row >= col)) {
               const cuDoubleComplex v = cmul(P.beta, P.cin[row * P.cin_rs + (long long)col * P.cin_cs]);
               accr[mb][nb8][e] = v.x;
               acci[mb][nb8][e] = v.y;
@@ -315,7 +337,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
         for (int e = 0; e < 4; ++e) {
           const int row = wrow + mb * 16 + g + (e >> 1) * 8;
           const int col = wcol + nb8 * 8 + 2 * t + (e & 1);
-          if (row < P.m && col < P.n && (!P.lower_only || row >= col)) {
+          if (row < pm && col < P.n && (!P.lower_only || row >= col)) {
             cuDoubleComplex v = make_cuDoubleComplex(accr[mb][nb8][e], acci[mb][nb8][e]);
             if (!P.preload) v = cmul(P.alpha, v);
             if (has_cin) {
@@ -324,7 +346,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
               v.y += o.y;
             }
             if (P.real_diag && row == col) v.y = 0.0;
-            P.c[row * P.c_rs + (long long)col * P.c_cs] = v;
+            P.c[cshift + row * P.c_rs + (long long)col * P.c_cs] = v;
           }
         }
   }
