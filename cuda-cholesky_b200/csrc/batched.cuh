@@ -30,9 +30,9 @@ struct __cucholbatched_st {
   void* d_w;                 // inverses of the current step's diagonal blocks
   void* d_work;              // TRTRI X blocks, then L^H L (sum of n_b^2 elements)
   std::vector<void*> d_lists;
-  int persistent;            // FP64: the whole sequence is one persistent kernel (bpersist.cuh)
+  int persistent;            // the whole sequence is one persistent kernel (bpersist.cuh)
   int* d_next;               // its work-queue head
-  double* d_wp;              // its per-CTA inverses of the diagonal blocks (wp_tiles per CTA)
+  void* d_wp;                // its per-CTA inverses of the diagonal blocks (wp_tiles per CTA)
   int wp_tiles;
   bool dry;                  // recording pass 1: build and upload lists, launch nothing
   bool reuse;                // recording pass 2 (under capture): reuse the uploaded lists
@@ -102,11 +102,9 @@ CUresult record_persistent(CUcholBatched p, const BatchedShape<T>& sh, cudaStrea
 // Enqueue the whole batched sequence on stream s (used under stream capture).
 template <typename T>
 CUresult record_batched(CUcholBatched p, const BatchedShape<T>& sh, int nb, cudaStream_t s) {
-  if constexpr (std::is_same<T, double>::value) {
-    if (p->persistent) return record_persistent<T>(p, sh, s);
-  }
+  if (p->persistent) return record_persistent<T>(p, sh, s);
   CULAPACKhandle h = p->h;
-  using Smem = DiagSmem<T, kBatchedMaxNb>;
+  using Smem = BlockSmem<T, kBatchedMaxNb>;
   const int B = sh.batch;
   T* W = static_cast<T*>(p->d_w);
   T* work = static_cast<T*>(p->d_work);
@@ -300,10 +298,9 @@ __global__ void set_identity_kernel(T* a, const long long* __restrict__ off, con
 // (the kernels do the same work for any SPD input) and keep the fastest.
 template <typename T>
 CUresult tune_nb(CUcholBatched p, const BatchedShape<T>& sh, int* best_nb) {
-  // candidates: the grouped graphs with nb = 32 and 64, and (FP64) the persistent
-  // kernel, written nb = -1 here
-  std::vector<int> candidates = {32, 64};
-  if (std::is_same<T, double>::value) candidates.push_back(-1);
+  // candidates: the grouped graphs with nb = 32 and 64, and the persistent kernel,
+  // written nb = -1 here
+  const std::vector<int> candidates = {32, 64, -1};
   std::vector<long long> off(sh.batch);
   long long total = 0;
   for (int b = 0; b < sh.batch; ++b) { off[b] = total; total += (long long)sh.n[b] * sh.n[b]; }
@@ -417,7 +414,7 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
     delete p;
     return r;
   };
-  using Smem = DiagSmem<T, kBatchedMaxNb>;
+  using Smem = BlockSmem<T, kBatchedMaxNb>;
   if (cudaFuncSetAttribute(diag_factor_batched_kernel<T, kBatchedMaxNb, kDiagThreads2>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem::bytes) != cudaSuccess ||
       cudaFuncSetAttribute(diag_invert_batched_kernel<T, kBatchedMaxNb, kDiagThreads2>,
@@ -430,10 +427,9 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
   int nmax = 1;
   for (int b = 0; b < batch; ++b) nmax = std::max(nmax, n[b]);
   p->wp_tiles = (nmax + kBatchedMaxNb - 1) / kBatchedMaxNb;
-  if (std::is_same<T, double>::value &&
-      (dev_malloc(&p->d_next, sizeof(int)) != cudaSuccess ||
-       dev_malloc(&p->d_wp, sizeof(double) * (size_t)h->num_sms * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb) !=
-           cudaSuccess))
+  if (dev_malloc(&p->d_next, sizeof(int)) != cudaSuccess ||
+      dev_malloc(&p->d_wp, sizeof(T) * 2 * (size_t)h->num_sms * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb) !=
+          cudaSuccess)
     return fail(report(cudaGetLastError(), "cudaMalloc", __func__, __FILE__, __LINE__));
   if (nb == 0) {
     rc = tune_nb<T>(p, sh, &nb);
@@ -481,7 +477,7 @@ extern "C" CUCHOL_EXPORT CUresult cuCholBatchedResults(CUcholBatched p, long* in
 
 extern "C" CUCHOL_EXPORT CUresult cuCholBatchedGetBlockSize(CUcholBatched p, int* nb) {
   if (p == nullptr || nb == nullptr) return CUDA_ERROR_INVALID_VALUE;
-  *nb = p->persistent ? -1 : p->nb;
+  *nb = (p->persistent && p->type == 'D') ? -1 : p->nb;   // FP32: the persistent kernel's tile order
   return CUDA_SUCCESS;
 }
 

@@ -51,7 +51,7 @@ template <typename T>
 CUresult trsm_left(CULAPACKhandle h, const TriView<T>& v, int m, int n, T* B, long long brs, long long bcs,
                    cudaStream_t s) {
   constexpr int nb = Tune<T>::nb;
-  using Smem = DiagSmem<T, nb>;
+  using Smem = BlockSmem<T, nb>;
   const int nblk = (m + nb - 1) / nb;
   const long long ldw = (long long)round_up((size_t)nb, 2);
   // workspace: the inverted diagonal blocks (nb x nb each, column-major, in the

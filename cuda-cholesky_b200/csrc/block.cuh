@@ -345,4 +345,114 @@ __device__ __forceinline__ void factor_block(T* S, T* Lsh, RealOf<T>* rd, int n1
   __syncthreads();
 }
 
+// Shared memory of a block that is also inverted.
+template <typename T, int NB>
+struct BlockSmem {
+  static constexpr size_t F = (FactorSmem<T, NB>::bytes + 15) / 16 * 16;
+  static constexpr size_t RD = sizeof(T) * NB;
+  static constexpr size_t TMP = sizeof(T) * (NB / 2) * (NB / 2 + 1);
+  static constexpr size_t bytes = F + RD + TMP;
+};
+
+// In-place inverse of the lower triangular block in S (order n16, a multiple of 16 up to
+// NB, rd[i] = 1 / L(i, i)), by the whole CTA; TMP: (NB/2) x (NB/2 + 1) elements.  The
+// part above the diagonal is neither read nor written.  Starts and ends with a barrier.
+//
+// The 16 x 16 diagonal blocks first, a warp each (lane c: column c by substitution, in
+// registers), then pairs of inverted blocks of order b = 16, 32, ..:
+//   [L11 0; L21 L22]^-1 = [W11 0; -W22 L21 W11, W22],
+// all pairs of a level together, 4 x 4 outputs per thread.
+template <typename T, int NB, int NT>
+__device__ __forceinline__ void invert_block(T* S, int n16, const T* rd, T* TMP) {
+  constexpr int LD = FactorSmem<T, NB>::LD;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  __syncthreads();
+  for (int c0 = kSub * warp; c0 < n16; c0 += kSub * (NT / 32)) {
+    T* B = S + c0 * LD + c0;
+    const int c = lane & (kSub - 1);
+    T x[kSub];
+#pragma unroll
+    for (int i = 0; i < kSub; ++i) {
+      T a0 = zero<T>(), a1 = zero<T>();
+#pragma unroll
+      for (int k = 0; k < i; ++k) {
+        const T l = B[k * LD + i];
+        if (k >= c) { if (k & 1) fms(a1, l, x[k]); else fms(a0, l, x[k]); }
+      }
+      x[i] = (i < c) ? zero<T>() : (i == c) ? rd[c0 + i] : mul(add(a0, a1), rd[c0 + i]);
+    }
+    __syncwarp();
+    if (lane < kSub) {
+#pragma unroll
+      for (int i = 0; i < kSub; ++i)
+        if (i >= c) B[c * LD + i] = x[i];
+    }
+  }
+  __syncthreads();
+  for (int b = kSub; b < n16; b *= 2) {
+    const int q4 = b / 4, per = q4 * q4, pairs = (n16 - b + 2 * b - 1) / (2 * b), ldt = b + 1;
+    // T(r, c) = sum_{k >= c} L21(r, k) W11(k, c)
+    for (int e = t; e < pairs * per; e += NT) {
+      const int pr = e / per, f = e - pr * per, r = f % q4, cq = 4 * (f / q4);
+      const int c0 = 2 * b * pr, r0 = c0 + b;
+      const T* L = S + c0 * LD + r0;
+      const T* W = S + c0 * LD + c0;
+      T acc[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] = zero<T>();
+#pragma unroll 4
+      for (int k = cq; k < b; ++k) {
+        T x[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = (r0 + r + q4 * u < n16) ? L[k * LD + r + q4 * u] : zero<T>();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) y[v] = (k >= cq + v) ? W[(cq + v) * LD + k] : zero<T>();
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) mac(acc[u][v], x[u], y[v]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) TMP[pr * b * ldt + (cq + v) * ldt + r + q4 * u] = acc[u][v];
+    }
+    __syncthreads();
+    // W21(r, c) = -sum_{k <= r} W22(r, k) T(k, c)
+    for (int e = t; e < pairs * per; e += NT) {
+      const int pr = e / per, f = e - pr * per, r = f % q4, cq = 4 * (f / q4);
+      const int c0 = 2 * b * pr, r0 = c0 + b, nr = min(b, n16 - r0);
+      const T* W = S + r0 * LD + r0;
+      const T* X = TMP + pr * b * ldt;
+      T acc[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] = zero<T>();
+      const int ke = min(nr, r + 3 * q4 + 1);
+#pragma unroll 4
+      for (int k = 0; k < ke; ++k) {
+        T x[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = (k <= r + q4 * u && r + q4 * u < nr) ? W[k * LD + r + q4 * u] : zero<T>();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) y[v] = X[(cq + v) * ldt + k];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) fms(acc[u][v], x[u], y[v]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r + q4 * u < nr) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) S[(c0 + cq + v) * LD + r0 + r + q4 * u] = acc[u][v];
+        }
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace cuchol

@@ -1044,8 +1044,8 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
     }
   }
   constexpr int NB = Tune<T>::nb;
-  CUCHOL_CHECK_CU(set_smem<T>((const void*)diag_invert_kernel<T, NB, kDiagThreads2>, DiagSmem<T, NB>::bytes));
-  diag_invert_kernel<T, NB, kDiagThreads2><<<(n + nb - 1) / nb, kDiagThreads2, DiagSmem<T, NB>::bytes, sp>>>(
+  CUCHOL_CHECK_CU(set_smem<T>((const void*)diag_invert_kernel<T, NB, kDiagThreads2>, BlockSmem<T, NB>::bytes));
+  diag_invert_kernel<T, NB, kDiagThreads2><<<(n + nb - 1) / nb, kDiagThreads2, BlockSmem<T, NB>::bytes, sp>>>(
       A, rs, cs, n, nb, unit ? 1 : 0);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
@@ -1258,8 +1258,8 @@ CUresult trti22_run(CULAPACKhandle h, bool upper, bool unit, int n, const T* A, 
   if (inf != 0) return CUDA_SUCCESS;
   if (A != B) CUCHOL_CHECK_CU(copy_view<T>(h, A, ars, acs, B, brs, bcs, n, n, true, stream, nullptr));
   constexpr int NB = Tune<T>::nb;
-  CUCHOL_CHECK_CU(set_smem<T>((const void*)diag_invert_kernel<T, NB, kDiagThreads2>, DiagSmem<T, NB>::bytes));
-  diag_invert_kernel<T, NB, kDiagThreads2><<<1, kDiagThreads2, DiagSmem<T, NB>::bytes, stream>>>(
+  CUCHOL_CHECK_CU(set_smem<T>((const void*)diag_invert_kernel<T, NB, kDiagThreads2>, BlockSmem<T, NB>::bytes));
+  diag_invert_kernel<T, NB, kDiagThreads2><<<1, kDiagThreads2, BlockSmem<T, NB>::bytes, stream>>>(
       B, brs, bcs, n, n, unit ? 1 : 0);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());

@@ -1289,13 +1289,13 @@ CUresult mixed_refactor(CUcholMixed p, long* info) {
   // with one grouped launch per level and product, all NBT-blocks together (FP32).
   CUCHOL_CHECK(cudaMemsetAsync(p->Dinv, 0, sizeof(float) * (size_t)nT * NBT * NBT, sp));
   CUCHOL_CHECK_CU(set_smem<float>((const void*)diag_invert_kernel<float, SB, kDiagThreads2>,
-                                  DiagSmem<float, SB>::bytes));
+                                  BlockSmem<float, SB>::bytes));
   for (int I = 0; I < nT; ++I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0);
     float* Dn = p->Dinv + (size_t)I * NBT * NBT;
     CUCHOL_CHECK_CU(copy_view<float>(h, p->W + b0 + (long long)b0 * p->ldw, 1, p->ldw, Dn, 1, NBT, bI, bI, true, sp,
                                      nullptr));
-    diag_invert_kernel<float, SB, kDiagThreads2><<<(bI + SB - 1) / SB, kDiagThreads2, DiagSmem<float, SB>::bytes,
+    diag_invert_kernel<float, SB, kDiagThreads2><<<(bI + SB - 1) / SB, kDiagThreads2, BlockSmem<float, SB>::bytes,
                                                    sp>>>(Dn, 1, NBT, bI, SB, 0);
     ++h->launches;
     CUCHOL_CHECK(cudaGetLastError());
