@@ -9,15 +9,14 @@
 //     Per pivot the chain is one warp shuffle (the pivot), the reciprocal square root,
 //     one multiplication and one fused multiply-add: the next pivot d' = a' - |l|^2 needs
 //     only values of its own lane.  The column itself goes through shared memory to the
-//     other lanes in the shadow of the next pivot's square root.  The loop is rolled:
-//     every step shifts the register columns down by one (x[q] := x[q+1] - l v[q]), so
-//     one body of about 60 instructions serves all 16 steps and is fetched once.  (The
-//     kernels run once per block column from a cold instruction cache, where unrolled
-//     code costs more than the FMAs it saves.)
-//   * solve16 (one thread per row): the same shifted loop, right-looking.
+//     other lanes in the shadow of the next pivot's square root.  A warp issues in order,
+//     so this overlap exists only if the whole body is one basic block: no early exit on
+//     a bad pivot (its column is noted, the rest computes on rubbish that is not stored)
+//     and no slow path inside.
+//   * solve16 (one thread per row): right-looking substitution through 16 columns.
 //   * tile_update (one warp): C(32 x 16) -= P Q^H over 16 columns; FP64 on DMMA.
-// A column of L is kept twice: in place, and "shifted" in Lsh[j][q] = L(j+1+q, j), zero
-// past the block, so that the loops read it with aligned 16-byte loads.
+// The diagonal 16 x 16 block of L is kept a second time in Ld, column j at Ld[16 j], so
+// that the loops read it with aligned 16-byte loads.
 #pragma once
 #include <stdint.h>
 #include <type_traits>
@@ -49,28 +48,29 @@ constexpr int kSubRows = 32;         // rows factor16 covers: the 16 x 16 block 
 // touches 16 distinct 8-byte banks per half warp.
 constexpr int kLdPad = 4;
 
-// 1 / sqrt(d) for the pivot chain.  FP64: the hardware estimate y (relative error below
-// 2^-20) refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, to second order
-// (the dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations after the
-// estimate.  Outside a safe exponent range (where d y^2 could leave it) rsqrt().
+// 1 / sqrt(d) for the pivot chain, without branches.  FP64: the hardware estimate y
+// (relative error below 2^-20) refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2,
+// to second order (the dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations
+// after the estimate.  Right for every normal d and 0 for infinity, like rsqrt();
+// subnormal pivots (for which the estimate is infinite) are left to factor16_slow.
 __device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrtf(d); }
 __device__ __forceinline__ double pivot_rsqrt(double d) {
-  if (d >= 0x1p-900 && d <= 0x1p900) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-  }
-  return rsqrt(d);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d * y, y, 1.0);
+  const double r = fma(y * e, fma(0.375, e, 0.5), y);
+  return (__double2hiint(d) == 0x7ff00000) ? 0.0 : r;
 }
+__device__ __forceinline__ bool subnormal_pivot(float) { return false; }   // rsqrtf takes them
+__device__ __forceinline__ bool subnormal_pivot(double d) { return __double2hiint(d) < 0x00100000; }
 
-// 16 elements at a 16-byte aligned shared address.
-template <typename T>
+// Elements FROM .. 15 of 16 at a 16-byte aligned shared address, in 16-byte loads.
+template <int FROM, typename T>
 __device__ __forceinline__ void load_row16(const T* p, T (&v)[kSub]) {
   constexpr int per = 16 / sizeof(T);
   const int4* q = reinterpret_cast<const int4*>(p);
 #pragma unroll
-  for (int u = 0; u < kSub / per; ++u) {
+  for (int u = FROM / per; u < kSub / per; ++u) {
     const int4 w = q[u];
     memcpy(&v[u * per], &w, 16);
   }
@@ -92,63 +92,121 @@ __device__ __forceinline__ float minus_abs2(cuFloatComplex a, cuFloatComplex l) 
 __device__ __forceinline__ double minus_abs2(cuDoubleComplex a, cuDoubleComplex l) { return fma(-l.y, l.y, fma(-l.x, l.x, a.x)); }
 
 // One warp.  S: the sub-panel's top-left element (column-major, ld), rows 0 .. 31 of it,
-// of which those below nrows exist; factors the 16 columns in place, writes Lsh and the
+// of which those below nrows exist; factors the 16 columns in place, writes Ld and the
 // reciprocal pivots rd[0..15].  Returns the first failing column (pivot <= 0 or NaN) or
-// -1, the same in every lane; the columns before it are then done.
+// -1, the same in every lane; the columns before it are then done and the others as
+// they were.
+//
+// factor16_slow: the plain loop, for sub-panels with a subnormal pivot.
 template <typename T>
-__device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Lsh, RealOf<T>* rd) {
+__device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf<T>* rd) {
+  using R = RealOf<T>;
+  const int i = threadIdx.x & 31;
+  for (int j = 0; j < kSub; ++j) {
+    __syncwarp();
+    R d = re(S[j * ld + j]);
+    T a = (i < nrows) ? S[j * ld + i] : zero<T>();
+    for (int k = 0; k < j; ++k) {
+      const T ljk = S[k * ld + j];
+      d = minus_abs2(from_real<T>(d), ljk);
+      if (i < nrows) fms(a, S[k * ld + i], cj(ljk));
+    }
+    if (!(d > R(0))) return j;
+    const R r = R(1) / sqrt(d);
+    const T l = (i == j) ? from_real<T>(sqrt(d)) : scale(a, r);
+    __syncwarp();
+    if (i < nrows && i >= j) S[j * ld + i] = l;
+    if (i < kSub) Ld[j * kSub + i] = l;
+    if (i == 0) rd[j] = r;
+  }
+  __syncwarp();
+  return -1;
+}
+
+// Step J of factor16 and the ones after it: x the row, d the pivot of column J.
+template <int J, typename T>
+__device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> d, RealOf<T> r, int i, T* Ld, RealOf<T>* rd,
+                                               int& fail, bool& sub) {
+  using R = RealOf<T>;
+  if constexpr (J < kSub) {
+    fail = (fail < 0 && !(d > R(0))) ? J : fail;
+    sub = sub || subnormal_pivot(d);
+    x[J] = (i == J) ? from_real<T>(d * r) : scale(x[J], r);
+    R dn = R(1), rn = R(1);
+    if constexpr (J + 1 < kSub) {
+      dn = __shfl_sync(0xffffffffu, minus_abs2(x[J + 1], x[J]), J + 1);
+      rn = pivot_rsqrt(dn);
+    }
+    if (i < kSub) Ld[J * kSub + i] = x[J];
+    if (i == 0) rd[J] = r;
+    if constexpr (J + 1 < kSub) {
+      __syncwarp();
+      T v[kSub];
+      load_row16<J + 1>(Ld + J * kSub, v);
+#pragma unroll
+      for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
+      factor16_steps<J + 1>(x, dn, rn, i, Ld, rd, fail, sub);
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Ld, RealOf<T>* rd) {
   using R = RealOf<T>;
   const int i = threadIdx.x & 31;
   const bool mine = i < nrows;
   T x[kSub];
 #pragma unroll
   for (int q = 0; q < kSub; ++q) x[q] = mine ? S[q * ld + i] : zero<T>();
-  R dn = re(x[0]);
-#pragma unroll 1
-  for (int j = 0; j < kSub; ++j) {
-    const R d = __shfl_sync(0xffffffffu, dn, j);
-    if (!(d > R(0))) return j;
-    const R r = pivot_rsqrt(d);
-    const T l = (i == j) ? from_real<T>(d * r) : scale(x[0], r);
-    dn = minus_abs2(x[1], l);                  // the next pivot, on lane j + 1
-    if (mine && i >= j) S[j * ld + i] = l;
-    if (i < kSub) Lsh[j * kSub + ((i - j - 1) & (kSub - 1))] = (i > j) ? l : zero<T>();
-    if (i == 0) rd[j] = r;
-    __syncwarp();
-    T v[kSub];
-    load_row16(Lsh + j * kSub, v);
+  const R d = __shfl_sync(0xffffffffu, re(x[0]), 0);
+  int fail = -1;
+  bool sub = false;
+  factor16_steps<0>(x, d, pivot_rsqrt(d), i, Ld, rd, fail, sub);
+  // (rubbish after a failing column may look subnormal: only a sub-panel whose first
+  // bad pivot is subnormal and positive changes its outcome in the slow loop)
+  if (sub) return factor16_slow<T>(S, ld, nrows, Ld, rd);
 #pragma unroll
-    for (int q = 0; q < kSub - 1; ++q) {
-      T t = x[q + 1];
-      fms(t, l, cj(v[q]));
-      x[q] = t;
+  for (int q = 0; q < kSub; ++q)
+    if (mine && i >= q && (fail < 0 || q < fail)) S[q * ld + i] = x[q];
+  return fail;
+}
+
+template <int J, typename T>
+__device__ __forceinline__ void solve16_steps(T (&x)[kSub], const T* __restrict__ Ld, const RealOf<T>* __restrict__ rd) {
+  if constexpr (J < kSub) {
+    x[J] = scale(x[J], rd[J]);
+    if constexpr (J + 1 < kSub) {
+      T v[kSub];
+      load_row16<J + 1>(Ld + J * kSub, v);
+#pragma unroll
+      for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
+      solve16_steps<J + 1>(x, Ld, rd);
     }
   }
-  return -1;
 }
 
 // One thread: the row x of 16 columns (elements ld apart from S) solved against the
-// factored block: x := x L^-H, the first ncols columns of it.  Unrolled: 120 FMAs whose
-// chain is one multiplication and one FMA per column; the same loop rolled like
-// factor16's would issue twice as many.
+// factored block: x := x L^-H.  120 FMAs, whose chain is one multiplication and one FMA
+// per column.
 template <typename T>
-__device__ __forceinline__ void solve16(T* S, int ld, const T* __restrict__ Lsh, const RealOf<T>* __restrict__ rd,
-                                        int ncols = kSub) {
+__device__ __forceinline__ void solve16(T* S, int ld, const T* __restrict__ Ld, const RealOf<T>* __restrict__ rd) {
   T x[kSub];
 #pragma unroll
   for (int q = 0; q < kSub; ++q) x[q] = S[q * ld];
-#pragma unroll
-  for (int j = 0; j < kSub; ++j) {
-    if (j >= ncols) break;
-    T v[kSub];
-    load_row16(Lsh + j * kSub, v);             // only v[0 .. 14 - j] is used
-    x[j] = scale(x[j], rd[j]);
-#pragma unroll
-    for (int q = j + 1; q < kSub; ++q) fms(x[q], x[j], cj(v[q - j - 1]));
-  }
-  // stored at the end: a store between them would hold back the loads of Lsh
+  solve16_steps<0>(x, Ld, rd);
+  // stored at the end: a store between them would hold back the loads of Ld
 #pragma unroll
   for (int q = 0; q < kSub; ++q) S[q * ld] = x[q];
+}
+
+// The first ncols columns only (a block that failed there).
+template <typename T>
+__device__ __noinline__ void solve16_part(T* S, int ld, const T* Ld, const RealOf<T>* rd, int ncols) {
+  for (int j = 0; j < ncols; ++j) {
+    T x = S[j * ld];
+    for (int k = 0; k < j; ++k) fms(x, S[k * ld], cj(Ld[k * kSub + j]));
+    S[j * ld] = scale(x, rd[j]);
+  }
 }
 
 __device__ __forceinline__ void dmma16n8k4(double (&d)[4], double a0, double a1, double b) {
@@ -291,9 +349,9 @@ template <typename T, int NB>
 struct FactorSmem {
   static constexpr int LD = NB + kLdPad;
   static constexpr size_t S = sizeof(T) * NB * LD;
-  static constexpr size_t LSH = sizeof(T) * kSub * kSub;
+  static constexpr size_t LDS = sizeof(T) * kSub * kSub;
   static constexpr size_t RD = sizeof(RealOf<T>) * NB;
-  static constexpr size_t bytes = S + LSH + RD;
+  static constexpr size_t bytes = S + LDS + RD;
 };
 
 // Cholesky factor of the block in S (order n16, a multiple of 16 up to NB; lower part),
@@ -307,14 +365,14 @@ struct FactorSmem {
 // remaining row solves; the 32 x 16 elements warp 0 needs next are updated by all
 // threads; then warp 0 goes on while the other warps update the rest of the block.
 template <typename T, int NB, int NT, typename Done>
-__device__ __forceinline__ void factor_block(T* S, T* Lsh, RealOf<T>* rd, int n16, int* s_fail, Done done) {
+__device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16, int* s_fail, Done done) {
   constexpr int LD = FactorSmem<T, NB>::LD;
   const int t = threadIdx.x, warp = t >> 5;
   __syncthreads();
   for (int c0 = 0; c0 < n16; c0 += kSub) {
     const int c1 = c0 + kSub;
     if (warp == 0) {
-      const int f = factor16<T>(S + c0 * LD + c0, LD, n16 - c0, Lsh, rd + c0);
+      const int f = factor16<T>(S + c0 * LD + c0, LD, n16 - c0, Ld, rd + c0);
       if (t == 0 && f >= 0) *s_fail = c0 + f;
     } else if (c0 > 0) {
       // the rest of the update by the previous sub-panel: 32 x 16 tiles of the columns
@@ -331,8 +389,10 @@ __device__ __forceinline__ void factor_block(T* S, T* Lsh, RealOf<T>* rd, int n1
     }
     __syncthreads();
     const int fail = *s_fail;
-    const int ncols = fail < 0 ? kSub : fail - c0;
-    for (int r = c0 + kSubRows + t; r < n16; r += NT) solve16<T>(S + c0 * LD + r, LD, Lsh, rd + c0, ncols);
+    for (int r = c0 + kSubRows + t; r < n16; r += NT) {
+      if (fail < 0) solve16<T>(S + c0 * LD + r, LD, Ld, rd + c0);
+      else solve16_part<T>(S + c0 * LD + r, LD, Ld, rd + c0, fail - c0);
+    }
     __syncthreads();
     if (fail >= 0 || c1 >= n16) {
       done(c0, t, NT);

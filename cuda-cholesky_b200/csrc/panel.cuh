@@ -54,15 +54,15 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
   using F = FactorSmem<T, NB>;
   constexpr int LD = F::LD;
   T* S = reinterpret_cast<T*>(smem);
-  T* Lsh = reinterpret_cast<T*>(smem + F::S);
-  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem + F::S + F::LSH);
+  T* Ld = reinterpret_cast<T*>(smem + F::S);
+  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem + F::S + F::LDS);
   __shared__ int s_fail;
   __shared__ double s_log[NT / 32];
   const int tid = threadIdx.x, n16 = (jb + kSub - 1) & ~(kSub - 1);
   load_lower<T, TA, LD, NT>(S, A, rs, cs, jb, n16);
   if (tid == 0) s_fail = -1;
   cp_async_wait_all();
-  factor_block<T, NB, NT>(S, Lsh, rd, n16, &s_fail, [&](int c0, int t, int nt) {
+  factor_block<T, NB, NT>(S, Ld, rd, n16, &s_fail, [&](int c0, int t, int nt) {
     // columns c0 .. c0 + 15 of the factor back to A
     const int rows = jb - c0;
     if (rs == 1) {
@@ -121,7 +121,7 @@ __device__ __forceinline__ void diag_factor_block(T* __restrict__ A, long long r
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (!factor_diag<T, T, NB, NT>(smem_raw, A, rs, cs, jb, info_base, d_info, logdet) || W == nullptr) return;
   T* S = reinterpret_cast<T*>(smem_raw);
-  const T* rd = reinterpret_cast<const T*>(smem_raw + F::S + F::LSH);
+  const T* rd = reinterpret_cast<const T*>(smem_raw + F::S + F::LDS);
   T* TMP = reinterpret_cast<T*>(smem_raw + BlockSmem<T, NB>::F + BlockSmem<T, NB>::RD);
   invert_block<T, NB, NT>(S, (jb + kSub - 1) & ~(kSub - 1), rd, TMP);
   for (int e = threadIdx.x; e < NB * NB; e += NT) {

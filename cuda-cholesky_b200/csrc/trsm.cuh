@@ -31,7 +31,7 @@ enum : int {
 
 // Shared memory of the panel solve of R rows: the row tile Xs (column-major), the parts
 // of L below its 16 x 16 diagonal blocks (one column-major strip per sub-panel, from the
-// row below the block), the shifted diagonal blocks and the reciprocal pivots.
+// row below the block), the diagonal blocks and the reciprocal pivots.
 template <typename T, int NB, int R>
 struct SolveSmem {
   static constexpr bool dmma = std::is_same<T, double>::value;
@@ -44,9 +44,9 @@ struct SolveSmem {
     return kSub * (p * (NB - kSub + kLdPad) - kSub * (p * (p - 1) / 2));
   }
   static constexpr size_t L = sizeof(T) * strip_off(NP - 1);
-  static constexpr size_t LSH = sizeof(T) * NP * kSub * kSub;
+  static constexpr size_t LDS = sizeof(T) * NP * kSub * kSub;
   static constexpr size_t RD = sizeof(RealOf<T>) * NB;
-  static constexpr size_t bytes = X + L + LSH + RD;
+  static constexpr size_t bytes = X + L + LDS + RD;
 };
 
 // Panel solve X = B L^-H in place (L^-T for real types), row-parallel: B (m x jb,
@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(256)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* Xs = reinterpret_cast<T*>(smem_raw);                       // Xs[col * LDX + row]
   T* Ls = reinterpret_cast<T*>(smem_raw + SM::X);
-  T* Lsh = reinterpret_cast<T*>(smem_raw + SM::X + SM::L);
-  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem_raw + SM::X + SM::L + SM::LSH);
+  T* Ld = reinterpret_cast<T*>(smem_raw + SM::X + SM::L);
+  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem_raw + SM::X + SM::L + SM::LDS);
   if (cta_aborted(stop)) return;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int n16 = (jb + kSub - 1) & ~(kSub - 1);
@@ -99,11 +99,11 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
-  // the diagonal 16 x 16 blocks, shifted: global column j, row j + 1 + q
+  // the diagonal 16 x 16 blocks: column j at Ld[16 j], row i of its block
   for (int e = t; e < n16 * kSub; e += NT) {
-    const int j = e / kSub, q = e & (kSub - 1), i = j + 1 + q;
-    const bool v = q < kSub - 1 - (j & (kSub - 1)) && i < jb;
-    cp_async_elem<T>(&Lsh[e], v ? L + (long long)i * lrs + (long long)j * lcs : L, v);
+    const int j = e / kSub, i = (j & ~(kSub - 1)) + (e & (kSub - 1));
+    const bool v = i > j && i < jb;
+    cp_async_elem<T>(&Ld[e], v ? L + (long long)i * lrs + (long long)j * lcs : L, v);
   }
   // the strips of L below them
   if (lrs == 1) {
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256)
   for (int c0 = 0; c0 < n16; c0 += kSub) {
     const int p = c0 / kSub, c1 = c0 + kSub;
     if (warp < SW) {
-      solve16<T>(Xs + c0 * LDX + t, LDX, Lsh + p * kSub * kSub, rd + c0);
+      solve16<T>(Xs + c0 * LDX + t, LDX, Ld + p * kSub * kSub, rd + c0);
     } else if (p > 0) {
       // columns past this sub-panel, by the previous one
       int w = warp - SW;
