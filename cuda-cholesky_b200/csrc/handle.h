@@ -15,6 +15,7 @@ struct __culapackhandle_st {
   int* d_words;            // device scratch words: [0] info, [1] scan max, [2] scan min,
                            // [3] engine error (a bounded wait gave up)
   int* h_words;            // pinned mirror of d_words
+  double* h_norms;         // pinned scratch of the mixed solve (part of h_words' block)
   double* d_logdet;        // [0] fused potrf log det, [1] ?logdet result (double)
   float* d_logdet_f;       // ?logdet result (float)
   double* h_logdet;        // pinned mirror of d_logdet[0]

@@ -892,21 +892,30 @@ CUresult tcg_in_range(CULAPACKhandle h, const T* A, long long rs, long long cs, 
 // level s joins pairs of inverted blocks of order s.  Per level one launch packs, for
 // all pairs, inv(T22), T21 and inv(T11); one forms X = inv(T22) T21 straight into pack
 // form; one writes T21 := -X inv(T11).  *done = false when the workspace is refused.
+// Levels s < order only.
+inline int level_pairs(int n, int s) { return (n - s + 2 * s - 1) / (2 * s); }
+
 template <typename T>
-CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs, long long cs, bool* done) {
+size_t trtri_levels_bytes(int n, int order) {
+  // per level: inv(T22) and X (pairs * s rows), T21^T and inv(T11)^T (cx rows per row), all
+  // of pitch s * cx, hi and lo
+  constexpr int cx = real_per<T>();
+  size_t need = 0;
+  for (int s = Tune<T>::nb; s < std::min(n, order); s *= 2)
+    need = std::max(need, (size_t)level_pairs(n, s) * s * s * cx * (2 + 2 * cx) * 2);
+  return sizeof(float) * need;
+}
+
+template <typename T>
+CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs, long long cs, int order, bool* done) {
   constexpr int cx = real_per<T>(), nb = Tune<T>::nb;
   static_assert(nb == tcg::BM, "levels are multiples of the tile");
-  auto pairs = [&](int s) { return (n - s + 2 * s - 1) / (2 * s); };
-  // buffers of a level, in floats (hi and lo alike): inv(T22) and X (pairs*s rows), T21^T
-  // and inv(T11)^T (cx rows per row), all of pitch s*cx
-  size_t need = 0;
-  for (int s = nb; s < n; s *= 2) need = std::max(need, (size_t)pairs(s) * s * s * cx * (2 + 2 * cx) * 2);
-  *done = need == 0 || try_workspace(h, sizeof(float) * need);
+  *done = try_workspace(h, trtri_levels_bytes<T>(n, order));
   if (!*done) return CUDA_SUCCESS;
   cudaStream_t sp = h->s_panel;
   float* a = reinterpret_cast<float*>(A);
-  for (int s = nb; s < n; s *= 2) {
-    const int np = pairs(s), s2_last = std::min(s, n - 2 * s * (np - 1) - s);
+  for (int s = nb; s < std::min(n, order); s *= 2) {
+    const int np = level_pairs(n, s), s2_last = std::min(s, n - 2 * s * (np - 1) - s);
     const long long ld = (long long)s * cx;
     const size_t rows = (size_t)np * s, one = rows * ld;
     float* w = static_cast<float*>(h->ws);
@@ -986,7 +995,7 @@ CUresult trtri_levels_fp64(CULAPACKhandle h, bool unit, int n, T* A, long long l
   constexpr int nb = Tune<T>::nb;
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   for (int s = nb; s < n; s *= 2) {
-    const int np = (n - s + 2 * s - 1) / (2 * s), s2 = std::min(s, n - 2 * s * (np - 1) - s);
+    const int np = level_pairs(n, s), s2 = std::min(s, n - 2 * s * (np - 1) - s);
     const int m = np > 1 ? s : s2;
     const long long ldx = (long long)np * s;
     NodeLaunch nl{};
@@ -1054,7 +1063,7 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
     if (!h->force_simt && n > nb) {
       // X of the largest level, and an aligned copy of the triangle when A itself is not
       size_t x = 0;
-      for (int s = nb; s < n; s *= 2) x = std::max(x, (size_t)((n - s + 2 * s - 1) / (2 * s)) * s * s);
+      for (int s = nb; s < n; s *= 2) x = std::max(x, (size_t)level_pairs(n, s) * s * s);
       const bool direct = fp64_aligned(A, lda);
       const long long ldc = (long long)round_up((size_t)n, 2);
       const size_t need = sizeof(T) * (x + (direct ? 0 : (size_t)ldc * n));
@@ -1073,7 +1082,7 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
   }
   if constexpr (is_fp32<T>()) {
     bool done = false;
-    if (tensor) CUCHOL_CHECK_CU(trtri_levels_tcg<T>(h, unit, n, A, rs, cs, &done));
+    if (tensor) CUCHOL_CHECK_CU(trtri_levels_tcg<T>(h, unit, n, A, rs, cs, n, &done));
     if (done) return CUDA_SUCCESS;
   }
   std::vector<Node> nodes;
@@ -1365,7 +1374,8 @@ CUresult create_handle(CULAPACKhandle h) {
   CUCHOL_CHECK(cudaEventCreateWithFlags(&h->ev_update, cudaEventDisableTiming));
   CUCHOL_CHECK(dev_malloc(&h->d_words, 16 * sizeof(int)));
   CUCHOL_CHECK(cudaMemset(h->d_words, 0, 16 * sizeof(int)));
-  CUCHOL_CHECK(cudaMallocHost(&h->h_words, 16 * sizeof(int)));
+  CUCHOL_CHECK(cudaMallocHost(&h->h_words, 16 * sizeof(int) + 64 * sizeof(double)));
+  h->h_norms = reinterpret_cast<double*>(h->h_words + 16);
   CUCHOL_CHECK(dev_malloc(&h->d_logdet, 4 * sizeof(double)));
   CUCHOL_CHECK(dev_malloc(&h->d_logdet_f, 4 * sizeof(float)));
   CUCHOL_CHECK(cudaMallocHost(&h->h_logdet, 4 * sizeof(double)));

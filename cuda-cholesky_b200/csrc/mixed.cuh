@@ -719,34 +719,25 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // Y_K = alpha * (sum_{J <= K} U(K,J) + sum_{I >= K} V(I,K)) + beta * B_K, summed in
-// a fixed order (deterministic).  One CTA per SY-row block, thread = row.
+// a fixed order (deterministic).  One CTA per 16 rows, thread = (row, rhs), so a warp reads
+// whole 128-byte rows of the partials and enough CTAs are in flight to cover their latency
+// (a thread per row on one CTA per tile: n = 8192 75 us).
 // B may alias Y; ldy/ldb columns, only the first nrhs columns are written.
 __global__ void __launch_bounds__(kThreads)
     symv_reduce_kernel(const double* __restrict__ U, const double* __restrict__ V, int n, int ntile, double alpha,
                        double beta, const double* B, long long ldb, double* Y, long long ldy, int nrhs) {
-  const int K = blockIdx.x, t = threadIdx.x, i = K * SY + t;
-  double sum[NR];
-#pragma unroll
-  for (int c = 0; c < NR; ++c) sum[c] = 0.0;
-  for (int J = 0; J <= K; ++J) {
-    const double* p = U + ((size_t)(K * (K + 1) / 2 + J) * SY + t) * NR;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) sum[c] += p[c];
-  }
-  for (int I = K; I < ntile; ++I) {
-    const double* p = V + ((size_t)(I * (I + 1) / 2 + K) * SY + t) * NR;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) sum[c] += p[c];
-  }
-  if (i >= n) return;
-#pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    if (c < nrhs) {
-      double y = alpha * sum[c];
-      if (beta != 0.0) y += beta * B[i + (long long)c * ldb];
-      Y[i + (long long)c * ldy] = y;
-    }
-  }
+  const int i = blockIdx.x * (kThreads / NR) + threadIdx.x / NR, c = threadIdx.x % NR;
+  const int K = i / SY, o = (i % SY) * NR + c;
+  double sum = 0.0;
+  const double* u = U + (size_t)(K * (K + 1) / 2) * SY * NR + o;
+#pragma unroll 8
+  for (int J = 0; J <= K; ++J) sum += u[(size_t)J * SY * NR];
+#pragma unroll 8
+  for (int I = K; I < ntile; ++I) sum += V[(size_t)(I * (I + 1) / 2 + K) * SY * NR + o];
+  if (i >= n || c >= nrhs) return;
+  double y = alpha * sum;
+  if (beta != 0.0) y += beta * B[i + (long long)c * ldb];
+  Y[i + (long long)c * ldy] = y;
 }
 
 // ---- PCG vector kernels (n x NR, column-major, leading dimension ld) ------------------
@@ -796,10 +787,24 @@ __global__ void __launch_bounds__(kThreads) dot_kernel(const double* __restrict_
   if (threadIdx.x < NR) part[blockIdx.x * NR + threadIdx.x] = sh[threadIdx.x];
 }
 
-__device__ __forceinline__ double sum_parts(const double* part, int nparts, int c) {
+// total[c] = sum of the kVecBlocks partials of right-hand side c, by the whole CTA in a
+// fixed order: thread (g, c) sums 16 consecutive partials, then thread c sums the 16
+// groups (one thread per c over all 256: a chain of 256 loads, 29 us).  Ends with a barrier.
+__device__ __forceinline__ void sum_parts(const double* part, double* grp /* [16][NR] */, double* total) {
+  static_assert(kVecBlocks == 256 && kThreads == 16 * NR, "16 groups of 16 partials");
+  const int g = threadIdx.x / NR, c = threadIdx.x % NR;
   double s = 0.0;
-  for (int b = 0; b < nparts; ++b) s += part[b * NR + c];
-  return s;
+#pragma unroll
+  for (int b = 0; b < 16; ++b) s += part[(16 * g + b) * NR + c];
+  grp[g * NR + c] = s;
+  __syncthreads();
+  if (g == 0) {
+    double t = 0.0;
+#pragma unroll
+    for (int b = 0; b < 16; ++b) t += grp[b * NR + c];
+    total[c] = t;
+  }
+  __syncthreads();
 }
 
 // alpha_c = rz_c / (p_c . q_c); x += alpha p; r -= alpha q; partial max |r|, max |x|
@@ -810,9 +815,11 @@ __global__ void __launch_bounds__(kThreads)
                      const double* __restrict__ rz, double* __restrict__ part_norm) {
   __shared__ double alpha[NR];
   __shared__ double sh[kThreads * (NR + 1)];
+  __shared__ double total[NR];
+  sum_parts(part_pq, sh, total);
   if (threadIdx.x < NR) {
     const int c = threadIdx.x;
-    const double pq = sum_parts(part_pq, kVecBlocks, c);
+    const double pq = total[c];
     alpha[c] = (pq > 0.0 && rz[c] > 0.0) ? rz[c] / pq : 0.0;
   }
   __syncthreads();
@@ -858,13 +865,14 @@ __global__ void __launch_bounds__(kThreads) norms_kernel(const double* __restric
   if (threadIdx.x < NR) part_norm[blockIdx.x * 2 * NR + NR + threadIdx.x] = sh[threadIdx.x];
 }
 
-// out[0..2NR) = max over the partials (one CTA)
-__global__ void norms_final_kernel(const double* __restrict__ part_norm, int nparts, double* __restrict__ out) {
-  const int c = threadIdx.x;
-  if (c >= 2 * NR) return;
+// out[0..2NR) = max over the partials (one CTA of 2 NR warps, a warp per value)
+__global__ void __launch_bounds__(64 * NR) norms_final_kernel(const double* __restrict__ part_norm, int nparts,
+                                                              double* __restrict__ out) {
+  const int c = threadIdx.x >> 5;
   double m = 0.0;
-  for (int b = 0; b < nparts; ++b) m = fmax(m, part_norm[b * 2 * NR + c]);
-  out[c] = m;
+  for (int b = threadIdx.x & 31; b < nparts; b += 32) m = fmax(m, part_norm[b * 2 * NR + c]);
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) out[c] = m;
 }
 
 // rz_new = sum of part_rz; beta = rz_new / rz_old (0 when restart or rz_old == 0);
@@ -873,10 +881,11 @@ __global__ void __launch_bounds__(kThreads)
     update_p_kernel(double* __restrict__ p, const double* __restrict__ z, int n, long long ld,
                     const double* __restrict__ part_rz, const double* __restrict__ rz_old,
                     double* __restrict__ rz_new, int restart) {
-  __shared__ double beta[NR];
+  __shared__ double beta[NR], total[NR], grp[kThreads];
+  sum_parts(part_rz, grp, total);
   if (threadIdx.x < NR) {
     const int c = threadIdx.x;
-    const double rn = sum_parts(part_rz, kVecBlocks, c);
+    const double rn = total[c];
     beta[c] = (!restart && rz_old[c] > 0.0) ? rn / rz_old[c] : 0.0;
     if (blockIdx.x == 0) rz_new[c] = rn;
   }
@@ -885,6 +894,11 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int c = 0; c < NR; ++c) p[i + c * ld] = fma(beta[c], p[i + c * ld], z[i + c * ld]);
   }
+}
+
+__global__ void ones_kernel(double* __restrict__ x, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) x[i] = 1.0;
 }
 
 // dst (ld) = src (lds) for columns < ncols, zero for the rest of the NR columns
@@ -919,8 +933,7 @@ struct __cucholmixed_st {
   float* W;                   // FP32 factor of S A S + shift I (lower, ldw)
   long long ldw;
   double* s;                  // the scaling S
-  float* Dinv;                // inverses of W's NBT x NBT diagonal blocks (ld NBT)
-  float* dtmp;                // doubling scratch (n * NBT / 4)
+  float* Dinv;                // inverses of W's NBT x NBT diagonal blocks (ld NBT, NBT (NBT + 1) apart)
   float* gpart;               // split-k partial sums of the preconditioner GEMVs
   double anorm;               // |A|_inf
   double shift;               // shift of the factor that succeeded
@@ -930,7 +943,8 @@ struct __cucholmixed_st {
   float *t, *y, *zf;          // preconditioner vectors (FP32)
   double *U, *V;              // symmetric-product partials
   double *part, *part_norm, *rz, *norms;
-  double* h_norms;            // pinned mirror of norms
+  double* h_norms;            // pinned mirror of norms (the handle's)
+  char* arena;                // the one allocation behind all of the above
   unsigned* ctr;              // triangular-solve counters
   int* err;                   // a bounded wait gave up
 };
@@ -972,7 +986,7 @@ CUresult symv(const double* A, long long rs, long long cs, int n, const double* 
   symv_tiles_kernel<<<T * (T + 1) / 2, kThreads, kSymvSmem, s>>>(A, lda, upper, n, X, ldx, nrhs, absval, vec16, U,
                                                                   V);
   CUCHOL_CHECK(cudaGetLastError());
-  symv_reduce_kernel<<<T, kThreads, 0, s>>>(U, V, n, T, alpha, beta, B, ldb, Y, ldy, nrhs);
+  symv_reduce_kernel<<<T * SY * NR / kThreads, kThreads, 0, s>>>(U, V, n, T, alpha, beta, B, ldb, Y, ldy, nrhs);
   CUCHOL_CHECK(cudaGetLastError());
   return CUDA_SUCCESS;
 }
@@ -1035,7 +1049,7 @@ CUresult precond(CUcholMixed p, const double* R, double* Z, cudaStream_t s) {
   CUCHOL_CHECK(cudaGetLastError());
   for (int I = 0; I < nT; ++I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0), rest = n - b0 - bI;
-    const float* D = p->Dinv + (size_t)I * NBT * NBT;
+    const float* D = p->Dinv + (size_t)I * NBT * (NBT + 1);
     CUCHOL_CHECK_CU(gemv(false, D, NBT, bI, bI, p->t + b0, 1.f, 0.f, nullptr, p->y + b0));
     if (rest > 0)
       CUCHOL_CHECK_CU(gemv(false, p->W + (b0 + bI) + (long long)b0 * ldw, ldw, rest, bI, p->y + b0, -1.f, 1.f,
@@ -1043,7 +1057,7 @@ CUresult precond(CUcholMixed p, const double* R, double* Z, cudaStream_t s) {
   }
   for (int I = nT - 1; I >= 0; --I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0);
-    const float* D = p->Dinv + (size_t)I * NBT * NBT;
+    const float* D = p->Dinv + (size_t)I * NBT * (NBT + 1);
     CUCHOL_CHECK_CU(gemv(true, D, NBT, bI, bI, p->y + b0, 1.f, 0.f, nullptr, p->zf + b0));
     if (b0 > 0) CUCHOL_CHECK_CU(gemv(true, p->W + b0, ldw, b0, bI, p->zf + b0, -1.f, 1.f, p->y, p->y));
   }
@@ -1171,62 +1185,16 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
 
 void free_mixed(CUcholMixed p) {
   if (p == nullptr) return;
-  cudaFree(p->W);
-  cudaFree(p->s);
-  cudaFree(p->Dinv);
-  cudaFree(p->dtmp);
-  cudaFree(p->gpart);
-  cudaFree(p->x);
-  cudaFree(p->t);
-  cudaFree(p->U);
-  cudaFree(p->V);
-  cudaFree(p->part);
-  cudaFree(p->ctr);
-  cudaFreeHost(p->h_norms);
+  cudaFree(p->arena);
   delete p;
 }
 
 // Largest column max |v(:, c)| for c < 2 NR of the partials -> host (synchronises s).
 CUresult fetch_norms(CUcholMixed p, cudaStream_t s) {
-  norms_final_kernel<<<1, 2 * NR, 0, s>>>(p->part_norm, kVecBlocks, p->norms);
+  norms_final_kernel<<<1, 64 * NR, 0, s>>>(p->part_norm, kVecBlocks, p->norms);
   CUCHOL_CHECK(cudaGetLastError());
   CUCHOL_CHECK(cudaMemcpyAsync(p->h_norms, p->norms, 2 * NR * sizeof(double), cudaMemcpyDeviceToHost, s));
   CUCHOL_CHECK(cudaStreamSynchronize(s));
-  return CUDA_SUCCESS;
-}
-
-// The doubling levels of the NBT-block inverses (see mixed_refactor); the products
-// B inv(A) of one level (at most n * NBT / 4 elements) go to the plan's scratch.
-CUresult dinv_doubling(CUcholMixed p, cudaStream_t s) {
-  const int n = p->n, nT = (n + NBT - 1) / NBT;
-  const long long ldw = p->ldw;
-  for (int sz = SB; sz < NBT; sz *= 2) {
-    std::vector<GemmProblem<float>> first, second;
-    float* tmp = p->dtmp;
-    for (int I = 0; I < nT; ++I) {
-      const int b0 = I * NBT, bI = std::min(NBT, n - b0);
-      float* D = p->Dinv + (size_t)I * NBT * NBT;
-      for (int o = 0; o + sz < bI; o += 2 * sz) {
-        const int cs = std::min(sz, bI - o - sz);
-        GemmProblem<float> t1 = problem<float>();   // T = B inv(A), cs x sz
-        t1.a = p->W + (b0 + o + sz) + (long long)(b0 + o) * ldw; t1.a_rs = 1; t1.a_ks = ldw;
-        t1.b = D + o + (long long)o * NBT; t1.b_rs = NBT; t1.b_ks = 1;
-        t1.c = tmp; t1.c_rs = 1; t1.c_cs = cs;
-        t1.m = cs; t1.n = sz; t1.k = sz;
-        GemmProblem<float> t2 = problem<float>();   // X = -inv(C) T
-        t2.a = D + (o + sz) + (long long)(o + sz) * NBT; t2.a_rs = 1; t2.a_ks = NBT;
-        t2.b = tmp; t2.b_rs = cs; t2.b_ks = 1;
-        t2.c = D + (o + sz) + (long long)o * NBT; t2.c_rs = 1; t2.c_cs = NBT;
-        t2.m = cs; t2.n = sz; t2.k = cs;
-        t2.alpha = -1.f;
-        first.push_back(t1);
-        second.push_back(t2);
-        tmp += (size_t)cs * sz;
-      }
-    }
-    CUCHOL_CHECK_CU(gemm_group<float>(p->h, first, s, nullptr));
-    CUCHOL_CHECK_CU(gemm_group<float>(p->h, second, s, nullptr));
-  }
   return CUDA_SUCCESS;
 }
 
@@ -1255,8 +1223,8 @@ CUresult mixed_refactor(CUcholMixed p, long* info) {
   // |A|_inf = max row sum of |A| (x is zero: column 0 set to ones)
   CUCHOL_CHECK(cudaMemsetAsync(p->x, 0, sizeof(double) * p->ld * NR, sp));
   {
-    std::vector<double> ones(n, 1.0);
-    CUCHOL_CHECK(cudaMemcpyAsync(p->x, ones.data(), sizeof(double) * n, cudaMemcpyHostToDevice, sp));
+    ones_kernel<<<(n + 255) / 256, 256, 0, sp>>>(p->x, n);
+    CUCHOL_CHECK(cudaGetLastError());
     CUCHOL_CHECK_CU(symv(p->A, p->rs, p->cs, n, p->x, p->ld, 1, 1, 1.0, 0.0, nullptr, 0, p->r, p->ld, p->U, p->V,
                          sp));
     CUCHOL_CHECK(cudaMemsetAsync(p->r + p->ld, 0, sizeof(double) * p->ld * (NR - 1), sp));
@@ -1283,24 +1251,28 @@ CUresult mixed_refactor(CUcholMixed p, long* info) {
     *info = finfo;
     return CUDA_SUCCESS;
   }
-  // inverses of the NBT-wide diagonal blocks of the factor: the 128-wide diagonal
-  // blocks inverted in place (one CTA each), then recursive doubling
-  //   inv([A 0; B C]) = [inv(A) 0; -inv(C) B inv(A), inv(C)]
-  // with one grouped launch per level and product, all NBT-blocks together (FP32).
-  CUCHOL_CHECK(cudaMemsetAsync(p->Dinv, 0, sizeof(float) * (size_t)nT * NBT * NBT, sp));
-  CUCHOL_CHECK_CU(set_smem<float>((const void*)diag_invert_kernel<float, SB, kDiagThreads2>,
-                                  BlockSmem<float, SB>::bytes));
+  // Inverses of the NBT-wide diagonal blocks of the factor.  Block I starts at
+  // I * NBT * (NBT + 1), so all of them together look like the diagonal blocks of one
+  // matrix of order n and leading dimension NBT, and ?trtri's first levels (128-wide
+  // leaves, then pairs up to NBT, on the TF32 tensor cores) invert them in place.
+  CUCHOL_CHECK(cudaMemsetAsync(p->Dinv, 0, sizeof(float) * (size_t)nT * NBT * (NBT + 1), sp));
   for (int I = 0; I < nT; ++I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0);
-    float* Dn = p->Dinv + (size_t)I * NBT * NBT;
-    CUCHOL_CHECK_CU(copy_view<float>(h, p->W + b0 + (long long)b0 * p->ldw, 1, p->ldw, Dn, 1, NBT, bI, bI, true, sp,
-                                     nullptr));
-    diag_invert_kernel<float, SB, kDiagThreads2><<<(bI + SB - 1) / SB, kDiagThreads2, BlockSmem<float, SB>::bytes,
-                                                   sp>>>(Dn, 1, NBT, bI, SB, 0);
-    ++h->launches;
-    CUCHOL_CHECK(cudaGetLastError());
+    CUCHOL_CHECK_CU(copy_view<float>(h, p->W + b0 + (long long)b0 * p->ldw, 1, p->ldw,
+                                     p->Dinv + (size_t)I * NBT * (NBT + 1), 1, NBT, bI, bI, true, sp, nullptr));
   }
-  CUCHOL_CHECK_CU(dinv_doubling(p, sp));
+  CUCHOL_CHECK_CU(set_smem<float>((const void*)diag_invert_kernel<float, SB, kDiagThreads2>,
+                                  BlockSmem<float, SB>::bytes));
+  diag_invert_kernel<float, SB, kDiagThreads2><<<(n + SB - 1) / SB, kDiagThreads2, BlockSmem<float, SB>::bytes, sp>>>(
+      p->Dinv, 1, NBT, n, SB, 0);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  bool leveled = false;
+  CUCHOL_CHECK_CU(trtri_levels_tcg<float>(h, false, n, p->Dinv, 1, NBT, NBT, &leveled));
+  if (!leveled) {
+    CUCHOL_CHECK_CU(ensure_workspace(h, trtri_levels_bytes<float>(n, NBT)));
+    CUCHOL_CHECK_CU(trtri_levels_tcg<float>(h, false, n, p->Dinv, 1, NBT, NBT, &leveled));
+  }
   CUCHOL_CHECK(cudaStreamSynchronize(sp));
   *info = 0;
   return CUDA_SUCCESS;
@@ -1327,38 +1299,49 @@ CUresult mixed_create(CUcholMixed* out, CULAPACKhandle h, CBlasUplo uplo, size_t
     free_mixed(p);
     return ::cuchol::report(e, "cudaMalloc", __func__, __FILE__, __LINE__);
   };
-  cudaError_t e;
-  if ((e = dev_malloc(&p->W, sizeof(float) * p->ldw * n)) != cudaSuccess) return fail(e);
-  if ((e = dev_malloc(&p->s, sizeof(double) * n)) != cudaSuccess) return fail(e);
+  // one device block for everything (an allocation costs about as much as a refinement
+  // step, and freeing one waits for the device); pieces on 256-byte boundaries
   const int nT = (n + NBT - 1) / NBT;
-  if ((e = dev_malloc(&p->Dinv, sizeof(float) * (size_t)nT * NBT * NBT)) != cudaSuccess) return fail(e);
-  if ((e = dev_malloc(&p->dtmp, sizeof(float) * (size_t)n * NBT / 4 + 256)) != cudaSuccess) return fail(e);
   // split k only when a GEMV has fewer than 2 * SMs row blocks: at most NBT / 256 splits
   const size_t gpart = (size_t)(NBT / 256) * (2 * h->num_sms + 1) * GR * NR;
-  if ((e = dev_malloc(&p->gpart, sizeof(float) * gpart)) != cudaSuccess) return fail(e);
-  // x r z p q b in one block, then the reduction scratch
-  if ((e = dev_malloc(&p->x, sizeof(double) * 6 * p->ld * NR)) != cudaSuccess) return fail(e);
+  const size_t ptile = (size_t)T * (T + 1) / 2 * SY * NR;
+  const size_t nred = kVecBlocks * NR + kVecBlocks * 2 * NR + 2 * NR + 2 * NR;
+  size_t total = 0;
+  auto carve = [&](size_t bytes) {
+    const size_t at = total;
+    total += round_up(bytes, 256);
+    return at;
+  };
+  const size_t oW = carve(sizeof(float) * p->ldw * n), os = carve(sizeof(double) * n),
+               oD = carve(sizeof(float) * (size_t)nT * NBT * (NBT + 1)), og = carve(sizeof(float) * gpart),
+               ox = carve(sizeof(double) * 6 * p->ld * NR), ot = carve(sizeof(float) * 3 * p->ld * NR),
+               oU = carve(sizeof(double) * ptile), oV = carve(sizeof(double) * ptile), op = carve(sizeof(double) * nred),
+               oc = carve(16 * sizeof(unsigned));
+  cudaError_t e;
+  if ((e = dev_malloc(&p->arena, total)) != cudaSuccess) return fail(e);
+  p->W = reinterpret_cast<float*>(p->arena + oW);
+  p->s = reinterpret_cast<double*>(p->arena + os);
+  p->Dinv = reinterpret_cast<float*>(p->arena + oD);
+  p->gpart = reinterpret_cast<float*>(p->arena + og);
+  p->x = reinterpret_cast<double*>(p->arena + ox);   // x r z p q b
   p->r = p->x + p->ld * NR;
   p->z = p->r + p->ld * NR;
   p->p = p->z + p->ld * NR;
   p->q = p->p + p->ld * NR;
   p->b = p->q + p->ld * NR;
-  if ((e = dev_malloc(&p->t, sizeof(float) * 3 * p->ld * NR)) != cudaSuccess) return fail(e);
+  p->t = reinterpret_cast<float*>(p->arena + ot);
   p->y = p->t + p->ld * NR;
   p->zf = p->y + p->ld * NR;
-  const size_t ptile = (size_t)T * (T + 1) / 2 * SY * NR;
-  if ((e = dev_malloc(&p->U, sizeof(double) * ptile)) != cudaSuccess) return fail(e);
-  if ((e = dev_malloc(&p->V, sizeof(double) * ptile)) != cudaSuccess) return fail(e);
-  if ((e = dev_malloc(&p->part, sizeof(double) * (kVecBlocks * NR + kVecBlocks * 2 * NR + 2 * NR + 2 * NR))) !=
-      cudaSuccess)
-    return fail(e);
+  p->U = reinterpret_cast<double*>(p->arena + oU);
+  p->V = reinterpret_cast<double*>(p->arena + oV);
+  p->part = reinterpret_cast<double*>(p->arena + op);
   p->part_norm = p->part + kVecBlocks * NR;
   p->rz = p->part_norm + kVecBlocks * 2 * NR;
   p->norms = p->rz + 2 * NR;
-  if ((e = dev_malloc(&p->ctr, 16 * sizeof(unsigned))) != cudaSuccess) return fail(e);
+  p->ctr = reinterpret_cast<unsigned*>(p->arena + oc);
   p->err = reinterpret_cast<int*>(p->ctr + 8);
   if ((e = cudaMemset(p->ctr, 0, 16 * sizeof(unsigned))) != cudaSuccess) return fail(e);
-  if ((e = cudaMallocHost(&p->h_norms, 2 * NR * sizeof(double))) != cudaSuccess) return fail(e);
+  p->h_norms = h->h_norms;
 
   p->shift_request = shift_in;
   *out = p;
