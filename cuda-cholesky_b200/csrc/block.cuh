@@ -37,6 +37,15 @@ __device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool valid) 
                  : "memory");
   }
 }
+// The first `bytes` (0 .. 16) of a 16-byte piece, the rest zero; both addresses 16-byte
+// aligned.
+__device__ __forceinline__ void cp_async_piece(void* dst, const void* src, int bytes) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool aligned16(const void* p, long long stride_bytes) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)stride_bytes) & 15) == 0;
+}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
 }
@@ -48,21 +57,24 @@ constexpr int kSubRows = 32;         // rows factor16 covers: the 16 x 16 block 
 // touches 16 distinct 8-byte banks per half warp.
 constexpr int kLdPad = 4;
 
-// 1 / sqrt(d) for the pivot chain, without branches.  FP64: the hardware estimate y
-// (relative error below 2^-20) refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2,
-// to second order (the dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations
-// after the estimate.  Right for every normal d and 0 for infinity, like rsqrt();
-// subnormal pivots (for which the estimate is infinite) are left to factor16_slow.
-__device__ __forceinline__ float pivot_rsqrt(float d) { return rsqrtf(d); }
+// 1 / sqrt(d) for the pivot chain, for normal positive finite d, without branches.  FP32:
+// the hardware estimate.  FP64: the hardware estimate y (relative error below 2^-20)
+// refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, to second order (the
+// dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations after the estimate.
+__device__ __forceinline__ float pivot_rsqrt(float d) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return y;
+}
 __device__ __forceinline__ double pivot_rsqrt(double d) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d * y, y, 1.0);
-  const double r = fma(y * e, fma(0.375, e, 0.5), y);
-  return (__double2hiint(d) == 0x7ff00000) ? 0.0 : r;
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
-__device__ __forceinline__ bool subnormal_pivot(float) { return false; }   // rsqrtf takes them
-__device__ __forceinline__ bool subnormal_pivot(double d) { return __double2hiint(d) < 0x00100000; }
+// Not a normal positive finite number (one integer subtraction and comparison).
+__device__ __forceinline__ bool odd_pivot(float d) { return (unsigned)(__float_as_int(d) - 0x00800000) >= 0x7f000000u; }
+__device__ __forceinline__ bool odd_pivot(double d) { return (unsigned)(__double2hiint(d) - 0x00100000) >= 0x7fe00000u; }
 
 // Elements FROM .. 15 of 16 at a 16-byte aligned shared address, in 16-byte loads.
 template <int FROM, typename T>
@@ -97,7 +109,9 @@ __device__ __forceinline__ double minus_abs2(cuDoubleComplex a, cuDoubleComplex 
 // -1, the same in every lane; the columns before it are then done and the others as
 // they were.
 //
-// factor16_slow: the plain loop, for sub-panels with a subnormal pivot.
+// factor16_slow: the plain loop.  factor16 leaves every sub-panel with a pivot that is
+// not a normal positive number to it (non-SPD blocks, infinities, subnormals), so the
+// fast code carries one integer test per pivot and no failure handling.
 template <typename T>
 __device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf<T>* rd) {
   using R = RealOf<T>;
@@ -123,18 +137,18 @@ __device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf
   return -1;
 }
 
-// Step J of factor16 and the ones after it: x the row, d the pivot of column J.
+// Step J of factor16 and the ones after it: x the row, r the reciprocal square root of
+// the pivot of column J.  (On lane J the update formula makes x[J] the pivot itself, so
+// x[J] r is the diagonal element; complex types drop its imaginary part when it is stored.)
 template <int J, typename T>
-__device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> d, RealOf<T> r, int i, T* Ld, RealOf<T>* rd,
-                                               int& fail, bool& sub) {
+__device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i, T* Ld, RealOf<T>* rd, bool& odd) {
   using R = RealOf<T>;
   if constexpr (J < kSub) {
-    fail = (fail < 0 && !(d > R(0))) ? J : fail;
-    sub = sub || subnormal_pivot(d);
-    x[J] = (i == J) ? from_real<T>(d * r) : scale(x[J], r);
-    R dn = R(1), rn = R(1);
+    x[J] = scale(x[J], r);
+    R rn = R(1);
     if constexpr (J + 1 < kSub) {
-      dn = __shfl_sync(0xffffffffu, minus_abs2(x[J + 1], x[J]), J + 1);
+      const R dn = __shfl_sync(0xffffffffu, minus_abs2(x[J + 1], x[J]), J + 1);
+      odd = odd || odd_pivot(dn);
       rn = pivot_rsqrt(dn);
     }
     if (i < kSub) Ld[J * kSub + i] = x[J];
@@ -145,7 +159,7 @@ __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> d, RealOf
       load_row16<J + 1>(Ld + J * kSub, v);
 #pragma unroll
       for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
-      factor16_steps<J + 1>(x, dn, rn, i, Ld, rd, fail, sub);
+      factor16_steps<J + 1>(x, rn, i, Ld, rd, odd);
     }
   }
 }
@@ -159,29 +173,35 @@ __device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Ld, RealOf<T
 #pragma unroll
   for (int q = 0; q < kSub; ++q) x[q] = mine ? S[q * ld + i] : zero<T>();
   const R d = __shfl_sync(0xffffffffu, re(x[0]), 0);
-  int fail = -1;
-  bool sub = false;
-  factor16_steps<0>(x, d, pivot_rsqrt(d), i, Ld, rd, fail, sub);
-  // (rubbish after a failing column may look subnormal: only a sub-panel whose first
-  // bad pivot is subnormal and positive changes its outcome in the slow loop)
-  if (sub) return factor16_slow<T>(S, ld, nrows, Ld, rd);
+  bool odd = odd_pivot(d);
+  if constexpr (Traits<T>::complex) {
+    if (i == 0) x[0].y = 0;
+  }
+  factor16_steps<0>(x, pivot_rsqrt(d), i, Ld, rd, odd);
+  if (odd) return factor16_slow<T>(S, ld, nrows, Ld, rd);
 #pragma unroll
-  for (int q = 0; q < kSub; ++q)
-    if (mine && i >= q && (fail < 0 || q < fail)) S[q * ld + i] = x[q];
-  return fail;
+  for (int q = 0; q < kSub; ++q) {
+    if constexpr (Traits<T>::complex) {
+      if (i == q) x[q].y = 0;
+    }
+    if (mine && i >= q) S[q * ld + i] = x[q];
+  }
+  return -1;
 }
 
+// Step J of solve16 and the ones after it: v holds column J of the block.  The next
+// column is loaded one step ahead and no further: left alone the compiler hoists all 64
+// loads to the front and spills.
 template <int J, typename T>
-__device__ __forceinline__ void solve16_steps(T (&x)[kSub], const T* __restrict__ Ld, const RealOf<T>* __restrict__ rd) {
+__device__ __forceinline__ void solve16_steps(T (&x)[kSub], const T (&v)[kSub], const T* Ld, const RealOf<T>* rd) {
   if constexpr (J < kSub) {
+    T w[kSub];
+    if constexpr (J + 2 < kSub) load_row16<J + 2>(Ld + (J + 1) * kSub, w);
     x[J] = scale(x[J], rd[J]);
-    if constexpr (J + 1 < kSub) {
-      T v[kSub];
-      load_row16<J + 1>(Ld + J * kSub, v);
+    asm volatile("" ::: "memory");
 #pragma unroll
-      for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
-      solve16_steps<J + 1>(x, Ld, rd);
-    }
+    for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
+    solve16_steps<J + 1>(x, w, Ld, rd);
   }
 }
 
@@ -189,12 +209,12 @@ __device__ __forceinline__ void solve16_steps(T (&x)[kSub], const T* __restrict_
 // factored block: x := x L^-H.  120 FMAs, whose chain is one multiplication and one FMA
 // per column.
 template <typename T>
-__device__ __forceinline__ void solve16(T* S, int ld, const T* __restrict__ Ld, const RealOf<T>* __restrict__ rd) {
-  T x[kSub];
+__device__ __forceinline__ void solve16(T* S, int ld, const T* Ld, const RealOf<T>* rd) {
+  T x[kSub], v[kSub];
 #pragma unroll
   for (int q = 0; q < kSub; ++q) x[q] = S[q * ld];
-  solve16_steps<0>(x, Ld, rd);
-  // stored at the end: a store between them would hold back the loads of Ld
+  load_row16<1>(Ld, v);
+  solve16_steps<0>(x, v, Ld, rd);
 #pragma unroll
   for (int q = 0; q < kSub; ++q) S[q * ld] = x[q];
 }
@@ -206,6 +226,27 @@ __device__ __noinline__ void solve16_part(T* S, int ld, const T* Ld, const RealO
     T x = S[j * ld];
     for (int k = 0; k < j; ++k) fms(x, S[k * ld], cj(Ld[k * kSub + j]));
     S[j * ld] = scale(x, rd[j]);
+  }
+}
+
+// 4 elements at a 16-byte aligned shared address.
+template <typename T>
+__device__ __forceinline__ void load4(const T* p, T (&v)[4]) {
+  const int4* q = reinterpret_cast<const int4*>(p);
+#pragma unroll
+  for (int u = 0; u < (int)sizeof(T) / 4; ++u) {
+    const int4 w = q[u];
+    memcpy(reinterpret_cast<char*>(v) + 16 * u, &w, 16);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store4(T* p, const T (&v)[4]) {
+  int4* q = reinterpret_cast<int4*>(p);
+#pragma unroll
+  for (int u = 0; u < (int)sizeof(T) / 4; ++u) {
+    int4 w;
+    memcpy(&w, reinterpret_cast<const char*>(v) + 16 * u, 16);
+    q[u] = w;
   }
 }
 
@@ -258,50 +299,24 @@ __device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, 
         for (int e = 0; e < 4; ++e) C[(8 * b + 2 * t + (e & 1)) * ldc + 16 * a + g + 8 * (e >> 1)] -= acc[a][b][e];
     }
   } else {
-    // lane: rows lr + 8u, columns lc + 4v
+    // lane: rows 4 lr .. + 3, columns 4 lc .. + 3, all shared accesses in 16-byte pieces
     const int lr = lane & 7, lc = lane >> 3;
-    const int nu = nr > 16 ? 4 : 2;
+    if (4 * lr >= nr) return;
     T acc[4][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int v = 0; v < 4; ++v) load4(C + (4 * lc + v) * ldc + 4 * lr, acc[v]);
+#pragma unroll 4
+    for (int k = 0; k < kSub; ++k) {
+      T a[4], b[4];
+      load4(P + k * ldp + 4 * lr, a);
+      load4(Q + k * ldq + 4 * lc, b);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = zero<T>();
-    if (nu == 4) {
-#pragma unroll 8
-      for (int k = 0; k < kSub; ++k) {
-        T a[4], b[4];
+      for (int v = 0; v < 4; ++v)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = P[k * ldp + lr + 8 * u];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) b[v] = cj(Q[k * ldq + lc + 4 * v]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) fms(acc[u][v], a[u], b[v]);
-      }
-    } else {
-#pragma unroll 8
-      for (int k = 0; k < kSub; ++k) {
-        T a[2], b[4];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) a[u] = P[k * ldp + lr + 8 * u];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) b[v] = cj(Q[k * ldq + lc + 4 * v]);
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) fms(acc[u][v], a[u], b[v]);
-      }
+        for (int u = 0; u < 4; ++u) fms(acc[v][u], a[u], cj(b[v]));
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (u < nu) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          T* c = C + (lc + 4 * v) * ldc + lr + 8 * u;
-          *c = add(*c, acc[u][v]);
-        }
-      }
+    for (int v = 0; v < 4; ++v) store4(C + (4 * lc + v) * ldc + 4 * lr, acc[v]);
   }
 }
 

@@ -16,9 +16,10 @@ struct __culapackhandle_st {
                            // [3] engine error (a bounded wait gave up)
   int* h_words;            // pinned mirror of d_words
   double* h_norms;         // pinned scratch of the mixed solve (part of h_words' block)
-  double* d_logdet;        // [0] fused potrf log det, [1] ?logdet result (double)
+  double* d_result;        // ?logdet result (double)
+  double* d_logdet;        // fused potrf log det (behind d_words, in the same block)
   float* d_logdet_f;       // ?logdet result (float)
-  double* h_logdet;        // pinned mirror of d_logdet[0]
+  double* h_logdet;        // pinned mirror of d_logdet (behind h_words)
   double* d_part;          // ?logdet partial sums (kLogdetMaxBlocks)
   unsigned int* d_counter; // ?logdet retirement counter
   void* ws;                // grow-only workspace

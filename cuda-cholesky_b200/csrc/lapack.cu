@@ -496,14 +496,15 @@ CUresult set_smem(const void* fn, size_t bytes) {
 constexpr int kDiagThreads2 = 256;
 
 // Factor of the jb x jb diagonal block at A (logical lower view), queued on s; T: the
-// computing type, TA: the storage type.
+// computing type, TA: the storage type.  first: the factorization's first block, which
+// starts the info word and the log det.
 template <typename T, typename TA, int NB>
-CUresult diag_factor(CULAPACKhandle h, TA* A, long long rs, long long cs, int jb, long long info_base,
+CUresult diag_factor(CULAPACKhandle h, TA* A, long long rs, long long cs, int jb, long long info_base, bool first,
                      double* logdet, cudaStream_t s) {
   constexpr int smem = (int)FactorSmem<T, NB>::bytes;
   auto* kernel = diag_factor_kernel<T, TA, NB, kDiagThreads2>;
   CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
-  kernel<<<1, kDiagThreads2, smem, s>>>(A, rs, cs, jb, info_base, h->d_words, logdet);
+  kernel<<<1, kDiagThreads2, smem, s>>>(A, rs, cs, jb, info_base, first ? 1 : 0, h->d_words, logdet);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
   return CUDA_SUCCESS;
@@ -693,6 +694,13 @@ bool try_workspace(CULAPACKhandle h, size_t bytes) {
   return true;
 }
 
+// Words and fused log det to the host, with the synchronisation.
+CUresult fetch_words(CULAPACKhandle h, cudaStream_t s) {
+  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 16 * sizeof(int) + sizeof(double), cudaMemcpyDeviceToHost, s));
+  CUCHOL_CHECK(cudaStreamSynchronize(s));
+  return check_engine(h);
+}
+
 // ---- ?POTRF ---------------------------------------------------------------------
 // Right-looking blocked Cholesky, outer blocks of NB = sub*nb columns (each factored
 // as sub nb-wide sub-panels; sub from the tuning table, 2 to 8 by n for FP64),
@@ -719,13 +727,20 @@ bool try_workspace(CULAPACKhandle h, size_t bytes) {
 // own columns); the columns right of it are neither read nor written.
 using FinalColumns = std::function<CUresult(int c, int jb, cudaStream_t s)>;
 
+// Up to this order the chain of panels is the whole time: every step is queued on one
+// stream (diagonal block, solve, update of everything to the right), because a cross-stream
+// wait costs more than the overlap gives.
+constexpr int kOneStreamOrder = 1536;
+
 template <typename T>
 CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, long* info, double* logdet_out,
                    const FinalColumns* on_final = nullptr, int ncols = -1) {
   if (ncols < 0 || ncols > n) ncols = n;
   constexpr int nb = Tune<T>::nb;
   // outer block: sub diagonal blocks, from the handle's override or the tuning table
-  const int NB = (h->potrf_sub > 0 ? h->potrf_sub : tuned_potrf_sub(type_char<T>(), n)) * nb;
+  // small orders: outer blocks of one diagonal block and no second stream
+  const bool alone = h->potrf_sub == 0 && n <= kOneStreamOrder && on_final == nullptr && ncols == n;
+  const int NB = (h->potrf_sub > 0 ? h->potrf_sub : alone ? 1 : tuned_potrf_sub(type_char<T>(), n)) * nb;
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel, su = h->s_update;
@@ -750,12 +765,9 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   float* qbuf[4];
   for (int i = 0; i < 4; ++i) qbuf[i] = static_cast<float*>(h->ws) + i * qsize;
 
-  CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
-  CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
-  // the update stream starts after the panel stream's initialisation
-  CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
-  CUCHOL_CHECK(cudaStreamWaitEvent(su, h->ev_panel, 0));
-  CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
+  // the first diagonal kernel writes the info word and the log det, the later ones read
+  // and add to them; the update stream starts behind a panel event
+  CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));
 
   const T minus_one = from_real<T>(RealOf<T>(-1)), one = from_real<T>(RealOf<T>(1));
   // C -= Phat Phat^H on the lower trapezoid m x ncols of A with its corner on the
@@ -791,7 +803,7 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;                 // rows below this diagonal block
-      CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, h->d_logdet, sp)));
+      CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, c == 0, h->d_logdet, sp)));
       if (mr == 0) {
         if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
         break;
@@ -809,7 +821,7 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
         CUCHOL_CHECK_CU((panel_solve<T, T, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs,
                                                             P + s0 + (long long)s0 * ldp, 1, ldp, nullptr, sp)));
       }
-      CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
+      if (!alone) CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
       if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
       if (s0 + nb < jB) {
         // the outer block's remaining sub-panel columns (rows c + nb .., P rows s0 ..)
@@ -818,6 +830,10 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
       }
     }
     if (m == 0 || mc == 0) break;
+    if (alone) {
+      CUCHOL_CHECK_CU(update(P, Qh, Ql, j + NB, m, mc, NB - nb, 0, jB, sp));
+      continue;
+    }
     // lookahead: next outer block (P rows from j + NB, k = jB), after the previous
     // trailing update
     const int jB2 = std::min(NB, mc);
@@ -831,12 +847,11 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     // always recorded: it also covers the copies that still read P
     CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
   }
-  CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
-  CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, d_info, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_logdet, h->d_logdet, sizeof(double), cudaMemcpyDeviceToHost, sp));
-  CUCHOL_CHECK(cudaStreamSynchronize(sp));
-  CUCHOL_CHECK_CU(check_engine(h));
+  if (!alone) {
+    CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
+    CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
+  }
+  CUCHOL_CHECK_CU(fetch_words(h, sp));
   *info = h->h_words[0];
   if (logdet_out != nullptr) *logdet_out = h->h_logdet[0];
   return CUDA_SUCCESS;
@@ -962,9 +977,7 @@ CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs
     g.neg = 1;
     CUCHOL_CHECK_CU(tcg_launch(h, PackRef{x, x + one, (long long)rows, ld, 1}, rb2, g, sp, nullptr));
   }
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-  CUCHOL_CHECK(cudaStreamSynchronize(sp));
-  return check_engine(h);
+  return fetch_words(h, sp);
 }
 
 template <typename T> constexpr bool is_fp64() { return std::is_same<T, double>::value || std::is_same<T, cuDoubleComplex>::value; }
@@ -1074,9 +1087,7 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
         CUCHOL_CHECK_CU(trtri_levels_fp64<T>(h, unit, n, W, direct ? lda : ldc, upper, X, sp));
         if (!direct)
           CUCHOL_CHECK_CU(copy_view<T>(h, W, upper ? ldc : 1, upper ? 1 : ldc, A, rs, cs, n, n, true, sp, nullptr));
-        CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-        CUCHOL_CHECK(cudaStreamSynchronize(sp));
-        return check_engine(h);
+        return fetch_words(h, sp);
       }
     }
   }
@@ -1181,9 +1192,7 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
       g.lower_only = 1; g.real_diag = 1;
       CUCHOL_CHECK_CU(tcg_launch(h, PackRef{w, w + one, (long long)n * cx, ld, cx}, PackRef{w, w + one, (long long)n * cx, ld, 1},
                                  g, sp, nullptr));
-      CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-      CUCHOL_CHECK(cudaStreamSynchronize(sp));
-      return check_engine(h);
+      return fetch_words(h, sp);
     }
   }
   const int w = lauum_width<T>(h, n);
@@ -1220,9 +1229,7 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
       sum_slabs_kernel<T><<<dim3(nt, nt), 256, 0, sp>>>(W, ldw, nl.nd.c_node, slabs, slab, A, rs, cs, n);
       ++h->launches;
       CUCHOL_CHECK(cudaGetLastError());
-      CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-      CUCHOL_CHECK(cudaStreamSynchronize(sp));
-      return check_engine(h);
+      return fetch_words(h, sp);
     }
   }
   CUCHOL_CHECK_CU(ensure_workspace(h, sizeof(T) * (size_t)ldw * w));
@@ -1279,14 +1286,14 @@ CUresult trti22_run(CULAPACKhandle h, bool upper, bool unit, int n, const T* A, 
 template <typename T, typename Out>
 CUresult logdet_run(CULAPACKhandle h, const T* x, long long incx, long long n, Out* result, cudaStream_t stream) {
   const int blocks = (int)std::min<long long>((n + 255) / 256, std::min(kLogdetMaxBlocks, 2 * h->num_sms));
-  logdet_kernel<T, 256><<<blocks, 256, 0, stream>>>(x, incx, n, h->d_part, h->d_counter, h->d_logdet + 1);
+  logdet_kernel<T, 256><<<blocks, 256, 0, stream>>>(x, incx, n, h->d_part, h->d_counter, h->d_result);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
   if constexpr (sizeof(Out) == sizeof(double)) {
-    CUCHOL_CHECK(cudaMemcpyAsync(result, h->d_logdet + 1, sizeof(double), cudaMemcpyDeviceToHost, stream));
+    CUCHOL_CHECK(cudaMemcpyAsync(result, h->d_result, sizeof(double), cudaMemcpyDeviceToHost, stream));
   } else {
     // narrow on the device so the host copy stays asynchronous
-    narrow_double_kernel<<<1, 1, 0, stream>>>(h->d_logdet + 1, h->d_logdet_f);
+    narrow_double_kernel<<<1, 1, 0, stream>>>(h->d_result, h->d_logdet_f);
     ++h->launches;
     CUCHOL_CHECK(cudaGetLastError());
     CUCHOL_CHECK(cudaMemcpyAsync(result, h->d_logdet_f, sizeof(float), cudaMemcpyDeviceToHost, stream));
@@ -1309,9 +1316,8 @@ void release_handle(CULAPACKhandle h) {
   cudaFree(h->ws);
   cudaFree(h->d_words);
   cudaFreeHost(h->h_words);
-  cudaFree(h->d_logdet);
+  cudaFree(h->d_result);
   cudaFree(h->d_logdet_f);
-  cudaFreeHost(h->h_logdet);
   cudaFree(h->d_part);
   cudaFree(h->d_counter);
   cudaFree(h->desc_dev);
@@ -1324,6 +1330,8 @@ void release_handle(CULAPACKhandle h) {
 }
 
 CUresult create_handle(CULAPACKhandle h);
+
+constexpr size_t kWordBytes = 16 * sizeof(int);
 
 }  // namespace
 
@@ -1372,13 +1380,15 @@ CUresult create_handle(CULAPACKhandle h) {
   CUCHOL_CHECK(cudaStreamCreateWithPriority(&h->s_update, cudaStreamDefault, mid));
   CUCHOL_CHECK(cudaEventCreateWithFlags(&h->ev_panel, cudaEventDisableTiming));
   CUCHOL_CHECK(cudaEventCreateWithFlags(&h->ev_update, cudaEventDisableTiming));
-  CUCHOL_CHECK(dev_malloc(&h->d_words, 16 * sizeof(int)));
-  CUCHOL_CHECK(cudaMemset(h->d_words, 0, 16 * sizeof(int)));
-  CUCHOL_CHECK(cudaMallocHost(&h->h_words, 16 * sizeof(int) + 64 * sizeof(double)));
-  h->h_norms = reinterpret_cast<double*>(h->h_words + 16);
-  CUCHOL_CHECK(dev_malloc(&h->d_logdet, 4 * sizeof(double)));
+  // the words and, behind them, the log det values: one copy brings both to the host
+  CUCHOL_CHECK(dev_malloc(&h->d_words, kWordBytes + sizeof(double)));
+  CUCHOL_CHECK(cudaMemset(h->d_words, 0, kWordBytes + sizeof(double)));
+  h->d_logdet = reinterpret_cast<double*>(h->d_words + 16);
+  CUCHOL_CHECK(cudaMallocHost(&h->h_words, kWordBytes + 68 * sizeof(double)));
+  h->h_logdet = reinterpret_cast<double*>(h->h_words + 16);
+  h->h_norms = h->h_logdet + 4;
+  CUCHOL_CHECK(dev_malloc(&h->d_result, sizeof(double)));
   CUCHOL_CHECK(dev_malloc(&h->d_logdet_f, 4 * sizeof(float)));
-  CUCHOL_CHECK(cudaMallocHost(&h->h_logdet, 4 * sizeof(double)));
   CUCHOL_CHECK(dev_malloc(&h->d_part, kLogdetMaxBlocks * sizeof(double)));
   CUCHOL_CHECK(dev_malloc(&h->d_counter, sizeof(unsigned int)));
   CUCHOL_CHECK(cudaMemset(h->d_counter, 0, sizeof(unsigned int)));

@@ -87,37 +87,29 @@ __global__ void build_kernel(const double* __restrict__ a, long long rs, long lo
 
 // Inverse of the 64 x 64 diagonal blocks of a lower-triangular L (logical view
 // L(i, j) = L[i*rs + j*cs]); DI[b] is column-major 64 x 64 with zeros above the
-// diagonal.  Rows past n of the last block are given a unit diagonal.  One CTA per
-// block, one thread per column of the inverse (forward substitution).
+// diagonal.  Rows past n of the last block are given a unit diagonal.  One CTA per block,
+// in shared memory in 16-wide steps (block.cuh).  (A thread per column with a division
+// per row: 53 us FP64.)
 template <typename T>
-__global__ void __launch_bounds__(BS) block_inverse_kernel(const T* __restrict__ L, long long rs, long long cs,
-                                                           int n, T* __restrict__ DI) {
+__global__ void __launch_bounds__(kThreads) block_inverse_kernel(const T* __restrict__ L, long long rs, long long cs,
+                                                                 int n, T* __restrict__ DI) {
+  using BM = BlockSmem<T, BS>;
+  constexpr int LD = FactorSmem<T, BS>::LD;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Ls = reinterpret_cast<T*>(smem_raw);   // [BS][BS + 1], row-major
-  T* X = Ls + BS * (BS + 1);                // [BS][BS + 1]
+  T* S = reinterpret_cast<T*>(smem_raw);
+  T* rd = reinterpret_cast<T*>(smem_raw + BM::F);
+  T* TMP = reinterpret_cast<T*>(smem_raw + BM::F + BM::RD);
   const int b = blockIdx.x, i0 = b * BS, t = threadIdx.x;
-  const bool row_contig = (rs == 1);
-  for (int e = t; e < BS * BS; e += BS) {
-    const int i = row_contig ? (e % BS) : (e / BS), j = row_contig ? (e / BS) : (e % BS);
-    T v = T(0);
-    if (i0 + i < n && i >= j) v = L[(long long)(i0 + i) * rs + (long long)(i0 + j) * cs];
-    if (i0 + i >= n && i == j) v = T(1);
-    Ls[i * (BS + 1) + j] = v;
-  }
+  load_lower<T, T, BS, kThreads>(S, L + (long long)i0 * (rs + cs), rs, cs, min(BS, n - i0), BS);
+  cp_async_wait_all();
   __syncthreads();
-  const int c = t;   // column of the inverse
-  for (int i = 0; i < BS; ++i) {
-    T x = T(0);
-    if (i >= c) {
-      T acc = (i == c) ? T(1) : T(0);
-      for (int k = c; k < i; ++k) acc -= Ls[i * (BS + 1) + k] * X[k * (BS + 1) + c];
-      x = acc / Ls[i * (BS + 1) + i];
-    }
-    X[i * (BS + 1) + c] = x;
-  }
-  __syncthreads();
+  if (t < BS) rd[t] = T(1) / S[t * LD + t];
+  invert_block<T, BS, kThreads>(S, BS, rd, TMP);
   T* out = DI + (size_t)b * BS * BS;
-  for (int e = t; e < BS * BS; e += BS) out[e] = X[(e % BS) * (BS + 1) + e / BS];
+  for (int e = t; e < BS * BS; e += kThreads) {
+    const int r = e % BS, c = e / BS;
+    out[e] = (r >= c) ? S[c * LD + r] : T(0);
+  }
 }
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -957,14 +949,14 @@ constexpr size_t kSymvSmem = kSymvSmemBytes;
 
 template <typename T>
 CUresult block_inverse(const T* L, long long rs, long long cs, int n, T* DI, cudaStream_t s) {
-  const size_t smem = 2 * sizeof(T) * BS * (BS + 1);
+  const size_t smem = BlockSmem<T, BS>::bytes;
   static bool attr = false;
   if (!attr) {
     CUCHOL_CHECK(cudaFuncSetAttribute(block_inverse_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     attr = true;
   }
-  block_inverse_kernel<T><<<(n + BS - 1) / BS, BS, smem, s>>>(L, rs, cs, n, DI);
+  block_inverse_kernel<T><<<(n + BS - 1) / BS, kThreads, smem, s>>>(L, rs, cs, n, DI);
   CUCHOL_CHECK(cudaGetLastError());
   return CUDA_SUCCESS;
 }
@@ -1136,11 +1128,7 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
   CUCHOL_CHECK_CU(ensure_workspace(h, 2 * qbytes));
   char* ws = static_cast<char*>(h->ws);
   Op* Q[2] = {reinterpret_cast<Op*>(ws), reinterpret_cast<Op*>(ws + qbytes)};
-  CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
-  CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
-  CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
-  CUCHOL_CHECK(cudaStreamWaitEvent(su, h->ev_panel, 0));
-  CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
+  CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));   // (the update stream starts behind a panel event)
   auto at = [&](long long i, long long j) { return W + i + j * ldw; };
 
   for (int j = 0, step = 0; j < n; j += OB, ++step) {
@@ -1150,7 +1138,7 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
     const int q_rows = n - j - SB;   // P / Q row r = global row j + SB + r
     for (int s0 = 0; s0 < jB; s0 += SB) {
       const int c = j + s0, jb = std::min(SB, j + jB - c), mr = n - c - jb;
-      CUCHOL_CHECK_CU((diag_factor<double, float, SB>(h, at(c, c), 1, ldw, jb, c, h->d_logdet, sp)));
+      CUCHOL_CHECK_CU((diag_factor<double, float, SB>(h, at(c, c), 1, ldw, jb, c, c == 0, h->d_logdet, sp)));
       if (mr == 0) break;
       // panel rows c + jb .. n-1 solved in place; they are Q rows s0 .., columns s0 ..
       Op* Qs = Qj + (long long)s0 * ldq + s0;
@@ -1176,9 +1164,7 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
   }
   CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
   CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, d_info, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-  CUCHOL_CHECK(cudaStreamSynchronize(sp));
-  CUCHOL_CHECK_CU(check_engine(h));
+  CUCHOL_CHECK_CU(fetch_words(h, sp));
   *info = h->h_words[0];
   return CUDA_SUCCESS;
 }
@@ -1461,9 +1447,7 @@ CUresult potrs_run(CULAPACKhandle h, bool upper, int n, int nrhs, const T* A, lo
     CUCHOL_CHECK(cudaGetLastError());
     h->launches += 2;
   }
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, h->d_words, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  CUCHOL_CHECK(cudaStreamSynchronize(s));
-  return check_engine(h);
+  return fetch_words(h, s);
 }
 
 }  // namespace mx

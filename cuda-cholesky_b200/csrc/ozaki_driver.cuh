@@ -70,11 +70,7 @@ CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long lo
   int* ebuf[2] = {reinterpret_cast<int*>(ws + pbytes + 2 * sbytes),
                   reinterpret_cast<int*>(ws + pbytes + 2 * sbytes + ebytes)};
 
-  CUCHOL_CHECK(cudaMemsetAsync(d_info, 0, sizeof(int), sp));
-  CUCHOL_CHECK(cudaMemsetAsync(h->d_logdet, 0, sizeof(double), sp));
-  CUCHOL_CHECK(cudaEventRecord(h->ev_panel, sp));
-  CUCHOL_CHECK(cudaStreamWaitEvent(su, h->ev_panel, 0));
-  CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
+  CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));   // (the update stream starts behind a panel event)
 
   for (int j = 0, step = 0; j < n; j += NB, ++step) {
     const int jB = std::min(NB, n - j);
@@ -83,7 +79,7 @@ CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long lo
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;
-      CUCHOL_CHECK_CU((diag_factor<double, double, nb>(h, at(c, c), rs, cs, jb, c, h->d_logdet, sp)));
+      CUCHOL_CHECK_CU((diag_factor<double, double, nb>(h, at(c, c), rs, cs, jb, c, c == 0, h->d_logdet, sp)));
       if (mr == 0) break;
       double* Ps = P + s0 + (long long)s0 * ldp;   // P(r, .) = rows from j + nb
       CUCHOL_CHECK_CU((panel_solve<double, double, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Ps, 1, ldp,
@@ -119,9 +115,7 @@ CUresult potrf_ozaki_run(CULAPACKhandle h, bool upper, int n, double* A, long lo
   }
   CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
   CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
-  CUCHOL_CHECK(cudaMemcpyAsync(h->h_words, d_info, 4 * sizeof(int), cudaMemcpyDeviceToHost, sp));
-  CUCHOL_CHECK(cudaStreamSynchronize(sp));
-  CUCHOL_CHECK_CU(check_engine(h));
+  CUCHOL_CHECK_CU(fetch_words(h, sp));
   *info = h->h_words[0];
   return CUDA_SUCCESS;
 }

@@ -19,28 +19,53 @@
 namespace cuchol {
 
 // Lower part of the logical block A(r, c) (strides rs, cs) -> S (column-major, ld LD),
-// order jb padded to n16 with the identity.
-template <typename T, typename TA, int LD, int NT>
+// order jb padded to n16 with the identity.  Index arithmetic with compile-time extents
+// and several copies in flight per thread: with a loop per column this load took as long
+// as 60 pivots.  Aligned columns come in 16-byte pieces (the first piece of a column may
+// bring elements from above the diagonal along, which nothing reads).
+template <typename T, typename TA, int NB, int NT>
 __device__ __forceinline__ void load_lower(T* S, const TA* __restrict__ A, long long rs, long long cs, int jb, int n16) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto put = [&](int r, int c) {
-    const bool v = r < jb && c < jb;
-    if constexpr (std::is_same<T, TA>::value) {
-      if (v || r != c) cp_async_elem<T>(&S[c * LD + r], v ? A + r * rs + c * cs : A, v);
-      else S[c * LD + r] = from_real<T>(RealOf<T>(1));
-    } else {
-      S[c * LD + r] = v ? (T)A[r * rs + c * cs] : T(r == c ? 1 : 0);
+  constexpr int LD = FactorSmem<T, NB>::LD;
+  const int t = threadIdx.x;
+  // the identity past jb
+  for (int e = t; e < n16 * (n16 - jb); e += NT) {
+    const int r = jb + e / n16, c = e % n16;
+    if (r >= c) S[c * LD + r] = from_real<T>(RealOf<T>(r == c ? 1 : 0));
+  }
+  if constexpr (std::is_same<T, TA>::value) {
+    constexpr int V = 16 / sizeof(T);
+    if (V > 1 && rs == 1 && aligned16(A, cs * (long long)sizeof(T))) {
+      constexpr int PC = NB / V;                 // pieces of a column
+#pragma unroll 8
+      for (int u = 0; u < NB * PC / NT; ++u) {
+        const int e = t + u * NT, r = (e % PC) * V, c = e / PC;
+        if (r + V > c && r < jb && c < jb) {
+          // a piece that crosses jb would overwrite the identity's zeros with zeros
+          cp_async_piece(&S[c * LD + r], A + r + c * cs, min(16, (jb - r) * (int)sizeof(T)));
+        }
+      }
+      return;
     }
-  };
-  if (rs == 1) {               // rows contiguous: a warp per column
-    for (int c = warp; c < n16; c += NT / 32)
-      for (int r = (c & ~31) + lane; r < n16; r += 32)
-        if (r >= c) put(r, c);
-  } else {                     // columns contiguous: 4 rows x 8 columns per warp and step
-    const int dr = lane >> 3, dc = lane & 7;
-    for (int r0 = 4 * warp; r0 < n16; r0 += 4 * (NT / 32))
-      for (int c0 = 0; c0 <= r0 + 3; c0 += 8)
-        if (r0 + dr >= c0 + dc) put(r0 + dr, c0 + dc);
+    if (rs == 1) {
+#pragma unroll 8
+      for (int u = 0; u < NB * NB / NT; ++u) {
+        const int e = t + u * NT, r = e % NB, c = e / NB;
+        if (r >= c && r < jb) cp_async_elem<T>(&S[c * LD + r], A + r + c * cs, true);
+      }
+    } else {
+      // columns contiguous: a warp takes 8 columns of 4 rows (64-byte pieces of rows)
+#pragma unroll 8
+      for (int u = 0; u < NB * NB / NT; ++u) {
+        const int e = t + u * NT, c = (e & 7) + 8 * ((e >> 5) % (NB / 8)), r = ((e >> 3) & 3) + 4 * (e / (4 * NB));
+        if (r >= c && r < jb) cp_async_elem<T>(&S[c * LD + r], A + r * rs + c * cs, true);
+      }
+    }
+  } else {
+#pragma unroll 8
+    for (int u = 0; u < NB * NB / NT; ++u) {
+      const int e = t + u * NT, r = e % NB, c = e / NB;
+      if (r >= c && r < jb) S[c * LD + r] = (T)A[r * rs + c * cs];
+    }
   }
 }
 
@@ -59,7 +84,7 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
   __shared__ int s_fail;
   __shared__ double s_log[NT / 32];
   const int tid = threadIdx.x, n16 = (jb + kSub - 1) & ~(kSub - 1);
-  load_lower<T, TA, LD, NT>(S, A, rs, cs, jb, n16);
+  load_lower<T, TA, NB, NT>(S, A, rs, cs, jb, n16);
   if (tid == 0) s_fail = -1;
   cp_async_wait_all();
   factor_block<T, NB, NT>(S, Ld, rd, n16, &s_fail, [&](int c0, int t, int nt) {
@@ -101,9 +126,16 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
 // double 52 -> .
 template <typename T, typename TA, int NB, int NT>
 __global__ void __launch_bounds__(NT)
-diag_factor_kernel(TA* __restrict__ A, long long rs, long long cs, int jb, long long info_base,
+diag_factor_kernel(TA* __restrict__ A, long long rs, long long cs, int jb, long long info_base, int first,
                    int* __restrict__ d_info, double* __restrict__ logdet) {
-  if (cta_aborted(d_info)) return;   // an earlier block already failed
+  if (first) {                       // starts the words: no launch of its own clears them
+    if (threadIdx.x == 0) {
+      *d_info = 0;
+      *logdet = 0.0;
+    }
+  } else if (cta_aborted(d_info)) {
+    return;                          // an earlier block already failed
+  }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   factor_diag<T, TA, NB, NT>(smem_raw, A, rs, cs, jb, info_base, d_info, logdet);
 }
@@ -190,7 +222,7 @@ __device__ __forceinline__ void diag_invert_block(T* __restrict__ B, long long r
   T* rd = reinterpret_cast<T*>(smem_raw + BlockSmem<T, NB>::F);
   T* TMP = reinterpret_cast<T*>(smem_raw + BlockSmem<T, NB>::F + BlockSmem<T, NB>::RD);
   const int n16 = (jb + kSub - 1) & ~(kSub - 1);
-  load_lower<T, T, LD, NT>(S, B, rs, cs, jb, n16);
+  load_lower<T, T, NB, NT>(S, B, rs, cs, jb, n16);
   cp_async_wait_all();
   __syncthreads();
   for (int i = threadIdx.x; i < n16; i += NT) rd[i] = unit ? from_real<T>(RealOf<T>(1)) : recip(S[i * LD + i]);

@@ -36,7 +36,7 @@ template <typename T, int NB, int R>
 struct SolveSmem {
   static constexpr bool dmma = std::is_same<T, double>::value;
   static constexpr int NP = NB / kSub;
-  static constexpr int LDX = R + (dmma ? kLdPad : 1);
+  static constexpr int LDX = R + kLdPad;
   static constexpr size_t X = (sizeof(T) * NB * LDX + 15) / 16 * 16;
   // strip p: rows 16(p+1) .. NB-1, ld = NB - 16(p+1) + kLdPad, 16 columns
   __host__ __device__ static constexpr int strip_ld(int p) { return NB - kSub * (p + 1) + kLdPad; }
@@ -78,42 +78,81 @@ __global__ void __launch_bounds__(256)
   const long long row0 = (long long)blockIdx.x * R;
   const int rows = min((long long)R, m - row0);
 
-  // Everything comes in with cp.async, a warp walking its columns (or rows) with one
-  // pointer: no index divisions, and no load waits for another.
-  if (brs == 1) {                                // row tile: a warp per column
-    for (int c = warp; c < n16; c += NT / 32) {
-      const T* src = B + row0 + (long long)c * bcs;
-#pragma unroll
-      for (int r = lane; r < R; r += 32) {
-        const bool v = r < rows && c < jb;
-        cp_async_elem<T>(&Xs[c * LDX + r], v ? src + r : B, v);
-      }
+  RealOf<T> dl = RealOf<T>(1);
+  if (t < jb) dl = re(L[(long long)t * (lrs + lcs)]);
+  // Everything else comes in with cp.async, several copies in flight per thread and in
+  // 16-byte pieces where the storage allows (columns contiguous in memory and aligned).
+  constexpr int V = 16 / sizeof(T);
+  if (V > 1 && brs == 1 && aligned16(B, bcs * (long long)sizeof(T))) {
+    constexpr int PC = R / V;                    // pieces of a column of the row tile
+#pragma unroll 4
+    for (int e = t; e < n16 * PC; e += NT) {
+      const int r = (e % PC) * V, c = e / PC;
+      const int bytes = (c < jb) ? max(0, min(16, (rows - r) * (int)sizeof(T))) : 0;
+      cp_async_piece(&Xs[c * LDX + r], bytes ? B + row0 + r + (long long)c * bcs : B, bytes);
+    }
+  } else if (brs == 1) {
+#pragma unroll 4
+    for (int e = t; e < n16 * R; e += NT) {
+      const int r = e % R, c = e / R;
+      const bool v = r < rows && c < jb;
+      cp_async_elem<T>(&Xs[c * LDX + r], v ? B + row0 + r + (long long)c * bcs : B, v);
     }
   } else {                                       // 4 rows x 8 columns per warp and step
     const int dr = lane >> 3, dc = lane & 7;
     for (int r = 4 * warp + dr; r < R; r += 4 * (NT / 32)) {
       const T* src = B + (row0 + r) * brs;
+#pragma unroll 4
       for (int c = dc; c < n16; c += 8) {
         const bool v = r < rows && c < jb;
         cp_async_elem<T>(&Xs[c * LDX + r], v ? src + (long long)c * bcs : B, v);
       }
     }
   }
-  // the diagonal 16 x 16 blocks: column j at Ld[16 j], row i of its block
-  for (int e = t; e < n16 * kSub; e += NT) {
-    const int j = e / kSub, i = (j & ~(kSub - 1)) + (e & (kSub - 1));
-    const bool v = i > j && i < jb;
-    cp_async_elem<T>(&Ld[e], v ? L + (long long)i * lrs + (long long)j * lcs : L, v);
+  const bool lvec = V > 1 && lrs == 1 && aligned16(L, lcs * (long long)sizeof(T));
+  // the diagonal 16 x 16 blocks: column j at Ld[16 j], row i of its block (on and above
+  // the diagonal nothing reads)
+  if (lvec) {
+    constexpr int PC = kSub / V;
+#pragma unroll 4
+    for (int e = t; e < n16 * PC; e += NT) {
+      const int j = e / PC, i = (j & ~(kSub - 1)) + (e % PC) * V;
+      const int bytes = (j < jb) ? max(0, min(16, (jb - i) * (int)sizeof(T))) : 0;
+      cp_async_piece(&Ld[e * V], bytes ? L + i + (long long)j * lcs : L, bytes);
+    }
+  } else {
+#pragma unroll 4
+    for (int e = t; e < n16 * kSub; e += NT) {
+      const int j = e / kSub, i = (j & ~(kSub - 1)) + (e & (kSub - 1));
+      const bool v = i > j && i < jb;
+      cp_async_elem<T>(&Ld[e], v ? L + (long long)i * lrs + (long long)j * lcs : L, v);
+    }
   }
-  // the strips of L below them
-  if (lrs == 1) {
+  // the strips of L below them: row r0 = 16 (p + 1) on of column j in strip p
+  if (lvec) {
+#pragma unroll 2
     for (int j = warp; j < n16 - kSub; j += NT / 32) {
-      const int r0 = (j & ~(kSub - 1)) + kSub, p = j / kSub;
+      const int p = j / kSub, r0 = kSub * (p + 1);
       T* S = Ls + SM::strip_off(p) + (j & (kSub - 1)) * SM::strip_ld(p) - r0;
       const T* src = L + (long long)j * lcs;
-      for (int r = r0 + lane; r < n16; r += 32) {
-        const bool v = r < jb;
-        cp_async_elem<T>(&S[r], v ? src + r : L, v);
+#pragma unroll
+      for (int u = 0; u < (NB / V + 31) / 32; ++u) {
+        const int r = r0 + (lane + 32 * u) * V;
+        if (r < n16) {
+          const int bytes = max(0, min(16, (jb - r) * (int)sizeof(T)));
+          cp_async_piece(&S[r], bytes ? src + r : L, bytes);
+        }
+      }
+    }
+  } else if (lrs == 1) {
+    for (int j = warp; j < n16 - kSub; j += NT / 32) {
+      const int p = j / kSub, r0 = kSub * (p + 1);
+      T* S = Ls + SM::strip_off(p) + (j & (kSub - 1)) * SM::strip_ld(p) - r0;
+      const T* src = L + (long long)j * lcs;
+#pragma unroll
+      for (int u = 0; u < NB / 32; ++u) {
+        const int r = r0 + lane + 32 * u;
+        if (r < n16) cp_async_elem<T>(&S[r], r < jb ? src + r : L, r < jb);
       }
     }
   } else {
@@ -121,6 +160,7 @@ __global__ void __launch_bounds__(256)
     for (int r = kSub + 4 * warp + dr; r < n16; r += 4 * (NT / 32)) {
       const T* src = L + (long long)r * lrs;
       const int ce = r & ~(kSub - 1);
+#pragma unroll 4
       for (int j = dc; j < ce; j += 8) {
         const int p = j / kSub;
         const bool v = r < jb;
@@ -129,7 +169,7 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
-  if (t < n16) rd[t] = (t < jb) ? RealOf<T>(1) / re(L[(long long)t * (lrs + lcs)]) : RealOf<T>(0);
+  if (t < n16) rd[t] = (t < jb) ? RealOf<T>(1) / dl : RealOf<T>(0);
   cp_async_wait_all();
   __syncthreads();
 
@@ -163,16 +203,12 @@ __global__ void __launch_bounds__(256)
         for (int r = lane; r < R; r += 32)
           if (r < rows) dst[r] = conv(Xs[c * LDX + r]);
       }
-    } else if (SM::dmma) {
+    } else {                                     // 4 rows x 8 columns per warp and step
       const int dr = lane >> 3, dc = lane & 7;
       for (int r = 4 * warp + dr; r < rows; r += 4 * (NT / 32)) {
         auto* dst = out + (row0 + r) * rs_;
+#pragma unroll 4
         for (int c = dc; c < jb; c += 8) dst[(long long)c * cs_] = conv(Xs[c * LDX + r]);
-      }
-    } else {
-      for (int r = warp; r < rows; r += NT / 32) {
-        auto* dst = out + (row0 + r) * rs_;
-        for (int c = lane; c < jb; c += 32) dst[(long long)c * cs_] = conv(Xs[c * LDX + r]);
       }
     }
   };
@@ -181,8 +217,8 @@ __global__ void __launch_bounds__(256)
     put(out2, o_rs, o_cs, [](T v) { return to_op<O2>((float)v); });
   } else if constexpr (MODE == OUT_SPLIT && Traits<T>::complex) {
     // two rows of the split per row: (re, im) and (-im, re); o_rs floats per row of the split
-    for (int r = warp; r < rows; r += NT / 32)
-    for (int c = lane; c < jb; c += 32) {
+    for (int r = 4 * warp + (lane >> 3); r < rows; r += 4 * (NT / 32))
+    for (int c = lane & 7; c < jb; c += 8) {
       const T v = Xs[c * LDX + r];
       const float re = (float)v.x, im = (float)v.y, rh = round_tf32(re), ih = round_tf32(im);
       const float rl = round_tf32(re - rh), il = round_tf32(im - ih);
