@@ -305,7 +305,8 @@ __device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, 
     T acc[4][4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) load4(C + (4 * lc + v) * ldc + 4 * lr, acc[v]);
-#pragma unroll 4
+    constexpr int U = sizeof(T) == 4 ? 16 : sizeof(T) == 8 ? 4 : 2;   // operand loads in flight
+#pragma unroll U
     for (int k = 0; k < kSub; ++k) {
       T a[4], b[4];
       load4(P + k * ldp + 4 * lr, a);
@@ -359,17 +360,19 @@ __device__ __forceinline__ void strip_update(T* C, int ldc, const T* P, int ldp,
   }
 }
 
-// Shared memory of the factor of one block of order up to NB.
-template <typename T, int NB>
+// Shared memory of the factor of one block of order up to NB, with R more rows below it
+// that are solved along.
+template <typename T, int NB, int R = 0>
 struct FactorSmem {
-  static constexpr int LD = NB + kLdPad;
+  static constexpr int LD = NB + R + kLdPad;
   static constexpr size_t S = sizeof(T) * NB * LD;
   static constexpr size_t LDS = sizeof(T) * kSub * kSub;
   static constexpr size_t RD = sizeof(RealOf<T>) * NB;
   static constexpr size_t bytes = S + LDS + RD;
 };
 
-// Cholesky factor of the block in S (order n16, a multiple of 16 up to NB; lower part),
+// Cholesky factor of the block in S (order n16, a multiple of 16 up to NB; lower part) and
+// the solve of the rows below it (rows n16 .. nrow - 1; nrow a multiple of 16; none: n16),
 // by the whole CTA of NT threads, NT / 32 >= 2 warps.  rd[c] = 1 / L(c, c).  done(c0)
 // is called by the threads of warps 1 .. (t - 32 counts them) as soon as the columns
 // c0 .. c0 + 15 are final, and by all warps for the last ones, with (thread, threads).
@@ -379,15 +382,15 @@ struct FactorSmem {
 // Per sub-panel: warp 0 factors the diagonal 16 x 16 (and 16 rows below); one thread per
 // remaining row solves; the 32 x 16 elements warp 0 needs next are updated by all
 // threads; then warp 0 goes on while the other warps update the rest of the block.
-template <typename T, int NB, int NT, typename Done>
-__device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16, int* s_fail, Done done) {
-  constexpr int LD = FactorSmem<T, NB>::LD;
+template <typename T, int NB, int R, int NT, typename Done>
+__device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16, int nrow, int* s_fail, Done done) {
+  constexpr int LD = FactorSmem<T, NB, R>::LD;
   const int t = threadIdx.x, warp = t >> 5;
   __syncthreads();
   for (int c0 = 0; c0 < n16; c0 += kSub) {
     const int c1 = c0 + kSub;
     if (warp == 0) {
-      const int f = factor16<T>(S + c0 * LD + c0, LD, n16 - c0, Ld, rd + c0);
+      const int f = factor16<T>(S + c0 * LD + c0, LD, nrow - c0, Ld, rd + c0);
       if (t == 0 && f >= 0) *s_fail = c0 + f;
     } else if (c0 > 0) {
       // the rest of the update by the previous sub-panel: 32 x 16 tiles of the columns
@@ -395,16 +398,16 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
       const int cp = c0 - kSub;
       int w = warp - 1;
       for (int cb = c0; cb < n16; cb += kSub)
-        for (int rb = (cb == c0) ? c0 + kSubRows : cb; rb < n16; rb += 32) {
+        for (int rb = (cb == c0) ? c0 + kSubRows : cb; rb < nrow; rb += 32) {
           if (w == 0)
-            tile_update<T>(S + cb * LD + rb, LD, S + cp * LD + rb, LD, S + cp * LD + cb, LD, n16 - rb);
+            tile_update<T>(S + cb * LD + rb, LD, S + cp * LD + rb, LD, S + cp * LD + cb, LD, nrow - rb);
           w = (w == 0) ? NT / 32 - 2 : w - 1;
         }
       done(cp, t - 32, NT - 32);
     }
     __syncthreads();
     const int fail = *s_fail;
-    for (int r = c0 + kSubRows + t; r < n16; r += NT) {
+    for (int r = c0 + kSubRows + t; r < nrow; r += NT) {
       if (fail < 0) solve16<T>(S + c0 * LD + r, LD, Ld, rd + c0);
       else solve16_part<T>(S + c0 * LD + r, LD, Ld, rd + c0, fail - c0);
     }
@@ -414,7 +417,7 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
       break;
     }
     // the 32 x 16 elements the next factor16 works on
-    strip_update<T, kSubRows, NT>(S + c1 * LD + c1, LD, S + c0 * LD + c1, LD, S + c0 * LD + c1, LD, n16 - c1);
+    strip_update<T, kSubRows, NT>(S + c1 * LD + c1, LD, S + c0 * LD + c1, LD, S + c0 * LD + c1, LD, nrow - c1);
     __syncthreads();
   }
   __syncthreads();

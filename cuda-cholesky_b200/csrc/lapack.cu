@@ -495,16 +495,21 @@ CUresult set_smem(const void* fn, size_t bytes) {
 // ---- diagonal block and panel solve ------------------------------------------------
 constexpr int kDiagThreads2 = 256;
 
+// Threads of the diagonal kernel: the FP32 types' updates beside the pivots (4 x 4 outputs
+// per thread) are bound by the latency of their shared loads and gain from sixteen warps
+// (128 columns, complex 45 -> 41 us); FP64's run on DMMA and do not (33 against 37 us).
+template <typename T> constexpr int panel_threads() { return sizeof(RealOf<T>) == 4 ? 512 : 256; }
+
 // Factor of the jb x jb diagonal block at A (logical lower view), queued on s; T: the
 // computing type, TA: the storage type.  first: the factorization's first block, which
 // starts the info word and the log det.
 template <typename T, typename TA, int NB>
 CUresult diag_factor(CULAPACKhandle h, TA* A, long long rs, long long cs, int jb, long long info_base, bool first,
                      double* logdet, cudaStream_t s) {
-  constexpr int smem = (int)FactorSmem<T, NB>::bytes;
-  auto* kernel = diag_factor_kernel<T, TA, NB, kDiagThreads2>;
+  constexpr int smem = (int)FactorSmem<T, NB>::bytes, threads = panel_threads<T>();
+  auto* kernel = diag_factor_kernel<T, TA, NB, threads>;
   CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
-  kernel<<<1, kDiagThreads2, smem, s>>>(A, rs, cs, jb, info_base, first ? 1 : 0, h->d_words, logdet);
+  kernel<<<1, threads, smem, s>>>(A, rs, cs, jb, info_base, first ? 1 : 0, h->d_words, logdet);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
   return CUDA_SUCCESS;
@@ -524,6 +529,36 @@ CUresult panel_solve(CULAPACKhandle h, T* B, int m, int jb, const T* L, long lon
     attr = true;
   }
   kernel<<<(m + R - 1) / R, 256, smem, s>>>(B, rs, cs, m, jb, L, rs, cs, out2, o_rs, o_cs, h->d_words, out3);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
+// The diagonal block and the m rows below it in one launch (panel_kernel), queued on s.
+constexpr int kFusedRows = 32;
+template <typename T, typename O2, int MODE, int NB>
+CUresult panel_fused(CULAPACKhandle h, T* A, int m, long long rs, long long cs, O2* out2, long long o_rs, long long o_cs,
+                     O2* out3, T* D, long long info_base, bool first, double* logdet, cudaStream_t s) {
+  constexpr int R = kFusedRows, smem = (int)FactorSmem<T, NB, R>::bytes, threads = sizeof(T) == 16 ? 256 : 512;
+  auto* kernel = panel_kernel<T, O2, MODE, NB, R, threads>;
+  static bool attr = false;
+  if (!attr) {
+    CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
+    CUCHOL_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    attr = true;
+  }
+  kernel<<<(m + R - 1) / R, threads, smem, s>>>(A, rs, cs, m, out2, o_rs, o_cs, out3, D, info_base, first ? 1 : 0,
+                                                h->d_words, logdet);
+  ++h->launches;
+  CUCHOL_CHECK(cudaGetLastError());
+  return CUDA_SUCCESS;
+}
+
+// Blocks b0 .. b0 + count - 1 of the factors in D (whose slot 0 is block dfirst) to A.
+template <typename T, int NB>
+CUresult copy_diag(CULAPACKhandle h, const T* D, T* A, long long rs, long long cs, int dfirst, int b0, int count,
+                   cudaStream_t s) {
+  copy_diag_kernel<T, NB><<<count, 256, 0, s>>>(D, dfirst, A, rs, cs, b0, h->d_words);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
   return CUDA_SUCCESS;
@@ -759,8 +794,14 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   const bool tc3_tma = tc3 && n % 4 == 0 && tc3_usable(reinterpret_cast<const float*>(A), lda);
   const long long ldq = (long long)round_up((size_t)NB, 32) * cx;
   const size_t qsize = (size_t)n * cx * ldq;   // floats of one buffer
-  const size_t ws = tc3 ? sizeof(float) * 4 * qsize : sizeof(T) * (2 * (size_t)ldp * NB);
-  CUCHOL_CHECK_CU(ensure_workspace(h, ws));
+  const size_t ws = round_up(tc3 ? sizeof(float) * 4 * qsize : sizeof(T) * (2 * (size_t)ldp * NB), 256);
+  // one launch per diagonal block and its rows while those fill at most one CTA per SM;
+  // its factors wait in D
+  const int fused_rows = kFusedRows * h->num_sms;
+  const size_t dblocks = (size_t)(std::min(n, fused_rows + nb) / nb + 1);
+  CUCHOL_CHECK_CU(ensure_workspace(h, ws + sizeof(T) * dblocks * nb * nb));
+  int dfirst = -1, dnext = -1;   // diagonal blocks whose factors are in D (block b in slot b - dfirst)
+  T* dbuf = reinterpret_cast<T*>(static_cast<char*>(h->ws) + ws);
   T* pbuf[2] = {static_cast<T*>(h->ws), static_cast<T*>(h->ws) + (size_t)ldp * NB};
   float* qbuf[4];
   for (int i = 0; i < 4; ++i) qbuf[i] = static_cast<float*>(h->ws) + i * qsize;
@@ -803,7 +844,28 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;                 // rows below this diagonal block
-      CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, c == 0, h->d_logdet, sp)));
+      const bool fused = jb == nb && mr > 0 && mr <= fused_rows;
+      if (fused) {
+        if (dfirst < 0) dfirst = c / nb;
+        dnext = c / nb + 1;
+        T* D = dbuf + (size_t)(c / nb - dfirst) * nb * nb;
+        if constexpr (is_fp32<T>()) {
+          if (tc3) {
+            const long long qo = (long long)s0 * cx * ldq + s0 * cx;
+            CUCHOL_CHECK_CU((panel_fused<T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
+                                                                  c == 0, h->d_logdet, sp)));
+          }
+        }
+        if (!tc3)
+          CUCHOL_CHECK_CU((panel_fused<T, T, OUT_COPY, nb>(h, at(c, c), mr, rs, cs, P + s0 + (long long)s0 * ldp, 1, ldp,
+                                                           nullptr, D, c, c == 0, h->d_logdet, sp)));
+        if (on_final) {              // the block column goes to the caller now
+          CUCHOL_CHECK_CU((copy_diag<T, nb>(h, dbuf, A, rs, cs, dfirst, c / nb, 1, sp)));
+          dfirst = -1;
+        }
+      } else {
+        CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, c == 0, h->d_logdet, sp)));
+      }
       if (mr == 0) {
         if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
         break;
@@ -811,7 +873,8 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
       // panel solve into P: rows c + jb .. n-1 are P rows s0 .. (P starts at j + nb)
       // row-parallel triangular solve: A21 := A21 L11^-H in place, and into P (or its
       // hi / lo split into Q)
-      if (tc3) {
+      if (fused) {
+      } else if (tc3) {
         if constexpr (is_fp32<T>()) {
           const long long qo = (long long)s0 * cx * ldq + s0 * cx;
           CUCHOL_CHECK_CU((panel_solve<T, float, OUT_SPLIT, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Qh + qo, ldq,
@@ -851,6 +914,7 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
     CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
   }
+  if (dfirst >= 0) CUCHOL_CHECK_CU((copy_diag<T, nb>(h, dbuf, A, rs, cs, dfirst, dfirst, dnext - dfirst, sp)));
   CUCHOL_CHECK_CU(fetch_words(h, sp));
   *info = h->h_words[0];
   if (logdet_out != nullptr) *logdet_out = h->h_logdet[0];

@@ -23,9 +23,8 @@ namespace cuchol {
 // and several copies in flight per thread: with a loop per column this load took as long
 // as 60 pivots.  Aligned columns come in 16-byte pieces (the first piece of a column may
 // bring elements from above the diagonal along, which nothing reads).
-template <typename T, typename TA, int NB, int NT>
+template <typename T, typename TA, int NB, int NT, int LD = FactorSmem<T, NB>::LD>
 __device__ __forceinline__ void load_lower(T* S, const TA* __restrict__ A, long long rs, long long cs, int jb, int n16) {
-  constexpr int LD = FactorSmem<T, NB>::LD;
   const int t = threadIdx.x;
   // the identity past jb
   for (int e = t; e < n16 * (n16 - jb); e += NT) {
@@ -69,6 +68,21 @@ __device__ __forceinline__ void load_lower(T* S, const TA* __restrict__ A, long 
   }
 }
 
+// *logdet += 2 sum log L(j,j) of the factored block, one column per thread, reduced in a
+// fixed order (deterministic).
+template <typename T, int NB, int LD>
+__device__ __forceinline__ void add_logdet(const T* S, int jb, double* s_log, double* __restrict__ logdet) {
+  const int tid = threadIdx.x;
+  double s = (tid < jb) ? log((double)re(S[tid * LD + tid])) : 0.0;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((tid & 31) == 0) s_log[tid >> 5] = s;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < (NB + 31) / 32; ++w) s += s_log[w];
+    *logdet += 2.0 * s;
+  }
+}
+
 // Cholesky factor of one jb x jb diagonal block, jb <= NB, in place, by the whole CTA;
 // T: computing type, TA: storage type; smem: FactorSmem<T, NB>::bytes, which keep the
 // factor (S) and the reciprocal pivots.  On failure at local column k: *d_info =
@@ -87,7 +101,7 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
   load_lower<T, TA, NB, NT>(S, A, rs, cs, jb, n16);
   if (tid == 0) s_fail = -1;
   cp_async_wait_all();
-  factor_block<T, NB, NT>(S, Ld, rd, n16, &s_fail, [&](int c0, int t, int nt) {
+  factor_block<T, NB, 0, NT>(S, Ld, rd, n16, n16, &s_fail, [&](int c0, int t, int nt) {
     // columns c0 .. c0 + 15 of the factor back to A
     const int rows = jb - c0;
     if (rs == 1) {
@@ -107,17 +121,7 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
     if (tid == 0) atomicCAS(d_info, 0, (int)(info_base + s_fail + 1));
     return false;
   }
-  if (logdet != nullptr) {
-    // 2 sum log L(j,j), one column per thread, reduced in a fixed order (deterministic)
-    double s = (tid < jb) ? log((double)re(S[tid * LD + tid])) : 0.0;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((tid & 31) == 0) s_log[tid >> 5] = s;
-    __syncthreads();
-    if (tid == 0) {
-      for (int w = 1; w < (NB + 31) / 32; ++w) s += s_log[w];
-      *logdet += 2.0 * s;
-    }
-  }
+  if (logdet != nullptr) add_logdet<T, NB, LD>(S, jb, s_log, logdet);
   return true;
 }
 

@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include "block.cuh"
+#include "panel.cuh"
 #include "scalar.cuh"
 
 namespace cuchol {
@@ -28,6 +29,17 @@ enum : int {
   OUT_SPLIT = 2,     // out2 = hi = tf32(X), out3 = lo = tf32(X - hi): X = hi + lo to 2^-22
                      // (complex: the two-row form of tcgemm.cuh)
 };
+
+// A complex value into the two-row split: (re, im) at o and (-im, re) one row further.
+template <typename T>
+__device__ __forceinline__ void put_split(T v, float* hi, float* lo, long long o, long long row) {
+  const float re = (float)v.x, im = (float)v.y, rh = round_tf32(re), ih = round_tf32(im);
+  const float rl = round_tf32(re - rh), il = round_tf32(im - ih);
+  *reinterpret_cast<float2*>(hi + o) = make_float2(rh, ih);
+  *reinterpret_cast<float2*>(hi + o + row) = make_float2(-ih, rh);
+  *reinterpret_cast<float2*>(lo + o) = make_float2(rl, il);
+  *reinterpret_cast<float2*>(lo + o + row) = make_float2(-il, rl);
+}
 
 // Shared memory of the panel solve of R rows: the row tile Xs (column-major), the parts
 // of L below its 16 x 16 diagonal blocks (one column-major strip per sub-panel, from the
@@ -219,14 +231,7 @@ __global__ void __launch_bounds__(256)
     // two rows of the split per row: (re, im) and (-im, re); o_rs floats per row of the split
     for (int r = 4 * warp + (lane >> 3); r < rows; r += 4 * (NT / 32))
     for (int c = lane & 7; c < jb; c += 8) {
-      const T v = Xs[c * LDX + r];
-      const float re = (float)v.x, im = (float)v.y, rh = round_tf32(re), ih = round_tf32(im);
-      const float rl = round_tf32(re - rh), il = round_tf32(im - ih);
-      const long long o = 2 * (row0 + r) * o_rs + 2 * c;
-      *reinterpret_cast<float2*>(out2 + o) = make_float2(rh, ih);
-      *reinterpret_cast<float2*>(out2 + o + o_rs) = make_float2(-ih, rh);
-      *reinterpret_cast<float2*>(out3 + o) = make_float2(rl, il);
-      *reinterpret_cast<float2*>(out3 + o + o_rs) = make_float2(-il, rl);
+      put_split(Xs[c * LDX + r], out2, out3, 2 * (row0 + r) * o_rs + 2 * c, o_rs);
     }
   } else if constexpr (MODE == OUT_SPLIT) {
     put(out2, o_rs, o_cs, [](T v) { return round_tf32((float)v); });
@@ -236,6 +241,117 @@ __global__ void __launch_bounds__(256)
     });
   } else {
     put(out2, o_rs, o_cs, [](T v) { return v; });
+  }
+}
+
+// The diagonal block and the rows below it in one launch, for panels of few rows: every
+// CTA factors the NB x NB block for itself, with R of the m rows below it as R more rows of
+// its sub-panels, so the rows are solved in the shadow of the pivots and the step has one
+// launch instead of two and no pass of the factor through memory.  The block in A must stay
+// as it is while CTAs still load it: CTA 0 writes the factor to D (column-major, ld NB),
+// and copy_diag_kernel takes it to A later.  Outputs for the rows as trsm_rows_kernel.
+// Worth it while the CTAs fit the GPU at once (each is as long as the factor).
+template <typename T, typename O2, int MODE, int NB, int R, int NT>
+__global__ void __launch_bounds__(NT)
+    panel_kernel(T* __restrict__ A, long long rs, long long cs, int m, O2* __restrict__ out2, long long o_rs,
+                 long long o_cs, O2* __restrict__ out3, T* __restrict__ D, long long info_base, int first,
+                 int* __restrict__ d_info, double* __restrict__ logdet) {
+  using F = FactorSmem<T, NB, R>;
+  constexpr int LD = F::LD, V = 16 / sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* S = reinterpret_cast<T*>(smem_raw);
+  T* Ld = reinterpret_cast<T*>(smem_raw + F::S);
+  RealOf<T>* rd = reinterpret_cast<RealOf<T>*>(smem_raw + F::S + F::LDS);
+  __shared__ int s_fail;
+  __shared__ double s_log[NT / 32];
+  const int t = threadIdx.x;
+  if (first) {                       // starts the words; the other CTAs do not read them
+    if (blockIdx.x == 0 && t == 0) {
+      *d_info = 0;
+      *logdet = 0.0;
+    }
+  } else if (cta_aborted(d_info)) {
+    return;
+  }
+  const long long row0 = (long long)blockIdx.x * R;
+  const int rows = min((long long)R, m - row0);
+  T* B = A + NB * rs;                // the rows below the block
+  load_lower<T, T, NB, NT, LD>(S, A, rs, cs, NB, NB);
+  if (V > 1 && rs == 1 && aligned16(B, cs * (long long)sizeof(T))) {
+    constexpr int PC = R / V;
+#pragma unroll 4
+    for (int u = 0; u < NB * PC / NT; ++u) {
+      const int e = t + u * NT, r = (e % PC) * V, c = e / PC;
+      const int bytes = max(0, min(16, (rows - r) * (int)sizeof(T)));
+      cp_async_piece(&S[c * LD + NB + r], bytes ? B + row0 + r + (long long)c * cs : B, bytes);
+    }
+  } else if (rs == 1) {
+#pragma unroll 4
+    for (int u = 0; u < NB * R / NT; ++u) {
+      const int e = t + u * NT, r = e % R, c = e / R;
+      cp_async_elem<T>(&S[c * LD + NB + r], r < rows ? B + row0 + r + (long long)c * cs : B, r < rows);
+    }
+  } else {
+#pragma unroll 4
+    for (int u = 0; u < NB * R / NT; ++u) {
+      const int e = t + u * NT, c = (e & 7) + 8 * ((e >> 5) % (NB / 8)), r = ((e >> 3) & 3) + 4 * (e / (4 * NB));
+      cp_async_elem<T>(&S[c * LD + NB + r], r < rows ? B + (row0 + r) * rs + (long long)c * cs : B, r < rows);
+    }
+  }
+  if (t == 0) s_fail = -1;
+  cp_async_wait_all();
+  factor_block<T, NB, R, NT>(S, Ld, rd, NB, NB + R, &s_fail, [&](int c0, int tt, int nt) {
+    const T* X = S + c0 * LD + NB;
+    if (blockIdx.x == 0)
+      for (int e = tt; e < NB * kSub; e += nt) {
+        const int r = e % NB, c = c0 + e / NB;
+        if (r >= c) D[r + c * NB] = S[c * LD + r];
+      }
+    auto put = [&](auto* out, long long rs_, long long cs_, auto conv) {
+#pragma unroll 4
+      for (int e = tt; e < R * kSub; e += nt) {
+        const int r = (rs_ == 1) ? e % R : e / kSub, c = (rs_ == 1) ? e / R : e % kSub;
+        if (r < rows) out[(row0 + r) * rs_ + (long long)(c0 + c) * cs_] = conv(X[c * LD + r]);
+      }
+    };
+    put(B, rs, cs, [](T v) { return v; });
+    if constexpr (MODE == OUT_SPLIT && Traits<T>::complex) {
+#pragma unroll 2
+      for (int e = tt; e < R * kSub; e += nt) {
+        const int r = e / kSub, c = e % kSub;
+        if (r < rows) put_split(X[c * LD + r], out2, out3, 2 * (row0 + r) * o_rs + 2 * (c0 + c), o_rs);
+      }
+    } else if constexpr (MODE == OUT_SPLIT) {
+      put(out2, o_rs, o_cs, [](T v) { return round_tf32((float)v); });
+      put(out3, o_rs, o_cs, [](T v) {
+        const float hi = round_tf32((float)v);
+        return round_tf32((float)v - hi);
+      });
+    } else {
+      put(out2, o_rs, o_cs, [](T v) { return v; });
+    }
+  });
+  if (blockIdx.x != 0) return;
+  if (s_fail >= 0) {
+    if (t == 0) atomicCAS(d_info, 0, (int)(info_base + s_fail + 1));
+  } else if (logdet != nullptr) {
+    add_logdet<T, NB, LD>(S, NB, s_log, logdet);
+  }
+}
+
+// The factored diagonal blocks first_block + blockIdx.x from D (slot 0: block slot0) to A: the lower triangle of every
+// block before the one that failed, and of that one the columns before the failing one.
+template <typename T, int NB>
+__global__ void __launch_bounds__(256)
+    copy_diag_kernel(const T* __restrict__ D, int slot0, T* __restrict__ A, long long rs, long long cs, int first_block,
+                     const int* __restrict__ d_info) {
+  const int b = first_block + blockIdx.x, info = *d_info;
+  const int cols = (info == 0) ? NB : min(NB, info - 1 - b * NB);
+  const T* d = D + (size_t)(b - slot0) * NB * NB;
+  T* a = A + (long long)b * NB * (rs + cs);
+  for (int e = threadIdx.x; e < NB * NB; e += 256) {
+    const int r = (rs == 1) ? e % NB : e / NB, c = (rs == 1) ? e / NB : e % NB;
+    if (r >= c && c < cols) a[r * rs + c * cs] = d[r + c * NB];
   }
 }
 
