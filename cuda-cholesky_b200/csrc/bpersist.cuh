@@ -6,9 +6,9 @@
 // largest first (the longest-processing-time rule: the last matrices taken are the
 // cheapest, so the CTAs finish together), and runs the blocked algorithms on the
 // matrix in place as a sequence of phases over 64 x 64 tiles:
-//   ?potrf  for each block column k: the diagonal block factored (and its inverse W
-//           formed) in shared memory; panel tiles L_ik = A_ik W^T; trailing tiles
-//           A_ij -= L_ik L_jk^T (lower part of the diagonal tiles only);
+//   ?potrf  for each block column k: its tiles A_ik -= sum_{l < k} L_il L_kl^T; the
+//           diagonal block factored (and its inverse W formed) in shared memory; panel
+//           tiles L_ik = A_ik W^T;
 //   ?trtri  every diagonal tile replaced by the inverse that the factor formed for its
 //           panel (kept aside until the factor has succeeded); then, block column j from the last
 //           to the first, X_ij = sum_{l=j+1..i} inv(L)_il L_lj (rows from the bottom
@@ -50,14 +50,16 @@ struct Opnd {
   int m, kk, tri;
 };
 
-// Output of a job: C(r, c) at p[r * rs + c * cs], r < m, c < n;
-// C := alpha * acc + beta * C, lower: only r >= c.
+// Output of a job: C(r, c) at p[r * rs + c * cs], r < m, c < n (lower: only r >= c);
+// C := acc, -acc (neg), or C - acc (sub: the accumulators then start at -C, so that the sum
+// runs down to the Schur complement as step-by-step updates do and does not cancel at its
+// end: FP32 log dets of ill-conditioned kernels lost half a digit otherwise).
 template <typename T>
 struct Out {
   T* p;
   long long rs, cs;
   int m, n;
-  T alpha, beta;
+  int neg, sub;
   int lower;
 };
 
@@ -128,7 +130,7 @@ template <> struct Acc<double> {
     }
   }
   template <typename F>
-  __device__ __forceinline__ void each(F f) const {
+  __device__ __forceinline__ void each(F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int r0 = (warp & 1) * 32, c0 = (warp >> 1) * 16;
 #pragma unroll
@@ -164,7 +166,7 @@ template <> struct Acc<float> {
     }
   }
   template <typename F>
-  __device__ __forceinline__ void each(F f) const {
+  __device__ __forceinline__ void each(F f) {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -179,7 +181,14 @@ template <typename T, typename NT, typename TF, typename OF>
 __device__ __forceinline__ void run_phase(int njobs, NT nterms, TF term, OF out, T* ring) {
   if (njobs <= 0) return;
   Acc<T> acc;
-  acc.clear();
+  auto start = [&](int j) {
+    const Out<T> o = out(j);
+    acc.clear();
+    if (o.sub)
+      acc.each([&](int r, int c, T& x) {
+        if (r < o.m && c < o.n && (!o.lower || r >= c)) x = -o.p[r * o.rs + c * o.cs];
+      });
+  };
   int job = 0, tt = 0, k0 = 0, st = 0, jn = nterms(0);   // the item being multiplied
   Opnd<T> A, B;
   term(0, 0, A, B);
@@ -189,6 +198,7 @@ __device__ __forceinline__ void run_phase(int njobs, NT nterms, TF term, OF out,
   };
   issue(0, 0);
   cp_commit();
+  start(0);
   while (true) {
     // the next item: 32 k further, the next term, or the next job
     int nj = job, nt = tt, nk = k0 + KS;
@@ -211,16 +221,12 @@ __device__ __forceinline__ void run_phase(int njobs, NT nterms, TF term, OF out,
     __syncthreads();                                 // stage st is refilled next
     if (nj != job) {
       const Out<T> o = out(job);
-      acc.each([&](int r, int c, T x) {
-        if (r < o.m && c < o.n && (!o.lower || r >= c)) {
-          T* q = o.p + r * o.rs + c * o.cs;
-          T y = o.alpha * x;
-          if (o.beta != T(0)) y = fma(o.beta, *q, y);
-          *q = y;
-        }
+      const bool neg = o.neg || o.sub;
+      acc.each([&](int r, int c, T& x) {
+        if (r < o.m && c < o.n && (!o.lower || r >= c)) o.p[r * o.rs + c * o.cs] = neg ? -x : x;
       });
-      acc.clear();
       if (!more) break;
+      start(nj);
       jn = nterms(nj);
     }
     job = nj;
@@ -244,44 +250,40 @@ __device__ void process(const MatDesc<T>& M, long long rs, long long cs, bool in
   // below it and, with the inverse to follow, for ?trtri
   auto Wk = [&](int k) { return W + (inverse ? (size_t)k * NB * NB : 0); };
 
-  // ---- ?potrf ----
+  // ---- ?potrf, left-looking: block column k takes all its updates at once, so a tile is
+  // read and written once per step and not once per earlier column ----
   for (int k = 0; k < nt; ++k) {
     const int jb = ext(k);
-    const bool below = (k + 1 < nt);
-    cuchol::diag_factor_block<T, NB, THREADS>(tl(k, k), rs, cs, jb, (below || inverse) ? Wk(k) : nullptr,
-                                                   NB, (long long)k * NB, M.info, M.logdet);
+    const int m = nt - k - 1;                        // tiles below the diagonal one
+    // A_ik -= sum_{l < k} L_il L_kl^T, i = k .. (the diagonal tile's lower part)
+    if (k > 0)
+      run_phase<T>(
+          m + 1, [&](int) { return k; },
+          [&](int q, int l, Opnd<T>& A, Opnd<T>& B) {
+            const int i = k + q;
+            A = Opnd<T>{tl(i, l), rs, cs, ext(i), NB, TRI_NONE};
+            B = Opnd<T>{tl(k, l), rs, cs, jb, NB, TRI_NONE};
+          },
+          [&](int q) {
+            const int i = k + q;
+            return Out<T>{tl(i, k), rs, cs, ext(i), jb, 0, 1, q == 0};
+          },
+          ring);
+    cuchol::diag_factor_block<T, NB, THREADS>(tl(k, k), rs, cs, jb, (m > 0 || inverse) ? Wk(k) : nullptr, NB,
+                                              (long long)k * NB, M.info, M.logdet);
     __syncthreads();
     if (cuchol::cta_aborted(M.info)) return;         // this matrix's factor failed
-    if (!below) break;
-    const int m = nt - k - 1;
     // panel: L_ik = A_ik W^T, i = k+1 ..
     run_phase<T>(
         m, [](int) { return 1; },
         [&](int j, int, Opnd<T>& A, Opnd<T>& B) {
           const int i = k + 1 + j;
           A = Opnd<T>{tl(i, k), rs, cs, ext(i), jb, TRI_NONE};
-          B = Opnd<T>{Wk(k), 1, NB, jb, jb, TRI_NONE};    // B(c, kk) = W(c, kk): zeros above the diagonal
+          B = Opnd<T>{Wk(k), 1, NB, jb, jb, TRI_NONE};   // B(c, kk) = W(c, kk): zeros above the diagonal
         },
         [&](int j) {
           const int i = k + 1 + j;
-          return Out<T>{tl(i, k), rs, cs, ext(i), jb, T(1), T(0), 0};
-        },
-        ring);
-    // trailing: A_ij -= L_ik L_jk^T, k < j <= i (jobs in order j = k+1.., i = j..)
-    run_phase<T>(
-        m * (m + 1) / 2, [](int) { return 1; },
-        [&](int q, int, Opnd<T>& A, Opnd<T>& B) {
-          int jj = 0;
-          while (q >= m - jj) { q -= m - jj; ++jj; }
-          const int j = k + 1 + jj, i = j + q;
-          A = Opnd<T>{tl(i, k), rs, cs, ext(i), jb, TRI_NONE};
-          B = Opnd<T>{tl(j, k), rs, cs, ext(j), jb, TRI_NONE};
-        },
-        [&](int q) {
-          int jj = 0;
-          while (q >= m - jj) { q -= m - jj; ++jj; }
-          const int j = k + 1 + jj, i = j + q;
-          return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), T(-1), T(1), i == j};
+          return Out<T>{tl(i, k), rs, cs, ext(i), jb, 0, 0, 0};
         },
         ring);
   }
@@ -312,7 +314,7 @@ __device__ void process(const MatDesc<T>& M, long long rs, long long cs, bool in
         },
         [&](int q) {
           const int i = nt - 1 - q;
-          return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), T(1), T(0), 0};
+          return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), 0, 0, 0};
         },
         ring);
     // inv(L)_ij = -X_ij inv(L_jj): B(c, kk) = inv(L_jj)(kk, c), nonzero for kk >= c
@@ -325,7 +327,7 @@ __device__ void process(const MatDesc<T>& M, long long rs, long long cs, bool in
         },
         [&](int q) {
           const int i = j + 1 + q;
-          return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), T(-1), T(0), 0};
+          return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), 1, 0, 0};
         },
         ring);
   }
@@ -351,7 +353,7 @@ __device__ void process(const MatDesc<T>& M, long long rs, long long cs, bool in
         int j = 0;
         while (q >= nt - j) { q -= nt - j; ++j; }
         const int i = j + q;
-        return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), T(1), T(0), i == j};
+        return Out<T>{tl(i, j), rs, cs, ext(i), ext(j), 0, 0, i == j};
       },
       ring);
 }
