@@ -94,6 +94,7 @@ CUresult launch_list(CULAPACKhandle h, std::vector<GemmProblem<T>>& ps, CUcholBa
 
 namespace {
 
+constexpr int kPersistentCtas = 3;   // CTAs per SM of the persistent form
 constexpr int kBatchedMaxNb = 64;   // a 64-wide SIMT tile holds a whole panel: in-place solve
 
 template <typename T>
@@ -428,7 +429,7 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
   for (int b = 0; b < batch; ++b) nmax = std::max(nmax, n[b]);
   p->wp_tiles = (nmax + kBatchedMaxNb - 1) / kBatchedMaxNb;
   if (dev_malloc(&p->d_next, sizeof(int)) != cudaSuccess ||
-      dev_malloc(&p->d_wp, sizeof(T) * 2 * (size_t)h->num_sms * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb) !=
+      dev_malloc(&p->d_wp, sizeof(T) * kPersistentCtas * (size_t)h->num_sms * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb) !=
           cudaSuccess)
     return fail(report(cudaGetLastError(), "cudaMalloc", __func__, __FILE__, __LINE__));
   if (nb == 0) {

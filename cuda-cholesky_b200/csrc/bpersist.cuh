@@ -1,8 +1,8 @@
 // Persistent form of the batched plan (included at the end of lapack.cu, after
 // batched.cuh): one launch factors, log-dets and inverts every matrix of the batch.
 //
-// Each CTA (two per SM: while one is in a diagonal step or at a barrier the other has
-// tile products to run) takes whole matrices from a work queue ordered by size,
+// Each CTA (three of four warps per SM: while one is in a diagonal step or at a barrier the
+// others have tile products to run) takes whole matrices from a work queue ordered by size,
 // largest first (the longest-processing-time rule: the last matrices taken are the
 // cheapest, so the CTAs finish together), and runs the blocked algorithms on the
 // matrix in place as a sequence of phases over 64 x 64 tiles:
@@ -19,8 +19,8 @@
 //           after it.
 // The jobs of a phase are independent of each other (by the orders above), so the
 // operand tiles of the next 32 k are fetched (cp.async, two-stage ring) while the
-// current ones are multiplied: FP64 on the tensor cores (mma.sync m16n8k4, eight warps of
-// 32 x 16 outputs), FP32 with 4 x 4 outputs per thread.  Phases are separated by barriers.
+// current ones are multiplied: FP64 on the tensor cores (mma.sync m16n8k4, four warps of
+// 32 x 32 outputs), FP32 with 8 x 4 outputs per thread.  Phases are separated by barriers.
 // The diagonal steps are those of panel.cuh.  A matrix whose factor fails keeps its info
 // word and is left as the factor left it.
 #pragma once
@@ -28,7 +28,7 @@
 namespace {
 namespace bpk {
 
-constexpr int NB = 64, THREADS = 256, LDS = 68;      // tile order; staged rows padded to 68
+constexpr int NB = 64, THREADS = 128, CTAS = kPersistentCtas, LDS = 68;      // tile order; staged rows padded to 68
 constexpr int KS = 32;                                // k per stage
 constexpr int TILE = KS * LDS;                        // elements per staged operand tile
 template <typename T> constexpr size_t ring_bytes() { return 2 * 2 * TILE * sizeof(T); }   // 2 stages x (A, B)
@@ -77,22 +77,26 @@ __device__ __forceinline__ void stage(const Opnd<T>& o, int k0, T* X) {
   if (o.rs == 1) {
     const int r = t & (NB - 1);
     const T* src = o.p + r + (long long)(k0 + (t >> 6)) * o.ks;
-    const long long step = 4 * o.ks;
+    const long long step = 2 * o.ks;
+    const bool rv = r < o.m;
+    // k <= hi and k >= lo are kept
+    const int hi = min(o.kk - 1, o.tri == TRI_LOWER ? r : NB), lo = o.tri == TRI_UPPER ? r : 0;
 #pragma unroll
-    for (int u = 0; u < KS / 4; ++u, src += step) {
-      const int kl = (t >> 6) + 4 * u, k = k0 + kl;
-      const bool v = r < o.m && k < o.kk && (o.tri == TRI_NONE || (o.tri == TRI_LOWER ? k <= r : k >= r));
+    for (int u = 0; u < KS / 2; ++u, src += step) {
+      const int kl = (t >> 6) + 2 * u, k = k0 + kl;
+      const bool v = rv && k <= hi && k >= lo;
       cp_async_elem<T>(&X[kl * LDS + r], v ? src : o.p, v);
     }
   } else {
-    const int kl0 = (t & 7) + 8 * ((t >> 5) & 3), k = k0 + kl0;
-    const int r0 = ((t >> 3) & 3) + 4 * (t >> 7);
+    const int kl0 = (t & 7) + 8 * (t >> 5), k = k0 + kl0, r0 = (t >> 3) & 3;
     const T* src = o.p + (long long)r0 * o.rs + (long long)k * o.ks;
-    const long long step = 8 * o.rs;
+    const long long step = 4 * o.rs;
+    // rows lo <= r < hi are kept
+    const int hi = (k < o.kk) ? min(o.m, o.tri == TRI_UPPER ? k + 1 : NB) : 0, lo = o.tri == TRI_LOWER ? k : 0;
 #pragma unroll
-    for (int u = 0; u < NB / 8; ++u, src += step) {
-      const int r = r0 + 8 * u;
-      const bool v = r < o.m && k < o.kk && (o.tri == TRI_NONE || (o.tri == TRI_LOWER ? k <= r : k >= r));
+    for (int u = 0; u < NB / 4; ++u, src += step) {
+      const int r = r0 + 4 * u;
+      const bool v = r < hi && r >= lo;
       cp_async_elem<T>(&X[kl0 * LDS + r], v ? src : o.p, v);
     }
   }
@@ -101,77 +105,87 @@ __device__ __forceinline__ void stage(const Opnd<T>& o, int k0, T* X) {
 // 64 x 64 accumulators of the CTA.
 template <typename T> struct Acc;
 
-// FP64: warp w holds rows 32 (w & 1) .. + 31, columns 16 (w >> 1) .. + 15 as DMMA
-// fragments (g, t) of lane = 4 g + t.
+// FP64: warp w holds rows 32 (w & 1) .. + 31, columns 32 (w >> 1) .. + 31 as DMMA fragments
+// (g, t) of lane = 4 g + t.  A lane takes rows 2g, 2g + 1 of an m16 block's half and columns
+// 2g, 2g + 1 of a pair of n8 blocks, so each fragment pair is one 16-byte shared load
+// (a quarter warp touches chunks 2t + g: conflict-free), four loads per eight MMAs.
 template <> struct Acc<double> {
-  double v[2][2][4];
+  double v[2][4][4];
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int c = 0; c < 4; ++c) v[a][b][c] = 0.0;
   }
   // += A B^T for the staged tiles
   __device__ __forceinline__ void mma(const double* As, const double* Bs) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int r0 = (warp & 1) * 32, c0 = (warp >> 1) * 16;
+    const int r0 = (warp & 1) * 32, c0 = (warp >> 1) * 32;
 #pragma unroll 4
     for (int k4 = 0; k4 < KS; k4 += 4) {
-      const double* a = As + (k4 + t) * LDS + r0 + g;
-      const double* b = Bs + (k4 + t) * LDS + c0 + g;
-      const double a00 = a[0], a01 = a[8], a10 = a[16], a11 = a[24];
-      const double b0 = b[0], b1 = b[8];
-      cuchol::dmma_m16n8k4(v[0][0], a00, a01, b0);
-      cuchol::dmma_m16n8k4(v[0][1], a00, a01, b1);
-      cuchol::dmma_m16n8k4(v[1][0], a10, a11, b0);
-      cuchol::dmma_m16n8k4(v[1][1], a10, a11, b1);
+      const double* a = As + (k4 + t) * LDS + r0 + 2 * g;
+      const double* b = Bs + (k4 + t) * LDS + c0 + 2 * g;
+      const double2 a0 = *reinterpret_cast<const double2*>(a), a1 = *reinterpret_cast<const double2*>(a + 16);
+      const double2 b0 = *reinterpret_cast<const double2*>(b), b1 = *reinterpret_cast<const double2*>(b + 16);
+      cuchol::dmma_m16n8k4(v[0][0], a0.x, a0.y, b0.x);
+      cuchol::dmma_m16n8k4(v[0][1], a0.x, a0.y, b0.y);
+      cuchol::dmma_m16n8k4(v[0][2], a0.x, a0.y, b1.x);
+      cuchol::dmma_m16n8k4(v[0][3], a0.x, a0.y, b1.y);
+      cuchol::dmma_m16n8k4(v[1][0], a1.x, a1.y, b0.x);
+      cuchol::dmma_m16n8k4(v[1][1], a1.x, a1.y, b0.y);
+      cuchol::dmma_m16n8k4(v[1][2], a1.x, a1.y, b1.x);
+      cuchol::dmma_m16n8k4(v[1][3], a1.x, a1.y, b1.y);
     }
   }
+  // f(row, column, value): fragment element e is row 2g + (e >> 1) and MMA column
+  // 2t + (e & 1), which is column 2 (2t + (e & 1)) + (block & 1) of its pair
   template <typename F>
   __device__ __forceinline__ void each(F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int r0 = (warp & 1) * 32, c0 = (warp >> 1) * 16;
+    const int r0 = (warp & 1) * 32, c0 = (warp >> 1) * 32;
 #pragma unroll
     for (int mb = 0; mb < 2; ++mb)
 #pragma unroll
-      for (int nb8 = 0; nb8 < 2; ++nb8)
+      for (int nb8 = 0; nb8 < 4; ++nb8)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) f(r0 + mb * 16 + g + (e >> 1) * 8, c0 + nb8 * 8 + 2 * t + (e & 1), v[mb][nb8][e]);
+        for (int e = 0; e < 4; ++e)
+          f(r0 + mb * 16 + 2 * g + (e >> 1), c0 + (nb8 >> 1) * 16 + 4 * t + 2 * (e & 1) + (nb8 & 1), v[mb][nb8][e]);
   }
 };
 
-// FP32: thread (tx, ty) holds rows 4 tx .. + 3, columns 4 ty .. + 3 (two 16-byte shared
-// loads per 16 FMAs).
+// FP32: thread (tx, ty) holds rows 4 tx .. + 3 and 32 + 4 tx .. + 3, columns 4 ty .. + 3
+// (three 16-byte shared loads per 32 FMAs).
 template <> struct Acc<float> {
-  float v[4][4];
+  float v[8][4];
   __device__ __forceinline__ void clear() {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 8; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) v[a][b] = 0.f;
   }
   __device__ __forceinline__ void mma(const float* As, const float* Bs) {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
 #pragma unroll 8
     for (int k = 0; k < KS; ++k) {
       const float4 a = *reinterpret_cast<const float4*>(As + k * LDS + 4 * tx);
+      const float4 d = *reinterpret_cast<const float4*>(As + k * LDS + 32 + 4 * tx);
       const float4 b = *reinterpret_cast<const float4*>(Bs + k * LDS + 4 * ty);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+      const float av[8] = {a.x, a.y, a.z, a.w, d.x, d.y, d.z, d.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[i][j] = fmaf(av[i], bv[j], v[i][j]);
     }
   }
   template <typename F>
   __device__ __forceinline__ void each(F f) {
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) f(4 * tx + i, 4 * ty + j, v[i][j]);
+      for (int i = 0; i < 8; ++i) f(4 * tx + (i & 3) + 32 * (i >> 2), 4 * ty + j, v[i][j]);
   }
 };
 
@@ -362,7 +376,7 @@ __device__ void process(const MatDesc<T>& M, long long rs, long long cs, bool in
 // wbuf: per CTA, ntmax inverse blocks of NB x NB (ntmax = block columns of the largest
 // matrix).
 template <typename T>
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(THREADS, CTAS)
     persistent_kernel(const MatDesc<T>* __restrict__ mats, const int* __restrict__ order, int batch, int* next,
                       int upper, int inverse, T* wbuf, int ntmax) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -422,7 +436,7 @@ CUresult record_persistent(CUcholBatched p, const BatchedShape<T>& sh, cudaStrea
   CUCHOL_CHECK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * B, s));
   CUCHOL_CHECK(cudaMemsetAsync(p->d_logdet, 0, sizeof(double) * B, s));
   CUCHOL_CHECK(cudaMemsetAsync(p->d_next, 0, sizeof(int), s));
-  const int grid = std::min(B, 2 * h->num_sms);
+  const int grid = std::min(B, bpk::CTAS * h->num_sms);
   bpk::persistent_kernel<T><<<grid, bpk::THREADS, bpk::smem_bytes<T>(), s>>>(
       dm, dord, B, p->d_next, sh.upper ? 1 : 0, (sh.flags & 4) ? 1 : 0, static_cast<T*>(p->d_wp), p->wp_tiles);
   ++h->launches;
