@@ -426,12 +426,12 @@ CUresult record_persistent(CUcholBatched p, const BatchedShape<T>& sh, cudaStrea
   const int* dord = upload(p, order, &rc);
   if (dord == nullptr) return rc == CUDA_SUCCESS ? CUDA_ERROR_OUT_OF_MEMORY : rc;
   if (p->dry) return CUDA_SUCCESS;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(bpk::persistent_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)bpk::smem_bytes<T>()));
     CUCHOL_CHECK(cudaFuncSetAttribute(bpk::persistent_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr = true;
+    attr.done(h->device);
   }
   CUCHOL_CHECK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * B, s));
   CUCHOL_CHECK(cudaMemsetAsync(p->d_logdet, 0, sizeof(double) * B, s));

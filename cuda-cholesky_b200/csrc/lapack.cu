@@ -108,6 +108,17 @@ template <typename T> constexpr char type_char() {
        : std::is_same<T, cuFloatComplex>::value ? 'C' : 'Z';
 }
 
+// Kernel attributes hold per device: whether a launcher's have been set on this one.  (Two
+// threads may both set them; neither launches before they are set.)
+class DeviceOnce {
+ public:
+  bool needed(int device) const { return (mask_.load() >> (device & 63) & 1) == 0; }
+  void done(int device) { mask_.fetch_or(1ull << (device & 63)); }
+
+ private:
+  std::atomic<unsigned long long> mask_{0};
+};
+
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // ---- tile engine launcher -------------------------------------------------------
@@ -192,14 +203,14 @@ template <int LA, int LB, bool TRI, int MB>
 CUresult launch_dmma(CULAPACKhandle h, const CUtensorMap& ma, const CUtensorMap& mb, const dmma::Params& q,
                      int tiles, cudaStream_t s, const int* abort) {
   constexpr int smem = dmma::Shape<MB>::SMEM_BYTES;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(dmma::gemm_kernel<LA, LB, TRI, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       smem));
     // several CTAs per SM: ask for the whole unified L1/shared carve-out
     CUCHOL_CHECK(cudaFuncSetAttribute(dmma::gemm_kernel<LA, LB, TRI, MB>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr = true;
+    attr.done(h->device);
   }
   dmma::gemm_kernel<LA, LB, TRI, MB><<<tiles, dmma::THREADS, smem, s>>>(ma, mb, q, abort);
   ++h->launches;
@@ -318,13 +329,13 @@ template <int LA, int LB, bool TRI, int MB>
 CUresult launch_zmma(CULAPACKhandle h, const CUtensorMap& ma, const CUtensorMap& mb, const zmma::Params& q,
                      int tiles, cudaStream_t s, const int* abort) {
   constexpr int smem = zmma::Shape<MB>::SMEM_BYTES;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(zmma::gemm_kernel<LA, LB, TRI, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       smem));
     CUCHOL_CHECK(cudaFuncSetAttribute(zmma::gemm_kernel<LA, LB, TRI, MB>,
                                       cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr = true;
+    attr.done(h->device);
   }
   zmma::gemm_kernel<LA, LB, TRI, MB><<<tiles, zmma::THREADS, smem, s>>>(ma, mb, q, abort);
   ++h->launches;
@@ -508,7 +519,11 @@ CUresult diag_factor(CULAPACKhandle h, TA* A, long long rs, long long cs, int jb
                      double* logdet, cudaStream_t s) {
   constexpr int smem = (int)FactorSmem<T, NB>::bytes, threads = panel_threads<T>();
   auto* kernel = diag_factor_kernel<T, TA, NB, threads>;
-  CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
+    CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
+    attr.done(h->device);
+  }
   kernel<<<1, threads, smem, s>>>(A, rs, cs, jb, info_base, first ? 1 : 0, h->d_words, logdet);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
@@ -521,12 +536,12 @@ CUresult panel_solve(CULAPACKhandle h, T* B, int m, int jb, const T* L, long lon
                      long long o_rs, long long o_cs, O2* out3, cudaStream_t s) {
   constexpr int R = 32, smem = (int)SolveSmem<T, NB, R>::bytes;
   auto* kernel = trsm_rows_kernel<T, O2, MODE, NB, R>;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
     // several CTAs per SM: ask for the whole unified L1/shared carve-out
     CUCHOL_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr = true;
+    attr.done(h->device);
   }
   kernel<<<(m + R - 1) / R, 256, smem, s>>>(B, rs, cs, m, jb, L, rs, cs, out2, o_rs, o_cs, h->d_words, out3);
   ++h->launches;
@@ -541,11 +556,11 @@ CUresult panel_fused(CULAPACKhandle h, T* A, int m, long long rs, long long cs, 
                      O2* out3, T* D, long long info_base, bool first, double* logdet, cudaStream_t s) {
   constexpr int R = kFusedRows, smem = (int)FactorSmem<T, NB, R>::bytes, threads = sizeof(T) == 16 ? 256 : 512;
   auto* kernel = panel_kernel<T, O2, MODE, NB, R, threads>;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
     CUCHOL_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    attr = true;
+    attr.done(h->device);
   }
   kernel<<<(m + R - 1) / R, threads, smem, s>>>(A, rs, cs, m, out2, o_rs, o_cs, out3, D, info_base, first ? 1 : 0,
                                                 h->d_words, logdet);
@@ -654,12 +669,11 @@ CUresult tcg_launch(CULAPACKhandle h, const PackRef& A, const PackRef& B, tcg::P
     return CUDA_ERROR_INVALID_VALUE;
   p.tiles_m = (p.m + tcg::BM - 1) / tcg::BM;
   p.tiles_n = (p.n + tcg::BN - 1) / tcg::BN;
-  p.vec = (p.cs == p.cx) && aligned16(p.c) && (p.rs % 4) == 0 && (p.c_node % 4) == 0;
   p.err = h->d_words + 3;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(tcg::gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcg::SMEM_BYTES));
-    attr = true;
+    attr.done(h->device);
   }
   tcg::gemm_kernel<<<p.nodes * p.tiles_m * p.tiles_n, tcg::THREADS, tcg::SMEM_BYTES, s>>>(ah, al, bh, bl, p, stop);
   ++h->launches;
@@ -808,7 +822,7 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
 
   // the first diagonal kernel writes the info word and the log det, the later ones read
   // and add to them; the update stream starts behind a panel event
-  CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));
+  if (!alone) CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));
 
   const T minus_one = from_real<T>(RealOf<T>(-1)), one = from_real<T>(RealOf<T>(1));
   // C -= Phat Phat^H on the lower trapezoid m x ncols of A with its corner on the
@@ -844,19 +858,17 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
     for (int s0 = 0; s0 < jB; s0 += nb) {
       const int c = j + s0, jb = std::min(nb, j + jB - c);
       const int mr = n - c - jb;                 // rows below this diagonal block
-      const bool fused = jb == nb && mr > 0 && mr <= fused_rows;
+      const bool fused = jb == nb && mr > 0 && mr <= fused_rows && (tc3 || !is_fp32<T>());
       if (fused) {
         if (dfirst < 0) dfirst = c / nb;
         dnext = c / nb + 1;
         T* D = dbuf + (size_t)(c / nb - dfirst) * nb * nb;
         if constexpr (is_fp32<T>()) {
-          if (tc3) {
-            const long long qo = (long long)s0 * cx * ldq + s0 * cx;
-            CUCHOL_CHECK_CU((panel_fused<T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
-                                                                  c == 0, h->d_logdet, sp)));
-          }
+          const long long qo = (long long)s0 * cx * ldq + s0 * cx;
+          CUCHOL_CHECK_CU((panel_fused<T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
+                                                                c == 0, h->d_logdet, sp)));
         }
-        if (!tc3)
+        if constexpr (!is_fp32<T>())
           CUCHOL_CHECK_CU((panel_fused<T, T, OUT_COPY, nb>(h, at(c, c), mr, rs, cs, P + s0 + (long long)s0 * ldp, 1, ldp,
                                                            nullptr, D, c, c == 0, h->d_logdet, sp)));
         if (on_final) {              // the block column goes to the caller now
@@ -873,14 +885,13 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
       // panel solve into P: rows c + jb .. n-1 are P rows s0 .. (P starts at j + nb)
       // row-parallel triangular solve: A21 := A21 L11^-H in place, and into P (or its
       // hi / lo split into Q)
-      if (fused) {
-      } else if (tc3) {
+      if (!fused && tc3) {
         if constexpr (is_fp32<T>()) {
           const long long qo = (long long)s0 * cx * ldq + s0 * cx;
           CUCHOL_CHECK_CU((panel_solve<T, float, OUT_SPLIT, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs, Qh + qo, ldq,
                                                                 1, Ql + qo, sp)));
         }
-      } else {
+      } else if (!fused) {
         CUCHOL_CHECK_CU((panel_solve<T, T, OUT_COPY, nb>(h, at(c + jb, c), mr, jb, at(c, c), rs, cs,
                                                             P + s0 + (long long)s0 * ldp, 1, ldp, nullptr, sp)));
       }
@@ -1267,10 +1278,12 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
     // n down to one tile, and without slabs the launch takes as long as an SM's share
     // of the longest ones (n = 2048: 285 us for 82 us of FP64 work).
     const long long tiles = (long long)((n + 63) / 64) * ((n + 63) / 64 + 1) / 2;
-    const int want = (int)std::min<long long>((24LL * h->num_sms + tiles - 1) / tiles, std::max(1, n / 512));
-    const int slab = (int)round_up((size_t)(n + want - 1) / want, 128), slabs = (n + slab - 1) / slab;
+    const size_t product = sizeof(T) * (size_t)ldw * n;
     const bool direct = fp64_aligned(A, lda);
-    const size_t need = sizeof(T) * (size_t)ldw * n * (slabs + (direct ? 0 : 1));
+    const long long fit = (long long)(kLauumWorkspace / product) - (direct ? 0 : 1);
+    const int want = (int)std::max(1LL, std::min({(24LL * h->num_sms + tiles - 1) / tiles, (long long)n / 512, fit}));
+    const int slab = (int)round_up((size_t)(n + want - 1) / want, 128), slabs = (n + slab - 1) / slab;
+    const size_t need = product * (slabs + (direct ? 0 : 1));
     if (!h->force_simt && h->lauum_cols == 0 && (slabs > 1 || !direct) && need <= kLauumWorkspace && try_workspace(h, need)) {
       T* W = static_cast<T*>(h->ws);
       T* S = W + (size_t)ldw * n * slabs;

@@ -52,9 +52,9 @@ struct Params {
   int k, k_last;                // real k (a multiple of BK or zero-padded in the packs)
   int kmode, cx;
   int a_row0, b_row0, a_node, b_node, k0;   // k0: first k in the packs
-  float* c;                     // output, in floats; element (i, col, part) at i*rs + col*cs + part
+  float* c;                     // output, in floats; element (i, col, part) at i*rs + col*cs + part;
+                                // rs or cs is cx
   long long rs, cs, c_node;     // in floats
-  int vec;                      // C's rows are contiguous along columns and 16-byte aligned
   int beta, neg;                // C := (beta ? C : 0) + (neg ? -1 : 1) * acc
   int lower_only, real_diag;
   float *xhi, *xlo;             // if not null: the product goes here, split, as an A pack of row
@@ -175,46 +175,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       s_consumed = kk;
     }
   } else {
-    // epilogue warps: tile row of this lane; 128 real columns in registers
-    const int r = i0 + 32 * warp + lane;
-    const bool row_ok = r < m;
-    float* cq = p.c + (long long)q * p.c_node;
-    const bool colmaj = p.rs == p.cx;
+    // epilogue warps: 32 tile rows each, a row per lane, its 128 real columns in registers
     float acc[BN];
-    auto keep = [&](int col) { return col < p.n && row_ok && (!p.lower_only || r * p.cx + p.cx - 1 >= col); };
-    // C first, while the operands are on their way: acc = -+C, so that the result is +-acc
-    if (p.beta && p.xhi == nullptr && p.vec) {
 #pragma unroll
-      for (int j = 0; j < BN; j += 4) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (keep(j0 + j + 3)) {
-          v = *reinterpret_cast<const float4*>(cq + r * p.rs + j0 + j);
-        } else {
-          if (keep(j0 + j)) v.x = cq[r * p.rs + j0 + j];
-          if (keep(j0 + j + 1)) v.y = cq[r * p.rs + j0 + j + 1];
-          if (keep(j0 + j + 2)) v.z = cq[r * p.rs + j0 + j + 2];
-        }
-        acc[j] = p.neg ? -v.x : v.x;
-        acc[j + 1] = p.neg ? -v.y : v.y;
-        acc[j + 2] = p.neg ? -v.z : v.z;
-        acc[j + 3] = p.neg ? -v.w : v.w;
-      }
-    } else if (p.beta && p.xhi == nullptr) {
-#pragma unroll
-      for (int j = 0; j < BN; ++j) {
-        const int col = j0 + j;
-        float v = 0.f;
-        if (keep(col)) {
-          const long long off = (p.cx == 2) ? (long long)(col >> 1) * p.cs + (col & 1) : (long long)col * p.cs;
-          v = cq[r * p.rs + off];
-        }
-        acc[j] = p.neg ? -v : v;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-    }
+    for (int j = 0; j < BN; ++j) acc[j] = 0.f;
     bool ok = true;
+#pragma unroll 1
     for (int c = 0; c < nch; ++c) {
       const int b = c & 1;
       if (!tc::mbar_wait(&acc_full[b], (c >> 1) & 1)) {
@@ -236,64 +202,65 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     if (!ok) s_fail = 1;
     if (ok) {
+      // The ring is idle now (every MMA has read its operands): the rows go through it, so
+      // that the output loops are rolled, coalesced in either storage, and short.  Straight
+      // code over 128 registers, with C read into them first, was bound by instruction
+      // fetch: 26 us for a launch of one wave with k = 128.
+      float* st = reinterpret_cast<float*>(base) + warp * (BN * 33);     // st[col * 33 + row]
+#pragma unroll
+      for (int j = 0; j < BN; ++j) st[j * 33 + lane] = p.neg ? -acc[j] : acc[j];
+      __syncwarp();
+      const int r0 = i0 + 32 * warp, rows = min(32, m - r0), cols = min(BN, p.n - j0);
+      float* cq = p.c + (long long)q * p.c_node;
+      // C(r, col) in floats: += (no load to wait for; one CTA owns the element) or =
+      auto put = [&](float* o, float v) {
+        if (p.beta) atomicAdd(o, v);
+        else *o = v;
+      };
+      auto keep = [&](int r, int col) { return !p.lower_only || r * p.cx + p.cx - 1 >= col; };
       if (p.xhi != nullptr) {
-        if (row_ok) {
-          const long long o = (long long)(q * p.a_node + r) * p.xld + j0;
+#pragma unroll 2
+        for (int r = 0; r < rows; ++r) {
+          const long long o = (long long)(q * p.a_node + r0 + r) * p.xld + j0;
 #pragma unroll
-          for (int j = 0; j < BN; j += 4) {
-            if (j0 + j < p.n) {
-              float4 h, l;
-              float* hp = &h.x;
-              float* lp = &l.x;
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const float x = (p.neg ? -acc[j + u] : acc[j + u]);
-                hp[u] = round_tf32(x);
-                lp[u] = round_tf32(x - hp[u]);
-              }
-              *reinterpret_cast<float4*>(p.xhi + o + j) = h;
-              *reinterpret_cast<float4*>(p.xlo + o + j) = l;
+          for (int u = 0; u < BN / 32; ++u) {
+            const int c = lane + 32 * u;
+            if (c < cols) {
+              const float x = st[c * 33 + r], h = round_tf32(x);
+              p.xhi[o + c] = h;
+              p.xlo[o + c] = round_tf32(x - h);
             }
           }
         }
-      } else if (p.vec) {
-#pragma unroll
-        for (int j = 0; j < BN; j += 4) {
-          const int col = j0 + j;
-          float4 v = p.neg ? make_float4(-acc[j], -acc[j + 1], -acc[j + 2], -acc[j + 3])
-                           : make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-          if (p.real_diag && p.cx == 2) {
-            if (r == (col >> 1)) v.y = 0.f;
-            if (r == (col >> 1) + 1) v.w = 0.f;
-          }
-          float* o = cq + r * p.rs + col;
-          if (keep(col + 3)) {
-            *reinterpret_cast<float4*>(o) = v;
-          } else {
-            if (keep(col)) o[0] = v.x;
-            if (keep(col + 1)) o[1] = v.y;
-            if (keep(col + 2)) o[2] = v.z;
-          }
-        }
-      } else if (p.cx == 2 && colmaj) {
-#pragma unroll
-        for (int j = 0; j < BN; j += 2) {
-          const int col = j0 + j;
-          if (keep(col)) {
-            float2 v = make_float2(p.neg ? -acc[j] : acc[j], p.neg ? -acc[j + 1] : acc[j + 1]);
-            if (p.real_diag && r == (col >> 1)) v.y = 0.f;
-            *reinterpret_cast<float2*>(cq + r * p.rs + (long long)(col >> 1) * p.cs) = v;
+      } else if (p.rs == p.cx && p.cx == 1) {       // rows contiguous
+        float* o = cq + r0 + lane + (long long)j0 * p.cs;
+        const int r = r0 + lane;
+#pragma unroll 4
+        for (int c = 0; c < cols; ++c, o += p.cs)
+          if (lane < rows && keep(r, j0 + c)) put(o, st[c * 33 + lane]);
+      } else if (p.rs == p.cx) {                    // complex, rows contiguous: 16 rows x (re, im) per step
+        const int part = lane & 1;
+#pragma unroll 4
+        for (int e = 0; e < cols; ++e) {            // e: column pair e / 2, half e % 2 of the rows
+          const int c = (e & ~1) + part, rl = (lane >> 1) + 16 * (e & 1), r = r0 + rl, col = j0 + c;
+          if (rl < rows && keep(r, col)) {
+            float v = st[c * 33 + rl];
+            float* o = cq + r * p.rs + (long long)(col >> 1) * p.cs + part;
+            if (p.real_diag && part && r == (col >> 1)) *o = 0.f;
+            else put(o, v);
           }
         }
-      } else {
+      } else {                                      // columns contiguous (complex: re, im adjacent)
+#pragma unroll 2
+        for (int r = 0; r < rows; ++r) {
+          float* o = cq + (r0 + r) * p.rs + j0;
 #pragma unroll
-        for (int j = 0; j < BN; ++j) {
-          const int col = j0 + j;
-          if (keep(col)) {
-            const long long off = (p.cx == 2) ? (long long)(col >> 1) * p.cs + (col & 1) : (long long)col * p.cs;
-            float v = p.neg ? -acc[j] : acc[j];
-            if (p.real_diag && p.cx == 2 && (col & 1) && r == (col >> 1)) v = 0.f;
-            cq[r * p.rs + off] = v;
+          for (int u = 0; u < BN / 32; ++u) {
+            const int c = lane + 32 * u, col = j0 + c;
+            if (c < cols && keep(r0 + r, col)) {
+              if (p.real_diag && p.cx == 2 && (col & 1) && r0 + r == (col >> 1)) o[c] = 0.f;
+              else put(o + c, st[c * 33 + r]);
+            }
           }
         }
       }
