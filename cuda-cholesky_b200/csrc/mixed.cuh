@@ -141,6 +141,36 @@ __device__ __forceinline__ unsigned wait_ready(const unsigned* ready, unsigned n
 // for J < I as the y_J are published (the counter ready = number of finished
 // blocks), then applies DI_I.
 // Counters: ctr[0] ticket, ctr[1] ready; both zero at launch.
+// How the 256 threads share a 64-row step: four row sets of 64 threads take four
+// right-hand sides each and, with eight or fewer of them, a half or a quarter of the 64
+// columns (one warp per scheduler then runs 16 to 32 FP64 FMAs per column set instead of
+// 64, on the chain that every later block waits for).
+struct TrsvSplit {
+  int g, part, c0, c1, groups;
+  __device__ __forceinline__ TrsvSplit(int nrhs, int set) {
+    groups = nrhs <= 4 ? 1 : nrhs <= 8 ? 2 : 4;
+    g = set % groups;
+    part = set / groups;
+    const int w = BS * groups / 4;
+    c0 = part * w;
+    c1 = c0 + w;
+  }
+};
+// v of the sets with part 0 += those of the other parts, in order; by the whole CTA.
+template <typename T>
+__device__ __forceinline__ void trsv_combine(const TrsvSplit& sp, T (&v)[4], T* Red /* [4][BS][4] */, int r) {
+  if (sp.groups == 4) return;
+  const int set = sp.part * sp.groups + sp.g;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) Red[(set * 4 + k) * BS + r] = v[k];
+  __syncthreads();
+  if (sp.part == 0) {
+    for (int q = 1; q < 4 / sp.groups; ++q)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] += Red[((q * sp.groups + sp.g) * 4 + k) * BS + r];
+  }
+}
+
 template <typename T, typename VB>
 __global__ void __launch_bounds__(kThreads)
     trsv_fwd_kernel(const T* __restrict__ L, long long rs, long long cs, int n, const T* __restrict__ DI,
@@ -150,8 +180,11 @@ __global__ void __launch_bounds__(kThreads)
   auto Ls = reinterpret_cast<T(*)[BS + 1]>(smem_raw);           // [BS][BS + 1]
   auto Ds = reinterpret_cast<T(*)[BS + 1]>(smem_raw + sizeof(T) * BS * (BS + 1));
   auto Vs = reinterpret_cast<T(*)[NR]>(smem_raw + 2 * sizeof(T) * BS * (BS + 1));
+  T* Red = reinterpret_cast<T*>(smem_raw + 2 * sizeof(T) * BS * (BS + 1)) + BS * NR;
   __shared__ unsigned s_I, s_known;
-  const int t = threadIdx.x, r = t & (BS - 1), g = t >> 6;
+  const int t = threadIdx.x, r = t & (BS - 1);
+  const TrsvSplit sp(nrhs, t >> 6);
+  const int g = sp.g;                                            // right-hand sides 4g .. 4g + 3
   if (t == 0) {
     s_I = atomicAdd(&ctr[0], 1u);
     s_known = 0;
@@ -167,7 +200,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int c = g * 4 + k;
-    acc[k] = (i < n && c < nrhs) ? (T)(sc != nullptr ? sc[i] * (double)B[i + c * ldb] : (double)B[i + c * ldb])
+    acc[k] = (sp.part == 0 && i < n && c < nrhs) ? (T)(sc != nullptr ? sc[i] * (double)B[i + c * ldb] : (double)B[i + c * ldb])
                                  : T(0);
   }
   // prefetch of the next L block: element e = t + 256 q
@@ -201,7 +234,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
 #pragma unroll 8
-    for (int cc = 0; cc < BS; ++cc) {
+    for (int cc = sp.c0; cc < sp.c1; ++cc) {
       const T l = Ls[r][cc];
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc[k] -= l * Vs[cc][g * 4 + k];
@@ -209,21 +242,25 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
   }
   // y_I = DI_I acc
+  trsv_combine(sp, acc, Red, r);
+  if (sp.part == 0) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) Vs[r][g * 4 + k] = acc[k];
+    for (int k = 0; k < 4; ++k) Vs[r][g * 4 + k] = acc[k];
+  }
   __syncthreads();
   T y[4] = {T(0), T(0), T(0), T(0)};
-  for (int cc = 0; cc <= r; ++cc) {
+#pragma unroll 8
+  for (int cc = sp.c0; cc < sp.c1; ++cc) {
     const T d = Ds[r][cc];
+    if (cc <= r) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) y[k] += d * Vs[cc][g * 4 + k];
+      for (int k = 0; k < 4; ++k) y[k] += d * Vs[cc][g * 4 + k];
+    }
   }
-  if (i < n) {
+  trsv_combine(sp, y, Red, r);
+  if (sp.part == 0) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) __stcg(&Y[i + (long long)(g * 4 + k) * ldy], y[k]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) __stcg(&Y[i + (long long)(g * 4 + k) * ldy], T(0));
+    for (int k = 0; k < 4; ++k) __stcg(&Y[i + (long long)(g * 4 + k) * ldy], i < n ? y[k] : T(0));
   }
   __threadfence();
   __syncthreads();
@@ -242,9 +279,12 @@ __global__ void __launch_bounds__(kThreads)
   auto Ls = reinterpret_cast<T(*)[BS + 1]>(smem_raw);           // Ls[c][r] = L(J*BS + c, I*BS + r)
   auto Ds = reinterpret_cast<T(*)[BS + 1]>(smem_raw + sizeof(T) * BS * (BS + 1));   // Ds[r][c] = DI_I(c, r)
   auto Vs = reinterpret_cast<T(*)[NR]>(smem_raw + 2 * sizeof(T) * BS * (BS + 1));
+  T* Red = reinterpret_cast<T*>(smem_raw + 2 * sizeof(T) * BS * (BS + 1)) + BS * NR;
   __shared__ unsigned s_I, s_known;
   const int nblk = (n + BS - 1) / BS;
-  const int t = threadIdx.x, r = t & (BS - 1), g = t >> 6;
+  const int t = threadIdx.x, r = t & (BS - 1);
+  const TrsvSplit sp(nrhs, t >> 6);
+  const int g = sp.g;
   if (t == 0) {
     s_I = atomicAdd(&ctr[0], 1u);
     s_known = 0;
@@ -258,7 +298,7 @@ __global__ void __launch_bounds__(kThreads)
   const bool row_contig = (rs == 1);
   T acc[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) acc[k] = (i < n) ? Y[i + (long long)(g * 4 + k) * ldy] : T(0);
+  for (int k = 0; k < 4; ++k) acc[k] = (sp.part == 0 && i < n) ? Y[i + (long long)(g * 4 + k) * ldy] : T(0);
   T pre[BS * BS / kThreads];
   auto fetch = [&](int J) {
 #pragma unroll
@@ -287,7 +327,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
 #pragma unroll 8
-    for (int cc = 0; cc < BS; ++cc) {
+    for (int cc = sp.c0; cc < sp.c1; ++cc) {
       const T l = Ls[cc][r];
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc[k] -= l * Vs[cc][g * 4 + k];
@@ -295,18 +335,26 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
   }
   // z_I = DI_I^T acc
+  trsv_combine(sp, acc, Red, r);
+  if (sp.part == 0) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) Vs[r][g * 4 + k] = acc[k];
+    for (int k = 0; k < 4; ++k) Vs[r][g * 4 + k] = acc[k];
+  }
   __syncthreads();
   T z[4] = {T(0), T(0), T(0), T(0)};
-  for (int cc = r; cc < BS; ++cc) {
+#pragma unroll 8
+  for (int cc = sp.c0; cc < sp.c1; ++cc) {
     const T d = Ds[r][cc];
+    if (cc >= r) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) z[k] += d * Vs[cc][g * 4 + k];
+      for (int k = 0; k < 4; ++k) z[k] += d * Vs[cc][g * 4 + k];
+    }
   }
+  trsv_combine(sp, z, Red, r);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int c = g * 4 + k;
+    if (sp.part != 0) continue;
     __stcg(&Zt[i + (long long)c * ldy], (i < n) ? z[k] : T(0));
     if (i < n && c < nrhs) Z[i + (long long)c * ldz] = (VZ)((sc != nullptr) ? sc[i] * (double)z[k] : (double)z[k]);
   }
@@ -984,7 +1032,7 @@ CUresult symv(const double* A, long long rs, long long cs, int n, const double* 
 }
 
 template <typename T>
-constexpr size_t trsv_smem() { return sizeof(T) * (2 * BS * (BS + 1) + BS * NR); }
+constexpr size_t trsv_smem() { return sizeof(T) * (2 * BS * (BS + 1) + BS * NR + 16 * BS); }
 
 // Opt in to the triangular solves' shared memory (above 48 KB for FP64).
 template <typename T, typename V>
