@@ -32,15 +32,14 @@ struct TuneRow {
   int sub;
 };
 
-// FP64 ?potrf, B200, rows from tune.py with the 64 x 64-tile DMMA updates: outer
-// blocks of 2 / 2 / 5 / 8 diagonal blocks at n = 4096 / 8192 / 16384 / 32768 (best
-// 3.99, 10.78, 54.33, 382.6 ms; at 16384 the other widths gave 57.1 (2), 55.3 (3),
-// 54.8 (4), 54.4 (6), 54.9 (8)), split at the geometric midpoints.  C: the rows tune.py wrote from n = 4096 / 8192 / 16384 (best
-// cpotrf 7.34 / 29.82 / 196.8 ms; outer block 2 gave 208.5 ms at n = 16384).  Z on
-// the complex FP64 tensor-core engine: best 9.93 / 37.56 / 223.9 ms with 2 / 6 / 12
-// (outer block 2 gave 293.5 ms at 16384).  S on the split TF32 tensor-core updates:
-// flat in the width up to n = 8192 (2.78 / 6.09 ms), best 4 at 16384 (16.69 ms; 1
-// gave 22.37) and within 1% of the best at 32768 (88.74 ms).
+// ?potrf, ms on a B200 by the width of the outer block; the rows split at the geometric
+// midpoints of the orders measured, and lie within 1.3% of the best width at each:
+//   D  n = 8192   8.68 (2)  8.57 (3)  8.65 (4)
+//      n = 16384  54.7 (2)  52.7 (3)  51.95 (4)  51.67 (5)  51.47 (6)      n = 32768  378.6 (6)  376.2 (8)
+//   S  n = 16384  14.1 (2)  12.6 (3)  11.9 (4)  11.85 (6)                  n = 32768  84.1 (4)  85.1 (6)
+//   C  n = 4096  2.32 (2)  2.33 (3)  2.34 (4)      n = 8192  7.59 (3)  7.49 (4)  7.58 (6)  7.87 (8)
+//      n = 16384  48.2 (4)  46.8 (6)  46.8 (8)
+//   Z  n = 4096  6.6 (2 .. 6)      n = 8192  33.0 (4)  32.4 (6)
 // cuDpotrfOzaki: 8 (1024 columns) below n = 49152, 16 from there on (n = 8192 / 32768 /
 // 65536: 10.8 / 255 / 2028 ms with 8; 11.7 / 255 / 1926 ms with 16; 4 gave 282 ms and
 // 2344 ms at the two larger orders).
