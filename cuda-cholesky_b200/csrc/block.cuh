@@ -58,10 +58,9 @@ constexpr int kSubRows = 32;         // rows factor16 covers: the 16 x 16 block 
 constexpr int kLdPad = 4;
 
 // 1 / sqrt(d) for the pivot chain, for normal positive finite d, without branches.  FP32:
-// the hardware estimate.  FP64: the hardware estimate y refined by the Taylor series of
-// (1 - e)^(-1/2), e = 1 - d y^2, to third order: five dependent FP64 operations after the
-// estimate.  To second order the dropped 5/16 e^3 showed: the factor of n = 100 was 1.5e-16
-// from the exact one in place of 1.0e-16.
+// the hardware estimate.  FP64: the hardware estimate y (relative error below 2^-20)
+// refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, to second order (the
+// dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations after the estimate.
 __device__ __forceinline__ float pivot_rsqrt(float d) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
@@ -71,7 +70,7 @@ __device__ __forceinline__ double pivot_rsqrt(double d) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d * y, y, 1.0);
-  return fma(y * e, fma(fma(0.3125, e, 0.375), e, 0.5), y);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 // Not a normal positive finite number (one integer subtraction and comparison).
 __device__ __forceinline__ bool odd_pivot(float d) { return (unsigned)(__float_as_int(d) - 0x00800000) >= 0x7f000000u; }
