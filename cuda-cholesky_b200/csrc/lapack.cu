@@ -551,11 +551,11 @@ CUresult panel_solve(CULAPACKhandle h, T* B, int m, int jb, const T* L, long lon
 
 // The diagonal block and the m rows below it in one launch (panel_kernel), queued on s.
 constexpr int kFusedRows = 32;
-template <typename T, typename O2, int MODE, int NB>
-CUresult panel_fused(CULAPACKhandle h, T* A, int m, long long rs, long long cs, O2* out2, long long o_rs, long long o_cs,
-                     O2* out3, T* D, long long info_base, bool first, double* logdet, cudaStream_t s) {
+template <typename T, typename TA, typename O2, int MODE, int NB>
+CUresult panel_fused(CULAPACKhandle h, TA* A, int m, long long rs, long long cs, O2* out2, long long o_rs, long long o_cs,
+                     O2* out3, TA* D, long long info_base, bool first, double* logdet, cudaStream_t s) {
   constexpr int R = kFusedRows, smem = (int)FactorSmem<T, NB, R>::bytes, threads = sizeof(T) == 16 ? 256 : 512;
-  auto* kernel = panel_kernel<T, O2, MODE, NB, R, threads>;
+  auto* kernel = panel_kernel<T, TA, O2, MODE, NB, R, threads>;
   static DeviceOnce attr;
   if (attr.needed(h->device)) {
     CUCHOL_CHECK_CU(set_smem<T>((const void*)kernel, smem));
@@ -865,11 +865,11 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
         T* D = dbuf + (size_t)(c / nb - dfirst) * nb * nb;
         if constexpr (is_fp32<T>()) {
           const long long qo = (long long)s0 * cx * ldq + s0 * cx;
-          CUCHOL_CHECK_CU((panel_fused<T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
+          CUCHOL_CHECK_CU((panel_fused<T, T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
                                                                 c == 0, h->d_logdet, sp)));
         }
         if constexpr (!is_fp32<T>())
-          CUCHOL_CHECK_CU((panel_fused<T, T, OUT_COPY, nb>(h, at(c, c), mr, rs, cs, P + s0 + (long long)s0 * ldp, 1, ldp,
+          CUCHOL_CHECK_CU((panel_fused<T, T, T, OUT_COPY, nb>(h, at(c, c), mr, rs, cs, P + s0 + (long long)s0 * ldp, 1, ldp,
                                                            nullptr, D, c, c == 0, h->d_logdet, sp)));
         if (on_final) {              // the block column goes to the caller now
           CUCHOL_CHECK_CU((copy_diag<T, nb>(h, dbuf, A, rs, cs, dfirst, c / nb, 1, sp)));

@@ -1173,9 +1173,15 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
   const long long ldq = OB;
   const size_t rows = round_up((size_t)n, 128) + 128;
   const size_t qbytes = round_up(sizeof(Op) * rows * ldq, 256);
-  CUCHOL_CHECK_CU(ensure_workspace(h, 2 * qbytes));
+  // Block and panel in one launch while its CTAs fit the GPU, as in ?potrf: there 33 us in
+  // place of 34 + 14 and a gap.  Those factors wait in D, from block dfirst on.
+  const int fused_rows = kFusedRows * h->num_sms;
+  int dfirst = -1, dcount = 0;
+  const size_t dbytes = sizeof(float) * SB * SB * (size_t)(std::min(n, fused_rows + SB) / SB + 1);
+  CUCHOL_CHECK_CU(ensure_workspace(h, 2 * qbytes + dbytes));
   char* ws = static_cast<char*>(h->ws);
   Op* Q[2] = {reinterpret_cast<Op*>(ws), reinterpret_cast<Op*>(ws + qbytes)};
+  float* D = reinterpret_cast<float*>(ws + 2 * qbytes);
   CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));   // (the update stream starts behind a panel event)
   auto at = [&](long long i, long long j) { return W + i + j * ldw; };
 
@@ -1186,12 +1192,18 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
     const int q_rows = n - j - SB;   // P / Q row r = global row j + SB + r
     for (int s0 = 0; s0 < jB; s0 += SB) {
       const int c = j + s0, jb = std::min(SB, j + jB - c), mr = n - c - jb;
-      CUCHOL_CHECK_CU((diag_factor<double, float, SB>(h, at(c, c), 1, ldw, jb, c, c == 0, h->d_logdet, sp)));
-      if (mr == 0) break;
       // panel rows c + jb .. n-1 solved in place; they are Q rows s0 .., columns s0 ..
       Op* Qs = Qj + (long long)s0 * ldq + s0;
-      CUCHOL_CHECK_CU((panel_solve<float, Op, OUT_ROUND, SB>(h, at(c + jb, c), mr, jb, at(c, c), 1, ldw, Qs, ldq, 1,
-                                                             nullptr, sp)));
+      if (mr > 0 && mr <= fused_rows) {              // (rows below it: the block is a whole one)
+        if (dfirst < 0) dfirst = c / SB;
+        CUCHOL_CHECK_CU((panel_fused<double, float, Op, OUT_ROUND, SB>(
+            h, at(c, c), mr, 1, ldw, Qs, ldq, 1, nullptr, D + (size_t)dcount++ * SB * SB, c, c == 0, h->d_logdet, sp)));
+      } else {
+        CUCHOL_CHECK_CU((diag_factor<double, float, SB>(h, at(c, c), 1, ldw, jb, c, c == 0, h->d_logdet, sp)));
+        if (mr == 0) break;
+        CUCHOL_CHECK_CU((panel_solve<float, Op, OUT_ROUND, SB>(h, at(c + jb, c), mr, jb, at(c, c), 1, ldw, Qs, ldq, 1,
+                                                               nullptr, sp)));
+      }
       if (s0 + SB < jB)   // the outer block's remaining columns by this sub-panel
         CUCHOL_CHECK_CU(tc_update<Op>(h, Qs, ldq, q_rows - s0, jb, 0, 0, at(c + jb, c + jb), ldw, mr,
                                       jB - s0 - SB, sp, d_info));
@@ -1212,6 +1224,7 @@ CUresult mixed_factor(CULAPACKhandle h, int n, float* W, long long ldw, long* in
   }
   CUCHOL_CHECK(cudaEventRecord(h->ev_update, su));
   CUCHOL_CHECK(cudaStreamWaitEvent(sp, h->ev_update, 0));
+  if (dcount > 0) CUCHOL_CHECK_CU((copy_diag<float, SB>(h, D, W, 1, ldw, dfirst, dfirst, dcount, sp)));
   CUCHOL_CHECK_CU(fetch_words(h, sp));
   *info = h->h_words[0];
   return CUDA_SUCCESS;

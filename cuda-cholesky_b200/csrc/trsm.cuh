@@ -251,10 +251,11 @@ __global__ void __launch_bounds__(256)
 // as it is while CTAs still load it: CTA 0 writes the factor to D (column-major, ld NB),
 // and copy_diag_kernel takes it to A later.  Outputs for the rows as trsm_rows_kernel.
 // Worth it while the CTAs fit the GPU at once (each is as long as the factor).
-template <typename T, typename O2, int MODE, int NB, int R, int NT>
+// T: the computing type; TA: the storage type of A and D (float under double only with rs = 1).
+template <typename T, typename TA, typename O2, int MODE, int NB, int R, int NT>
 __global__ void __launch_bounds__(NT)
-    panel_kernel(T* __restrict__ A, long long rs, long long cs, int m, O2* __restrict__ out2, long long o_rs,
-                 long long o_cs, O2* __restrict__ out3, T* __restrict__ D, long long info_base, int first,
+    panel_kernel(TA* __restrict__ A, long long rs, long long cs, int m, O2* __restrict__ out2, long long o_rs,
+                 long long o_cs, O2* __restrict__ out3, TA* __restrict__ D, long long info_base, int first,
                  int* __restrict__ d_info, double* __restrict__ logdet) {
   using F = FactorSmem<T, NB, R>;
   constexpr int LD = F::LD, V = 16 / sizeof(T);
@@ -275,9 +276,11 @@ __global__ void __launch_bounds__(NT)
   }
   const long long row0 = (long long)blockIdx.x * R;
   const int rows = min((long long)R, m - row0);
-  T* B = A + NB * rs;                // the rows below the block
-  load_lower<T, T, NB, NT, LD>(S, A, rs, cs, NB, NB);
-  if (V > 1 && rs == 1 && aligned16(B, cs * (long long)sizeof(T))) {
+  TA* B = A + NB * rs;               // the rows below the block
+  load_lower<T, TA, NB, NT, LD>(S, A, rs, cs, NB, NB);
+  if constexpr (!std::is_same<T, TA>::value) {
+    load_widened<R, NB, NT, LD, false>(S + NB, B + row0, cs, rows, NB);
+  } else if (V > 1 && rs == 1 && aligned16(B, cs * (long long)sizeof(T))) {
     constexpr int PC = R / V;
 #pragma unroll 4
     for (int u = 0; u < NB * PC / NT; ++u) {
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(NT)
     if (blockIdx.x == 0)
       for (int e = tt; e < NB * kSub; e += nt) {
         const int r = e % NB, c = c0 + e / NB;
-        if (r >= c) D[r + c * NB] = S[c * LD + r];
+        if (r >= c) D[r + c * NB] = (TA)S[c * LD + r];
       }
     auto put = [&](auto* out, long long rs_, long long cs_, auto conv) {
 #pragma unroll 4
@@ -314,8 +317,10 @@ __global__ void __launch_bounds__(NT)
         if (r < rows) out[(row0 + r) * rs_ + (long long)(c0 + c) * cs_] = conv(X[c * LD + r]);
       }
     };
-    put(B, rs, cs, [](T v) { return v; });
-    if constexpr (MODE == OUT_SPLIT && Traits<T>::complex) {
+    put(B, rs, cs, [](T v) { return (TA)v; });
+    if constexpr (MODE == OUT_ROUND) {
+      put(out2, o_rs, o_cs, [](T v) { return to_op<O2>((float)v); });
+    } else if constexpr (MODE == OUT_SPLIT && Traits<T>::complex) {
 #pragma unroll 2
       for (int e = tt; e < R * kSub; e += nt) {
         const int r = e / kSub, c = e % kSub;
