@@ -391,44 +391,61 @@ constexpr int GSTAGE = GR * GMP + GR * GVP;             // floats per stage
 constexpr size_t kGemvSmem = sizeof(float) * (GST * GSTAGE + 4 * GR * NR);
 
 // The 4 partial 4 x 4 blocks of every thread -> out (alpha, beta), rows/columns
-// [o0, o0 + 64) of the output; with a split k range (part != null) the raw sums go to
-// part[o][c] of this split instead, for gemv_reduce_kernel.
+// [o0, o0 + 64) of the output.  With a split k range (gridDim.y > 1) the raw sums go to
+// part[split][block][c][o], and the last CTA of the block to arrive at count[block] adds the
+// splits in order and resets the count: a second launch for this took 3.7 us and a gap of
+// the 15 to 25 us of a product.
+constexpr int kGemvSplits = NBT / 256;                  // at most
 __device__ __forceinline__ void gemv_finish(float (&acc)[4][4], float* Red, int ig, int cg, int ks, int o0, int m,
                                             float alpha, float beta, const float* in, float* out, long long ldv,
-                                            float* part) {
-  const int t = threadIdx.x;
+                                            float* part, unsigned* count) {
+  const int t = threadIdx.x, o = t & 63, c0 = (t >> 6) * 4, r = o0 + o;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) Red[(ks * GR + 4 * ig + i) * NR + 4 * cg + j] = acc[i][j];
   __syncthreads();
+  float sum[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int o = t & 63, c = (t >> 6) * 4 + q, r = o0 + o;
-    const float sum = ((Red[(0 * GR + o) * NR + c] + Red[(1 * GR + o) * NR + c]) +
-                       (Red[(2 * GR + o) * NR + c] + Red[(3 * GR + o) * NR + c]));
-    if (part != nullptr) {
-      part[(long long)r * NR + c] = sum;
-    } else if (r < m) {
-      float v = alpha * sum;
-      if (beta != 0.f) v = fmaf(beta, in[r + (long long)c * ldv], v);
-      out[r + (long long)c * ldv] = v;
+    const int c = c0 + q;
+    sum[q] = ((Red[(0 * GR + o) * NR + c] + Red[(1 * GR + o) * NR + c]) +
+              (Red[(2 * GR + o) * NR + c] + Red[(3 * GR + o) * NR + c]));
+  }
+  const int ns = gridDim.y;
+  if (ns > 1) {
+    const long long step = (long long)gridDim.x * GR * NR;
+    float* mine = part + (long long)blockIdx.x * GR * NR + c0 * GR + o;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mine[blockIdx.y * step + q * GR] = sum[q];
+    __threadfence();
+    __shared__ bool s_last;
+    __syncthreads();
+    if (t == 0) s_last = atomicAdd(&count[blockIdx.x], 1u) == (unsigned)ns - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float v[kGemvSplits];
+#pragma unroll
+      for (int u = 0; u < kGemvSplits; ++u) v[u] = u < ns ? __ldcg(mine + u * step + q * GR) : 0.f;
+      sum[q] = 0.f;
+#pragma unroll
+      for (int u = 0; u < kGemvSplits; ++u) sum[q] += v[u];
     }
+    if (t == 0) count[blockIdx.x] = 0;
+  }
+  if (r >= m) return;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long e = r + (long long)(c0 + q) * ldv;
+    float v = alpha * sum[q];
+    if (beta != 0.f) v = fmaf(beta, in[e], v);
+    out[e] = v;
   }
 }
 
-// out(r, c) = alpha * sum_s part[s][r][c] + beta * in(r, c), the splits in order.
-__global__ void gemv_reduce_kernel(const float* __restrict__ part, int nsplit, long long mp, int m, float alpha,
-                                   float beta, const float* in, float* out, long long ldv) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= (long long)m * NR) return;
-  const int r = (int)(e / NR), c = (int)(e % NR);
-  float sum = 0.f;
-  for (int q = 0; q < nsplit; ++q) sum += part[((long long)q * mp + r) * NR + c];
-  float v = alpha * sum;
-  if (beta != 0.f) v = fmaf(beta, in[r + (long long)c * ldv], v);
-  out[r + (long long)c * ldv] = v;
-}
 
 // 16 consecutive k of the stage: thread block (ig, cg) += A4(ig rows) x V4(cg rhs).
 __device__ __forceinline__ void gemv_mac(const float* Ms, const float* Vs, int ig, int cg, int ks,
@@ -464,14 +481,16 @@ __device__ __forceinline__ void gemv_issue_v(float* Vs, const float* v, long lon
 // x 4 right-hand sides over a quarter of each chunk.
 __global__ void __launch_bounds__(kThreads)
     gemv_n_kernel(const float* __restrict__ M, long long ldm, int m, int kk, const float* __restrict__ v,
-                  float alpha, float beta, const float* in, float* out, long long ldv, int kc, float* part) {
+                  float alpha, float beta, const float* in, float* out, long long ldv, int kc, float* part,
+                  unsigned* count, int tri) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* ring = reinterpret_cast<float*>(smem_raw);
   float* Red = ring + GST * GSTAGE;
   const int t = threadIdx.x, ig = t & 15, cg = (t >> 4) & 3, ks = t >> 6;
   const int r0 = blockIdx.x * GR;
-  // this CTA's k range [kb, ke): split blockIdx.y of width kc (a multiple of 64)
-  const int kb = blockIdx.y * kc, ke = min(kk, kb + kc);
+  // this CTA's k range [kb, ke): split blockIdx.y of width kc (a multiple of 64); of a
+  // lower triangular M only the columns up to the block's last row
+  const int kb = (int)blockIdx.y * kc, ke = min(tri ? min(kk, r0 + GR) : kk, kb + kc);
   const int nch = (ke - kb + GR - 1) / GR;
   auto issue = [&](int ch) {
     float* Ms = ring + (ch % GST) * GSTAGE;
@@ -501,8 +520,7 @@ __global__ void __launch_bounds__(kThreads)
     gemv_mac(Ms, Ms + GR * GMP, ig, cg, ks, acc);
   }
   cp_async_wait<0>();
-  gemv_finish(acc, Red, ig, cg, ks, r0, m, alpha, beta, in, out, ldv,
-              part ? part + (long long)blockIdx.y * gridDim.x * GR * NR : nullptr);
+  gemv_finish(acc, Red, ig, cg, ks, r0, m, alpha, beta, in, out, ldv, part, count);
 }
 
 // out(j, c) = alpha * sum_k M(k, j) v(k, c) + beta * in(j, c), j < m, k < kk (the
@@ -511,13 +529,15 @@ __global__ void __launch_bounds__(kThreads)
 // with one 16-byte load.
 __global__ void __launch_bounds__(kThreads)
     gemv_t_kernel(const float* __restrict__ M, long long ldm, int m, int kk, const float* __restrict__ v,
-                  float alpha, float beta, const float* in, float* out, long long ldv, int kc, float* part) {
+                  float alpha, float beta, const float* in, float* out, long long ldv, int kc, float* part,
+                  unsigned* count, int tri) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* ring = reinterpret_cast<float*>(smem_raw);
   float* Red = ring + GST * GSTAGE;
   const int t = threadIdx.x, jg = t & 15, cg = (t >> 4) & 3, ks = t >> 6;
   const int j0 = blockIdx.x * GR;
-  const int kb = blockIdx.y * kc, ke = min(kk, kb + kc);
+  // of a lower triangular M only the rows from the block's first column on
+  const int k1 = (int)blockIdx.y * kc, kb = max(k1, tri ? j0 : 0), ke = min(kk, k1 + kc);
   const int nch = (ke - kb + GR - 1) / GR;
   auto issue = [&](int ch) {
     float* Ms = ring + (ch % GST) * GSTAGE;
@@ -545,8 +565,7 @@ __global__ void __launch_bounds__(kThreads)
     gemv_mac(Ms, Ms + GR * GMP, jg, cg, ks, acc);
   }
   cp_async_wait<0>();
-  gemv_finish(acc, Red, jg, cg, ks, j0, m, alpha, beta, in, out, ldv,
-              part ? part + (long long)blockIdx.y * gridDim.x * GR * NR : nullptr);
+  gemv_finish(acc, Red, jg, cg, ks, j0, m, alpha, beta, in, out, ldv, part, count);
 }
 
 // t = (float)(s .* r) (NR columns)
@@ -986,6 +1005,7 @@ struct __cucholmixed_st {
   double* h_norms;            // pinned mirror of norms (the handle's)
   char* arena;                // the one allocation behind all of the above
   unsigned* ctr;              // triangular-solve counters
+  unsigned* gcount;           // arrivals per output block of a split GEMV (zero between launches)
   int* err;                   // a bounded wait gave up
 };
 
@@ -1061,28 +1081,23 @@ CUresult precond(CUcholMixed p, const double* R, double* Z, cudaStream_t s) {
   const long long ld = p->ld, ldw = p->ldw;
   const int nT = (n + NBT - 1) / NBT, vb = 4 * p->h->num_sms;
   // one GEMV; with fewer than two CTAs per SM the k range is split (chunks of 256 or
-  // more) and the partial sums reduced in order by a second launch
-  auto gemv = [&](bool trans, const float* M, long long ldm, int m, int kk, const float* v, float alpha,
+  // more) and the partial sums are added in order by the last CTA of each block
+  auto gemv = [&](bool trans, bool tri, const float* M, long long ldm, int m, int kk, const float* v, float alpha,
                   float beta, const float* in, float* out) -> CUresult {
     const int blocks = (m + GR - 1) / GR, want = 2 * p->h->num_sms;
     int split = 1;
     if (blocks < want) split = std::max(1, std::min((want + blocks - 1) / blocks, kk / 256));
     const int kc = (int)round_up((size_t)((kk + split - 1) / split), GR);
     split = (kk + kc - 1) / kc;
-    float* part = split > 1 ? p->gpart : nullptr;
     const dim3 grid(blocks, split);
     if (trans)
-      gemv_t_kernel<<<grid, kThreads, kGemvSmem, s>>>(M, ldm, m, kk, v, alpha, beta, in, out, ld, kc, part);
+      gemv_t_kernel<<<grid, kThreads, kGemvSmem, s>>>(M, ldm, m, kk, v, alpha, beta, in, out, ld, kc, p->gpart,
+                                                      p->gcount, tri);
     else
-      gemv_n_kernel<<<grid, kThreads, kGemvSmem, s>>>(M, ldm, m, kk, v, alpha, beta, in, out, ld, kc, part);
+      gemv_n_kernel<<<grid, kThreads, kGemvSmem, s>>>(M, ldm, m, kk, v, alpha, beta, in, out, ld, kc, p->gpart,
+                                                      p->gcount, tri);
     CUCHOL_CHECK(cudaGetLastError());
     ++p->h->launches;
-    if (split > 1) {
-      gemv_reduce_kernel<<<(m * NR + 255) / 256, 256, 0, s>>>(part, split, (long long)blocks * GR, m, alpha, beta,
-                                                              in, out, ld);
-      CUCHOL_CHECK(cudaGetLastError());
-      ++p->h->launches;
-    }
     return CUDA_SUCCESS;
   };
   scale_in_kernel<<<vb, 256, 0, s>>>(R, p->s, n, ld, p->t);
@@ -1090,16 +1105,16 @@ CUresult precond(CUcholMixed p, const double* R, double* Z, cudaStream_t s) {
   for (int I = 0; I < nT; ++I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0), rest = n - b0 - bI;
     const float* D = p->Dinv + (size_t)I * NBT * (NBT + 1);
-    CUCHOL_CHECK_CU(gemv(false, D, NBT, bI, bI, p->t + b0, 1.f, 0.f, nullptr, p->y + b0));
+    CUCHOL_CHECK_CU(gemv(false, true, D, NBT, bI, bI, p->t + b0, 1.f, 0.f, nullptr, p->y + b0));
     if (rest > 0)
-      CUCHOL_CHECK_CU(gemv(false, p->W + (b0 + bI) + (long long)b0 * ldw, ldw, rest, bI, p->y + b0, -1.f, 1.f,
+      CUCHOL_CHECK_CU(gemv(false, false, p->W + (b0 + bI) + (long long)b0 * ldw, ldw, rest, bI, p->y + b0, -1.f, 1.f,
                            p->t + b0 + bI, p->t + b0 + bI));
   }
   for (int I = nT - 1; I >= 0; --I) {
     const int b0 = I * NBT, bI = std::min(NBT, n - b0);
     const float* D = p->Dinv + (size_t)I * NBT * (NBT + 1);
-    CUCHOL_CHECK_CU(gemv(true, D, NBT, bI, bI, p->y + b0, 1.f, 0.f, nullptr, p->zf + b0));
-    if (b0 > 0) CUCHOL_CHECK_CU(gemv(true, p->W + b0, ldw, b0, bI, p->zf + b0, -1.f, 1.f, p->y, p->y));
+    CUCHOL_CHECK_CU(gemv(true, true, D, NBT, bI, bI, p->y + b0, 1.f, 0.f, nullptr, p->zf + b0));
+    if (b0 > 0) CUCHOL_CHECK_CU(gemv(true, false, p->W + b0, ldw, b0, bI, p->zf + b0, -1.f, 1.f, p->y, p->y));
   }
   scale_out_kernel<<<vb, 256, 0, s>>>(p->zf, p->s, n, ld, Z);
   CUCHOL_CHECK(cudaGetLastError());
@@ -1363,7 +1378,7 @@ CUresult mixed_create(CUcholMixed* out, CULAPACKhandle h, CBlasUplo uplo, size_t
                oD = carve(sizeof(float) * (size_t)nT * NBT * (NBT + 1)), og = carve(sizeof(float) * gpart),
                ox = carve(sizeof(double) * 6 * p->ld * NR), ot = carve(sizeof(float) * 3 * p->ld * NR),
                oU = carve(sizeof(double) * ptile), oV = carve(sizeof(double) * ptile), op = carve(sizeof(double) * nred),
-               oc = carve(16 * sizeof(unsigned));
+               oc = carve((16 + 2 * h->num_sms) * sizeof(unsigned));
   cudaError_t e;
   if ((e = dev_malloc(&p->arena, total)) != cudaSuccess) return fail(e);
   p->W = reinterpret_cast<float*>(p->arena + oW);
@@ -1387,7 +1402,8 @@ CUresult mixed_create(CUcholMixed* out, CULAPACKhandle h, CBlasUplo uplo, size_t
   p->norms = p->rz + 2 * NR;
   p->ctr = reinterpret_cast<unsigned*>(p->arena + oc);
   p->err = reinterpret_cast<int*>(p->ctr + 8);
-  if ((e = cudaMemset(p->ctr, 0, 16 * sizeof(unsigned))) != cudaSuccess) return fail(e);
+  p->gcount = p->ctr + 16;
+  if ((e = cudaMemset(p->ctr, 0, (16 + 2 * h->num_sms) * sizeof(unsigned))) != cudaSuccess) return fail(e);
   p->h_norms = h->h_norms;
 
   p->shift_request = shift_in;

@@ -145,3 +145,42 @@ def test_potrs_right_hand_side_groups(handle, uplo, nrhs):
         assert rc == 0 and info == 0
         ref = np.linalg.solve(A, B)
         assert np.linalg.norm(X.cpu().numpy().T - ref) <= 2.0 ** -53 * 8 * (32 + np.sqrt(n)) * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("prec", [cc.MIXED_BF16, cc.MIXED_TF32])
+@pytest.mark.parametrize("n,nrhs,uplo", [(127, 1, "L"), (128, 1, "L"), (129, 2, "U"), (255, 3, "L"), (641, 16, "U"),
+                                         (2047, 5, "L"), (2048, 1, "U"), (2049, 16, "L"), (2400, 17, "L"),
+                                         (4864, 2, "U"), (4865, 2, "L"), (6200, 3, "L")])
+def test_mixed_launch_limits(handle, prec, n, nrhs, uplo):
+    """The mixed factor's panels (the block and its rows in one launch while they fit the
+    GPU, 4864 = 148 x 32 + 128) and the preconditioner's products (2048-wide steps, their
+    triangular blocks, split or not): W W^T against S A S + shift I to the rounding of the
+    operands, and the refined solution to the criterion that ends the refinement."""
+    import torch
+    A = matgen.spd_device("d", n, seed=n).contiguous()
+    H = matgen.hermitian_of(A, uplo)
+    plan = cc.MixedPlan(handle, uplo, n, A.data_ptr(), n, prec)
+    assert plan.info == 0
+    w, ldw, s, anorm, shift = plan.factor()
+    torch.cuda.synchronize()
+
+    def view(ptr, count, typestr):
+        raw = type("Raw", (), {"__cuda_array_interface__": {"shape": (count,), "typestr": typestr,
+                                                            "data": (ptr, False), "version": 2}})
+        return torch.as_tensor(raw(), device="cuda").clone()
+    L = torch.tril(view(w, n * ldw, "<f4").reshape(n, ldw)[:, :n].T).double()
+    S = view(s, n, "<f8")
+    M = S[:, None] * H * S[None, :] + shift * torch.eye(n, dtype=torch.float64, device="cuda")
+    # every product rounds two operands to u: |E| <= 2u |L| |L|^T, whose Frobenius norm is at
+    # most |L|_F^2 = trace(M) <= sqrt(n) |M|_F; the roundings are independent, so sqrt(n) u falls
+    # to a small multiple of u
+    u = 2.0 ** -8 if prec == cc.MIXED_BF16 else 2.0 ** -11
+    assert float(torch.linalg.norm(M - L @ L.T) / torch.linalg.norm(M)) <= 4 * u
+    B = torch.as_tensor(np.random.default_rng(n).standard_normal((nrhs, n)), device="cuda")
+    X = torch.zeros_like(B)
+    it, berr = plan.solve(nrhs, B.data_ptr(), n, X.data_ptr(), n)
+    tol = np.sqrt(n) * 2.0 ** -53
+    assert it > 0 and berr <= tol
+    R = torch.abs(B - X @ H).amax(1) / (torch.abs(H).sum(1).max() * torch.abs(X).amax(1) + torch.abs(B).amax(1))
+    assert float(R.max()) <= 2 * tol
+    plan.close()
