@@ -16,7 +16,8 @@
 //   * solve16 (one thread per row): right-looking substitution through 16 columns.
 //   * tile_update (one warp): C(32 x 16) -= P Q^H over 16 columns; FP64 on DMMA.
 // The diagonal 16 x 16 block of L is kept a second time in Ld, column j at Ld[16 j], so
-// that the loops read it with aligned 16-byte loads.
+// that the loops read it with aligned 16-byte loads; its diagonal holds the pivots (the
+// squares of the diagonal elements).
 #pragma once
 #include <stdint.h>
 #include <type_traits>
@@ -59,8 +60,9 @@ constexpr int kLdPad = 4;
 
 // 1 / sqrt(d) for the pivot chain, for normal positive finite d, without branches.  FP32:
 // the hardware estimate.  FP64: the hardware estimate y (relative error below 2^-20)
-// refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, to second order (the
-// dropped term is 5/16 e^3 < 2^-60): four dependent FP64 operations after the estimate.
+// refined by the Taylor series of (1 - e)^(-1/2), e = 1 - d y^2, |e| < 2^-19, to second
+// order (the dropped term is 5/16 e^3 < 2^-58): four dependent FP64 operations after the
+// estimate.
 __device__ __forceinline__ float pivot_rsqrt(float d) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
@@ -130,7 +132,7 @@ __device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf
     const T l = (i == j) ? from_real<T>(sqrt(d)) : scale(a, r);
     __syncwarp();
     if (i < nrows && i >= j) S[j * ld + i] = l;
-    if (i < kSub) Ld[j * kSub + i] = l;
+    if (i < kSub) Ld[j * kSub + i] = (i == j) ? from_real<T>(d) : l;
     if (i == 0) rd[j] = r;
   }
   __syncwarp();
@@ -138,12 +140,12 @@ __device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf
 }
 
 // Step J of factor16 and the ones after it: x the row, r the reciprocal square root of
-// the pivot of column J.  (On lane J the update formula makes x[J] the pivot itself, so
-// x[J] r is the diagonal element; complex types drop its imaginary part when it is stored.)
+// the pivot of column J.  (On lane J the update formula makes x[J] the pivot itself.)
 template <int J, typename T>
 __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i, T* Ld, RealOf<T>* rd, bool& odd) {
   using R = RealOf<T>;
   if constexpr (J < kSub) {
+    if (i == J) Ld[J * kSub + J] = from_real<T>(re(x[J]));
     x[J] = scale(x[J], r);
     R rn = R(1);
     if constexpr (J + 1 < kSub) {
@@ -151,7 +153,7 @@ __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i,
       odd = odd || odd_pivot(dn);
       rn = pivot_rsqrt(dn);
     }
-    if (i < kSub) Ld[J * kSub + i] = x[J];
+    if (i < kSub && i != J) Ld[J * kSub + i] = x[J];
     if (i == 0) rd[J] = r;
     if constexpr (J + 1 < kSub) {
       __syncwarp();
@@ -174,17 +176,11 @@ __device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Ld, RealOf<T
   for (int q = 0; q < kSub; ++q) x[q] = mine ? S[q * ld + i] : zero<T>();
   const R d = __shfl_sync(0xffffffffu, re(x[0]), 0);
   bool odd = odd_pivot(d);
-  if constexpr (Traits<T>::complex) {
-    if (i == 0) x[0].y = 0;
-  }
   factor16_steps<0>(x, pivot_rsqrt(d), i, Ld, rd, odd);
   if (odd) return factor16_slow<T>(S, ld, nrows, Ld, rd);
 #pragma unroll
   for (int q = 0; q < kSub; ++q) {
-    if constexpr (Traits<T>::complex) {
-      if (i == q) x[q].y = 0;
-    }
-    if (mine && i >= q) S[q * ld + i] = x[q];
+    if (mine && i > q) S[q * ld + i] = x[q];
   }
   return -1;
 }
@@ -262,7 +258,10 @@ __device__ __forceinline__ void dmma16n8k4(double (&d)[4], double a0, double a1,
 // neither read nor written.
 // The tile is 32 x 16 because eight warps then cover 128 x 32 or 64 x 64 with every
 // lane holding 4 x 4 outputs.  FP64 runs on DMMA: the same flop rate as DFMA, but 6
-// shared loads per 4 k instead of 32.
+// shared loads per 4 k instead of 32.  The 16 products are summed from zero and subtracted
+// once: product by product from C an FP32 factor of order 100 errs by 1.05e-7 instead of
+// 0.51e-7 (against FP64), a complex one by 1.28e-7 instead of 0.58e-7, and C held from the
+// start costs panel_kernel<float> 48 bytes of spills (n = 1000: 379 us instead of 345).
 template <typename T>
 __device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, const T* Q, int ldq, int nr) {
   const int lane = threadIdx.x & 31;
@@ -304,7 +303,9 @@ __device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, 
     if (4 * lr >= nr) return;
     T acc[4][4];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) load4(C + (4 * lc + v) * ldc + 4 * lr, acc[v]);
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[v][u] = zero<T>();
     constexpr int U = sizeof(T) == 4 ? 16 : sizeof(T) == 8 ? 4 : 2;   // operand loads in flight
 #pragma unroll U
     for (int k = 0; k < kSub; ++k) {
@@ -314,10 +315,16 @@ __device__ __forceinline__ void tile_update(T* C, int ldc, const T* P, int ldp, 
 #pragma unroll
       for (int v = 0; v < 4; ++v)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) fms(acc[v][u], a[u], cj(b[v]));
+        for (int u = 0; u < 4; ++u) mac(acc[v][u], a[u], cj(b[v]));
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) store4(C + (4 * lc + v) * ldc + 4 * lr, acc[v]);
+    for (int v = 0; v < 4; ++v) {
+      T c[4];
+      load4(C + (4 * lc + v) * ldc + 4 * lr, c);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) c[u] = sub(c[u], acc[v][u]);
+      store4(C + (4 * lc + v) * ldc + 4 * lr, c);
+    }
   }
 }
 
@@ -347,15 +354,15 @@ __device__ __forceinline__ void strip_update(T* C, int ldc, const T* P, int ldp,
     for (int w = warp; w < (R / 32) * 8; w += NT / 32) {
       const int r = 32 * (w >> 3) + lane, c = 2 * (w & 7);
       if (r >= nr) continue;
-      T a0 = C[c * ldc + r], a1 = C[(c + 1) * ldc + r];
+      T a0 = zero<T>(), a1 = zero<T>();
 #pragma unroll
       for (int k = 0; k < kSub; ++k) {
         const T p = P[k * ldp + r];
-        fms(a0, p, cj(Q[k * ldq + c]));
-        fms(a1, p, cj(Q[k * ldq + c + 1]));
+        mac(a0, p, cj(Q[k * ldq + c]));
+        mac(a1, p, cj(Q[k * ldq + c + 1]));
       }
-      C[c * ldc + r] = a0;
-      C[(c + 1) * ldc + r] = a1;
+      C[c * ldc + r] = sub(C[c * ldc + r], a0);
+      C[(c + 1) * ldc + r] = sub(C[(c + 1) * ldc + r], a1);
     }
   }
 }
@@ -407,6 +414,11 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
     }
     __syncthreads();
     const int fail = *s_fail;
+    // the diagonal, rounded once: the pivot times its reciprocal root, as the columns are
+    // scaled, is up to an ulp off (n = 16 .. 200 FP64: error of the factor 6% larger)
+    static_assert(NB + R - kSubRows <= NT - kSub, "these threads have no row to solve");
+    const int i = t - (NT - kSub);
+    if (i >= 0 && (fail < 0 || c0 + i < fail)) S[(c0 + i) * LD + c0 + i] = from_real<T>(sqrt(re(Ld[i * kSub + i])));
     for (int r = c0 + kSubRows + t; r < nrow; r += NT) {
       if (fail < 0) solve16<T>(S + c0 * LD + r, LD, Ld, rd + c0);
       else solve16_part<T>(S + c0 * LD + r, LD, Ld, rd + c0, fail - c0);
