@@ -954,8 +954,12 @@ int build_tree(int o, int s, int nb, std::vector<Node>& out) {
   return hgt;
 }
 
-// FP32 orders from which ?trtri and ?lauum run on the TF32 tensor cores.
-constexpr int kTcgMinOrder = 256;
+// FP32 orders from which ?trtri and ?lauum run on the TF32 tensor cores: where the split
+// products are both no less accurate than the SIMT engine (against FP64) and no slower.  ?potri,
+// tensor cores / SIMT, B200: S n = 257 2.58e-7 / 2.47e-7 and 218 / 185 us, 320 2.64e-7 / 2.77e-7
+// and 220 / 207, 384 2.65e-7 / 3.14e-7 and 228 / 232, 1000 2.83e-7 / 4.91e-7 and 282 / 1006;
+// C n = 257 3.22e-7 / 4.39e-7 and 237 / 238 us, 1000 3.76e-7 / 8.87e-7 and 360 / 1009.
+template <typename T> constexpr int tcg_min_order() { return Traits<T>::complex ? 256 : 384; }
 
 // Whether the split products are safe for the triangle of A: every entry finite and at
 // most 2^62, every diagonal entry (unless unit) at least 2^-62, so that no hi part
@@ -1125,7 +1129,7 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
   *info = 0;
   bool tensor = false;
   if constexpr (is_fp32<T>()) {
-    if (!h->force_simt && n >= kTcgMinOrder) CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, unit, &tensor));
+    if (!h->force_simt && n >= tcg_min_order<T>()) CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, unit, &tensor));
   }
   if (!unit) {
     int init[3] = {0, 0, INT_MAX};
@@ -1243,7 +1247,7 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
     const long long ld = (long long)round_up((size_t)n, 32) * cx;
     const size_t one = (size_t)n * cx * ld;
     bool tensor = false;
-    if (!h->force_simt && n >= kTcgMinOrder && h->lauum_cols == 0)
+    if (!h->force_simt && n >= tcg_min_order<T>() && h->lauum_cols == 0)
       CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, false, &tensor));
     if (tensor && try_workspace(h, sizeof(float) * 2 * one)) {
       float* w = static_cast<float*>(h->ws);

@@ -8,11 +8,13 @@
 // hi hi^T (the dropped lo lo^T is below 2^-22 of the product).
 //
 // Accumulation.  The tensor core truncates when it adds to its FP32 accumulator, which
-// over thousands of k would bias the sums.  So an accumulator in tensor memory only runs
-// over kChunk k blocks (64 k); four epilogue warps then add it, rounded to nearest, to
-// FP32 registers while the next chunk runs in the other half of the tensor memory.  That
-// is blocked summation: measured against 64 bits its error is below that of one FMA
-// chain per element.
+// biases long sums.  So an accumulator in tensor memory only runs over one k block (32 k:
+// four additions of the large products); eight epilogue warps then add it, rounded to
+// nearest, to FP32 registers while the next k block runs in the other accumulator.  That is
+// blocked summation: its error is below that of one FMA chain per element (tcg_min_order
+// has the figures).  Accumulators of two k blocks, read by four warps: ?potri of order 300
+// 6.3e-7 in place of 2.9e-7 (the FMA chains: 3.0e-7), complex ?potri of order 4096 3.89 in
+// place of 4.00 ms.
 //
 // Complex.  With a complex number stored as two adjacent k values, a complex product is
 // a real one of twice the k: Re C = (ar, ai) . (br, -bi), Im C = (ar, ai) . (bi, br).
@@ -21,8 +23,8 @@
 // are Re and Im of column j.  Conjugated views flip the sign of the stored imaginary
 // part.  All of it is the packs' business: the kernel only knows real products.
 //
-// One CTA per 128 x 128 real tile: warp 4 streams operand tiles with TMA into a 3-stage
-// ring, warp 5 issues the MMAs, warps 0..3 accumulate and write C.  Triangular operands
+// One CTA per 128 x 128 real tile: warp 8 streams operand tiles with TMA into a 3-stage
+// ring, warp 9 issues the MMAs, warps 0..7 accumulate and write C.  Triangular operands
 // are zero outside their triangle in the pack; k blocks that are zero for a whole tile
 // are skipped.  What bounds it: operand traffic.  A k block of 32 moves 64 KB through L2
 // and shared memory for 783 tensor cycles.
@@ -37,9 +39,10 @@ constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3;
 constexpr int TILE_BYTES = BM * BK * 4;                      // 16 KB: one operand part
 constexpr int STAGE_BYTES = 4 * TILE_BYTES;                  // Ahi Alo Bhi Blo
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
-constexpr int THREADS = 192;
-constexpr int TMEM_COLS = 256;                               // two accumulators
-constexpr int kChunk = 2;                                    // k blocks per accumulator
+constexpr int EPI_WARPS = 8, EPI_COLS = 64;                  // epilogue warps, and real columns of each
+constexpr int THREADS = 32 * (EPI_WARPS + 2);
+constexpr int NACC = 2;                                      // accumulators (four: no faster)
+constexpr int TMEM_COLS = NACC * BN;
 
 enum : int { K_FULL = 0, K_A_LOWER = 1, K_LAUUM = 2, K_B_UPPER = 3 };
 
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const __grid_constant__ CUtensorMap mbhi, const __grid_constant__ CUtensorMap mblo, const Params p,
                 const int* stop) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], acc_full[NACC], acc_empty[NACC];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_fail, s_issued, s_consumed;
   if (cta_aborted(stop)) return;
@@ -97,7 +100,6 @@ __global__ void __launch_bounds__(THREADS, 1)
   int kb, ke;
   k_range(p, i0, j0, last ? p.k_last : p.k, kb, ke);
   const int nkb = ke > kb ? (ke - kb + BK - 1) / BK : 0;
-  const int nch = (nkb + kChunk - 1) / kChunk;
 
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -106,9 +108,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       tc::mbar_init(&full[s], 1);
       tc::mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < NACC; ++b) {
       tc::mbar_init(&acc_full[b], 1);
-      tc::mbar_init(&acc_empty[b], 4);
+      tc::mbar_init(&acc_empty[b], EPI_WARPS);
     }
     s_fail = 0;
     s_issued = 0;
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   tc::fence_after();
   const uint32_t tmem = tmem_slot;
 
-  if (warp == 4) {
+  if (warp == EPI_WARPS) {
     if (lane == 0) {                              // TMA producer
       const int ar = p.a_row0 + q * p.a_node + i0, br = p.b_row0 + q * p.b_node + j0;
       int kk = 0;
@@ -141,56 +143,54 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       s_issued = kk;
     }
-  } else if (warp == 5) {
+  } else if (warp == EPI_WARPS + 1) {
     if (lane == 0) {                              // MMA issuer
       int kk = 0;
       bool ok = true;
-      for (int c = 0; c < nch && ok; ++c) {
-        const int b = c & 1;
-        if (c >= 2 && !tc::mbar_wait(&acc_empty[b], ((c >> 1) & 1) ^ 1)) ok = false;
+      for (; kk < nkb; ++kk) {
+        const int b = kk % NACC, s = kk % STAGES;
+        if ((kk >= NACC && !tc::mbar_wait(&acc_empty[b], ((kk / NACC) & 1) ^ 1)) ||
+            !tc::mbar_wait(&full[s], (kk / STAGES) & 1)) {
+          ok = false;
+          break;
+        }
         tc::fence_after();
         const uint32_t d = tmem + b * BN;
-        for (int u = 0; u < kChunk && kk < nkb && ok; ++u, ++kk) {
-          const int s = kk % STAGES;
-          if (!tc::mbar_wait(&full[s], (kk / STAGES) & 1)) {
-            ok = false;
-            break;
-          }
-          tc::fence_after();
-          const uint32_t ah = tc::smem_u32(base + s * STAGE_BYTES), al = ah + TILE_BYTES, bh = al + TILE_BYTES,
-                         bl = bh + TILE_BYTES;
-          // the small products first: they meet a small accumulator
+        const uint32_t ah = tc::smem_u32(base + s * STAGE_BYTES), al = ah + TILE_BYTES, bh = al + TILE_BYTES,
+                       bl = bh + TILE_BYTES;
+        // the small products first: they meet a small accumulator
 #pragma unroll
-          for (int x = 0; x < BK * 4 / 32; ++x)
-            tc::mma<float>(d, tc::smem_desc(al + 32 * x), tc::smem_desc(bh + 32 * x), (u | x) != 0 ? 1u : 0u);
+        for (int x = 0; x < BK * 4 / 32; ++x)
+          tc::mma<float>(d, tc::smem_desc(al + 32 * x), tc::smem_desc(bh + 32 * x), x != 0 ? 1u : 0u);
 #pragma unroll
-          for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bl + 32 * x), 1u);
+        for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bl + 32 * x), 1u);
 #pragma unroll
-          for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bh + 32 * x), 1u);
-          tc::mma_commit(&empty[s]);
-        }
+        for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bh + 32 * x), 1u);
+        tc::mma_commit(&empty[s]);
         tc::mma_commit(&acc_full[b]);
       }
       if (!ok) s_fail = 1;
       s_consumed = kk;
     }
   } else {
-    // epilogue warps: 32 tile rows each, a row per lane, its 128 real columns in registers
-    float acc[BN];
+    // epilogue warps: 32 tile rows each (a row per lane), and half of their real columns in
+    // registers
+    const int wrow = 32 * (warp & 3), wcol = EPI_COLS * (warp >> 2);
+    float acc[EPI_COLS];
 #pragma unroll
-    for (int j = 0; j < BN; ++j) acc[j] = 0.f;
+    for (int j = 0; j < EPI_COLS; ++j) acc[j] = 0.f;
     bool ok = true;
 #pragma unroll 1
-    for (int c = 0; c < nch; ++c) {
-      const int b = c & 1;
-      if (!tc::mbar_wait(&acc_full[b], (c >> 1) & 1)) {
+    for (int kk = 0; kk < nkb; ++kk) {
+      const int b = kk % NACC;
+      if (!tc::mbar_wait(&acc_full[b], (kk / NACC) & 1)) {
         ok = false;
         break;
       }
       tc::fence_after();
-      const uint32_t src = tmem + b * BN + ((uint32_t)(32 * warp) << 16);
+      const uint32_t src = tmem + b * BN + wcol + ((uint32_t)wrow << 16);
 #pragma unroll
-      for (int g = 0; g < BN / 32; ++g) {
+      for (int g = 0; g < EPI_COLS / 32; ++g) {
         float v[32];
         tc::tmem_ld32(src + 32 * g, v);
 #pragma unroll
@@ -206,11 +206,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       // that the output loops are rolled, coalesced in either storage, and short.  Straight
       // code over 128 registers, with C read into them first, was bound by instruction
       // fetch: 26 us for a launch of one wave with k = 128.
-      float* st = reinterpret_cast<float*>(base) + warp * (BN * 33);     // st[col * 33 + row]
+      float* st = reinterpret_cast<float*>(base) + warp * (EPI_COLS * 33);     // st[col * 33 + row]
 #pragma unroll
-      for (int j = 0; j < BN; ++j) st[j * 33 + lane] = p.neg ? -acc[j] : acc[j];
+      for (int j = 0; j < EPI_COLS; ++j) st[j * 33 + lane] = p.neg ? -acc[j] : acc[j];
       __syncwarp();
-      const int r0 = i0 + 32 * warp, rows = min(32, m - r0), cols = min(BN, p.n - j0);
+      const int r0 = i0 + wrow, rows = min(32, m - r0), c0 = j0 + wcol, cols = min(EPI_COLS, p.n - c0);
       float* cq = p.c + (long long)q * p.c_node;
       // C(r, col) in floats: += (no load to wait for; one CTA owns the element) or =
       auto put = [&](float* o, float v) {
@@ -232,9 +232,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (p.xhi != nullptr) {
 #pragma unroll 2
         for (int r = 0; r < rows; ++r) {
-          const long long o = (long long)(q * p.a_node + r0 + r) * p.xld + j0;
+          const long long o = (long long)(q * p.a_node + r0 + r) * p.xld + c0;
 #pragma unroll
-          for (int u = 0; u < BN / 32; ++u) {
+          for (int u = 0; u < EPI_COLS / 32; ++u) {
             const int c = lane + 32 * u;
             if (c < cols) {
               const float x = st[c * 33 + r], h = round_tf32(x);
@@ -244,35 +244,35 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       } else if (p.rs == p.cx && p.cx == 1) {       // rows contiguous
-        float* o = cq + r0 + lane + (long long)j0 * p.cs;
+        float* o = cq + r0 + lane + (long long)c0 * p.cs;
         const int r = r0 + lane;
 #pragma unroll 4
         for (int c = 0; c < cols; ++c, o += p.cs)
-          if (lane < rows && keep(r, j0 + c)) put(o, st[c * 33 + lane]);
+          if (lane < rows && keep(r, c0 + c)) put(o, st[c * 33 + lane]);
       } else if (p.rs == p.cx) {                    // complex, rows contiguous: a row per lane
         const int r = r0 + lane;
-        float* o = cq + r * p.rs + (long long)(j0 >> 1) * p.cs;
+        float* o = cq + r * p.rs + (long long)(c0 >> 1) * p.cs;
 #pragma unroll 4
         for (int c = 0; c < cols; c += 2, o += p.cs)
-          if (lane < rows && keep(r, j0 + c)) put2(o, st[c * 33 + lane], st[(c + 1) * 33 + lane], r == ((j0 + c) >> 1));
+          if (lane < rows && keep(r, c0 + c)) put2(o, st[c * 33 + lane], st[(c + 1) * 33 + lane], r == ((c0 + c) >> 1));
       } else if (p.cx == 2) {                       // complex, columns contiguous: a column per lane
 #pragma unroll 2
         for (int r = 0; r < rows; ++r) {
-          float* o = cq + (r0 + r) * p.rs + j0;
+          float* o = cq + (r0 + r) * p.rs + c0;
 #pragma unroll
-          for (int u = 0; u < BN / 64; ++u) {
-            const int c = 2 * lane + 64 * u, col = j0 + c;
+          for (int u = 0; u < EPI_COLS / 64; ++u) {
+            const int c = 2 * lane + 64 * u, col = c0 + c;
             if (c < cols && keep(r0 + r, col)) put2(o + c, st[c * 33 + r], st[(c + 1) * 33 + r], r0 + r == (col >> 1));
           }
         }
       } else {                                      // columns contiguous
 #pragma unroll 2
         for (int r = 0; r < rows; ++r) {
-          float* o = cq + (r0 + r) * p.rs + j0;
+          float* o = cq + (r0 + r) * p.rs + c0;
 #pragma unroll
-          for (int u = 0; u < BN / 32; ++u) {
+          for (int u = 0; u < EPI_COLS / 32; ++u) {
             const int c = lane + 32 * u;
-            if (c < cols && keep(r0 + r, j0 + c)) put(o + c, st[c * 33 + r]);
+            if (c < cols && keep(r0 + r, c0 + c)) put(o + c, st[c * 33 + r]);
           }
         }
       }

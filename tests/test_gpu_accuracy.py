@@ -1,6 +1,9 @@
-"""Rounding errors of the panel kernels against wider arithmetic: the diagonal and the column
-scaling of a pivot, and the updates inside a diagonal block."""
+"""Rounding errors of the panel kernels and of the split TF32 products, against wider
+arithmetic: the diagonal and the column scaling of a pivot, the updates inside a diagonal
+block, and the FP32 inverse against the plain FP32 engine's."""
 from __future__ import annotations
+
+import os
 
 import numpy as np
 import pytest
@@ -82,3 +85,28 @@ def test_pivot_roots(handle, p, n):
         ref = b.astype(wide) / np.sqrt(d.astype(wide))
         assert np.max(np.abs(F[i + 1, i].astype(wide) / ref - 1)) <= bound
         assert np.count_nonzero(np.tril(F, -1)) == n // 2
+
+
+@pytest.mark.parametrize("n", [257, 300, 384, 513, 1000])
+@pytest.mark.parametrize("p", "sc")
+def test_split_inverse_no_worse_than_simt(handle, p, n):
+    """?potri of the same factor on the TF32 tensor cores and on the FP32 engine: the split
+    products' sums, rounded to nearest every 32 k, err no more than one FMA chain per element."""
+    os.environ["CUCHOLESKY_FORCE_SIMT"] = "1"
+    try:
+        simt = cc.Handle()
+    finally:
+        del os.environ["CUCHOLESKY_FORCE_SIMT"]
+    err = {}
+    for seed in range(3):
+        L = np.linalg.cholesky(_matrix(p, n, seed).astype(np.complex128 if p == "c" else np.float64))
+        T = np.asfortranarray(L.astype(matgen.dtype_of(p)))
+        W = np.linalg.inv(T.astype(L.dtype))
+        ref = np.tril(W.conj().T @ W)
+        for name, h in (("split", handle), ("simt", simt)):
+            D = cc.to_device_colmajor(T)
+            assert cc.potri(h, D, n) == 0
+            got = np.tril(cc.to_host_colmajor(D)).astype(L.dtype)
+            err.setdefault(name, []).append(np.linalg.norm(got - ref) / np.linalg.norm(ref))
+    simt.close()
+    assert np.mean(err["split"]) <= 1.05 * np.mean(err["simt"]), err
