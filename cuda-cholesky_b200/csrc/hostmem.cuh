@@ -184,6 +184,27 @@ inline bool host_args(const char* name, size_t n, size_t lda, long pos, long* in
   return true;
 }
 
+// Whether the panels of the FP32 matrix A may use split products, from the whole diagonal,
+// which no panel holds: read here, or on the GPU when A is not in host memory.
+template <typename T>
+CUresult host_split(CULAPACKhandle h, const T* A, size_t lda, size_t n, Split* split) {
+  cudaPointerAttributes a;
+  CUCHOL_CHECK(cudaPointerGetAttributes(&a, A));
+  bool ok = true;
+  if (a.type == cudaMemoryTypeHost) {
+    for (size_t i = 0; i < n; ++i) ok = ok && tcg::diag_in_range(re(A[i * (lda + 1)]));
+  } else {
+    tcg::diag_range_kernel<<<1, 1024, 0, h->s_panel>>>(reinterpret_cast<const float*>(A),
+                                                       (long long)(lda + 1) * real_per<T>(), (int)n, h->d_words, h->d_logdet);
+    ++h->launches;
+    CUCHOL_CHECK(cudaGetLastError());
+    CUCHOL_CHECK_CU(fetch_words(h, h->s_panel));
+    ok = h->h_words[0] == 0;
+  }
+  *split = ok ? Split::YES : Split::NO;
+  return CUDA_SUCCESS;
+}
+
 template <typename T>
 CUresult host_potrf_run(CUmultiGPULAPACKhandle hh, bool upper, size_t n, T* A, size_t lda, long* info) {
   CULAPACKhandle h = hh->h;
@@ -211,6 +232,8 @@ CUresult host_potrf_run(CUmultiGPULAPACKhandle hh, bool upper, size_t n, T* A, s
     CUCHOL_CHECK_CU(copy_panel<T>(D, ldd, A, lda, n, upper, plan[r], plan[r + 1], hh->s_copy, &hh->h2d_bytes));
     CUCHOL_CHECK(cudaEventRecord(hh->ev_in[r], hh->s_copy));
   }
+  Split split = Split::NO;
+  if constexpr (is_fp32<T>()) CUCHOL_CHECK_CU(host_split<T>(h, A, lda, n, &split));
   while (hh->ev_a.size() < panels) {
     cudaEvent_t e;
     CUCHOL_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -276,7 +299,7 @@ CUresult host_potrf_run(CUmultiGPULAPACKhandle hh, bool upper, size_t n, T* A, s
     };
     long pinfo = 0;
     CUCHOL_CHECK_CU(potrf_run<T>(h, upper, (int)(n - c0), at(c0, c0), (long long)ldd, &pinfo, nullptr, &back,
-                                 (int)w));
+                                 (int)w, split));
     if (pinfo != 0) {
       *info = (long)c0 + pinfo;
       return CUDA_SUCCESS;

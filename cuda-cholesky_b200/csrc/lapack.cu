@@ -781,9 +781,14 @@ using FinalColumns = std::function<CUresult(int c, int jb, cudaStream_t s)>;
 // wait costs more than the overlap gives.
 constexpr int kOneStreamOrder = 1536;
 
+// Whether the FP32 types' updates may run as split products (tcg::diag_in_range): CHECK
+// looks at A's diagonal on the GPU and, out of range, starts over on the SIMT engine with A
+// untouched; a caller that hands over a part of a matrix has looked itself.
+enum class Split { CHECK, YES, NO };
+
 template <typename T>
 CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, long* info, double* logdet_out,
-                   const FinalColumns* on_final = nullptr, int ncols = -1) {
+                   const FinalColumns* on_final = nullptr, int ncols = -1, Split split = Split::CHECK) {
   if (ncols < 0 || ncols > n) ncols = n;
   constexpr int nb = Tune<T>::nb;
   // outer block: sub diagonal blocks, from the handle's override or the tuning table
@@ -804,7 +809,8 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   // TMA clips its last row piece to 16 bytes, not to elements, and would add to the
   // padding rows below an order that is not a multiple of four.
   constexpr int cx = real_per<T>();
-  const bool tc3 = is_fp32<T>() && !h->force_simt && n > 128;
+  const bool tc3 = is_fp32<T>() && !h->force_simt && n > 128 && split != Split::NO;
+  const bool check = tc3 && split == Split::CHECK;
   const bool tc3_tma = tc3 && n % 4 == 0 && tc3_usable(reinterpret_cast<const float*>(A), lda);
   const long long ldq = (long long)round_up((size_t)NB, 32) * cx;
   const size_t qsize = (size_t)n * cx * ldq;   // floats of one buffer
@@ -820,8 +826,13 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   float* qbuf[4];
   for (int i = 0; i < 4; ++i) qbuf[i] = static_cast<float*>(h->ws) + i * qsize;
 
-  // the first diagonal kernel writes the info word and the log det, the later ones read
-  // and add to them; the update stream starts behind a panel event
+  // the range check or else the first diagonal kernel writes the info word and the log det,
+  // the later ones read and add to them; the update stream starts behind a panel event
+  if (check) {
+    tcg::diag_range_kernel<<<1, 1024, 0, sp>>>(reinterpret_cast<const float*>(A), (rs + cs) * cx, n, d_info, h->d_logdet);
+    ++h->launches;
+    CUCHOL_CHECK(cudaGetLastError());
+  }
   if (!alone) CUCHOL_CHECK(cudaEventRecord(h->ev_update, sp));
 
   const T minus_one = from_real<T>(RealOf<T>(-1)), one = from_real<T>(RealOf<T>(1));
@@ -866,17 +877,17 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
         if constexpr (is_fp32<T>()) {
           const long long qo = (long long)s0 * cx * ldq + s0 * cx;
           CUCHOL_CHECK_CU((panel_fused<T, T, float, OUT_SPLIT, nb>(h, at(c, c), mr, rs, cs, Qh + qo, ldq, 1, Ql + qo, D, c,
-                                                                c == 0, h->d_logdet, sp)));
+                                                                !check && c == 0, h->d_logdet, sp)));
         }
         if constexpr (!is_fp32<T>())
           CUCHOL_CHECK_CU((panel_fused<T, T, T, OUT_COPY, nb>(h, at(c, c), mr, rs, cs, P + s0 + (long long)s0 * ldp, 1, ldp,
-                                                           nullptr, D, c, c == 0, h->d_logdet, sp)));
+                                                           nullptr, D, c, !check && c == 0, h->d_logdet, sp)));
         if (on_final) {              // the block column goes to the caller now
           CUCHOL_CHECK_CU((copy_diag<T, nb>(h, dbuf, A, rs, cs, dfirst, c / nb, 1, sp)));
           dfirst = -1;
         }
       } else {
-        CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, c == 0, h->d_logdet, sp)));
+        CUCHOL_CHECK_CU((diag_factor<T, T, nb>(h, at(c, c), rs, cs, jb, c, !check && c == 0, h->d_logdet, sp)));
       }
       if (mr == 0) {
         if (on_final) CUCHOL_CHECK_CU((*on_final)(c, jb, sp));
@@ -927,6 +938,8 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   }
   if (dfirst >= 0) CUCHOL_CHECK_CU((copy_diag<T, nb>(h, dbuf, A, rs, cs, dfirst, dfirst, dnext - dfirst, sp)));
   CUCHOL_CHECK_CU(fetch_words(h, sp));
+  if (check && h->h_words[0] == tcg::kOutOfRange)
+    return potrf_run<T>(h, upper, n, A, lda, info, logdet_out, on_final, ncols, Split::NO);
   *info = h->h_words[0];
   if (logdet_out != nullptr) *logdet_out = h->h_logdet[0];
   return CUDA_SUCCESS;

@@ -395,5 +395,31 @@ __global__ void __launch_bounds__(256) range_kernel(const float* __restrict__ a,
   if (!ok) atomicExch(bad, 1);
 }
 
+// Range of ?potrf's split products, read off the diagonal of A: |l_ij|^2 <= a_ii, so in a
+// factorization that succeeds
+//   no value overflows while a_ii <= 2^126;
+//   what the hi lo products and the FP32 output drop below 2^-126 is at most 2^-126 per product,
+//   which for fewer than 2^20 of them stays under the FP32 rounding 2^-24 sqrt(a_ii a_jj)
+//   while a_ii >= 2^-80.
+// Entries that are not positive end the factorization at their column or before, whatever
+// the products of their rows are.
+constexpr float kDiagMin = 0x1p-80f, kDiagMax = 0x1p126f;
+__host__ __device__ inline bool diag_in_range(float d) { return !(d > 0.f) || (d >= kDiagMin && d <= kDiagMax); }
+
+// Starts a factorization's words: info := 0, or kOutOfRange (which the kernels that follow take
+// for a failure, so they leave A as it is), and log det := 0.  One CTA.
+constexpr int kOutOfRange = -1;
+__global__ void __launch_bounds__(1024) diag_range_kernel(const float* __restrict__ a, long long stride, int n,
+                                                          int* __restrict__ info, double* __restrict__ logdet) {
+  bool bad = false;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += 1024) bad |= !diag_in_range(a[i * stride]);
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    *info = any ? kOutOfRange : 0;
+    *logdet = 0.0;
+  }
+}
+
 }  // namespace tcg
 }  // namespace cuchol

@@ -1,0 +1,101 @@
+"""Calls at the limits of the kernels they would take: ranges of FP32 entries, memory that is
+refused or tight, failing pivots on either side of a launch rule."""
+from __future__ import annotations
+
+import os
+
+import numpy as np
+import pytest
+
+import cucholesky as cc
+from cucholesky import matgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def simt():
+    """A handle whose products all run on the plain FP32 engine."""
+    os.environ["CUCHOLESKY_FORCE_SIMT"] = "1"
+    try:
+        h = cc.Handle()
+    finally:
+        del os.environ["CUCHOLESKY_FORCE_SIMT"]
+    yield h
+    h.close()
+
+
+def _factor_error(A, F, uplo):
+    """|F - L| / |L| against FP64 (A and F as numpy arrays of an FP32 type)."""
+    w = np.complex128 if np.iscomplexobj(A) else np.float64
+    L = np.linalg.cholesky(A.astype(w))
+    F = np.tril(F) if uplo == "L" else np.triu(F).conj().T
+    return np.linalg.norm(F.astype(w) - L) / np.linalg.norm(L)
+
+
+# Split products lose what falls below 2^-126: entries about 2^-110 are where that shows
+# first (3e-6), entries above 2^126 overflow.  Both take the FP32 engine, bit for bit.
+@pytest.mark.parametrize("case", ["small", "one small row", "large", "infinite"])
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("p,uplo,n", [("s", "L", 300), ("s", "U", 700), ("c", "L", 300), ("c", "U", 700)])
+def test_potrf_range_rule(handle, simt, p, uplo, n, pad, case):
+    A = matgen.spd(p, n, seed=n)
+    A = A / np.abs(np.diag(A)).max()
+    if case == "one small row":
+        A[n // 2] *= np.float32(2.0 ** -55)
+        A[:, n // 2] *= np.float32(2.0 ** -55)
+    elif case == "small":
+        A = A * np.float32(2.0 ** -110)
+    elif case == "large":
+        A = A * np.float32(2.0 ** 127)
+    else:
+        A[n // 2, n // 2] = np.inf
+    T = np.zeros((n + pad, n), A.dtype, order="F")
+    T[:n] = A
+    out = []
+    for h in (handle, simt):
+        D = cc.to_device_colmajor(T)
+        info = cc.potrf(h, D, n, uplo)
+        out.append((info, cc.to_host_colmajor(D)))
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1], equal_nan=True)
+    if case in ("small", "large"):
+        assert out[0][0] == 0 and _factor_error(A, out[0][1][:n], uplo) <= 4 * 2.0 ** -24
+    # a failing pivot is found all the same
+    k = n - 5
+    B = T.copy(order="F")
+    B[k, k] = -1.0
+    if case != "infinite":
+        assert cc.potrf(handle, cc.to_device_colmajor(B), n, uplo) == k + 1
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -79, 2.0 ** 125])
+@pytest.mark.parametrize("p,n", [("s", 301), ("c", 300)])
+def test_potrf_split_products_within_range(handle, p, n, scale):
+    """Just inside the range the error is that of the unscaled matrix (powers of two are exact)."""
+    A = matgen.spd(p, n, seed=n)
+    A = (A / np.abs(np.diag(A)).max()).astype(A.dtype)   # the diagonal at most 1
+    A[np.arange(n), np.arange(n)] = np.maximum(np.diag(A).real, 0.5)
+    err = []
+    for s in (1.0, scale):
+        D = cc.to_device_colmajor(np.asfortranarray((A * s).astype(A.dtype)))
+        assert cc.potrf(handle, D, n) == 0
+        err.append(_factor_error(A * s if s == 1.0 else (A * s).astype(A.dtype), cc.to_host_colmajor(D), "L"))
+    assert err[1] <= 1.1 * err[0] + 2.0 ** -26
+
+
+@pytest.mark.parametrize("memory", ["pinned", "device"])
+@pytest.mark.parametrize("p,uplo", [("s", "U"), ("c", "L")])
+def test_host_potrf_range_rule(p, uplo, memory):
+    """The streamed host-memory factor (n >= 2048: a panel, then the rest) of small entries."""
+    import torch
+    n = 2100
+    A = matgen.spd(p, n, seed=4)
+    A = (A * np.float32(2.0 ** -110)).astype(A.dtype)
+    T = torch.from_numpy(np.ascontiguousarray(A.T))
+    T = T.pin_memory() if memory == "pinned" else T.cuda()
+    gpus = cc.MultiGPU([0])
+    hh = cc.HostHandle(gpus)
+    rc, info = cc.call_host(hh, p.upper(), "potrf", uplo, n, T.data_ptr(), n)
+    torch.cuda.synchronize()
+    assert rc == 0 and info == 0
+    assert _factor_error(A, T.cpu().numpy().T, uplo) <= 4 * 2.0 ** -24
