@@ -727,9 +727,9 @@ CUresult tcg_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
 // Grows the workspace like ensure_workspace, but an allocation that fails is not an
 // error: false, and the caller takes a path that needs less.
 constexpr size_t kTcgWorkspace = size_t(8) << 30;
-bool try_workspace(CULAPACKhandle h, size_t bytes) {
+bool try_workspace(CULAPACKhandle h, size_t bytes, size_t limit = kTcgWorkspace) {
   if (bytes <= h->ws_bytes) return true;
-  if (bytes > kTcgWorkspace || cudaStreamSynchronize(h->s_panel) != cudaSuccess ||
+  if (bytes > limit || cudaStreamSynchronize(h->s_panel) != cudaSuccess ||
       cudaStreamSynchronize(h->s_update) != cudaSuccess)
     return false;
   void* p = nullptr;
@@ -809,17 +809,20 @@ CUresult potrf_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, lon
   // TMA clips its last row piece to 16 bytes, not to elements, and would add to the
   // padding rows below an order that is not a multiple of four.
   constexpr int cx = real_per<T>();
-  const bool tc3 = is_fp32<T>() && !h->force_simt && n > 128 && split != Split::NO;
-  const bool check = tc3 && split == Split::CHECK;
-  const bool tc3_tma = tc3 && n % 4 == 0 && tc3_usable(reinterpret_cast<const float*>(A), lda);
+  bool tc3 = is_fp32<T>() && !h->force_simt && n > 128 && split != Split::NO;
+  const bool tc3_tma = tc3 && cx == 1 && n % 4 == 0 && tc3_usable(reinterpret_cast<const float*>(A), lda);
   const long long ldq = (long long)round_up((size_t)NB, 32) * cx;
   const size_t qsize = (size_t)n * cx * ldq;   // floats of one buffer
-  const size_t ws = round_up(tc3 ? sizeof(float) * 4 * qsize : sizeof(T) * (2 * (size_t)ldp * NB), 256);
   // one launch per diagonal block and its rows while those fill at most one CTA per SM;
   // its factors wait in D
   const int fused_rows = kFusedRows * h->num_sms;
-  const size_t dblocks = (size_t)(std::min(n, fused_rows + nb) / nb + 1);
-  CUCHOL_CHECK_CU(ensure_workspace(h, ws + sizeof(T) * dblocks * nb * nb));
+  const size_t dbytes = sizeof(T) * (size_t)(std::min(n, fused_rows + nb) / nb + 1) * nb * nb;
+  auto panels = [&](bool q) { return round_up(q ? sizeof(float) * 4 * qsize : sizeof(T) * (2 * (size_t)ldp * NB), 256); };
+  // complex splits take four times the memory of P: refused, the SIMT engine's updates
+  if (tc3 && !tc3_tma) tc3 = try_workspace(h, panels(true) + dbytes, SIZE_MAX);
+  const size_t ws = panels(tc3);
+  CUCHOL_CHECK_CU(ensure_workspace(h, ws + dbytes));
+  const bool check = tc3 && split == Split::CHECK;
   int dfirst = -1, dnext = -1;   // diagonal blocks whose factors are in D (block b in slot b - dfirst)
   T* dbuf = reinterpret_cast<T*>(static_cast<char*>(h->ws) + ws);
   T* pbuf[2] = {static_cast<T*>(h->ws), static_cast<T*>(h->ws) + (size_t)ldp * NB};

@@ -99,3 +99,27 @@ def test_host_potrf_range_rule(p, uplo, memory):
     torch.cuda.synchronize()
     assert rc == 0 and info == 0
     assert _factor_error(A, T.cpu().numpy().T, uplo) <= 4 * 2.0 ** -24
+
+
+def _refuse_allocation(after):
+    import ctypes as C
+    f = cc.lib().cuLAPACKFailAllocation
+    f.argtypes, f.restype = [C.c_int], C.c_int
+    assert f(after) == 0
+
+
+@pytest.mark.parametrize("p,pad", [("c", 0), ("s", 1)])
+def test_potrf_without_memory_for_the_splits(simt, p, pad):
+    """The operand splits take more memory than the panel: refused, the call still succeeds."""
+    n = 300
+    T = matgen.spd(p, n, seed=6, lda=n + pad)
+    h = cc.Handle()
+    D, S = cc.to_device_colmajor(T), cc.to_device_colmajor(T)
+    _refuse_allocation(0)
+    try:
+        assert cc.potrf(h, D, n) == 0
+    finally:
+        _refuse_allocation(-1)
+    assert cc.potrf(simt, S, n) == 0
+    assert np.array_equal(cc.to_host_colmajor(D), cc.to_host_colmajor(S))
+    h.close()
