@@ -647,11 +647,12 @@ template <typename T> constexpr bool is_fp32() { return std::is_same<T, float>::
 template <typename T> constexpr int real_per() { return Traits<T>::complex ? 2 : 1; }
 
 // A pack (k-major, `rows` rows of pitch ld floats) as a TMA map of 128-row x 32-k tiles;
-// step 2 takes every other row (the A form of a complex B pack).
-bool make_pack_map(CUtensorMap* map, const float* base, long long rows, long long ld, int step) {
+// step 2 takes every other row (the A form of a complex B pack).  skip: the base lies that
+// many floats into the first row.
+bool make_pack_map(CUtensorMap* map, const float* base, long long rows, long long ld, int step, long long skip) {
   EncodeTiledFn fn = encode_tiled();
   if (fn == nullptr) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)((rows + step - 1) / step)};
+  const cuuint64_t dims[2] = {(cuuint64_t)(ld - skip), (cuuint64_t)((rows + step - 1) / step)};
   const cuuint64_t str[1] = {(cuuint64_t)ld * step * sizeof(float)};
   const cuuint32_t box[2] = {(cuuint32_t)tcg::BK, (cuuint32_t)tcg::BM}, es[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, str, box, es,
@@ -659,13 +660,15 @@ bool make_pack_map(CUtensorMap* map, const float* base, long long rows, long lon
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct PackRef { const float *hi, *lo; long long rows, ld; int step; };
+struct PackRef { const float *hi, *lo; long long rows, ld; int step; long long skip = 0; };
 
 CUresult tcg_launch(CULAPACKhandle h, const PackRef& A, const PackRef& B, tcg::Params p, cudaStream_t s,
                     const int* stop) {
   CUtensorMap ah, al, bh, bl;
-  if (!make_pack_map(&ah, A.hi, A.rows, A.ld, A.step) || !make_pack_map(&al, A.lo, A.rows, A.ld, A.step) ||
-      !make_pack_map(&bh, B.hi, B.rows, B.ld, B.step) || !make_pack_map(&bl, B.lo, B.rows, B.ld, B.step))
+  auto maps = [](CUtensorMap* hi, CUtensorMap* lo, const PackRef& r) {
+    return make_pack_map(hi, r.hi, r.rows, r.ld, r.step, r.skip) && make_pack_map(lo, r.lo, r.rows, r.ld, r.step, r.skip);
+  };
+  if (!maps(&ah, &al, A) || !maps(&bh, &bl, B))
     return CUDA_ERROR_INVALID_VALUE;
   p.tiles_m = (p.m + tcg::BM - 1) / tcg::BM;
   p.tiles_n = (p.n + tcg::BN - 1) / tcg::BN;
@@ -1005,15 +1008,42 @@ CUresult tcg_in_range(CULAPACKhandle h, const T* A, long long rs, long long cs, 
 // Levels s < order only.
 inline int level_pairs(int n, int s) { return (n - s + 2 * s - 1) / (2 * s); }
 
+// Level s of the FP32 levels: pairs, rows of the last pair's lower block, and its buffers in
+// floats (each twice, hi and lo), all k-major:
+//   ia  inv(T22), s rows per pair (the last one its own), pitch ldk
+//   x   X, the same rows, pitch s cx
+//   b1  T21^T, cx rows per column, pitch ldk
+//   b2  inv(T11)^T of `cols` columns at a time, cx rows per column, pitch s cx
+// The last pair may have one row below s columns: its inv(T22) and T21^T are as narrow, and
+// b2, all of T11 then, is split into column pieces above kTcgWorkspace.  (Every pair sized
+// s x s: strtri n = 16385 8 GiB, now 2.1; ctrtri 24 GiB, now 6.)
+template <typename T>
+struct TcgLevel {
+  int np, s2, cols;
+  long long ldk, ldx;
+  size_t rows, ia, x, b1, b2;
+  TcgLevel(int n, int s) : np(level_pairs(n, s)), s2(std::min(s, n - 2 * s * (np - 1) - s)), cols(s) {
+    constexpr int cx = real_per<T>();
+    ldk = cx * (np > 1 ? (long long)s : (long long)round_up((size_t)s2, 32));
+    ldx = (long long)s * cx;
+    rows = (size_t)(np - 1) * s + s2;
+    ia = rows * ldk;
+    x = rows * ldx;
+    b1 = (size_t)np * s * cx * ldk;
+    b2 = (size_t)np * cols * cx * ldx;
+    while (bytes() > kTcgWorkspace && cols > 4096) {
+      cols /= 2;
+      b2 /= 2;
+    }
+  }
+  size_t bytes() const { return sizeof(float) * 2 * (ia + x + b1 + b2); }
+};
+
 template <typename T>
 size_t trtri_levels_bytes(int n, int order) {
-  // per level: inv(T22) and X (pairs * s rows), T21^T and inv(T11)^T (cx rows per row), all
-  // of pitch s * cx, hi and lo
-  constexpr int cx = real_per<T>();
   size_t need = 0;
-  for (int s = Tune<T>::nb; s < std::min(n, order); s *= 2)
-    need = std::max(need, (size_t)level_pairs(n, s) * s * s * cx * (2 + 2 * cx) * 2);
-  return sizeof(float) * need;
+  for (int s = Tune<T>::nb; s < std::min(n, order); s *= 2) need = std::max(need, TcgLevel<T>(n, s).bytes());
+  return need;
 }
 
 template <typename T>
@@ -1025,52 +1055,69 @@ CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs
   cudaStream_t sp = h->s_panel;
   float* a = reinterpret_cast<float*>(A);
   for (int s = nb; s < std::min(n, order); s *= 2) {
-    const int np = level_pairs(n, s), s2_last = std::min(s, n - 2 * s * (np - 1) - s);
-    const long long ld = (long long)s * cx;
-    const size_t rows = (size_t)np * s, one = rows * ld;
-    float* w = static_cast<float*>(h->ws);
-    float *ia = w, *x = w + 2 * one, *b1 = w + 4 * one, *b2 = b1 + 2 * one * cx;   // each: hi, then lo
+    const TcgLevel<T> L(n, s);
+    const int m = L.np > 1 ? s : L.s2;
+    float *ia = static_cast<float*>(h->ws), *x = ia + 2 * L.ia, *b1 = x + 2 * L.x, *b2 = b1 + 2 * L.b1;   // each: hi, then lo
     auto at = [&](long long i, long long j) { return a + (i * rs + j * cs) * cx; };
     tcg::Packs ps{};
-    ps.count = 3;
-    for (int i = 0; i < 3; ++i) {
-      tcg::Pack& p = ps.p[i];
+    ps.count = 2;
+    for (tcg::Pack& p : ps.p) {
       p.cx = cx;
-      p.nodes = np;
+      p.nodes = L.np;
       p.node_rows = s;
       p.src_node = 2LL * s * (rs + cs) * cx;
-      p.ld = ld;
       p.rows = p.rows_last = p.kk = p.kk_last = s;
     }
     tcg::Pack& p0 = ps.p[0];                    // A(i, k) = inv(T22)(i, k)
     p0.src = at(s, s); p0.rs = rs * cx; p0.cs = cs * cx; p0.tri = TRI_LOWER; p0.unit = unit;
-    p0.rows_last = p0.kk_last = s2_last;
-    p0.hi = ia; p0.lo = ia + one;
+    p0.rows = p0.kk = m;
+    p0.rows_last = p0.kk_last = L.s2;
+    p0.hi = ia; p0.lo = ia + L.ia; p0.ld = L.ldk;
     tcg::Pack& p1 = ps.p[1];                    // B(j, k) = T21(k, j)
     p1.src = at(s, 0); p1.rs = cs * cx; p1.cs = rs * cx; p1.two = cx == 2;
-    p1.kk_last = s2_last;
-    p1.hi = b1; p1.lo = b1 + one * cx;
-    tcg::Pack& p2 = ps.p[2];                    // B(j, k) = inv(T11)(k, j)
-    p2.src = at(0, 0); p2.rs = cs * cx; p2.cs = rs * cx; p2.two = cx == 2; p2.tri = TRI_UPPER; p2.unit = unit;
-    p2.hi = b2; p2.lo = b2 + one * cx;
+    p1.kk = m;
+    p1.kk_last = L.s2;
+    p1.hi = b1; p1.lo = b1 + L.b1; p1.ld = L.ldk;
+    tcg::Pack& p2 = ps.p[2];                    // B(j, k) = inv(T11)(k, j), columns from j0
+    p2.rs = cs * cx; p2.cs = rs * cx; p2.two = cx == 2; p2.tri = TRI_UPPER; p2.unit = unit;
+    p2.src = at(0, 0);
+    p2.rows = p2.rows_last = p2.node_rows = L.cols;
+    p2.hi = b2; p2.lo = b2 + L.b2; p2.ld = L.ldx;
+    if (L.cols == s) ps.count = 3;
     CUCHOL_CHECK_CU(pack_launch(h, ps, sp));
     tcg::Params g{};
-    g.nodes = np;
-    g.m = s; g.m_last = s2_last; g.n = s * cx;
+    g.nodes = L.np;
+    g.m = m; g.m_last = L.s2; g.n = s * cx;
     g.cx = cx;
     g.a_node = s; g.b_node = s * cx;
     g.kmode = tcg::K_A_LOWER;
-    g.k = s * cx; g.k_last = s2_last * cx;
-    g.xhi = x; g.xlo = x + one; g.xld = ld;
-    const PackRef rb1{b1, b1 + one * cx, (long long)rows * cx, ld, 1}, rb2{b2, b2 + one * cx, (long long)rows * cx, ld, 1};
-    CUCHOL_CHECK_CU(tcg_launch(h, PackRef{ia, ia + one, (long long)rows, ld, 1}, rb1, g, sp, nullptr));
+    g.k = m * cx; g.k_last = L.s2 * cx;
+    g.xhi = x; g.xlo = x + L.x; g.xld = L.ldx;
+    const long long rows = (long long)L.rows;
+    CUCHOL_CHECK_CU(tcg_launch(h, PackRef{ia, ia + L.ia, rows, L.ldk, 1},
+                               PackRef{b1, b1 + L.b1, (long long)L.np * s * cx, L.ldk, 1}, g, sp, nullptr));
     g.xhi = g.xlo = nullptr;
     g.kmode = tcg::K_B_UPPER;
-    g.k_last = g.k;
-    g.c = at(s, 0);
+    g.n = L.cols * cx;
+    g.b_node = L.cols * cx;
     g.rs = rs * cx; g.cs = cs * cx; g.c_node = p0.src_node;
     g.neg = 1;
-    CUCHOL_CHECK_CU(tcg_launch(h, PackRef{x, x + one, (long long)rows, ld, 1}, rb2, g, sp, nullptr));
+    for (int j0 = 0; j0 < s; j0 += L.cols) {
+      if (L.cols < s) {
+        tcg::Packs piece{};
+        piece.count = 1;
+        piece.p[0] = p2;
+        piece.p[0].src = at(j0, j0);
+        piece.p[0].kk = piece.p[0].kk_last = s - j0;
+        CUCHOL_CHECK_CU(pack_launch(h, piece, sp));
+      }
+      // X from its column j0 on: inv(T11) is zero above its diagonal
+      g.k = g.k_last = (s - j0) * cx;
+      g.c = at(s, j0);
+      const float* xj = x + (long long)j0 * cx;
+      CUCHOL_CHECK_CU(tcg_launch(h, PackRef{xj, xj + L.x, rows, L.ldx, 1, (long long)j0 * cx},
+                                 PackRef{b2, b2 + L.b2, (long long)L.np * L.cols * cx, L.ldx, 1}, g, sp, nullptr));
+    }
   }
   return fetch_words(h, sp);
 }
@@ -1098,6 +1145,28 @@ CUresult gemm_nodes(CULAPACKhandle h, const GemmProblem<T>& p, const NodeLaunch&
 // workspace (the X of pair q are rows q s .. of it) and T21 := -X inv(T11).  One launch
 // per pair and product, as the recursive splits took for up to eight pairs, ran small
 // levels one after the other on a nearly idle GPU: n = 2048 30 launches, 970 us.
+// Rows of the X of level s (even: an operand's pitch).
+inline long long fp64_level_rows(int n, int s) {
+  const int np = level_pairs(n, s);
+  return (long long)round_up((size_t)(np - 1) * s + std::min(s, n - 2 * s * (np - 1) - s), 2);
+}
+template <typename T>
+size_t fp64_levels_elements(int n) {
+  size_t x = 0;
+  for (int s = Tune<T>::nb; s < n; s *= 2) x = std::max(x, (size_t)fp64_level_rows(n, s) * s);
+  return x;
+}
+
+// Workspace of ?trtri's level launches (FP64: with an aligned copy of the triangle when A itself
+// is not), 0 for the orders and handles that do not take them.
+template <typename T>
+size_t trtri_scratch(CULAPACKhandle h, int n, const T* A, long long lda) {
+  if (h->force_simt) return 0;
+  if (is_fp32<T>()) return n >= tcg_min_order<T>() ? trtri_levels_bytes<T>(n, n) : 0;
+  if (n <= Tune<T>::nb) return 0;
+  return sizeof(T) * (fp64_levels_elements<T>(n) + (fp64_aligned(A, lda) ? 0 : round_up((size_t)n, 2) * n));
+}
+
 template <typename T>
 CUresult trtri_levels_fp64(CULAPACKhandle h, bool unit, int n, T* A, long long lda, bool upper, T* X, cudaStream_t sp) {
   constexpr int nb = Tune<T>::nb;
@@ -1105,7 +1174,7 @@ CUresult trtri_levels_fp64(CULAPACKhandle h, bool unit, int n, T* A, long long l
   for (int s = nb; s < n; s *= 2) {
     const int np = level_pairs(n, s), s2 = std::min(s, n - 2 * s * (np - 1) - s);
     const int m = np > 1 ? s : s2;
-    const long long ldx = (long long)np * s;
+    const long long ldx = fp64_level_rows(n, s);
     NodeLaunch nl{};
     nl.nd.count = np;
     nl.nd.m_last = s2;
@@ -1169,13 +1238,11 @@ CUresult trtri_run(CULAPACKhandle h, bool upper, bool unit, int n, T* A, long lo
 
   if constexpr (is_fp64<T>()) {
     if (!h->force_simt && n > nb) {
-      // X of the largest level, and an aligned copy of the triangle when A itself is not
-      size_t x = 0;
-      for (int s = nb; s < n; s *= 2) x = std::max(x, (size_t)level_pairs(n, s) * s * s);
+      // X of the largest level, and the copy
+      const size_t x = fp64_levels_elements<T>(n);
       const bool direct = fp64_aligned(A, lda);
       const long long ldc = (long long)round_up((size_t)n, 2);
-      const size_t need = sizeof(T) * (x + (direct ? 0 : (size_t)ldc * n));
-      if (try_workspace(h, need)) {
+      if (try_workspace(h, trtri_scratch<T>(h, n, A, lda))) {
         T* X = static_cast<T*>(h->ws);
         T* W = direct ? A : X + x;
         if (!direct) CUCHOL_CHECK_CU(copy_view<T>(h, A, rs, cs, W, upper ? ldc : 1, upper ? 1 : ldc, n, n, true, sp, nullptr));

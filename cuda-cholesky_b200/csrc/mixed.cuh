@@ -1329,11 +1329,15 @@ CUresult mixed_refactor(CUcholMixed p, long* info) {
       p->Dinv, 1, NBT, n, SB, 0);
   ++h->launches;
   CUCHOL_CHECK(cudaGetLastError());
-  bool leveled = false;
-  CUCHOL_CHECK_CU(trtri_levels_tcg<float>(h, false, n, p->Dinv, 1, NBT, NBT, &leveled));
-  if (!leveled) {
-    CUCHOL_CHECK_CU(ensure_workspace(h, trtri_levels_bytes<float>(n, NBT)));
-    CUCHOL_CHECK_CU(trtri_levels_tcg<float>(h, false, n, p->Dinv, 1, NBT, NBT, &leveled));
+  // all blocks at once, or as many as there is memory for
+  auto bytes = [&](int blocks) { return trtri_levels_bytes<float>(std::min(n, blocks * NBT), NBT); };
+  int per = nT;
+  while (per > 1 && !try_workspace(h, bytes(per))) per = (per + 1) / 2;
+  CUCHOL_CHECK_CU(ensure_workspace(h, bytes(per)));
+  for (int I = 0; I < nT; I += per) {
+    bool done = false;
+    CUCHOL_CHECK_CU(trtri_levels_tcg<float>(h, false, std::min(n - I * NBT, per * NBT),
+                                            p->Dinv + (size_t)I * NBT * (NBT + 1), 1, NBT, NBT, &done));
   }
   CUCHOL_CHECK(cudaStreamSynchronize(sp));
   *info = 0;

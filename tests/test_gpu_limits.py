@@ -123,3 +123,62 @@ def test_potrf_without_memory_for_the_splits(simt, p, pad):
     assert cc.potrf(simt, S, n) == 0
     assert np.array_equal(cc.to_host_colmajor(D), cc.to_host_colmajor(S))
     h.close()
+
+
+def _held_after(call):
+    """Device memory that a fresh handle holds after call(handle)."""
+    import torch
+    h = cc.Handle()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    call(h)
+    torch.cuda.synchronize()
+    held = free0 - torch.cuda.mem_get_info()[0]
+    h.close()
+    return held
+
+
+@pytest.mark.parametrize("p,n,limit", [("s", 8193, 0.75), ("d", 8193, 0.65), ("c", 16385, 6.5)])
+def test_trtri_memory_with_a_last_pair_of_one_row(p, n, limit):
+    """One row past a power of two: the buffers of the last level are as narrow as its last
+    pair (GiB held by the handle; FP64 with 0.5 for an aligned copy), and the inverse is
+    right, also where the level's columns come in pieces (complex, above 8 GiB)."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    t = matgen.torch_dtype(p)
+    T = torch.randn((n, n), generator=g, device="cuda", dtype=t).div_(n)
+    T.diagonal().copy_(torch.rand(n, generator=g, device="cuda").add_(1))
+    X = T.clone()
+    held = _held_after(lambda h: cc.trtri(h, X, n))
+    assert held <= limit * 2 ** 30, held / 2 ** 30
+    wide = torch.complex128 if p == "c" else torch.float64
+    v = torch.randn((4, n), generator=g, device="cuda", dtype=wide)
+    w = v
+    for S in (X, T):                    # [j, i] = A(i, j): the lower triangle of A
+        w = w @ S.triu_().T.to(wide)
+    err = float(torch.linalg.norm(w - v) / torch.linalg.norm(v))
+    assert err <= {"s": 2.0 ** -20, "c": 2.0 ** -20, "d": 2.0 ** -48}[p], err
+
+
+def test_mixed_solve_when_its_workspace_is_refused():
+    """The plan's block inverses are formed for fewer blocks at a time."""
+    import torch
+    n = 4300
+    A = matgen.spd_device("d", n, seed=2).contiguous()
+    B = torch.randn((3, n), device="cuda", dtype=torch.float64)
+    X = torch.zeros_like(B)
+    for after in (1, 2, 3):
+        h = cc.Handle()
+        _refuse_allocation(after)
+        try:
+            rc, it, berr, info = cc.call_posv_mixed(h, "L", n, 3, A.data_ptr(), n, B.data_ptr(), n, X.data_ptr(), n)
+        finally:
+            _refuse_allocation(-1)
+        if rc == 0:
+            break
+        h.close()
+    assert rc == 0 and info == 0
+    R = B - X @ matgen.hermitian_of(A, "L")
+    assert float(R.abs().max()) <= 1e-11
+    h.close()
