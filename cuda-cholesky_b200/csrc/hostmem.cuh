@@ -370,8 +370,7 @@ CUresult host_potri(const char* name, CUmultiGPULAPACKhandle hh, CBlasUplo uplo,
   T* D;
   size_t ldd;
   CUresult r = stage_in<T>(hh, A, lda, n, upper, &D, &ldd);
-  if (r == CUDA_SUCCESS) r = trtri_run<T>(hh->h, upper, false, (int)n, D, (long long)ldd, info);
-  if (r == CUDA_SUCCESS && *info == 0) r = lauum_run<T>(hh->h, upper, (int)n, D, (long long)ldd);
+  if (r == CUDA_SUCCESS) r = potri_run<T>(hh->h, upper, (int)n, D, (long long)ldd, info);
   if (r == CUDA_SUCCESS && *info == 0)
     r = copy_triangle<T>(A, lda, D, ldd, n, upper, hh->s_copy, &hh->d2h_bytes);
   CUCHOL_CHECK_CU(finish(hh, r));

@@ -1319,20 +1319,48 @@ int lauum_width(CULAPACKhandle h, int n) {
   return (int)std::max<size_t>(256, cols / 256 * 256);
 }
 
+// The one-launch forms of ?lauum and what they take.  FP32: one pack of the whole triangle.
+// FP64, orders whose product fits the workspace: the k range in slabs, one node of one
+// launch each, summed in order on the way back into A.  The tiles' k ranges run from n down
+// to one tile, and without slabs the launch takes as long as an SM's share of the longest
+// ones (n = 2048: 285 us for 82 us of FP64 work).
+template <typename T>
+struct LauumPlan {
+  int slab = 0, slabs = 0;
+  size_t bytes = 0;              // 0: the blocked form
+  LauumPlan(CULAPACKhandle h, int n, const T* A, long long lda) {
+    if (h->force_simt || h->lauum_cols != 0) return;
+    if (is_fp32<T>()) {
+      constexpr size_t cx = real_per<T>();
+      if (n >= tcg_min_order<T>()) bytes = sizeof(float) * 2 * (n * cx) * (round_up((size_t)n, 32) * cx);
+      return;
+    }
+    const bool direct = fp64_aligned(A, lda);
+    const long long tiles = (long long)((n + 63) / 64) * ((n + 63) / 64 + 1) / 2;
+    const size_t product = sizeof(T) * round_up((size_t)n, 2) * n;
+    const long long fit = (long long)(kLauumWorkspace / product) - (direct ? 0 : 1);
+    const int want = (int)std::max(1LL, std::min({(24LL * h->num_sms + tiles - 1) / tiles, (long long)n / 512, fit}));
+    slab = (int)round_up((size_t)(n + want - 1) / want, 128);
+    slabs = (n + slab - 1) / slab;
+    const size_t need = product * (slabs + (direct ? 0 : 1));
+    if ((slabs > 1 || !direct) && need <= kLauumWorkspace) bytes = need;
+  }
+};
+
 template <typename T>
 CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
   const long long rs = upper ? lda : 1, cs = upper ? 1 : lda;
   auto at = [&](long long i, long long j) { return A + i * rs + j * cs; };
   cudaStream_t sp = h->s_panel;
+  const LauumPlan<T> plan(h, n, A, lda);
   if constexpr (is_fp32<T>()) {
-    // one pack of the whole triangle, from which the product is written straight over A
+    // from the pack the product is written straight over A
     constexpr int cx = real_per<T>();
     const long long ld = (long long)round_up((size_t)n, 32) * cx;
     const size_t one = (size_t)n * cx * ld;
     bool tensor = false;
-    if (!h->force_simt && n >= tcg_min_order<T>() && h->lauum_cols == 0)
-      CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, false, &tensor));
-    if (tensor && try_workspace(h, sizeof(float) * 2 * one)) {
+    if (plan.bytes > 0) CUCHOL_CHECK_CU(tcg_in_range<T>(h, A, rs, cs, n, false, &tensor));
+    if (tensor && try_workspace(h, plan.bytes)) {
       float* w = static_cast<float*>(h->ws);
       tcg::Packs ps{};
       ps.count = 1;
@@ -1360,18 +1388,9 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
   const int w = lauum_width<T>(h, n);
   const long long ldw = (long long)round_up((size_t)n, 2);
   if constexpr (is_fp64<T>()) {
-    // Orders whose product fits the workspace: the k range in slabs, one node of one
-    // launch each, summed in order on the way back into A.  The tiles' k ranges run from
-    // n down to one tile, and without slabs the launch takes as long as an SM's share
-    // of the longest ones (n = 2048: 285 us for 82 us of FP64 work).
-    const long long tiles = (long long)((n + 63) / 64) * ((n + 63) / 64 + 1) / 2;
-    const size_t product = sizeof(T) * (size_t)ldw * n;
     const bool direct = fp64_aligned(A, lda);
-    const long long fit = (long long)(kLauumWorkspace / product) - (direct ? 0 : 1);
-    const int want = (int)std::max(1LL, std::min({(24LL * h->num_sms + tiles - 1) / tiles, (long long)n / 512, fit}));
-    const int slab = (int)round_up((size_t)(n + want - 1) / want, 128), slabs = (n + slab - 1) / slab;
-    const size_t need = product * (slabs + (direct ? 0 : 1));
-    if (!h->force_simt && h->lauum_cols == 0 && (slabs > 1 || !direct) && need <= kLauumWorkspace && try_workspace(h, need)) {
+    if (plan.bytes > 0 && try_workspace(h, plan.bytes)) {
+      const int slab = plan.slab, slabs = plan.slabs;
       T* W = static_cast<T*>(h->ws);
       T* S = W + (size_t)ldw * n * slabs;
       if (!direct) CUCHOL_CHECK_CU(copy_view<T>(h, A, rs, cs, S, upper ? ldw : 1, upper ? 1 : ldw, n, n, true, sp, nullptr));
@@ -1639,6 +1658,17 @@ CUresult api_lauum(const char* name, CULAPACKhandle h, CBlasUplo uplo, size_t n,
   return lauum_run<T>(h, uplo == CBlasUpper, (int)n, reinterpret_cast<T*>(A), (long long)lda);
 }
 
+// ?potri: inverse of the triangle, then its product.  The workspace grows once, to the larger of
+// the two needs (a growth is an allocation, a free and with them two waits for the device, 1 to
+// 2 ms; refused, each part takes its own way).
+template <typename T>
+CUresult potri_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda, long* info) {
+  try_workspace(h, std::max(trtri_scratch<T>(h, n, A, lda), LauumPlan<T>(h, n, A, lda).bytes));
+  CUCHOL_CHECK_CU(trtri_run<T>(h, upper, false, n, A, lda, info));
+  if (*info != 0) return CUDA_SUCCESS;
+  return lauum_run<T>(h, upper, n, A, lda);
+}
+
 template <typename T>
 CUresult api_potri(const char* name, CULAPACKhandle h, CBlasUplo uplo, size_t n, CUdeviceptr A, size_t lda,
                    long* info) {
@@ -1650,10 +1680,7 @@ CUresult api_potri(const char* name, CULAPACKhandle h, CBlasUplo uplo, size_t n,
   }
   if (n == 0) return CUDA_SUCCESS;
   if (h == nullptr || bad_uplo(uplo) || n > (size_t)INT_MAX) return CUDA_ERROR_INVALID_VALUE;
-  const bool up = (uplo == CBlasUpper);
-  CUCHOL_CHECK_CU(trtri_run<T>(h, up, false, (int)n, reinterpret_cast<T*>(A), (long long)lda, info));
-  if (*info != 0) return CUDA_SUCCESS;
-  return lauum_run<T>(h, up, (int)n, reinterpret_cast<T*>(A), (long long)lda);
+  return potri_run<T>(h, uplo == CBlasUpper, (int)n, reinterpret_cast<T*>(A), (long long)lda, info);
 }
 
 template <typename T>

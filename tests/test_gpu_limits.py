@@ -182,3 +182,22 @@ def test_mixed_solve_when_its_workspace_is_refused():
     R = B - X @ matgen.hermitian_of(A, "L")
     assert float(R.abs().max()) <= 1e-11
     h.close()
+
+
+@pytest.mark.parametrize("p,n", [("z", 1100), ("c", 1000), ("d", 1100)])
+def test_first_potri_grows_the_workspace_once(p, n):
+    """A second growth would be refused here, and the product then take another route."""
+    L = np.linalg.cholesky(matgen.spd(p, n, seed=8).astype(np.complex128 if p in "cz" else np.float64))
+    T = np.asfortranarray(L.astype(matgen.dtype_of(p)))
+    out = []
+    for after in (1, -1):
+        h = cc.Handle()
+        D = cc.to_device_colmajor(T)
+        _refuse_allocation(after)
+        try:
+            assert cc.potri(h, D, n) == 0
+        finally:
+            _refuse_allocation(-1)
+        out.append(np.tril(cc.to_host_colmajor(D)))
+        h.close()
+    assert np.array_equal(out[0], out[1])
