@@ -95,6 +95,7 @@ CUresult launch_list(CULAPACKhandle h, std::vector<GemmProblem<T>>& ps, CUcholBa
 namespace {
 
 constexpr int kPersistentCtas = 3;   // CTAs per SM of the persistent form
+inline int persistent_grid(CULAPACKhandle h, int batch) { return std::min(batch, kPersistentCtas * h->num_sms); }
 constexpr int kBatchedMaxNb = 64;   // a 64-wide SIMT tile holds a whole panel: in-place solve
 
 template <typename T>
@@ -299,9 +300,10 @@ __global__ void set_identity_kernel(T* a, const long long* __restrict__ off, con
 // (the kernels do the same work for any SPD input) and keep the fastest.
 template <typename T>
 CUresult tune_nb(CUcholBatched p, const BatchedShape<T>& sh, int* best_nb) {
-  // candidates: the grouped graphs with nb = 32 and 64, and the persistent kernel,
-  // written nb = -1 here
-  const std::vector<int> candidates = {32, 64, -1};
+  // candidates: the grouped graphs with nb = 32 and 64, and, unless its workspace was
+  // refused, the persistent kernel, written nb = -1 here
+  std::vector<int> candidates = {32, 64};
+  if (p->d_wp != nullptr) candidates.push_back(-1);
   std::vector<long long> off(sh.batch);
   long long total = 0;
   for (int b = 0; b < sh.batch; ++b) { off[b] = total; total += (long long)sh.n[b] * sh.n[b]; }
@@ -427,14 +429,24 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
     return fail(report(cudaGetLastError(), "cudaMalloc", __func__, __FILE__, __LINE__));
   int nmax = 1;
   for (int b = 0; b < batch; ++b) nmax = std::max(nmax, n[b]);
-  p->wp_tiles = (nmax + kBatchedMaxNb - 1) / kBatchedMaxNb;
-  if (dev_malloc(&p->d_next, sizeof(int)) != cudaSuccess ||
-      dev_malloc(&p->d_wp, sizeof(T) * kPersistentCtas * (size_t)h->num_sms * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb) !=
-          cudaSuccess)
-    return fail(report(cudaGetLastError(), "cudaMalloc", __func__, __FILE__, __LINE__));
+  // The persistent form's workspace: per CTA that it launches the inverses of one matrix's
+  // diagonal blocks (without ?potri: of the present one).  Only for plans that may take the
+  // form; a refusal leaves the tuner the grouped ones.
+  if (nb <= 0) {
+    p->wp_tiles = (flags & 4) ? (nmax + kBatchedMaxNb - 1) / kBatchedMaxNb : 1;
+    const size_t bytes = sizeof(T) * persistent_grid(h, batch) * p->wp_tiles * kBatchedMaxNb * kBatchedMaxNb;
+    if (dev_malloc(&p->d_next, sizeof(int)) != cudaSuccess || dev_malloc(&p->d_wp, bytes) != cudaSuccess) {
+      const cudaError_t e = cudaGetLastError();
+      if (nb < 0) return fail(report(e, "cudaMalloc", __func__, __FILE__, __LINE__));
+    }
+  }
   if (nb == 0) {
     rc = tune_nb<T>(p, sh, &nb);
     if (rc != CUDA_SUCCESS) return fail(rc);
+  }
+  if (nb > 0) {
+    cudaFree(p->d_wp);
+    p->d_wp = nullptr;
   }
   p->persistent = (nb < 0);
   rc = build_graph<T>(p, sh, nb < 0 ? kBatchedMaxNb : nb);

@@ -436,7 +436,7 @@ CUresult record_persistent(CUcholBatched p, const BatchedShape<T>& sh, cudaStrea
   CUCHOL_CHECK(cudaMemsetAsync(p->d_info, 0, sizeof(int) * B, s));
   CUCHOL_CHECK(cudaMemsetAsync(p->d_logdet, 0, sizeof(double) * B, s));
   CUCHOL_CHECK(cudaMemsetAsync(p->d_next, 0, sizeof(int), s));
-  const int grid = std::min(B, bpk::CTAS * h->num_sms);
+  const int grid = persistent_grid(h, B);
   bpk::persistent_kernel<T><<<grid, bpk::THREADS, bpk::smem_bytes<T>(), s>>>(
       dm, dord, B, p->d_next, sh.upper ? 1 : 0, (sh.flags & 4) ? 1 : 0, static_cast<T*>(p->d_wp), p->wp_tiles);
   ++h->launches;

@@ -201,3 +201,60 @@ def test_first_potri_grows_the_workspace_once(p, n):
         out.append(np.tril(cc.to_host_colmajor(D)))
         h.close()
     assert np.array_equal(out[0], out[1])
+
+
+def _batch(p, n, batch):
+    import torch
+    mats = [matgen.spd(p, n, seed=b) for b in range(batch)]
+    flat, off, sizes = cc.pack_colmajor(mats, matgen.dtype_of(p))
+    return mats, torch.from_numpy(flat).cuda(), off, sizes
+
+
+@pytest.mark.parametrize("p", "sd")
+@pytest.mark.parametrize("flags,nb", [(7, 0), (7, 32), (3, 0), (7, -1)])
+def test_batched_plan_memory(p, flags, nb):
+    """Two matrices of order 3000: the plan holds the inverse's workspace and little more, not
+    inverse blocks for CTAs that never run."""
+    import torch
+    if p == "s" and nb == -1:
+        pytest.skip("not selectable for FP32")
+    n = 3000
+    h = cc.Handle()
+    buf = torch.zeros(2 * n * n, dtype=matgen.torch_dtype(p), device="cuda")
+    for o in (0, n * n):
+        buf[o:o + n * n].view(n, n).fill_diagonal_(1.0)
+    plans = []
+
+    def create(_):
+        plans.append(cc.BatchedPlan(h, buf, [n, n], [0, n * n], flags=flags, nb=nb))
+    held = _held_after(create)
+    work = 2 * n * n * buf.element_size() if flags & 4 else 0
+    assert held <= work + (48 << 20), held >> 20
+    plans[0].run()
+    info, _ = plans[0].results()
+    assert info == [0, 0]
+    plans[0].close()
+    h.close()
+
+
+@pytest.mark.parametrize("after", [4, 5])
+@pytest.mark.parametrize("p", "sd")
+def test_batched_plan_without_the_persistent_workspace(p, after):
+    """Refused, the tuner chooses among the grouped forms."""
+    mats, buf, off, sizes = _batch(p, 200, 5)
+    h = cc.Handle()
+    _refuse_allocation(after)
+    try:
+        plan = cc.BatchedPlan(h, buf, sizes, off, flags=7, nb=0)
+    finally:
+        _refuse_allocation(-1)
+    assert plan.nb in (32, 64)
+    plan.run()
+    info, logdet = plan.results()
+    for b, A in enumerate(mats):
+        inv = np.linalg.inv(A.astype(np.float64))
+        got = buf[off[b]:off[b] + 200 * 200].view(200, 200).T.cpu().numpy()
+        assert info[b] == 0
+        assert np.linalg.norm(np.tril(got - inv)) <= {"s": 2.0 ** -18, "d": 2.0 ** -47}[p] * np.linalg.norm(inv)
+    plan.close()
+    h.close()
