@@ -590,7 +590,7 @@ def batched_result(torch, cc, p, warmup, steps, peak, rank=0, world=1, pg=None, 
     else:
         n_failed = sum(1 for i in info if i != 0)
     ms = statistics.mean(times)
-    nb = plan.nb
+    nb = plan.form
     if rank != 0:
         plan.close()
         h.close()

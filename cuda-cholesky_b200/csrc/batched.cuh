@@ -369,9 +369,8 @@ template <typename T>
 CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUplo uplo, int batch,
                         const int* n, const CUdeviceptr* A, const int* lda, int flags, int nb) {
   // nb: 0 = tuned, 8..64 (multiple of 8) = the grouped graph with that block size,
-  // -1 = the persistent kernel (FP64 only)
-  const bool nb_ok = (nb == -1 && std::is_same<T, double>::value) ||
-                     (nb >= 0 && nb <= kBatchedMaxNb && (nb == 0 || nb % 8 == 0));
+  // -1 = the persistent kernel
+  const bool nb_ok = nb == -1 || (nb >= 0 && nb <= kBatchedMaxNb && nb % 8 == 0);
   if (out == nullptr || h == nullptr || batch <= 0 || n == nullptr || A == nullptr || lda == nullptr ||
       (uplo != CBlasLower && uplo != CBlasUpper) || !nb_ok)
     return CUDA_ERROR_INVALID_VALUE;
@@ -440,7 +439,8 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
       if (nb < 0) return fail(report(e, "cudaMalloc", __func__, __FILE__, __LINE__));
     }
   }
-  if (nb == 0) {
+  const bool tuned = nb == 0;
+  if (tuned) {
     rc = tune_nb<T>(p, sh, &nb);
     if (rc != CUDA_SUCCESS) return fail(rc);
   }
@@ -451,6 +451,8 @@ CUresult batched_create(CUcholBatched* out, CULAPACKhandle h, char type, CBlasUp
   p->persistent = (nb < 0);
   rc = build_graph<T>(p, sh, nb < 0 ? kBatchedMaxNb : nb);
   if (rc != CUDA_SUCCESS) return fail(rc);
+  // what cuCholBatchedGetBlockSize reports; FP32 plans that were tuned have always reported a width
+  p->nb = (tuned && nb < 0 && type == 'S') ? kBatchedMaxNb : nb;
   *out = p;
   return CUDA_SUCCESS;
 }
@@ -490,7 +492,13 @@ extern "C" CUCHOL_EXPORT CUresult cuCholBatchedResults(CUcholBatched p, long* in
 
 extern "C" CUCHOL_EXPORT CUresult cuCholBatchedGetBlockSize(CUcholBatched p, int* nb) {
   if (p == nullptr || nb == nullptr) return CUDA_ERROR_INVALID_VALUE;
-  *nb = (p->persistent && p->type == 'D') ? -1 : p->nb;   // FP32: the persistent kernel's tile order
+  *nb = p->nb;
+  return CUDA_SUCCESS;
+}
+
+extern "C" CUCHOL_EXPORT CUresult cuCholBatchedGetForm(CUcholBatched p, int* form) {
+  if (p == nullptr || form == nullptr) return CUDA_ERROR_INVALID_VALUE;
+  *form = p->persistent ? -1 : p->nb;
   return CUDA_SUCCESS;
 }
 

@@ -372,6 +372,15 @@ class BatchedPlan:
         lib().cuCholBatchedGetBlockSize(self._p, C.byref(v))
         return v.value
 
+    @property
+    def form(self) -> int:
+        """The nb that selects the form in use: 8..64 grouped, -1 the persistent kernel."""
+        v = C.c_int(0)
+        f = lib().cuCholBatchedGetForm
+        f.argtypes, f.restype = [C.c_void_p, C.POINTER(C.c_int)], C.c_int
+        f(self._p, C.byref(v))
+        return v.value
+
     def run(self, stream: int = 0) -> None:
         rc = lib().cuCholBatchedRun(self._p, C.c_void_p(stream))
         if rc != CUDA_SUCCESS:

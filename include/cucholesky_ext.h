@@ -50,13 +50,16 @@ CUresult cuLAPACKGetPotrfBlocks(CULAPACKhandle, char, size_t, int *);
  *     step, and each step is a few grouped launches over the batch (diagonal blocks,
  *     panel solves, trailing updates), followed, with CUCHOL_BATCHED_POTRI, by the
  *     grouped inverse;
- *   nb = -1 (FP64 only): one persistent kernel; each CTA takes whole matrices from a
- *     queue ordered by size, largest first, and factors, log-dets and inverts each in
- *     place with 64 x 64 tile products on the FP64 tensor cores.
+ *   nb = -1: one persistent kernel; each CTA takes whole matrices from a queue ordered
+ *     by size, largest first, and factors, log-dets and inverts each in place with
+ *     64 x 64 tile products (FP64 on the tensor cores).
  * nb = 0 lets the plan pick by timing the candidates (grouped with nb 32 and 64, and
- * the persistent kernel for FP64) on an identity batch of the same shapes.  The plan
- * keeps the pointers: run it again after refilling the same buffers.
- * cuCholBatchedGetBlockSize reports the chosen nb (-1: the persistent kernel).
+ * the persistent kernel) on an identity batch of the same shapes.  The plan keeps the
+ * pointers: run it again after refilling the same buffers.
+ * cuCholBatchedGetForm reports the form in use as the nb that selects it (8..64 grouped,
+ * -1 persistent): pass it to make the same plan again.  cuCholBatchedGetBlockSize
+ * reports the same, except that an FP32 plan whose tuner took the persistent kernel
+ * reports the width 64.
  *   cu?cholBatchedCreate  build (and tune) the plan; allocates its workspace
  *   cuCholBatchedRun      one graph launch on `stream`
  *   cuCholBatchedResults  waits, then copies info[b] (as ?potrf / ?potri) and
@@ -72,6 +75,7 @@ CUresult cuScholBatchedCreate(CUcholBatched *, CULAPACKhandle, CBlasUplo, int, c
 CUresult cuCholBatchedRun(CUcholBatched, CUstream);
 CUresult cuCholBatchedResults(CUcholBatched, long *, double *);
 CUresult cuCholBatchedGetBlockSize(CUcholBatched, int *);
+CUresult cuCholBatchedGetForm(CUcholBatched, int *);
 CUresult cuCholBatchedDestroy(CUcholBatched);
 
 /* log det from a strided FP64 diagonal, 2 * sum_i log(x[i*incx]), for callers that

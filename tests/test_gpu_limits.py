@@ -13,6 +13,9 @@ from cucholesky import matgen
 pytestmark = pytest.mark.gpu
 
 
+U = {"s": 2.0 ** -24, "d": 2.0 ** -53}
+
+
 @pytest.fixture(scope="module")
 def simt():
     """A handle whose products all run on the plain FP32 engine."""
@@ -216,8 +219,6 @@ def test_batched_plan_memory(p, flags, nb):
     """Two matrices of order 3000: the plan holds the inverse's workspace and little more, not
     inverse blocks for CTAs that never run."""
     import torch
-    if p == "s" and nb == -1:
-        pytest.skip("not selectable for FP32")
     n = 3000
     h = cc.Handle()
     buf = torch.zeros(2 * n * n, dtype=matgen.torch_dtype(p), device="cuda")
@@ -258,3 +259,57 @@ def test_batched_plan_without_the_persistent_workspace(p, after):
         assert np.linalg.norm(np.tril(got - inv)) <= {"s": 2.0 ** -18, "d": 2.0 ** -47}[p] * np.linalg.norm(inv)
     plan.close()
     h.close()
+
+
+def _check_inverse(A, got, uplo, u):
+    n = A.shape[0]
+    inv = np.linalg.inv(A.astype(np.float64))
+    keep = np.tril(np.ones((n, n), bool)) if uplo == "L" else np.triu(np.ones((n, n), bool))
+    # condition numbers of about 3: rounding errors of sums of up to n terms
+    assert np.linalg.norm(np.where(keep, got - inv, 0)) <= u * (32 + np.sqrt(n)) * np.linalg.norm(inv), n
+    assert np.array_equal(got[~keep], A[~keep])
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("flags", [7, 3])
+@pytest.mark.parametrize("p", "sd")
+def test_batched_persistent_form(handle, p, flags, uplo):
+    """nb = -1 for both types: matrices at the edges of the 64 x 64 tiles, one that fails, and
+    the factor alone."""
+    import torch
+    sizes = [1, 2, 16, 63, 64, 65, 127, 128, 129, 200, 256, 257, 500]
+    mats = [matgen.spd(p, n, seed=n) for n in sizes]
+    mats[9] = mats[9].copy(order="F")
+    mats[9][150, 150] = -1.0
+    flat, off, _ = cc.pack_colmajor(mats, matgen.dtype_of(p))
+    buf = torch.from_numpy(flat.copy()).cuda()
+    plan = cc.BatchedPlan(handle, buf, sizes, off, uplo=uplo, flags=flags, nb=-1)
+    assert plan.nb == -1 and plan.form == -1
+    for _ in range(2):
+        buf.copy_(torch.from_numpy(flat))
+        plan.run()
+        info, logdet = plan.results()
+        out = buf.cpu().numpy()
+        for b, (n, A, o) in enumerate(zip(sizes, mats, off)):
+            if b == 9:
+                assert info[b] == 151
+                continue
+            got = out[o:o + n * n].reshape(n, n).T
+            assert info[b] == 0
+            assert abs(logdet[b] - np.linalg.slogdet(A.astype(np.float64))[1]) <= 200 * n * U[p]
+            if flags & 4:
+                _check_inverse(A, got, uplo, U[p])
+            else:
+                assert matgen.backward_error(A, np.asfortranarray(got), uplo) <= 2
+    plan.close()
+
+
+@pytest.mark.parametrize("p", "sd")
+def test_batched_form_makes_the_plan_again(handle, p):
+    mats, buf, off, sizes = _batch(p, 130, 40)
+    plan = cc.BatchedPlan(handle, buf, sizes, off, flags=7, nb=0)
+    again = cc.BatchedPlan(handle, buf, sizes, off, flags=7, nb=plan.form)
+    assert again.form == plan.form and plan.form in (-1, 32, 64)
+    assert plan.nb == plan.form or (p == "s" and plan.nb == 64)
+    again.close()
+    plan.close()
