@@ -626,12 +626,12 @@ CUresult tc3_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
   prm.err = h->d_words + 3;
   const int tiles = prm.tiles_n * (prm.tiles_n + 1) / 2 + (prm.tiles_m - prm.tiles_n) * prm.tiles_n;
   constexpr int smem = tc::Ring<true>::SMEM;
-  static bool attr[2] = {false, false};
-  if (!attr[upper]) {
+  static DeviceOnce attr[2];
+  if (attr[upper].needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(upper ? (const void*)tc::update_kernel<float, true, true>
                                             : (const void*)tc::update_kernel<float, true, false>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr[upper] = true;
+    attr[upper].done(h->device);
   }
   if (upper)
     tc::update_kernel<float, true, true><<<tiles, tc::THREADS, smem, s>>>(mhi, mlo, mc, prm, stop);

@@ -1016,13 +1016,13 @@ inline int ntile_of(int n) { return (n + SY - 1) / SY; }
 constexpr size_t kSymvSmem = kSymvSmemBytes;
 
 template <typename T>
-CUresult block_inverse(const T* L, long long rs, long long cs, int n, T* DI, cudaStream_t s) {
+CUresult block_inverse(int device, const T* L, long long rs, long long cs, int n, T* DI, cudaStream_t s) {
   const size_t smem = BlockSmem<T, BS>::bytes;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(block_inverse_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-    attr = true;
+    attr.done(device);
   }
   block_inverse_kernel<T><<<(n + BS - 1) / BS, kThreads, smem, s>>>(L, rs, cs, n, DI);
   CUCHOL_CHECK(cudaGetLastError());
@@ -1030,14 +1030,14 @@ CUresult block_inverse(const T* L, long long rs, long long cs, int n, T* DI, cud
 }
 
 // Y = alpha A X + beta B for the symmetric A (one triangle, lower view rs, cs).
-CUresult symv(const double* A, long long rs, long long cs, int n, const double* X, long long ldx, int nrhs,
+CUresult symv(int device, const double* A, long long rs, long long cs, int n, const double* X, long long ldx, int nrhs,
               int absval, double alpha, double beta, const double* B, long long ldb, double* Y, long long ldy,
               double* U, double* V, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(symv_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kSymvSmem));
-    attr = true;
+    attr.done(device);
   }
   const int T = ntile_of(n);
   const int upper = (rs != 1);
@@ -1056,14 +1056,14 @@ constexpr size_t trsv_smem() { return sizeof(T) * (2 * BS * (BS + 1) + BS * NR +
 
 // Opt in to the triangular solves' shared memory (above 48 KB for FP64).
 template <typename T, typename V>
-CUresult trsv_attr() {
-  static bool done = false;
-  if (!done) {
+CUresult trsv_attr(int device) {
+  static DeviceOnce attr;
+  if (attr.needed(device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(trsv_fwd_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)trsv_smem<T>()));
     CUCHOL_CHECK(cudaFuncSetAttribute(trsv_bwd_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)trsv_smem<T>()));
-    done = true;
+    attr.done(device);
   }
   return CUDA_SUCCESS;
 }
@@ -1071,11 +1071,11 @@ CUresult trsv_attr() {
 // Z = S F^T F S R (the preconditioner; F = forward solve by the FP32 factor in
 // NBT-wide steps with the inverted diagonal blocks), 16 columns.
 CUresult precond(CUcholMixed p, const double* R, double* Z, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(p->h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(gemv_n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSmem));
     CUCHOL_CHECK(cudaFuncSetAttribute(gemv_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemvSmem));
-    attr = true;
+    attr.done(p->h->device);
   }
   const int n = p->n;
   const long long ld = p->ld, ldw = p->ldw;
@@ -1164,11 +1164,11 @@ CUresult tc_update(CULAPACKhandle h, const Op* q, long long ldq, int q_rows, int
   prm.tiles_n = (ncols + tc::BN - 1) / tc::BN;
   prm.err = h->d_words + 3;
   const int tiles = prm.tiles_n * (prm.tiles_n + 1) / 2 + (prm.tiles_m - prm.tiles_n) * prm.tiles_n;
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(tc::update_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc::SMEM_BYTES));
-    attr = true;
+    attr.done(h->device);
   }
   tc::update_kernel<Op><<<tiles, tc::THREADS, tc::SMEM_BYTES, s>>>(mq, mq, mc, prm, stop);
   ++h->launches;
@@ -1287,7 +1287,7 @@ CUresult mixed_refactor(CUcholMixed p, long* info) {
   {
     ones_kernel<<<(n + 255) / 256, 256, 0, sp>>>(p->x, n);
     CUCHOL_CHECK(cudaGetLastError());
-    CUCHOL_CHECK_CU(symv(p->A, p->rs, p->cs, n, p->x, p->ld, 1, 1, 1.0, 0.0, nullptr, 0, p->r, p->ld, p->U, p->V,
+    CUCHOL_CHECK_CU(symv(p->h->device, p->A, p->rs, p->cs, n, p->x, p->ld, 1, 1, 1.0, 0.0, nullptr, 0, p->r, p->ld, p->U, p->V,
                          sp));
     CUCHOL_CHECK(cudaMemsetAsync(p->r + p->ld, 0, sizeof(double) * p->ld * (NR - 1), sp));
     norms_kernel<<<kVecBlocks, kThreads, 0, sp>>>(p->r, nullptr, n, p->ld, p->part_norm);
@@ -1459,7 +1459,7 @@ CUresult mixed_solve(CUcholMixed p, int nrhs, const double* B, long long ldb, do
       CUCHOL_CHECK(cudaGetLastError());
       slot ^= 1;
       while (it < maxit) {
-        CUCHOL_CHECK_CU(symv(p->A, p->rs, p->cs, n, p->p, ld, NR, 0, 1.0, 0.0, nullptr, 0, p->q, ld, p->U, p->V, s));
+        CUCHOL_CHECK_CU(symv(p->h->device, p->A, p->rs, p->cs, n, p->p, ld, NR, 0, 1.0, 0.0, nullptr, 0, p->q, ld, p->U, p->V, s));
         dot_kernel<<<kVecBlocks, kThreads, 0, s>>>(p->p, p->q, n, ld, p->part);
         update_xr_kernel<<<kVecBlocks, kThreads, 0, s>>>(p->x, p->r, p->p, p->q, n, ld, p->part, p->rz + slot * NR,
                                                          p->part_norm);
@@ -1475,7 +1475,7 @@ CUresult mixed_solve(CUcholMixed p, int nrhs, const double* B, long long ldb, do
         slot ^= 1;
       }
       // FP64 residual from scratch: r = b - A x
-      CUCHOL_CHECK_CU(symv(p->A, p->rs, p->cs, n, p->x, ld, NR, 0, -1.0, 1.0, p->b, ld, p->r, ld, p->U, p->V, s));
+      CUCHOL_CHECK_CU(symv(p->h->device, p->A, p->rs, p->cs, n, p->x, ld, NR, 0, -1.0, 1.0, p->b, ld, p->r, ld, p->U, p->V, s));
       norms_kernel<<<kVecBlocks, kThreads, 0, s>>>(p->r, p->x, n, ld, p->part_norm);
       CUCHOL_CHECK(cudaGetLastError());
       CUCHOL_CHECK_CU(fetch_norms(p, s));
@@ -1514,8 +1514,8 @@ CUresult potrs_run(CULAPACKhandle h, bool upper, int n, int nrhs, const T* A, lo
   T* Y = reinterpret_cast<T*>(static_cast<char*>(h->ws) + di);
   unsigned* ctr = reinterpret_cast<unsigned*>(h->d_words + 8);   // words 8..11
   int* err = h->d_words + 3;
-  CUCHOL_CHECK_CU(block_inverse<T>(A, rs, cs, n, DI, s));
-  CUCHOL_CHECK_CU((trsv_attr<T, T>()));
+  CUCHOL_CHECK_CU(block_inverse<T>(h->device, A, rs, cs, n, DI, s));
+  CUCHOL_CHECK_CU((trsv_attr<T, T>(h->device)));
   for (int g0 = 0; g0 < nrhs; g0 += NR) {
     const int nc = std::min(NR, nrhs - g0);
     T* Bg = B + (long long)g0 * ldb;

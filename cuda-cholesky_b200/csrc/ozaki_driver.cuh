@@ -40,11 +40,11 @@ CUresult ozaki_update(CULAPACKhandle h, const int8_t* sl, int R, int S, long lon
   q.err = h->d_words + 3;
   int tiles = 0;
   for (int r = 0; r < q.tiles_m; ++r) tiles += std::min(q.tiles_n, (r * oz::BM + oz::BM - 1) / oz::BN + 1);
-  static bool attr = false;
-  if (!attr) {
+  static DeviceOnce attr;
+  if (attr.needed(h->device)) {
     CUCHOL_CHECK(cudaFuncSetAttribute(oz::update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       oz::SMEM_BYTES));
-    attr = true;
+    attr.done(h->device);
   }
   oz::update_kernel<<<tiles, oz::THREADS, oz::SMEM_BYTES, s>>>(map, map, q, R, stop);
   ++h->launches;

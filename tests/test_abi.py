@@ -279,3 +279,14 @@ def test_tuning_table_file(tmp_path):
         restore.write_text("\n".join(lines) + "\n")
         assert lib.cuLAPACKLoadTuning(str(restore).encode()) == 0
     assert [(t, n, sub(t, n)) for t in "SDCZ" for n in (100, 7000, 20000, 70000)] == builtin
+
+
+def test_kernel_attributes_are_kept_per_device():
+    """A kernel's shared-memory opt-in holds on the device it was made on: no launcher remembers
+    it in a flag of the process, which would leave a second device without it."""
+    src = os.path.join(ROOT, "cuda-cholesky_b200", "csrc")
+    for fn in sorted(os.listdir(src)):
+        if fn.endswith((".cu", ".cuh")):
+            text = open(os.path.join(src, fn)).read()
+            for m in re.finditer(r"cudaFuncSetAttribute\(", text):
+                assert "static bool" not in text[max(0, m.start() - 200):m.start()], (fn, text[:m.start()].count("\n") + 1)
