@@ -380,9 +380,10 @@ struct FactorSmem {
 
 // Cholesky factor of the block in S (order n16, a multiple of 16 up to NB; lower part) and
 // the solve of the rows below it (rows n16 .. nrow - 1; nrow a multiple of 16; none: n16),
-// by the whole CTA of NT threads, NT / 32 >= 2 warps.  rd[c] = 1 / L(c, c).  done(c0)
+// by the whole CTA of NT threads, NT / 32 >= 2 warps.  rd[c] = 1 / L(c, c).  done(c0, cols)
 // is called by the threads of warps 1 .. (t - 32 counts them) as soon as the columns
-// c0 .. c0 + 15 are final, and by all warps for the last ones, with (thread, threads).
+// c0 .. c0 + cols - 1 are final, and by all warps for the last ones, with (thread, threads);
+// cols is 16, or for the sub-panel that failed the columns before the failing one.
 // s_fail (shared, -1 at entry) becomes the first failing column.  Starts and ends with a
 // barrier.
 //
@@ -410,7 +411,7 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
             tile_update<T>(S + cb * LD + rb, LD, S + cp * LD + rb, LD, S + cp * LD + cb, LD, nrow - rb);
           w = (w == 0) ? NT / 32 - 2 : w - 1;
         }
-      done(cp, t - 32, NT - 32);
+      done(cp, kSub, t - 32, NT - 32);
     }
     __syncthreads();
     const int fail = *s_fail;
@@ -425,7 +426,7 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
     }
     __syncthreads();
     if (fail >= 0 || c1 >= n16) {
-      done(c0, t, NT);
+      done(c0, fail < 0 ? kSub : fail - c0, t, NT);
       break;
     }
     // the 32 x 16 elements the next factor16 works on

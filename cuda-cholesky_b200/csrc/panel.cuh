@@ -139,19 +139,19 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
   load_lower<T, TA, NB, NT>(S, A, rs, cs, jb, n16);
   if (tid == 0) s_fail = -1;
   cp_async_wait_all();
-  factor_block<T, NB, 0, NT>(S, Ld, rd, n16, n16, &s_fail, [&](int c0, int t, int nt) {
-    // columns c0 .. c0 + 15 of the factor back to A
-    const int rows = jb - c0;
+  factor_block<T, NB, 0, NT>(S, Ld, rd, n16, n16, &s_fail, [&](int c0, int cols, int t, int nt) {
+    // columns c0 .. c0 + cols - 1 of the factor back to A
+    const int rows = jb - c0, ce = min(jb, c0 + cols);
     if (rs == 1) {
       for (int e = t >> 5; e < 4 * kSub; e += nt >> 5) {       // a warp per column and quarter
         const int c = c0 + (e & (kSub - 1));
         const int r = c0 + 32 * (e / kSub) + (t & 31);
-        if (c < jb && r < jb && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
+        if (c < ce && r < jb && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
       }
     } else {
       for (int e = t; e < rows * kSub; e += nt) {
         const int c = c0 + (e & (kSub - 1)), r = c0 + e / kSub;
-        if (c < jb && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
+        if (c < ce && r >= c) A[r * rs + c * cs] = (TA)S[c * LD + r];
       }
     }
   });

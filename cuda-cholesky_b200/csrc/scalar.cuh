@@ -119,6 +119,19 @@ __device__ __forceinline__ bool cta_aborted(const int* a, const int* b = nullptr
   return s_abort_word != 0;
 }
 
+// The same for an info word that the kernel itself may set, to base + 1 or more: only what
+// was set before the launch counts, so that what a kernel does with its own failure does not
+// depend on when its CTAs start.
+__device__ __forceinline__ bool cta_aborted_before(const int* info, long long base) {
+  __shared__ int s_abort_word;
+  if (threadIdx.x == 0) {
+    const int v = *(volatile const int*)info;
+    s_abort_word = v != 0 && v <= base;
+  }
+  __syncthreads();
+  return s_abort_word != 0;
+}
+
 // Nanoseconds of the GPU's global timer (for waits bounded in time).
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;

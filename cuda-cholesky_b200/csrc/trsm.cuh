@@ -250,7 +250,9 @@ __global__ void __launch_bounds__(256)
 // launch instead of two and no pass of the factor through memory.  The block in A must stay
 // as it is while CTAs still load it: CTA 0 writes the factor to D (column-major, ld NB),
 // and copy_diag_kernel takes it to A later.  Outputs for the rows as trsm_rows_kernel.
-// Worth it while the CTAs fit the GPU at once (each is as long as the factor).
+// Worth it while the CTAs fit the GPU at once (each is as long as the factor).  A bad pivot: the
+// columns before it are finished in all rows, the others are left as they were (the kernels that
+// take two launches leave the rows below that block alone).
 // T: the computing type; TA: the storage type of A and D (float under double only with rs = 1).
 template <typename T, typename TA, typename O2, int MODE, int NB, int R, int NT>
 __global__ void __launch_bounds__(NT)
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(NT)
       *d_info = 0;
       *logdet = 0.0;
     }
-  } else if (cta_aborted(d_info)) {
+  } else if (cta_aborted_before(d_info, info_base)) {
     return;
   }
   const long long row0 = (long long)blockIdx.x * R;
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(NT)
   }
   if (t == 0) s_fail = -1;
   cp_async_wait_all();
-  factor_block<T, NB, R, NT>(S, Ld, rd, NB, NB + R, &s_fail, [&](int c0, int tt, int nt) {
+  factor_block<T, NB, R, NT>(S, Ld, rd, NB, NB + R, &s_fail, [&](int c0, int cols, int tt, int nt) {
     const T* X = S + c0 * LD + NB;
     if (blockIdx.x == 0)
       for (int e = tt; e < NB * kSub; e += nt) {
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll 4
       for (int e = tt; e < R * kSub; e += nt) {
         const int r = (rs_ == 1) ? e % R : e / kSub, c = (rs_ == 1) ? e / R : e % kSub;
-        if (r < rows) out[(row0 + r) * rs_ + (long long)(c0 + c) * cs_] = conv(X[c * LD + r]);
+        if (r < rows && c < cols) out[(row0 + r) * rs_ + (long long)(c0 + c) * cs_] = conv(X[c * LD + r]);
       }
     };
     put(B, rs, cs, [](T v) { return (TA)v; });
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll 2
       for (int e = tt; e < R * kSub; e += nt) {
         const int r = e / kSub, c = e % kSub;
-        if (r < rows) put_split(X[c * LD + r], out2, out3, 2 * (row0 + r) * o_rs + 2 * (c0 + c), o_rs);
+        if (r < rows && c < cols) put_split(X[c * LD + r], out2, out3, 2 * (row0 + r) * o_rs + 2 * (c0 + c), o_rs);
       }
     } else if constexpr (MODE == OUT_SPLIT) {
       put(out2, o_rs, o_cs, [](T v) { return round_tf32((float)v); });

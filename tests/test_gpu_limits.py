@@ -313,3 +313,34 @@ def test_batched_form_makes_the_plan_again(handle, p):
     assert plan.nb == plan.form or (p == "s" and plan.nb == 64)
     again.close()
     plan.close()
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("p", "sdcz")
+def test_contents_after_a_bad_pivot(handle, p, uplo):
+    """The columns before the bad pivot hold the factor, the others of its block what they held:
+    with rows below the block (one launch) and without (the block alone)."""
+    nb = 64 if p == "z" else 128
+    A = matgen.spd(p, 300, seed=12)
+    A = A if uplo == "L" else np.asfortranarray(A.conj().T)
+    for n in (nb, 300):
+        for k in (0, 5, 20, 31, 47, nb - 1):
+            G = A[:n, :n].copy(order="F")
+            D = cc.to_device_colmajor(G)
+            assert cc.potrf(handle, D, n, uplo) == 0
+            good = cc.to_host_colmajor(D)
+            B = G.copy(order="F")
+            B[k, k] = -1.0
+            D = cc.to_device_colmajor(B)
+            assert cc.potrf(handle, D, n, uplo) == k + 1
+            got = cc.to_host_colmajor(D)
+            if uplo == "U":
+                got, good, B = got.T, good.T, B.T
+            low = np.tril(np.ones((n, nb), bool))
+            done = low & (np.arange(nb) < k)
+            # up to the pivot's own row the factor does not depend on it (but for rounding: a
+            # sub-panel with a bad pivot goes through a plain loop)
+            rest = np.arange(n) != k
+            d = np.abs(np.where(done, got[:, :nb] - good[:, :nb], 0))[rest]
+            assert d.max() <= 64 * np.finfo(got.real.dtype).eps
+            assert np.array_equal(got[:, :nb][low & ~done], B[:, :nb][low & ~done])
