@@ -719,6 +719,7 @@ CUresult tcg_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
   p.c = reinterpret_cast<float*>(corner);
   p.rs = rs * cx;
   p.cs = cs * cx;
+  p.chunk = 2;
   p.beta = 1;
   p.neg = 1;
   p.lower_only = 1;
@@ -726,6 +727,14 @@ CUresult tcg_update(CULAPACKhandle h, const float* qhi, const float* qlo, long l
   return tcg_launch(h, PackRef{qhi, qlo, (long long)q_rows * cx, ldq, cx}, PackRef{qhi, qlo, (long long)q_rows * cx, ldq, 1},
                     p, s, stop);
 }
+
+// k blocks per accumulator of a ?trtri or ?lauum product whose sums run over k: two from
+// kLongSum on, where an FMA chain errs more than that (?potri against FP64, two blocks / SIMT
+// engine: S n = 1400 6.5e-7 / 5.9e-7, 2000 6.6e-7 / 7.3e-7, 3001 6.0e-7 / 9.1e-7; complex, of
+// twice the k, n = 1000 6.5e-7 / 6.0e-7, 1400 6.3e-7 / 7.3e-7).  ?potrf's updates take two: their
+// sums are one outer block long and the factor's error is that of its panels.
+constexpr int kLongSum = 4096;
+inline int sum_chunk(int k) { return k >= kLongSum ? 2 : 1; }
 
 // Grows the workspace like ensure_workspace, but an allocation that fails is not an
 // error: false, and the caller takes a path that needs less.
@@ -1092,6 +1101,7 @@ CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs
     g.a_node = s; g.b_node = s * cx;
     g.kmode = tcg::K_A_LOWER;
     g.k = m * cx; g.k_last = L.s2 * cx;
+    g.chunk = sum_chunk(g.k);
     g.xhi = x; g.xlo = x + L.x; g.xld = L.ldx;
     const long long rows = (long long)L.rows;
     CUCHOL_CHECK_CU(tcg_launch(h, PackRef{ia, ia + L.ia, rows, L.ldk, 1},
@@ -1113,6 +1123,7 @@ CUresult trtri_levels_tcg(CULAPACKhandle h, bool unit, int n, T* A, long long rs
       }
       // X from its column j0 on: inv(T11) is zero above its diagonal
       g.k = g.k_last = (s - j0) * cx;
+      g.chunk = sum_chunk(g.k);
       g.c = at(s, j0);
       const float* xj = x + (long long)j0 * cx;
       CUCHOL_CHECK_CU(tcg_launch(h, PackRef{xj, xj + L.x, rows, L.ldx, 1, (long long)j0 * cx},
@@ -1375,6 +1386,7 @@ CUresult lauum_run(CULAPACKhandle h, bool upper, int n, T* A, long long lda) {
       g.nodes = 1;
       g.m = g.m_last = n; g.n = n * cx;
       g.k = g.k_last = n * cx;
+      g.chunk = sum_chunk(g.k);
       g.kmode = tcg::K_LAUUM;
       g.cx = cx;
       g.c = reinterpret_cast<float*>(A);

@@ -8,13 +8,13 @@
 // hi hi^T (the dropped lo lo^T is below 2^-22 of the product).
 //
 // Accumulation.  The tensor core truncates when it adds to its FP32 accumulator, which
-// biases long sums.  So an accumulator in tensor memory only runs over one k block (32 k:
-// four additions of the large products); eight epilogue warps then add it, rounded to
-// nearest, to FP32 registers while the next k block runs in the other accumulator.  That is
-// blocked summation: its error is below that of one FMA chain per element (tcg_min_order
-// has the figures).  Accumulators of two k blocks, read by four warps: ?potri of order 300
-// 6.3e-7 in place of 2.9e-7 (the FMA chains: 3.0e-7), complex ?potri of order 4096 3.89 in
-// place of 4.00 ms.
+// biases long sums.  So an accumulator in tensor memory only runs over `chunk` k blocks of
+// 32; eight epilogue warps then add it, rounded to nearest, to FP32 registers while the next
+// ones run in the other accumulator.  That is blocked summation.  With one k block (four
+// additions of the large products) its error is below that of one FMA chain per element at
+// every order from tcg_min_order on, with two (twelve more) it is so for long sums only
+// (kLongSum), and half of the reads of tensor memory, which the products share with the MMAs,
+// go: strtri + slauum n = 16384 19.5 in place of 21 ms.
 //
 // Complex.  With a complex number stored as two adjacent k values, a complex product is
 // a real one of twice the k: Re C = (ar, ai) . (br, -bi), Im C = (ar, ai) . (bi, br).
@@ -58,6 +58,7 @@ struct Params {
   float* c;                     // output, in floats; element (i, col, part) at i*rs + col*cs + part;
                                 // rs or cs is cx
   long long rs, cs, c_node;     // in floats
+  int chunk;                    // k blocks per accumulator
   int beta, neg;                // C := (beta ? C : 0) + (neg ? -1 : 1) * acc
   int lower_only, real_diag;
   float *xhi, *xlo;             // if not null: the product goes here, split, as an A pack of row
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   int kb, ke;
   k_range(p, i0, j0, last ? p.k_last : p.k, kb, ke);
   const int nkb = ke > kb ? (ke - kb + BK - 1) / BK : 0;
+  const int nch = (nkb + p.chunk - 1) / p.chunk;
 
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -147,26 +149,29 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {                              // MMA issuer
       int kk = 0;
       bool ok = true;
-      for (; kk < nkb; ++kk) {
-        const int b = kk % NACC, s = kk % STAGES;
-        if ((kk >= NACC && !tc::mbar_wait(&acc_empty[b], ((kk / NACC) & 1) ^ 1)) ||
-            !tc::mbar_wait(&full[s], (kk / STAGES) & 1)) {
-          ok = false;
-          break;
-        }
-        tc::fence_after();
+      for (int c = 0; c < nch && ok; ++c) {
+        const int b = c % NACC;
+        if (c >= NACC && !tc::mbar_wait(&acc_empty[b], ((c / NACC) & 1) ^ 1)) ok = false;
         const uint32_t d = tmem + b * BN;
-        const uint32_t ah = tc::smem_u32(base + s * STAGE_BYTES), al = ah + TILE_BYTES, bh = al + TILE_BYTES,
-                       bl = bh + TILE_BYTES;
-        // the small products first: they meet a small accumulator
+        for (int u = 0; u < p.chunk && kk < nkb && ok; ++u, ++kk) {
+          const int s = kk % STAGES;
+          if (!tc::mbar_wait(&full[s], (kk / STAGES) & 1)) {
+            ok = false;
+            break;
+          }
+          tc::fence_after();
+          const uint32_t ah = tc::smem_u32(base + s * STAGE_BYTES), al = ah + TILE_BYTES, bh = al + TILE_BYTES,
+                         bl = bh + TILE_BYTES;
+          // the small products first: they meet a small accumulator
 #pragma unroll
-        for (int x = 0; x < BK * 4 / 32; ++x)
-          tc::mma<float>(d, tc::smem_desc(al + 32 * x), tc::smem_desc(bh + 32 * x), x != 0 ? 1u : 0u);
+          for (int x = 0; x < BK * 4 / 32; ++x)
+            tc::mma<float>(d, tc::smem_desc(al + 32 * x), tc::smem_desc(bh + 32 * x), (u | x) != 0 ? 1u : 0u);
 #pragma unroll
-        for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bl + 32 * x), 1u);
+          for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bl + 32 * x), 1u);
 #pragma unroll
-        for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bh + 32 * x), 1u);
-        tc::mma_commit(&empty[s]);
+          for (int x = 0; x < BK * 4 / 32; ++x) tc::mma<float>(d, tc::smem_desc(ah + 32 * x), tc::smem_desc(bh + 32 * x), 1u);
+          tc::mma_commit(&empty[s]);
+        }
         tc::mma_commit(&acc_full[b]);
       }
       if (!ok) s_fail = 1;
@@ -181,9 +186,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int j = 0; j < EPI_COLS; ++j) acc[j] = 0.f;
     bool ok = true;
 #pragma unroll 1
-    for (int kk = 0; kk < nkb; ++kk) {
-      const int b = kk % NACC;
-      if (!tc::mbar_wait(&acc_full[b], (kk / NACC) & 1)) {
+    for (int c = 0; c < nch; ++c) {
+      const int b = c % NACC;
+      if (!tc::mbar_wait(&acc_full[b], (c / NACC) & 1)) {
         ok = false;
         break;
       }
