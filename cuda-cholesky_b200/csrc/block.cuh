@@ -16,8 +16,13 @@
 //   * solve16 (one thread per row): right-looking substitution through 16 columns.
 //   * tile_update (one warp): C(32 x 16) -= P Q^H over 16 columns; FP64 on DMMA.
 // The diagonal 16 x 16 block of L is kept a second time in Ld, column j at Ld[16 j], so
-// that the loops read it with aligned 16-byte loads; its diagonal holds the pivots (the
-// squares of the diagonal elements).
+// that the loops read it with aligned 16-byte loads; with ROOT its diagonal holds the pivots
+// (the squares of the diagonal elements).
+// ROOT: the diagonal is the rounded square root of the pivot.  Without it is the pivot times its
+// reciprocal root, as the columns are scaled, up to an ulp off: the factor of order 16 to 200 errs
+// 6% more in FP64.  The batched kernels go without: there the root is on the chain of a block of
+// 64 (10,000 matrices in FP32 28.5 against 27.6 ms), and their errors are those of the
+// condition numbers.
 #pragma once
 #include <stdint.h>
 #include <type_traits>
@@ -141,11 +146,11 @@ __device__ __noinline__ int factor16_slow(T* S, int ld, int nrows, T* Ld, RealOf
 
 // Step J of factor16 and the ones after it: x the row, r the reciprocal square root of
 // the pivot of column J.  (On lane J the update formula makes x[J] the pivot itself.)
-template <int J, typename T>
+template <bool ROOT, int J, typename T>
 __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i, T* Ld, RealOf<T>* rd, bool& odd) {
   using R = RealOf<T>;
   if constexpr (J < kSub) {
-    if (i == J) Ld[J * kSub + J] = from_real<T>(re(x[J]));
+    if (ROOT && i == J) Ld[J * kSub + J] = from_real<T>(re(x[J]));
     x[J] = scale(x[J], r);
     R rn = R(1);
     if constexpr (J + 1 < kSub) {
@@ -153,7 +158,7 @@ __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i,
       odd = odd || odd_pivot(dn);
       rn = pivot_rsqrt(dn);
     }
-    if (i < kSub && i != J) Ld[J * kSub + i] = x[J];
+    if (i < kSub && !(ROOT && i == J)) Ld[J * kSub + i] = x[J];
     if (i == 0) rd[J] = r;
     if constexpr (J + 1 < kSub) {
       __syncwarp();
@@ -161,12 +166,12 @@ __device__ __forceinline__ void factor16_steps(T (&x)[kSub], RealOf<T> r, int i,
       load_row16<J + 1>(Ld + J * kSub, v);
 #pragma unroll
       for (int q = J + 1; q < kSub; ++q) fms(x[q], x[J], cj(v[q]));
-      factor16_steps<J + 1>(x, rn, i, Ld, rd, odd);
+      factor16_steps<ROOT, J + 1>(x, rn, i, Ld, rd, odd);
     }
   }
 }
 
-template <typename T>
+template <bool ROOT, typename T>
 __device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Ld, RealOf<T>* rd) {
   using R = RealOf<T>;
   const int i = threadIdx.x & 31;
@@ -176,11 +181,12 @@ __device__ __forceinline__ int factor16(T* S, int ld, int nrows, T* Ld, RealOf<T
   for (int q = 0; q < kSub; ++q) x[q] = mine ? S[q * ld + i] : zero<T>();
   const R d = __shfl_sync(0xffffffffu, re(x[0]), 0);
   bool odd = odd_pivot(d);
-  factor16_steps<0>(x, pivot_rsqrt(d), i, Ld, rd, odd);
+  static_assert(ROOT || !Traits<T>::complex, "the diagonal's imaginary part goes with the root");
+  factor16_steps<ROOT, 0>(x, pivot_rsqrt(d), i, Ld, rd, odd);
   if (odd) return factor16_slow<T>(S, ld, nrows, Ld, rd);
 #pragma unroll
   for (int q = 0; q < kSub; ++q) {
-    if (mine && i > q) S[q * ld + i] = x[q];
+    if (mine && (ROOT ? i > q : i >= q)) S[q * ld + i] = x[q];
   }
   return -1;
 }
@@ -390,7 +396,7 @@ struct FactorSmem {
 // Per sub-panel: warp 0 factors the diagonal 16 x 16 (and 16 rows below); one thread per
 // remaining row solves; the 32 x 16 elements warp 0 needs next are updated by all
 // threads; then warp 0 goes on while the other warps update the rest of the block.
-template <typename T, int NB, int R, int NT, typename Done>
+template <typename T, int NB, int R, int NT, bool ROOT = true, typename Done>
 __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16, int nrow, int* s_fail, Done done) {
   constexpr int LD = FactorSmem<T, NB, R>::LD;
   const int t = threadIdx.x, warp = t >> 5;
@@ -398,7 +404,7 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
   for (int c0 = 0; c0 < n16; c0 += kSub) {
     const int c1 = c0 + kSub;
     if (warp == 0) {
-      const int f = factor16<T>(S + c0 * LD + c0, LD, nrow - c0, Ld, rd + c0);
+      const int f = factor16<ROOT, T>(S + c0 * LD + c0, LD, nrow - c0, Ld, rd + c0);
       if (t == 0 && f >= 0) *s_fail = c0 + f;
     } else if (c0 > 0) {
       // the rest of the update by the previous sub-panel: 32 x 16 tiles of the columns
@@ -415,11 +421,11 @@ __device__ __forceinline__ void factor_block(T* S, T* Ld, RealOf<T>* rd, int n16
     }
     __syncthreads();
     const int fail = *s_fail;
-    // the diagonal, rounded once: the pivot times its reciprocal root, as the columns are
-    // scaled, is up to an ulp off (n = 16 .. 200 FP64: error of the factor 6% larger)
-    static_assert(NB + R - kSubRows <= NT - kSub, "these threads have no row to solve");
-    const int i = t - (NT - kSub);
-    if (i >= 0 && (fail < 0 || c0 + i < fail)) S[(c0 + i) * LD + c0 + i] = from_real<T>(sqrt(re(Ld[i * kSub + i])));
+    if constexpr (ROOT) {
+      static_assert(NB + R - kSubRows <= NT - kSub, "these threads have no row to solve");
+      const int i = t - (NT - kSub);
+      if (i >= 0 && (fail < 0 || c0 + i < fail)) S[(c0 + i) * LD + c0 + i] = from_real<T>(sqrt(re(Ld[i * kSub + i])));
+    }
     for (int r = c0 + kSubRows + t; r < nrow; r += NT) {
       if (fail < 0) solve16<T>(S + c0 * LD + r, LD, Ld, rd + c0);
       else solve16_part<T>(S + c0 * LD + r, LD, Ld, rd + c0, fail - c0);

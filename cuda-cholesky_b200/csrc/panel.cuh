@@ -125,7 +125,7 @@ __device__ __forceinline__ void add_logdet(const T* S, int jb, double* s_log, do
 // T: computing type, TA: storage type; smem: FactorSmem<T, NB>::bytes, which keep the
 // factor (S) and the reciprocal pivots.  On failure at local column k: *d_info =
 // info_base + k + 1 (if still 0), the columns before k are written back, false.
-template <typename T, typename TA, int NB, int NT>
+template <typename T, typename TA, int NB, int NT, bool ROOT = true>
 __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict__ A, long long rs, long long cs, int jb,
                                             long long info_base, int* __restrict__ d_info, double* __restrict__ logdet) {
   using F = FactorSmem<T, NB>;
@@ -139,7 +139,7 @@ __device__ __forceinline__ bool factor_diag(unsigned char* smem, TA* __restrict_
   load_lower<T, TA, NB, NT>(S, A, rs, cs, jb, n16);
   if (tid == 0) s_fail = -1;
   cp_async_wait_all();
-  factor_block<T, NB, 0, NT>(S, Ld, rd, n16, n16, &s_fail, [&](int c0, int cols, int t, int nt) {
+  factor_block<T, NB, 0, NT, ROOT>(S, Ld, rd, n16, n16, &s_fail, [&](int c0, int cols, int t, int nt) {
     // columns c0 .. c0 + cols - 1 of the factor back to A
     const int rows = jb - c0, ce = min(jb, c0 + cols);
     if (rs == 1) {
@@ -193,7 +193,7 @@ __device__ __forceinline__ void diag_factor_block(T* __restrict__ A, long long r
   constexpr int LD = F::LD;
   if (cta_aborted(d_info)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (!factor_diag<T, T, NB, NT>(smem_raw, A, rs, cs, jb, info_base, d_info, logdet) || W == nullptr) return;
+  if (!factor_diag<T, T, NB, NT, false>(smem_raw, A, rs, cs, jb, info_base, d_info, logdet) || W == nullptr) return;
   T* S = reinterpret_cast<T*>(smem_raw);
   const T* rd = reinterpret_cast<const T*>(smem_raw + F::S + F::LDS);
   T* TMP = reinterpret_cast<T*>(smem_raw + BlockSmem<T, NB>::F + BlockSmem<T, NB>::RD);

@@ -37,7 +37,8 @@ def _wide_factor(A):
     return np.tril(L)
 
 
-@pytest.mark.parametrize("p,n", [("s", 100), ("s", 129), ("s", 300), ("c", 100), ("c", 129), ("c", 300), ("z", 60)])
+@pytest.mark.parametrize("p,n", [("s", 100), ("s", 129), ("s", 300), ("d", 16), ("d", 100), ("c", 100), ("c", 129),
+                                 ("c", 300), ("z", 16), ("z", 60)])
 @pytest.mark.parametrize("uplo", "LU")
 def test_factor_rounding(handle, p, n, uplo):
     # An element takes one subtraction per 16 columns and at most 16 more inside its own, so in

@@ -344,3 +344,16 @@ def test_contents_after_a_bad_pivot(handle, p, uplo):
             d = np.abs(np.where(done, got[:, :nb] - good[:, :nb], 0))[rest]
             assert d.max() <= 64 * np.finfo(got.real.dtype).eps
             assert np.array_equal(got[:, :nb][low & ~done], B[:, :nb][low & ~done])
+
+
+@pytest.mark.parametrize("n", [40, 128])
+@pytest.mark.parametrize("p", "sc")
+def test_subnormal_and_large_fp32_pivots(handle, p, n):
+    """Pivots below 2^-126 hold fewer bits (2^-149 apart), those near 2^127 all of them."""
+    A = matgen.spd(p, n, seed=n)
+    A = A / np.abs(np.diag(A)).max()
+    for scale, bound in ((2.0 ** -130, 2.0 ** -19 * n), (2.0 ** 127, 4 * U["s"])):
+        B = (A * np.float32(scale)).astype(A.dtype)
+        D = cc.to_device_colmajor(B)
+        assert cc.potrf(handle, D, n) == 0
+        assert _factor_error(B, cc.to_host_colmajor(D), "L") <= bound
