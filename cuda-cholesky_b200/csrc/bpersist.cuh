@@ -408,7 +408,7 @@ namespace {
 
 // The persistent form as the plan's recorded sequence: per-matrix descriptors and
 // the size order uploaded once; per run, the result words and the queue head
-// cleared, then one launch (one CTA per SM).
+// cleared, then one launch (three CTAs per SM, no more than matrices).
 template <typename T>
 CUresult record_persistent(CUcholBatched p, const BatchedShape<T>& sh, cudaStream_t s) {
   CULAPACKhandle h = p->h;

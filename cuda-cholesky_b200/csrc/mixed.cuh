@@ -11,13 +11,13 @@
 //      the operand unit roundoff) and grows 8x after a breakdown.
 //   2. Right-looking blocked Cholesky of W with the two-stream schedule of ?potrf
 //      (outer blocks of 512 columns = four 128-column sub-panels, lookahead 1):
-//        - diagonal blocks in FP64 (the ?potrf diagonal kernel, FP32 in and out),
-//        - panel solve P = W21 inv(L11)^T in FP32 (SIMT engine) into a k-major
-//          buffer, then copied into W and rounded to the operand type Q (BF16 or
-//          TF32),
+//        - diagonal blocks in FP64 on FP32 storage, in one launch with the rows below
+//          while those fit the GPU (panel_kernel, FP64 too); otherwise the diagonal
+//          kernel and the row-parallel solve in FP32 (trsm_rows_kernel); either writes
+//          the rows into W and, rounded to BF16 or TF32, into the k-major operand Q,
 //        - trailing updates W22 -= Q Q^T on the tcgen05 tensor cores with FP32
 //          accumulation (tc.cuh).
-//   3. The inverses of W's 64 x 64 diagonal blocks (for the triangular solves).
+//   3. The inverses of W's 2048-wide diagonal blocks (for the preconditioner).
 // Solve (cuDcholMixedSolve): preconditioned conjugate gradients in FP64 on A x = b
 // with M^-1 = S L^-T L^-1 S, in groups of 16 right-hand sides, as iterative
 // refinement: the loop ends when every normwise backward error

@@ -33,13 +33,13 @@ struct TuneRow {
 };
 
 // ?potrf, ms on a B200 by the width of the outer block; the rows split at the geometric
-// midpoints of the orders measured, and lie within 1.3% of the best width at each:
-//   D  n = 8192   8.68 (2)  8.57 (3)  8.65 (4)
-//      n = 16384  54.7 (2)  52.7 (3)  51.95 (4)  51.67 (5)  51.47 (6)      n = 32768  378.6 (6)  376.2 (8)
-//   S  n = 16384  14.1 (2)  12.6 (3)  11.9 (4)  11.85 (6)                  n = 32768  84.1 (4)  85.1 (6)
-//   C  n = 4096  2.32 (2)  2.33 (3)  2.34 (4)      n = 8192  7.59 (3)  7.49 (4)  7.58 (6)  7.87 (8)
-//      n = 16384  48.2 (4)  46.8 (6)  46.8 (8)
-//   Z  n = 4096  6.6 (2 .. 6)      n = 8192  33.0 (4)  32.4 (6)
+// midpoints of the orders measured, and lie within 3% of the best width at each (Z n = 4096: 4%):
+//   D  n = 8192   8.58 (2)  8.35 (3)  8.36 (4)
+//      n = 16384  54.4 (2)  52.4 (3)  51.5 (4)  51.2 (5)  51.1 (6)         n = 32768  379.4 (6)  377.0 (8)
+//   S  n = 16384  13.5 (2)  12.0 (3)  11.4 (4)  11.3 (6)                   n = 32768  83 (4)  83.9 (6)
+//   C  n = 4096  2.33 (2)  2.35 (3)  2.36 (4)      n = 8192  7.40 (3)  7.34 (4)  7.43 (6)  7.66 (8)
+//      n = 16384  46 to 48 (4)  46.1 (6)  45 (8)
+//   Z  n = 4096  6.37 (2)  6.14 (3)  6.09 (4)  6.17 (6)      n = 8192  33.3 (4)  32.65 (6)
 // cuDpotrfOzaki: 8 (1024 columns) below n = 49152, 16 from there on (n = 8192 / 32768 /
 // 65536: 10.8 / 255 / 2028 ms with 8; 11.7 / 255 / 1926 ms with 16; 4 gave 282 ms and
 // 2344 ms at the two larger orders).
