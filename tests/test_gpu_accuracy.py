@@ -111,3 +111,33 @@ def test_split_inverse_no_worse_than_simt(handle, p, n):
             err.setdefault(name, []).append(np.linalg.norm(got - ref) / np.linalg.norm(ref))
     simt.close()
     assert np.mean(err["split"]) <= 1.05 * np.mean(err["simt"]), err
+
+
+@pytest.mark.parametrize("p,n,uplo", [("s", 4095, "L"), ("s", 4200, "U"), ("c", 2047, "U"), ("c", 2100, "L")])
+def test_split_inverse_of_long_sums(handle, p, n, uplo):
+    """On either side of the order from which an accumulator takes two k blocks (4096 real k):
+    the inverse errs less than the FP32 engine's."""
+    import torch
+    os.environ["CUCHOLESKY_FORCE_SIMT"] = "1"
+    try:
+        simt = cc.Handle()
+    finally:
+        del os.environ["CUCHOLESKY_FORCE_SIMT"]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    G = torch.randn((n, n), generator=g, device="cuda", dtype=torch.complex128 if p == "c" else torch.float64)
+    A = G @ G.conj().T / n + torch.eye(n, device="cuda", dtype=G.dtype)
+    T = torch.tril(torch.linalg.cholesky(A)).to(matgen.torch_dtype(p))     # the lower factor, [i, j]
+    ref = torch.cholesky_inverse(T.to(G.dtype))
+    # storage [j, i] = A(i, j): the lower factor for L, its conjugate transpose for U
+    stored = (T.T if uplo == "L" else T.conj()).resolve_conj().contiguous()
+    keep = torch.triu if uplo == "L" else torch.tril
+    want = keep(ref.T)
+    err = []
+    for h in (handle, simt):
+        D = stored.clone()
+        assert cc.potri(h, D, n, uplo) == 0
+        torch.cuda.synchronize()
+        err.append(float(torch.linalg.norm(keep(D).to(G.dtype) - want) / torch.linalg.norm(want)))
+    simt.close()
+    assert err[0] <= err[1], err

@@ -357,3 +357,23 @@ def test_subnormal_and_large_fp32_pivots(handle, p, n):
         D = cc.to_device_colmajor(B)
         assert cc.potrf(handle, D, n) == 0
         assert _factor_error(B, cc.to_host_colmajor(D), "L") <= bound
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan, 2.0 ** 70, "tiny"])
+@pytest.mark.parametrize("p", "sc")
+def test_inverse_range_rule(handle, simt, p, bad):
+    """?trtri and ?lauum of entries that the splits cannot hold, at an order where either type
+    would take them: the FP32 engine's results, bit for bit."""
+    n = 400
+    T = np.tril(np.linalg.cholesky(matgen.spd(p, n, seed=5))).astype(matgen.dtype_of(p), order="F")
+    if bad == "tiny":
+        T = np.asfortranarray(T * np.float32(2.0 ** -70))
+    else:
+        T[250, 50] = bad
+    for call in (cc.trtri, cc.lauum):
+        out = []
+        for h in (handle, simt):
+            D = cc.to_device_colmajor(T)
+            assert call(h, D, n, "L") == 0
+            out.append(cc.to_host_colmajor(D))
+        assert np.array_equal(out[0], out[1], equal_nan=True)
